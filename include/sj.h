@@ -236,8 +236,8 @@ sj_status sj_mlp_forward(const float *x, uint32_t m, const float *w, float *out,
  *
  * Every pointer is DEVICE memory owned by the caller: x (m x 16), y (m x 2),
  * w (SJ_MLP_NPARAM), loss (1 float, overwritten), grad (SJ_MLP_NPARAM).  The
- * per-sample activations live in a fixed array inside the library sized for
- * SJ_MLP_NOALLOC_MAX_SAMPLES samples (about 8.5 MB, held by every device that
+ * partial gradients live in a fixed array inside the library sized for
+ * SJ_MLP_NOALLOC_MAX_SAMPLES samples (about 5.5 MB, held by every device that
  * loads the library until the process exits); larger m is rejected with
  * SJ_ERR_BAD_INPUT.  Work is queued on `stream` (a cudaStream_t; NULL = the
  * default stream) and the call returns without synchronising.  The first call

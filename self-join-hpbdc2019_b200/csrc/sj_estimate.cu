@@ -57,75 +57,248 @@ __global__ void __launch_bounds__(128) k_mlp_infer(const float *__restrict__ fea
     for (int o = 0; o < SJ_NOUT; o++) out[(uint64_t)s * SJ_NOUT + o] = y[o];
 }
 
-// Per-sample forward + backward.  Loss = 1/(2m) * sum (y - t)^2.  Writes the
-// activations and pre-activation gradients the weight gradients need.
-__global__ void __launch_bounds__(128) k_mlp_backprop(const float *__restrict__ X, const float *__restrict__ Yt,
-                                                      uint32_t m, const float *__restrict__ wg,
-                                                      float *__restrict__ H1, float *__restrict__ G1,
-                                                      float *__restrict__ H2, float *__restrict__ G2,
-                                                      float *__restrict__ G3, float *__restrict__ loss)
+// Loss and gradient in two launches.  k_mlp_grad: a CTA takes tiles of GT
+// samples and runs the three layers forward and backward on them as small
+// matrix products out of shared memory (weights and activations stay there;
+// nothing per sample goes to global memory), keeping its sums of the weight
+// gradients in registers over all of its tiles; it then writes one partial
+// gradient (and loss).  k_mlp_grad_sum adds the partials in a fixed order, so
+// the result does not depend on scheduling.  Loss = 1/(2m) * sum (y - t)^2.
+//
+// Bound: latency -- 8192 samples are 0.24 GFLOP (3 us of the FP32 pipe) and
+// 0.6 MB of input.  Per-sample threads with their activations in local memory
+// and one thread per parameter summing all m samples in turn took 44 + 1063 us
+// at m = 8192 on a B200; this form takes 24.6 us for the call (both launches).
+constexpr int GT = 32;           // samples per tile
+constexpr int GTH = 256;         // threads: 16 x 16
+constexpr int GLD = SJ_HID + 4;  // row stride in shared memory: 16-byte accesses of 8 consecutive rows hit all banks
+constexpr int GXLD = SJ_NFEAT + 4;
+constexpr int GSTRIDE = NP + 1;  // a partial: the gradient, then the loss
+constexpr int GMAX_CTAS = 296;   // two CTAs on each of 148 SMs; more tiles are taken in turn
+static_assert(SJ_HID == 64 && SJ_NFEAT == 16 && SJ_NOUT == 2, "thread mapping of k_mlp_grad");
+
+struct __align__(16) GradSmem {
+    float w1[SJ_NFEAT][GLD], w2[SJ_HID][GLD], w3[SJ_HID * SJ_NOUT], b1[SJ_HID], b2[SJ_HID];
+    float x[GT][GXLD];
+    float a1[GT][GLD];           // relu(z1), later the gradient at z1
+    float a2[GT][GLD];           // relu(z2), later the gradient at z2
+    float g3[GT][SJ_NOUT];
+    float b3[SJ_NOUT];
+    float loss[GT];
+};
+
+// s[r][c] += the products of one 4-vector of a row with a 4 x 4 block
+__device__ __forceinline__ float dot4(float4 a, float4 b, float s)
 {
-    __shared__ float w[NP];
-    for (int i = threadIdx.x; i < NP; i += blockDim.x) w[i] = wg[i];
-    __syncthreads();
-    uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    float l = 0.f;
-    if (s < m) {
-        float x[SJ_NFEAT], z1[SJ_HID], z2[SJ_HID], y[SJ_NOUT], dy[SJ_NOUT], d2[SJ_HID];
-        for (int i = 0; i < SJ_NFEAT; i++) x[i] = X[(uint64_t)s * SJ_NFEAT + i];
-        mlp_forward(w, x, z1, z2, y);
-        const float inv = 1.0f / (float)m;
-        for (int o = 0; o < SJ_NOUT; o++) {
-            float e = y[o] - Yt[(uint64_t)s * SJ_NOUT + o];
-            l += 0.5f * e * e;
-            dy[o] = e * inv;
-            G3[(uint64_t)s * SJ_NOUT + o] = dy[o];
-        }
-        for (int i = 0; i < SJ_HID; i++) {
-            float g = 0.f;
-#pragma unroll
-            for (int o = 0; o < SJ_NOUT; o++) g = fmaf(dy[o], w[OW3 + i * SJ_NOUT + o], g);
-            d2[i] = z2[i] > 0.f ? g : 0.f;
-            H2[(uint64_t)s * SJ_HID + i] = fmaxf(z2[i], 0.f);
-            G2[(uint64_t)s * SJ_HID + i] = d2[i];
-        }
-        for (int i = 0; i < SJ_HID; i++) {
-            float g = 0.f;
-            for (int j = 0; j < SJ_HID; j++) g = fmaf(d2[j], w[OW2 + i * SJ_HID + j], g);
-            H1[(uint64_t)s * SJ_HID + i] = fmaxf(z1[i], 0.f);
-            G1[(uint64_t)s * SJ_HID + i] = z1[i] > 0.f ? g : 0.f;
-        }
-    }
-    // loss reduction
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0 && l != 0.f) atomicAdd(loss, l / (float)m);
+    return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s))));
 }
 
-// grad[param] = sum over samples of (input activation) x (output gradient);
-// one thread per parameter.  Inputs: X (m x 16), H1, H2 (m x 64);
-// gradients: G1, G2 (m x 64), G3 (m x 2).
-__global__ void __launch_bounds__(256) k_mlp_wgrad(const float *__restrict__ X, const float *__restrict__ H1,
-                                                   const float *__restrict__ H2, const float *__restrict__ G1,
-                                                   const float *__restrict__ G2, const float *__restrict__ G3,
-                                                   uint32_t m, float *__restrict__ grad)
+__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+
+__device__ __forceinline__ void axpy4(float a, float4 b, float (&s)[4])
 {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= NP) return;
-    const float *A = nullptr, *G = nullptr;
-    int ai = -1, gj, aw = 0, gw;
-    if (p < OB1) { A = X; aw = SJ_NFEAT; ai = (p - OW1) / SJ_HID; G = G1; gw = SJ_HID; gj = (p - OW1) % SJ_HID; }
-    else if (p < OW2) { G = G1; gw = SJ_HID; gj = p - OB1; }
-    else if (p < OB2) { A = H1; aw = SJ_HID; ai = (p - OW2) / SJ_HID; G = G2; gw = SJ_HID; gj = (p - OW2) % SJ_HID; }
-    else if (p < OW3) { G = G2; gw = SJ_HID; gj = p - OB2; }
-    else if (p < OB3) { A = H2; aw = SJ_HID; ai = (p - OW3) / SJ_NOUT; G = G3; gw = SJ_NOUT; gj = (p - OW3) % SJ_NOUT; }
-    else { G = G3; gw = SJ_NOUT; gj = p - OB3; }
-    float s = 0.f;
-    for (uint32_t k = 0; k < m; k++) {
-        float av = (ai >= 0) ? A[(uint64_t)k * aw + ai] : 1.0f;
-        s = fmaf(av, G[(uint64_t)k * gw + gj], s);
+    s[0] = fmaf(a, b.x, s[0]);
+    s[1] = fmaf(a, b.y, s[1]);
+    s[2] = fmaf(a, b.z, s[2]);
+    s[3] = fmaf(a, b.w, s[3]);
+}
+
+__global__ void __launch_bounds__(GTH, 2) k_mlp_grad(const float *__restrict__ X, const float *__restrict__ Yt,
+                                                     uint32_t m, const float *__restrict__ wg,
+                                                     float *__restrict__ part)
+{
+    __shared__ GradSmem sm;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    for (int i = tid; i < SJ_NFEAT * SJ_HID; i += GTH) sm.w1[i / SJ_HID][i % SJ_HID] = wg[OW1 + i];
+    for (int i = tid; i < SJ_HID * SJ_HID; i += GTH) sm.w2[i / SJ_HID][i % SJ_HID] = wg[OW2 + i];
+    if (tid < SJ_HID * SJ_NOUT) sm.w3[tid] = wg[OW3 + tid];
+    if (tid < SJ_HID) {
+        sm.b1[tid] = wg[OB1 + tid];
+        sm.b2[tid] = wg[OB2 + tid];
     }
-    grad[p] = s;
+    if (tid < SJ_NOUT) sm.b3[tid] = wg[OB3 + tid];
+    const float inv = 1.0f / (float)m;
+    float dw1[4] = {0.f, 0.f, 0.f, 0.f};                  // row ty, columns 4 tx ..
+    float dw2[4][4] = {};                                 // rows 4 ty .., columns 4 tx ..
+    float dw3 = 0.f, db = 0.f, db3 = 0.f, lsum = 0.f;     // by thread, see below
+    const uint32_t nTiles = (m + GT - 1) / GT;
+    for (uint32_t tile = blockIdx.x; tile < nTiles; tile += gridDim.x) {
+        const uint32_t s0 = tile * GT;
+        const uint32_t ns = min((uint32_t)GT, m - s0);
+        __syncthreads();   // the weights are there; the previous tile is done with the arrays
+        for (int i = tid; i < GT * SJ_NFEAT; i += GTH) {
+            const uint32_t r = i / SJ_NFEAT;
+            sm.x[r][i % SJ_NFEAT] = r < ns ? X[(uint64_t)s0 * SJ_NFEAT + i] : 0.f;
+        }
+        __syncthreads();
+        // layers 1 and 2: thread (ty, tx) has samples 2 ty, 2 ty + 1 and units 4 tx ..
+        {
+            float z[2][4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) z[0][c] = z[1][c] = sm.b1[4 * tx + c];
+#pragma unroll
+            for (int i = 0; i < SJ_NFEAT; i++) {
+                const float4 w = ld4(&sm.w1[i][4 * tx]);
+                axpy4(sm.x[2 * ty][i], w, z[0]);
+                axpy4(sm.x[2 * ty + 1][i], w, z[1]);
+            }
+#pragma unroll
+            for (int r = 0; r < 2; r++)
+#pragma unroll
+                for (int c = 0; c < 4; c++) sm.a1[2 * ty + r][4 * tx + c] = fmaxf(z[r][c], 0.f);
+        }
+        __syncthreads();
+        {
+            float z[2][4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) z[0][c] = z[1][c] = sm.b2[4 * tx + c];
+#pragma unroll 4
+            for (int i = 0; i < SJ_HID; i++) {
+                const float4 w = ld4(&sm.w2[i][4 * tx]);
+                axpy4(sm.a1[2 * ty][i], w, z[0]);
+                axpy4(sm.a1[2 * ty + 1][i], w, z[1]);
+            }
+#pragma unroll
+            for (int r = 0; r < 2; r++)
+#pragma unroll
+                for (int c = 0; c < 4; c++) sm.a2[2 * ty + r][4 * tx + c] = fmaxf(z[r][c], 0.f);
+        }
+        __syncthreads();
+        // output layer: threads 0..63 = (sample, output)
+        if (tid < GT * SJ_NOUT) {
+            const int r = tid / SJ_NOUT, o = tid % SJ_NOUT;
+            float y = sm.b3[o];
+            for (int i = 0; i < SJ_HID; i++) y = fmaf(sm.a2[r][i], sm.w3[i * SJ_NOUT + o], y);
+            const float e = (uint32_t)r < ns ? y - Yt[(uint64_t)(s0 + r) * SJ_NOUT + o] : 0.f;
+            lsum += 0.5f * e * e;
+            sm.g3[r][o] = e * inv;
+        }
+        __syncthreads();
+        // dW3 (threads 0..127: unit, output) and db3 (threads 128, 129)
+        if (tid < SJ_HID * SJ_NOUT) {
+            const int i = tid / SJ_NOUT, o = tid % SJ_NOUT;
+#pragma unroll 8
+            for (int r = 0; r < GT; r++) dw3 = fmaf(sm.a2[r][i], sm.g3[r][o], dw3);
+        } else if (tid < SJ_HID * SJ_NOUT + SJ_NOUT) {
+            for (int r = 0; r < GT; r++) db3 += sm.g3[r][tid - SJ_HID * SJ_NOUT];
+        }
+        __syncthreads();
+        // gradient at z2, in place
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const int s = 2 * ty + r;
+            const float e0 = sm.g3[s][0], e1 = sm.g3[s][1];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const int i = 4 * tx + c;
+                const float g = fmaf(e1, sm.w3[i * SJ_NOUT + 1], e0 * sm.w3[i * SJ_NOUT]);
+                sm.a2[s][i] = sm.a2[s][i] > 0.f ? g : 0.f;
+            }
+        }
+        __syncthreads();
+        // dW2; then the gradient at z1: thread (ty, tx) has samples 2 ty, 2 ty + 1 and units tx + 16 c
+#pragma unroll 4
+        for (int r = 0; r < GT; r++) {
+            const float4 h = ld4(&sm.a1[r][4 * ty]);
+            const float4 g = ld4(&sm.a2[r][4 * tx]);
+            axpy4(h.x, g, dw2[0]);
+            axpy4(h.y, g, dw2[1]);
+            axpy4(h.z, g, dw2[2]);
+            axpy4(h.w, g, dw2[3]);
+        }
+        float g1[2][4] = {};
+#pragma unroll 4
+        for (int j = 0; j < SJ_HID; j += 4) {
+            const float4 p = ld4(&sm.a2[2 * ty][j]), q = ld4(&sm.a2[2 * ty + 1][j]);
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const float4 w = ld4(&sm.w2[tx + 16 * c][j]);
+                g1[0][c] = dot4(p, w, g1[0][c]);
+                g1[1][c] = dot4(q, w, g1[1][c]);
+            }
+        }
+        __syncthreads();   // every thread has read the activations of layer 1
+#pragma unroll
+        for (int r = 0; r < 2; r++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                float &a = sm.a1[2 * ty + r][tx + 16 * c];
+                a = a > 0.f ? g1[r][c] : 0.f;
+            }
+        __syncthreads();
+        // dW1, db1 (threads 0..63) and db2 (threads 64..127)
+#pragma unroll 8
+        for (int r = 0; r < GT; r++) axpy4(sm.x[r][ty], ld4(&sm.a1[r][4 * tx]), dw1);
+        if (tid < SJ_HID) {
+            for (int r = 0; r < GT; r++) db += sm.a1[r][tid];
+        } else if (tid < 2 * SJ_HID) {
+            for (int r = 0; r < GT; r++) db += sm.a2[r][tid - SJ_HID];
+        }
+    }
+    float *const out = part + (uint64_t)blockIdx.x * GSTRIDE;
+#pragma unroll
+    for (int c = 0; c < 4; c++) out[OW1 + ty * SJ_HID + 4 * tx + c] = dw1[c];
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) out[OW2 + (4 * ty + r) * SJ_HID + 4 * tx + c] = dw2[r][c];
+    if (tid < SJ_HID * SJ_NOUT) out[OW3 + tid] = dw3;
+    else if (tid < SJ_HID * SJ_NOUT + SJ_NOUT) out[OB3 + tid - SJ_HID * SJ_NOUT] = db3;
+    if (tid < SJ_HID) out[OB1 + tid] = db;
+    else if (tid < 2 * SJ_HID) out[OB2 + tid - SJ_HID] = db;
+    // the loss: threads 0..63 hold (sample, output) parts
+    if (tid < 2 * 32) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+        if ((tid & 31) == 0) sm.loss[tid >> 5] = lsum;
+    }
+    __syncthreads();
+    if (tid == 0) out[NP] = (sm.loss[0] + sm.loss[1]) * inv;
+}
+
+// grad[p] = sum of the nPart partials of parameter p; entry NP is the loss.
+// A CTA has 32 parameters; its 8 warps take the partials in turn (coalesced
+// over the parameters) and meet in shared memory.
+__global__ void __launch_bounds__(256) k_mlp_grad_sum(const float *__restrict__ part, uint32_t nPart,
+                                                      float *__restrict__ grad, float *__restrict__ loss)
+{
+    __shared__ float red[8][32];
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    const uint32_t p = blockIdx.x * 32 + lane;
+    float s = 0.f;
+    if (p < GSTRIDE) {
+#pragma unroll 4
+        for (uint32_t k = w; k < nPart; k += 8) s += part[(uint64_t)k * GSTRIDE + p];
+    }
+    red[w][lane] = s;
+    __syncthreads();
+    if (w == 0 && p < GSTRIDE) {
+        float t = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; k++) t += red[k][lane];
+        if (p < NP) grad[p] = t;
+        else *loss = t;
+    }
+}
+
+uint32_t grad_ctas(uint32_t m)
+{
+    const uint32_t tiles = m / GT + (m % GT ? 1u : 0u);
+    return tiles < (uint32_t)GMAX_CTAS ? tiles : (uint32_t)GMAX_CTAS;
+}
+
+// part: grad_ctas(m) * GSTRIDE floats of scratch
+cudaError_t launch_grad(const float *x, const float *y, uint32_t m, const float *w, float *grad, float *loss,
+                        float *part, cudaStream_t s)
+{
+    const uint32_t n = grad_ctas(m);
+    k_mlp_grad<<<n, GTH, 0, s>>>(x, y, m, w, part);
+    sj_note_launch();
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    k_mlp_grad_sum<<<(GSTRIDE + 31) / 32, 256, 0, s>>>(part, n, grad, loss);
+    sj_note_launch();
+    return cudaGetLastError();
 }
 
 __global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ mm,
@@ -154,21 +327,14 @@ cudaError_t sj_launch_mlp_infer(const float *feat, uint32_t nCells, const float 
     return cudaGetLastError();
 }
 
-// Scratch for one training/gradient call: H1, G1, H2, G2 (m x 64 each), G3 (m x 2).
 static cudaError_t mlp_grad_impl(const float *x, const float *y, uint32_t m, const float *w, float *grad,
                                  float *lossOut, cudaStream_t s)
 {
-    float *buf = nullptr;
-    size_t per = (size_t)m * (4 * SJ_HID + SJ_NOUT);
-    cudaError_t e = cudaMallocAsync((void **)&buf, per * sizeof(float), s);
+    float *part = nullptr;
+    cudaError_t e = cudaMallocAsync((void **)&part, (size_t)grad_ctas(m) * GSTRIDE * sizeof(float), s);
     if (e != cudaSuccess) return e;
-    float *H1 = buf, *G1 = H1 + (size_t)m * SJ_HID, *H2 = G1 + (size_t)m * SJ_HID, *G2 = H2 + (size_t)m * SJ_HID,
-          *G3 = G2 + (size_t)m * SJ_HID;
-    cudaMemsetAsync(lossOut, 0, sizeof(float), s);
-    k_mlp_backprop<<<(m + 127) / 128, 128, 0, s>>>(x, y, m, w, H1, G1, H2, G2, G3, lossOut); sj_note_launch();
-    k_mlp_wgrad<<<(NP + 255) / 256, 256, 0, s>>>(x, H1, H2, G1, G2, G3, m, grad); sj_note_launch();
-    e = cudaGetLastError();
-    cudaFreeAsync(buf, s);
+    e = launch_grad(x, y, m, w, grad, lossOut, part, s);
+    cudaFreeAsync(part, s);
     return e;
 }
 
@@ -188,11 +354,12 @@ cudaError_t sj_launch_mlp_train_step(const float *x, const float *y, uint32_t m,
 }
 
 // ------------------------------------------------- allocation-free gradient --
-// Fixed scratch for sj_mlp_loss_grad_noalloc: the per-sample activations and
-// gradients (H1, G1, H2, G2 of SJ_HID floats and G3 of SJ_NOUT floats) of at
-// most SJ_MLP_NOALLOC_MAX_SAMPLES samples.  Every device that loads this
-// library holds it (about 8.5 MB) until the process exits.
-static __device__ __align__(256) float g_mlpNoallocScratch[SJ_MLP_NOALLOC_MAX_SAMPLES * (4 * SJ_HID + SJ_NOUT)];
+// Fixed scratch for sj_mlp_loss_grad_noalloc: the partial gradients of at most
+// SJ_MLP_NOALLOC_MAX_SAMPLES samples.  Every device that loads this library
+// holds it (about 5.5 MB) until the process exits.
+constexpr int kNoallocCtas = SJ_MLP_NOALLOC_MAX_SAMPLES / GT;
+static_assert(kNoallocCtas <= GMAX_CTAS && SJ_MLP_NOALLOC_MAX_SAMPLES % GT == 0, "one partial per tile");
+static __device__ __align__(256) float g_mlpNoallocScratch[kNoallocCtas * GSTRIDE];
 
 namespace {
 constexpr int kMaxDevices = 64;
@@ -241,22 +408,8 @@ extern "C" sj_status sj_mlp_loss_grad_noalloc(const float *x, const float *y, ui
         sj_set_error_message("sj_mlp_loss_grad_noalloc: a CUDA error from earlier work is pending");
         return SJ_ERR_CUDA;
     }
-    cudaStream_t s = (cudaStream_t)stream;
-    float *H1 = scratch, *G1 = H1 + (size_t)m * SJ_HID, *H2 = G1 + (size_t)m * SJ_HID, *G2 = H2 + (size_t)m * SJ_HID,
-          *G3 = G2 + (size_t)m * SJ_HID;
-    // the loss is accumulated with atomics: it must start at zero; the scratch
-    // rows are fully overwritten by every call
-    e = cudaMemsetAsync(loss, 0, sizeof(float), s);
-    if (e == cudaSuccess) {
-        k_mlp_backprop<<<(m + 127) / 128, 128, 0, s>>>(x, y, m, w, H1, G1, H2, G2, G3, loss);
-        sj_note_launch();
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) {
-        k_mlp_wgrad<<<(NP + 255) / 256, 256, 0, s>>>(x, H1, H2, G1, G2, G3, m, grad);
-        sj_note_launch();
-        e = cudaGetLastError();
-    }
+    // every partial and every output is overwritten by each call
+    e = launch_grad(x, y, m, w, grad, loss, scratch, (cudaStream_t)stream);
     if (e != cudaSuccess) {
         sj_set_error_message(cudaGetErrorString(e));
         return SJ_ERR_CUDA;
