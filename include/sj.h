@@ -95,7 +95,8 @@ typedef int (*sj_batch_cb)(const sj_batch *batch, void *user);
 typedef struct {
     uint64_t total_pairs;       /* totalNeighbors (main.cu:194) */
     uint64_t pair_hash;         /* order-independent set hash: wrapping sum of splitmix64(key<<32|val) */
-    uint64_t distance_calcs;    /* candidate evaluations performed (both passes counted once) */
+    uint64_t distance_calcs;    /* candidate evaluations of the traversal (those that the bounding boxes
+                                   of their points rule out included) */
     uint64_t full_stencil_calcs;/* evaluations a full-stencil traversal would do (work unit) */
     uint64_t refined_pairs;     /* FP32-borderline candidate pairs re-evaluated in FP64 */
     uint64_t num_batches;
@@ -111,7 +112,7 @@ typedef struct {
     float ms_join_kernels;      /* count + fill kernel time */
     float ms_fill_kernel;       /* fill kernel time alone */
     uint64_t kernel_launches;   /* this library's kernel launches during the last join */
-    float ms_expand;            /* key-array expansion from the batch's key runs */
+    float ms_expand;            /* always 0: the emission writes the key array */
     uint32_t exact_plan_batches;/* batches the same greedy plan needs with the measured per-task pairs
                                    in place of the predictions (the estimator-free reference count) */
 } sj_stats;

@@ -225,8 +225,10 @@ struct Ctx {
     bool indexed = false;
     sj_grid_dev g{};
     uint32_t nCells = 0;
-    DevBuf<uint32_t> ids;      // cell-sorted point ids
-    DevBuf<double> xs;         // cell-sorted coordinates, n x Dp
+    DevBuf<uint32_t> ids;      // cell-sorted point ids, ascending inside a cell (the exported order)
+    DevBuf<uint32_t> placeIds; // the join's order: cell-sorted, in spatial order inside a cell
+    const uint32_t *jids = nullptr;   // the join's order (placeIds or ids)
+    DevBuf<double> xs;         // coordinates in the join's order, n x Dp
     DevBuf<uint32_t> cellStart;
     DevBuf<uint64_t> cellLid;
     DevBuf<uint32_t> cellCoord;
@@ -248,6 +250,7 @@ struct Ctx {
     uint32_t nTasks = 0;
     DevBuf<sj_task> dTasks, dTasksAlt;
     DevBuf<float> dTaskPred, dTaskPredAlt;
+    DevBuf<uint32_t> smallPre, bigList, smallList;   // the tasks by count-pass kernel (sj_task_lists)
     DevBuf<uint32_t> tgGroupCnt, tgGroupBase, tgGroupLen, tgPosCnt, tgOrder, tgOrderAlt, tgItemCnt, tgItemStart,
         tgItemTasks, tgItemTaskStart, tgTot32;
     DevBuf<uint64_t> tgKeys, tgKeysAlt;
@@ -270,7 +273,7 @@ struct Ctx {
     DevBuf<uint32_t> keyStartAlt;
     std::vector<cudaEvent_t> syncEvents;   // stage boundaries of the synchronous phase
     DevBuf<uint8_t> scanTemp, scanTemp2;
-    DevBuf<uint32_t> total, total2;
+    DevBuf<uint32_t> total;
     DevBuf<unsigned long long> stat;   // see sj_join_args::stat
     DevBuf<uint32_t> queueHead;
     DevBuf<uint32_t> taskHits;
@@ -290,9 +293,6 @@ struct Ctx {
     int32_t *csrCols = nullptr;
     uint64_t csrCap = 0;
     DevBuf<uint32_t> csrFill;
-    DevBuf<uint4> longRuns;            // key expansion: runs too long for one warp
-    DevBuf<uint32_t> foldChunkKey;     // consumer fold: the key at each chunk's first slot
-    DevBuf<uint32_t> longCount;
     DevBuf<unsigned long long> batchTot;
     std::vector<cudaEvent_t> events;   // per-batch stage boundaries of the asynchronous phase
     PinBuf pinTotal, pinKey[2], pinVal[2], pinStart[2];
@@ -371,6 +371,56 @@ sj_status check_params(const sj_params &p)
 }
 
 // ---------------------------------------------------------------- index --
+// Bits that hold the values 0 .. count - 1 (at least 1).
+int bits_for(uint64_t count)
+{
+    int bits = 1;
+    while (bits < 64 && (1ULL << bits) < count) bits++;
+    return bits;
+}
+
+// The order of the points inside their cells (see sj_place_plan).  The count
+// pass rules out (32 queries x 32 candidates) tiles by the boxes of their
+// points, so the points of a cell are put in an order in which 32 consecutive
+// ones lie close together: each bit of the place halves the dimension along
+// which the bins are widest so far (a cell is eps wide in the indexed
+// dimensions, the data's range in the others).
+// Only where the cells hold 16 points or more on average: with fewer, 32
+// consecutive points span cells anyway and the extra sort does not pay.
+sj_place_plan place_plan(const Ctx &c)
+{
+    sj_place_plan pl{};
+    if (c.nCells == 0 || c.n / c.nCells < 16) return pl;
+    const sj_grid_dev &g = c.g;
+    double width[SJ_MAX_DIM];
+    for (int j = 0; j < g.D; j++) {
+        const double range = c.dataMax[j] - c.dataMin[j];
+        width[j] = j < g.k ? g.eps : range;
+        pl.lo[j] = c.dataMin[j];
+        pl.inv[j] = range > 0.0 ? 1.0 / range : 0.0;
+        if (!std::isfinite(range) || !std::isfinite(pl.inv[j])) width[j] = pl.inv[j] = 0.0;
+    }
+    // cell and place share a 32-bit key, sorted 8 bits a pass: fill up 24 or 32 bits
+    const int cellBits = bits_for(c.nCells);
+    const int bits = std::min(18, (cellBits + 12 <= 24 ? 24 : 32) - cellBits);
+    for (int b = 0; b < bits; b++) {
+        int d = 0;
+        for (int j = 1; j < g.D; j++)
+            if (width[j] > width[d]) d = j;
+        pl.dim[b] = (uint8_t)d;
+        pl.nb[d]++;
+        width[d] *= 0.5;
+    }
+    uint8_t used[SJ_MAX_DIM] = {0};
+    for (int b = 0; b < bits; b++) {
+        const int d = pl.dim[b];
+        used[d]++;
+        pl.shift[b] = (uint8_t)(pl.nb[d] - used[d]);
+    }
+    pl.bits = std::max(bits, 0);
+    return pl;
+}
+
 sj_status build_index(Ctx &c)
 {
     if (!c.havePoints) {
@@ -429,8 +479,7 @@ sj_status build_index(Ctx &c)
         return SJ_ERR_BAD_INPUT;
     }
     c.st.total_cells = mul;
-    int bits = 1;
-    while (bits < 64 && (1ULL << bits) < mul) bits++;
+    const int bits = bits_for(mul);
     // 3. keys, stable sort, run-length cells
     DevBuf<uint64_t> &keys = c.sKeys, &keysAlt = c.sKeysAlt;
     DevBuf<uint32_t> &valsAlt = c.sValsAlt, &flags = c.sFlags;
@@ -448,7 +497,7 @@ sj_status build_index(Ctx &c)
     int inAlt = 0;
     CK(sj_radix_sort_u64_u32(keys.p, c.ids.p, keysAlt.p, valsAlt.p, n, bits, tmp.p, &inAlt, c.s));
     uint64_t *sk = inAlt ? keysAlt.p : keys.p;
-    if (inAlt) CK(cudaMemcpyAsync(c.ids.p, valsAlt.p, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, c.s));
+    if (inAlt) c.ids.swap(valsAlt);
     CK(sj_launch_cell_flags(sk, n, flags.p, c.s));
     CK(sj_exclusive_scan_u32(flags.p, flags.p, n, tmp.p, nne.p, c.s));
     uint32_t hn[2] = {0, 0};
@@ -468,9 +517,28 @@ sj_status build_index(Ctx &c)
     uint32_t nn = (uint32_t)n;
     CK(cudaMemcpyAsync(c.cellStart.p + nCells, &nn, sizeof(uint32_t), cudaMemcpyHostToDevice, c.s));
     CK(sj_launch_cell_coords(c.cellLid.p, nCells, g, c.cellCoord.p, c.s));
-    // 4. cell-sorted coordinates
+    // 4. the join's order inside the cells and the coordinates in that order
+    c.jids = c.ids.p;
+    const sj_place_plan pl = place_plan(c);
+    if (pl.bits) {
+        // the buffer that does not hold the sorted cell ids is free
+        uint32_t *pk = reinterpret_cast<uint32_t *>(inAlt ? keys.p : keysAlt.p), *pkAlt = pk + n;
+        CK(c.placeIds.ensure(n));
+        CK(valsAlt.ensure(n));
+        CK(sj_launch_place_keys(c.pts.p, c.ids.p, sk, flags.p, n, g, pl, pk, c.placeIds.p, c.s));
+        int placeAlt = 0;
+        CK(sj_radix_sort_u32_u32(pk, c.placeIds.p, pkAlt, valsAlt.p, n, bits_for(nCells) + pl.bits, tmp.p, &placeAlt,
+                                 c.s));
+        if (placeAlt) {
+            c.placeIds.swap(valsAlt);
+            std::swap(pk, pkAlt);
+        }
+        CK(sj_launch_place_spread(pk, c.placeIds.p, c.cellStart.p, n, pl.bits, valsAlt.p, c.s));
+        c.placeIds.swap(valsAlt);
+        c.jids = c.placeIds.p;
+    }
     CK(c.xs.ensure(n * (uint64_t)g.Dp));
-    CK(sj_launch_gather(c.pts.p, c.ids.p, n, D, g.Dp, c.xs.p, c.s));
+    CK(sj_launch_gather(c.pts.p, c.jids, n, D, g.Dp, c.xs.p, c.s));
     c.indexed = true;
     c.nbrPattern = -1;
     c.haveMeas = false;
@@ -525,7 +593,9 @@ void join_args_base(Ctx &c, sj_join_args &a)
 {
     memset(&a, 0, sizeof(a));
     a.xs = c.xs.p;
-    a.ids = c.ids.p;
+    a.ids = c.jids;
+    a.pts = c.pts.p;
+    a.indexIds = c.ids.p;
     a.cellStart = c.cellStart.p;
     a.nbrStart = c.nbrStart.p;
     a.nbrCell = c.nbrCell.p;
@@ -544,9 +614,15 @@ void join_args_base(Ctx &c, sj_join_args &a)
 // d2 <= T.  y >= delta proves d2 > T when delta >= 2M + 2u (T + Ra^2 + M) (the
 // second term covers rounding tLo down).  Pairs with 0 < y < delta are
 // re-evaluated in FP64.
+// pruneT: two boxes of local FP32 coordinates whose squared distance s, in FP32,
+// exceeds T + 2M hold no pair that satisfies the predicate: rounding the
+// coordinates and the sum moves it by less than (D+6) u r^2 < M, the predicate's
+// own rounding by less than M.  Outside the range in which FP32 squares keep
+// that accuracy nothing is ruled out.
 struct FilterBounds {
     double margin;
     float delta;
+    float pruneT;
 };
 
 FilterBounds filter_bounds(const Ctx &c)
@@ -572,6 +648,11 @@ FilterBounds filter_bounds(const Ctx &c)
     float df = (float)d;
     if ((double)df < d) df = std::nextafter(df, INFINITY);
     b.delta = df;
+    b.pruneT = INFINITY;
+    if (g.eps >= 1e-15 && g.eps <= 1e15) {
+        const double pt = (T + 2.0 * b.margin) * (1.0 + std::ldexp(1.0, -20));
+        if (pt < 3.0e38) b.pruneT = std::nextafter((float)pt, INFINITY);
+    }
     return b;
 }
 
@@ -580,14 +661,16 @@ struct BatchRange {
     uint32_t t0, t1;
     double pred;      // planned batch: its predicted pairs; a part re-planned after an overflow: -1
     uint64_t exact;   // a re-planned part: its measured pairs (0 for a planned batch)
+    uint32_t big, small;   // tasks of each count-pass kernel (a re-planned part: upper bounds)
 };
 
-sj_status run_count(Ctx &c, sj_join_args &a, bool queue, cudaStream_t st = nullptr, int maxCtasPerSM = 0)
+sj_status run_count(Ctx &c, sj_join_args &a, bool queue, uint32_t nBig, uint32_t nSmall, cudaStream_t st = nullptr,
+                    int maxCtasPerSM = 0)
 {
     if (!st) st = c.s;
-    if (queue) CK(cudaMemsetAsync(c.queueHead.p, 0, sizeof(uint32_t), st));
-    CK(sj_launch_join(a, c.g, c.p.precision == SJ_PREC_FP32_REFINE ? 1 : 0, queue ? 1 : 0, c.numSM, maxCtasPerSM,
-                      st));
+    if (queue) CK(cudaMemsetAsync(c.queueHead.p, 0, sizeof(uint32_t) * 2, st));
+    CK(sj_launch_join(a, c.g, c.p.precision == SJ_PREC_FP32_REFINE ? 1 : 0, queue ? 1 : 0, nBig, nSmall, c.numSM,
+                      maxCtasPerSM, st));
     return SJ_OK;
 }
 
@@ -644,10 +727,11 @@ sj_status build_tasks_dev(Ctx &c, bool sym, uint64_t cap, bool byCost, int polic
         const double v = atof(ev);
         if (v >= 1.0) g.pairsPerTask = v;
     }
-    // evaluations per task at most: about 2 ms of one count-pass CTA, so a
-    // batch's tail is short next to its ~10^10 evaluations over ~740 CTAs.
+    // evaluations per task at most: about 2 ms of one count-pass CTA, and few
+    // enough that a join that is one batch still has some 16 tasks per resident
+    // CTA to level out (tasks differ by what their boxes rule out).
     // SJ_TASK_EVALS overrides it (0: no limit; a tuning knob)
-    g.evalsPerTask = 4.0e6;
+    g.evalsPerTask = std::min(4.0e6, std::max(262144.0, (double)c.st.full_stencil_calcs / (sym ? 24000.0 : 12000.0)));
     if (const char *ev = getenv("SJ_TASK_EVALS")) g.evalsPerTask = std::max(0.0, atof(ev));
     g.sym = sym ? 1 : 0;
     g.policy = policy;
@@ -750,6 +834,11 @@ sj_status build_tasks_dev(Ctx &c, bool sym, uint64_t cap, bool byCost, int polic
         nt = nOut;
     }
     c.nTasks = nt;
+    CK(c.smallPre.ensure((size_t)nt + 1));
+    CK(c.bigList.ensure(nt ? nt : 1));
+    CK(c.smallList.ensure(nt ? nt : 1));
+    CK(tmp.ensure(sj_scan_temp_bytes((uint64_t)nt + 1)));
+    CK(sj_task_lists(c.dTasks.p, nt, c.smallPre.p, c.bigList.p, c.smallList.p, tmp.p, s));
     return SJ_OK;
 }
 
@@ -793,17 +882,19 @@ sj_status plan_dev(Ctx &c, uint64_t cap, std::vector<BatchRange> &plan, uint64_t
     predTotal = (double)h.pred;
     const uint32_t nb = h.nb;
     if (nb == 0) return SJ_OK;
-    CK(c.planStats.ensure((size_t)nb * 5));
-    CK(sj_plan_stats(c.planStart.p, nb, off, c.planStats.p, c.s));
+    CK(c.planStats.ensure((size_t)nb * 6));
+    CK(sj_plan_stats(c.planStart.p, nb, off, c.smallPre.p, c.planStats.p, c.s));
     std::vector<uint32_t> start(nb + 1);
-    std::vector<unsigned long long> st((size_t)nb * 5);
+    std::vector<unsigned long long> st((size_t)nb * 6);
     CK(cudaMemcpyAsync(start.data(), c.planStart.p, sizeof(uint32_t) * (nb + 1), cudaMemcpyDeviceToHost, c.s));
-    CK(cudaMemcpyAsync(st.data(), c.planStats.p, sizeof(unsigned long long) * nb * 5, cudaMemcpyDeviceToHost, c.s));
+    CK(cudaMemcpyAsync(st.data(), c.planStats.p, sizeof(unsigned long long) * nb * 6, cudaMemcpyDeviceToHost, c.s));
     CK(cudaStreamSynchronize(c.s));
     plan.resize(nb);
     for (uint32_t b = 0; b < nb; b++) {
-        plan[b] = {start[b], start[b + 1], (double)st[(size_t)b * 5], 0};
-        for (int k = 0; k < 4; k++) maxes[k] = std::max<uint64_t>(maxes[k], st[(size_t)b * 5 + 1 + k]);
+        const unsigned long long *const sb = &st[(size_t)b * 6];
+        const uint32_t n = start[b + 1] - start[b], small = (uint32_t)sb[5];
+        plan[b] = {start[b], start[b + 1], (double)sb[0], 0, n - small, small};
+        for (int k = 0; k < 4; k++) maxes[k] = std::max<uint64_t>(maxes[k], sb[1 + k]);
     }
     return SJ_OK;
 }
@@ -836,13 +927,16 @@ sj_status estimate_rates(Ctx &c)
         const uint32_t nt = c.nTasks;
         CK(c.keyCount.ensure(c.n));
         CK(c.stat.ensure(8));
-        CK(c.queueHead.ensure(1));
+        CK(c.queueHead.ensure(2));
         CK(c.taskHits.ensure(nt ? nt : 1));
         CK(c.dTaskEvals.ensure(nt ? nt : 1));
         CK(c.dTaskRefined.ensure(nt ? nt : 1));
         sj_join_args a;
         join_args_base(c, a);
         a.tasks = c.dTasks.p;
+        a.smallPre = c.smallPre.p;
+        a.bigList = c.bigList.p;
+        a.smallList = c.smallList.p;
         a.queueHead = c.queueHead.p;
         a.keyCount = c.keyCount.p;   // cleared before the join's first count pass
         a.stat = c.stat.p;
@@ -852,9 +946,10 @@ sj_status estimate_rates(Ctx &c)
         const FilterBounds fb = filter_bounds(c);
         a.margin = fb.margin;
         a.delta = fb.delta;
+        a.pruneT = fb.pruneT;
         a.taskBegin = 0;
         a.taskEnd = nt;
-        CKS(run_count(c, a, true));
+        CKS(run_count(c, a, true, nt, nt));
         CK(c.sHits.ensure(2 * (size_t)(nc ? nc : 1)));
         CK(c.sCands.ensure(2 * (size_t)(nc ? nc : 1)));
         CK(c.sScalars.ensure(2 + sj_sample_totals_len()));
@@ -945,28 +1040,14 @@ sj_status replan_exact(const BatchRange &br, const std::vector<uint32_t> &taskHi
             return SJ_ERR_INTERNAL;
         }
         if (t > t0 && acc + h > cap) {
-            parts.push_back({t0, t, -1.0, acc});
+            parts.push_back({t0, t, -1.0, acc, t - t0, t - t0});
             t0 = t;
             acc = 0;
         }
         acc += h;
     }
-    parts.push_back({t0, br.t1, -1.0, acc});
+    parts.push_back({t0, br.t1, -1.0, acc, br.t1 - t0, br.t1 - t0});
     out.insert(out.end(), parts.begin(), parts.end());
-    return SJ_OK;
-}
-
-// Key array of the current batch (a.outKey, a.capacity) from a.keyStart and
-// the batch's scan total (default: c.total).
-sj_status expand_keys(Ctx &c, const sj_join_args &a, cudaStream_t st = nullptr, const uint32_t *scanTotal = nullptr)
-{
-    if (!st) st = c.s;
-    if (!scanTotal) scanTotal = c.total.p;
-    const size_t slots = sj_expand_long_slots(a.capacity);
-    CK(c.longRuns.ensure(slots));
-    CK(c.longCount.ensure(1));
-    CK(sj_expand_keys(a.keyStart, scanTotal, c.n, a.outKey, a.batchPairs, a.capacity, c.longRuns.p,
-                      (uint32_t)std::min<size_t>(c.longRuns.n, 0xffffffffu), c.longCount.p, c.numSM, st));
     return SJ_OK;
 }
 
@@ -1009,7 +1090,7 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
     CK(c.scanTemp.ensure(sj_scan_temp_bytes(n)));
     CK(c.total.ensure(1));
     CK(c.stat.ensure(8));
-    CK(c.queueHead.ensure(1));
+    CK(c.queueHead.ensure(2));
     CK(c.taskHits.ensure(nt ? nt : 1));
     CK(cudaMemsetAsync(c.taskHits.p, 0, sizeof(uint32_t) * (nt ? nt : 1), c.s));
     CK(c.dTaskEvals.ensure(nt ? nt : 1));
@@ -1029,6 +1110,9 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
     sj_join_args a;
     join_args_base(c, a);
     a.tasks = c.dTasks.p;
+    a.smallPre = c.smallPre.p;
+    a.bigList = c.bigList.p;
+    a.smallList = c.smallList.p;
     a.queueHead = c.queueHead.p;
     a.keyCount = c.keyCount.p;
     a.keyStart = c.keyStart.p;
@@ -1053,12 +1137,13 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
         const FilterBounds fb = filter_bounds(c);
         a.margin = fb.margin;
         a.delta = fb.delta;
+        a.pruneT = fb.pruneT;
     }
 
     std::vector<uint32_t> hTaskHits(nt);
     uint64_t pairsTotal = 0, batches = 0, retries = 0, errBatches = 0;
     double relErrSum = 0;
-    float msCount = 0, msScan = 0, msFill = 0, msDeliver = 0, msExpand = 0;
+    float msCount = 0, msScan = 0, msFill = 0, msDeliver = 0;
     int pinSel = 0;
     sj_status result = SJ_OK;
     CK(c.batchTot.ensure(plan.size() + 1));
@@ -1072,9 +1157,9 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
     };
 
     // ---- asynchronous phase: batches folded on the device (no host delivery).
-    // Every batch runs count -> scan -> emission -> fold without a host round
-    // trip; a batch whose count exceeds the output buffer skips its emission
-    // and fold.  Such batches are re-planned exactly from the count pass's
+    // Every batch runs count -> scan -> emission without a host round trip; a
+    // batch whose count exceeds the output buffer skips its emission.  Such
+    // batches are re-planned exactly from the count pass's
     // per-task pairs and run through the same pipeline in a further round (the
     // exact parts cannot overflow again).
     std::vector<BatchRange> stack;
@@ -1094,19 +1179,16 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
         a.outKey = c.outKey.p;
         a.outVal = c.outVal.p;
         a.capacity = bufCap;
-        CK(c.foldChunkKey.ensure(sj_fold_chunks(bufCap)));
         CK(c.batchTot.ensure(todo.size() + 1));
         CK(cudaMemsetAsync(c.batchTot.p, 0, sizeof(unsigned long long) * (todo.size() + 1), c.s));
         const size_t nplan = todo.size();
         // Two streams when the device has room for a second record set: the
-        // count pass and scan of each batch on the engine's stream, its key
-        // expansion, emission and fold on the second stream, so batch i + 1's
-        // count pass and scan run beside batch i's emission (and the launch
-        // tails of each stage fill with the other's work).  Batches alternate
-        // between two sets of count-pass records and two sets of key offsets
-        // and scan totals; batch i's count pass waits for batch i - 2's fold,
-        // the last reader of the set it reuses (the emission reads the
-        // records, the fold the key offsets and the scan total).
+        // count pass and scan of each batch on the engine's stream, its
+        // emission on the second stream, so batch i + 1's count pass and scan
+        // run beside batch i's emission (and the launch tails of each stage
+        // fill with the other's work).  Batches alternate between two sets of
+        // count-pass records and key offsets; batch i's count pass waits for
+        // batch i - 2's emission, the last reader of the set it reuses.
         // SJ_SERIAL=1 keeps every stage on the engine's stream (a diagnostic
         // knob: the per-stage CUDA-event times are then those of each stage alone)
         const char *serialEnv = getenv("SJ_SERIAL");
@@ -1119,7 +1201,6 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
             if (e == cudaSuccess) e = c.candRel2.ensure(maxCandRecs);
             if (e == cudaSuccess) e = c.emitHead.ensure(1);
             if (e == cudaSuccess) e = c.keyStart2.ensure(n);
-            if (e == cudaSuccess) e = c.total2.ensure(1);
             if (e != cudaSuccess) {
                 // no room for the second set: the batches run one after another
                 cudaGetLastError();
@@ -1143,7 +1224,7 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
                 if (s) cudaStreamSynchronize(s);
             }
         } drain{pipe ? sB : nullptr};
-        constexpr int EV = 8;   // events per batch
+        constexpr int EV = 6;   // events per batch
         while (c.events.size() < EV * nplan) {
             cudaEvent_t e;
             CK(cudaEventCreate(&e));
@@ -1158,7 +1239,6 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
             b.taskEnd = br.t1;
             b.batchPairs = c.batchTot.p + i;
             const bool second = pipe && (i & 1);
-            uint32_t *const scanTot = second ? c.total2.p : c.total.p;
             if (second) {
                 b.masks = c.masks2.p;
                 b.colMasks = c.colMasks2.p;
@@ -1167,28 +1247,23 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
                 b.candRel = c.candRel2.p;
                 b.keyStart = c.keyStart2.p;
             }
-            if (pipe && i > 1) CK(cudaStreamWaitEvent(sA, ev[EV * (i - 2) + 7], 0));   // set reused: fold i-2 done
+            if (pipe && i > 1) CK(cudaStreamWaitEvent(sA, ev[EV * (i - 2) + 5], 0));   // set reused: emission i-2 done
             CK(cudaEventRecord(e[0], sA));
-            CKS(run_count(c, b, queue, sA, pipe ? joinCtas : 0));
+            CKS(run_count(c, b, queue, br.big, br.small, sA, pipe ? joinCtas : 0));
             CK(cudaEventRecord(e[1], sA));
             CK(cudaEventRecord(e[2], sA));
-            CK(sj_exclusive_scan_u32_clear(c.keyCount.p, const_cast<uint32_t *>(b.keyStart), n, c.scanTemp.p, scanTot,
+            CK(sj_exclusive_scan_u32_clear(c.keyCount.p, const_cast<uint32_t *>(b.keyStart), n, c.scanTemp.p, c.total.p,
                                            sA));
             CK(cudaEventRecord(e[3], sA));
             if (pipe) CK(cudaStreamWaitEvent(sB, e[3], 0));
-            // emission (values), then the consumer fold, which reads the values
-            // back and writes the key array in the same pass
+            // emission: values, keys and the set hash of every pair
             CK(cudaEventRecord(e[4], sB));
-            CK(cudaEventRecord(e[5], sB));
             b.queueHead = pipe ? c.emitHead.p : c.queueHead.p;
             CK(cudaMemsetAsync(b.queueHead, 0, sizeof(uint32_t), sB));
-            CK(sj_launch_emit(b, c.numSM, pipe ? emitCtas : 0, sB));
-            CK(cudaEventRecord(e[6], sB));
-            CK(sj_fold(b.keyStart, scanTot, n, c.outVal.p, c.outKey.p, b.batchPairs, bufCap, c.foldChunkKey.p,
-                       c.stat.p + 4, c.numSM, sB));
-            CK(cudaEventRecord(e[7], sB));
+            CK(sj_launch_emit(b, 1, c.numSM, pipe ? emitCtas : 0, sB));
+            CK(cudaEventRecord(e[5], sB));
         }
-        if (pipe) CK(cudaStreamWaitEvent(sA, ev[EV * (nplan - 1) + 7], 0));
+        if (pipe) CK(cudaStreamWaitEvent(sA, ev[EV * (nplan - 1) + 5], 0));
         std::vector<unsigned long long> tot(nplan);
         CK(cudaMemcpyAsync(tot.data(), c.batchTot.p, sizeof(unsigned long long) * nplan, cudaMemcpyDeviceToHost,
                            c.s));
@@ -1198,17 +1273,13 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
         // sharing the device with the other stream's stage)
         for (size_t i = 0; i < nplan; i++) {
             const cudaEvent_t *e = ev + EV * i;
-            float tc, ts, tx, tf, th;
+            float tc, ts, tf;
             cudaEventElapsedTime(&tc, e[0], e[1]);
             cudaEventElapsedTime(&ts, e[2], e[3]);
-            cudaEventElapsedTime(&tx, e[4], e[5]);
-            cudaEventElapsedTime(&tf, e[5], e[6]);
-            cudaEventElapsedTime(&th, e[6], e[7]);
+            cudaEventElapsedTime(&tf, e[4], e[5]);
             msCount += tc;
             msScan += ts;
-            msExpand += tx;
             msFill += tf;
-            msDeliver += th;
         }
         // SJ_BATCH_LOG=<file>: one line per batch of this round appended to the
         // file (a diagnostic knob): tasks, pairs, record sizes, stage times
@@ -1223,17 +1294,15 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
                 for (size_t i = 0; i < nplan; i++) {
                     const BatchRange &br = todo[i];
                     const cudaEvent_t *e = ev + EV * i;
-                    float tc, tf, th;
+                    float tc, tf;
                     cudaEventElapsedTime(&tc, e[0], e[1]);
-                    cudaEventElapsedTime(&tf, e[5], e[6]);
-                    cudaEventElapsedTime(&th, e[6], e[7]);
+                    cudaEventElapsedTime(&tf, e[4], e[5]);
                     fprintf(lf,
                             "{\"round\": %d, \"batch\": %zu, \"t0\": %u, \"t1\": %u, \"pairs\": %llu, "
                             "\"row_words\": %llu, \"col_words\": %llu, \"query_recs\": %llu, \"cand_recs\": %llu, "
-                            "\"units\": %llu, \"count_ms\": %.4f, \"emit_ms\": %.4f, \"fold_ms\": %.4f}\n",
+                            "\"units\": %llu, \"count_ms\": %.4f, \"emit_ms\": %.4f}\n",
                             round, i, br.t0, br.t1, tot[i], ho[0][br.t1] - ho[0][br.t0], ho[1][br.t1] - ho[1][br.t0],
-                            ho[2][br.t1] - ho[2][br.t0], ho[3][br.t1] - ho[3][br.t0], ho[4][br.t1] - ho[4][br.t0], tc,
-                            tf, th);
+                            ho[2][br.t1] - ho[2][br.t0], ho[3][br.t1] - ho[3][br.t0], ho[4][br.t1] - ho[4][br.t0], tc, tf);
                 }
                 fclose(lf);
             }
@@ -1307,7 +1376,7 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
         a.keyStart = ksBuf;
         CK(cudaMemsetAsync(slot, 0, sizeof(unsigned long long), c.s));
         CK(cudaEventRecord(ev(0), c.s));
-        CKS(run_count(c, a, queue));
+        CKS(run_count(c, a, queue, br.big, br.small));
         CK(cudaEventRecord(ev(1), c.s));
         // this set's run offsets must have been copied out before the scan rewrites them
         if (setUsed[sel]) CK(cudaStreamWaitEvent(c.s, c.evStart[sel], 0));
@@ -1349,14 +1418,13 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
         a.outKey = c.outKey.p;
         a.outVal = valBuf;
         a.capacity = std::min<uint64_t>(c.outKey.n, sel ? c.outValAlt.n : c.outVal.n);
-        CKS(expand_keys(c, a));
         CK(cudaEventRecord(ev(3), c.s));
         // this set's values must have been copied out before the emission rewrites them
         if (setUsed[sel]) CK(cudaStreamWaitEvent(c.s, c.evVals[sel], 0));
         CK(cudaMemsetAsync(c.queueHead.p, 0, sizeof(uint32_t), c.s));
-        CK(sj_launch_emit(a, c.numSM, 0, c.s));
+        // host delivery expands the keys on the host, the CSR table has none
+        CK(sj_launch_emit(a, delivery == SJ_DELIVER_DEVICE ? 1 : 0, c.numSM, 0, c.s));
         CK(cudaEventRecord(ev(4), c.s));
-        CK(sj_hash_pairs(c.outKey.p, valBuf, cnt, c.stat.p + 4, c.s));
         if (delivery == SJ_DELIVER_CSR) {
             CK(sj_csr_append(ksBuf, c.total.p, n, valBuf, c.csrRowPtr, c.csrFill.p, c.csrCols, c.csrCap,
                              c.stat.p + 7, c.s));
@@ -1408,17 +1476,15 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
     CK(cudaStreamSynchronize(c.cs));
     CK(cudaStreamSynchronize(c.s));
     for (size_t i = 0; i < iter; i++) {
-        float t01 = 0, t12 = 0, t23 = 0, t34 = 0, t45 = 0;
+        float t01 = 0, t12 = 0, t34 = 0, t45 = 0;
         cudaEvent_t *e = c.syncEvents.data() + 6 * i;
         cudaEventElapsedTime(&t01, e[0], e[1]);
         cudaEventElapsedTime(&t12, e[1], e[2]);
         msCount += t01;
         msScan += t12;
         if (iterFull[i]) {
-            cudaEventElapsedTime(&t23, e[2], e[3]);
             cudaEventElapsedTime(&t34, e[3], e[4]);
             cudaEventElapsedTime(&t45, e[4], e[5]);
-            msExpand += t23;
             msFill += t34;
             msDeliver += t45;
         }
@@ -1473,7 +1539,7 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
     c.st.ms_deliver = msDeliver;
     c.st.ms_join_kernels = msCount + msFill;
     c.st.ms_fill_kernel = msFill;
-    c.st.ms_expand = msExpand;
+    c.st.ms_expand = 0;   // the emission writes the keys
     c.st.ms_total = total.stop(c.s);
     c.st.kernel_launches = sj_launch_total() - launches0;
     return result;
@@ -1490,12 +1556,15 @@ sj_status run_degrees(Ctx &c, uint32_t *degHost)
     const uint32_t nt = c.nTasks;
     CK(c.keyCount.ensure(n));
     CK(c.stat.ensure(8));
-    CK(c.queueHead.ensure(1));
+    CK(c.queueHead.ensure(2));
     CK(cudaMemsetAsync(c.keyCount.p, 0, sizeof(uint32_t) * n, c.s));
     CK(cudaMemsetAsync(c.stat.p, 0, sizeof(unsigned long long) * 8, c.s));
     sj_join_args a;
     join_args_base(c, a);
     a.tasks = c.dTasks.p;
+    a.smallPre = c.smallPre.p;
+    a.bigList = c.bigList.p;
+    a.smallList = c.smallList.p;
     a.queueHead = c.queueHead.p;
     a.keyCount = c.keyCount.p;
     a.stat = c.stat.p;
@@ -1503,6 +1572,7 @@ sj_status run_degrees(Ctx &c, uint32_t *degHost)
         const FilterBounds fb = filter_bounds(c);
         a.margin = fb.margin;
         a.delta = fb.delta;
+        a.pruneT = fb.pruneT;
     }
     CK(c.dTaskEvals.ensure(nt ? nt : 1));
     CK(c.dTaskRefined.ensure(nt ? nt : 1));
@@ -1510,7 +1580,7 @@ sj_status run_degrees(Ctx &c, uint32_t *degHost)
     a.taskRefined = c.dTaskRefined.p;
     a.taskBegin = 0;
     a.taskEnd = nt;
-    CKS(run_count(c, a, true));
+    CKS(run_count(c, a, true, nt, nt));
     // per-cell measured hits (the sum of the cell's points' degrees)
     CK(c.dCellHits.ensure(c.nCells ? c.nCells : 1));
     CK(sj_cell_hits(c.cellStart.p, c.ids.p, c.keyCount.p, c.nCells, c.dCellHits.p, c.s));

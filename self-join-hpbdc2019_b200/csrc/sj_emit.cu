@@ -1,10 +1,12 @@
-// The emission pass: (key, value) pairs from the count pass's hit masks.
+// The emission pass: the (key, value) pairs of a batch from the count pass's
+// hit masks, with the pairs' set hash.
 //
 // The count pass (sj_join.cu) leaves, per task of the batch:
-//   * every query's row hit mask per block of 32 stream positions, laid out
-//     [chunk of 64 blocks][query][block in chunk];
-//   * for a symmetric task the transposed (column) masks: per block and group
-//     of 32 queries, candidate j's query bits, laid out [block][group][j];
+//   * live bits per (block of 32 stream positions, group of 32 queries): whether
+//     the tile has any hit; only live tiles have hit words;
+//   * row words [block][query] (bit = stream position of the block) and, for a
+//     symmetric task, column words [block][group][position] (bit = query of the
+//     group);
 //   * per query the offset of the task's row run inside the query's key run,
 //     and per stream position the candidate's point id and the offset of its
 //     column run inside the candidate's key run.  Both offsets are the key's
@@ -15,68 +17,60 @@
 // come out ascending with each key's values contiguous -- the order
 // thrust::sort_by_key gives the reference (GPU.cu:2336) -- without a sort.
 //
-// Work is cut into warp units that any warp of any CTA takes from a counter:
-//   row unit    (task, group of 32 queries): the group's words of a chunk are
-//               contiguous; a window of 64 words (lane L holds words L and
-//               32 + L; one window spans several queries when the task has
-//               few blocks) is popcounted and scanned (both halves' counts
-//               packed in one 32-bit scan), its set bits are decoded into
-//               shared memory as 16-bit (query, stream position) entries in
-//               slot order, and the warp copies the entries out: consecutive
-//               entries of one query go to consecutive slots, so the stores
-//               are coalesced.
-//   column unit (symmetric task, block of 32 stream positions): lane j is
-//               candidate j; per query group its word is decoded lane-major
-//               and copied out the same way, each lane's run continuing across
-//               groups.
-// A window without any set bit costs one ballot.  Measured on one B200 and
-// not kept: two query groups per column window (c3 emission +5 %), and row
-// windows aligned to one query's words when a chunk has >= 32 blocks (c3
-// +13 %, no gain elsewhere).
-// Only the values are written here: the keys of a batch are its key runs in
-// key order, which sj_expand_keys writes sequentially (the emission's writes
-// land at scattered run positions, which HBM absorbs at a fraction of its
-// sequential rate, so writing the keys there too would cost more than the
-// separate sequential pass).  Every mask word is checked against its task's
-// sizes before it is decoded (bits past the stream end or for queries past the
-// tile, which a consistent count pass never sets, are dropped and raise an
-// error flag that the host reports), so the decoded entries need no checks.  No distance is evaluated, so the pass is the same for both
-// precisions.
+// Work is cut into warp units that warps take from a counter, UN at a time:
+//   row unit    (task, group of 32 queries): per 32 blocks, the words of the
+//               live blocks; the lines are the queries (key), the values the
+//               candidates' ids;
+//   column unit (symmetric task, block of 32 positions): the words of the live
+//               groups; the lines are the candidates, the values the queries'.
+// Both stage up to TW words of every line and the values they select from in
+// shared memory and go through emit_lines: a window holds the words of one line
+// (or of 2, 4 .. lines when few words are live), one per lane; their popcounts
+// are scanned, the set bits decoded into a list in slot order, and the warp
+// copies the list out line by line: consecutive entries go to consecutive
+// slots, so the stores are coalesced.  Key, value and the hash of the pair are
+// produced in the same pass.
+//
+// Bound: instruction issue.  With the points of a cell in spatial order the
+// live words are dense (10 to 26 bits on average on the exponential sets, and
+// over 80 % of the pairs lie in words of 16 bits or more), so a window of 32
+// words yields 300 to 800 pairs and the copy-out -- two shared loads, two stores
+// and the ~19 integer operations of splitmix64 with the key's part taken out --
+// is most of the work.  Hence words across the lanes with one scan a window, and
+// not a list per line (lanes idle for the fullest line: 2.1 against 1.4 warp
+// instructions a pair on 6-D data).
+// Every mask word is checked against its task's sizes before it is decoded (bits
+// past the stream end or for queries past the tile, which a consistent count
+// pass never sets, are dropped and raise an error flag that the host reports),
+// so the decoded entries need no checks.  No distance is evaluated, so the pass
+// is the same for both precisions.
 #include "sj_internal.h"
 
 #include <atomic>
 
 namespace {
 
-constexpr int EW = 256;             // threads per emission CTA (independent warps)
+constexpr int EW = 128;             // threads per emission CTA (independent warps)
 constexpr int ENW = EW / 32;
-constexpr int EM_CAP = 2048;        // staged entries per warp: one window of 64 words x 32 bits
+constexpr int EMIT_MINB = 7;        // resident CTAs per SM (26 KB of shared memory, 72 registers a thread)
+constexpr uint32_t UN = 4;          // consecutive units a warp takes at a time (1 near the end of the batch)
 constexpr uint32_t FULL = 0xffffffffu;
-#ifndef SJ_EMIT_UNROLL
-#define SJ_EMIT_UNROLL 4
-#endif
-constexpr int CO = SJ_EMIT_UNROLL;  // copy-out entries per lane whose loads are in flight together
-// Mask windows (rows) / query groups (columns) whose words are loaded ahead of
-// the one being decoded: the emission reads the hit masks once, in order, so
-// its loads can run this far ahead of the decode.
-#ifndef SJ_EMIT_PF
-#define SJ_EMIT_PF 4
-#endif
-constexpr int PF = SJ_EMIT_PF;
-#ifndef SJ_EMIT_MINB
-#define SJ_EMIT_MINB 4
-#endif
-// 1: a CTA takes EW/32 consecutive units per round (one atomic), 0: each warp
-// takes units on its own
-#ifndef SJ_EMIT_COOP
-#define SJ_EMIT_COOP 0
-#endif
+constexpr uint32_t TW = 16;         // words per line staged together: windows of two lines
+constexpr uint32_t LD = 4;          // words whose loads are in flight together
+constexpr uint32_t DENSE = 14;      // fullest word of a window above which every bit is tested in turn
+static_assert(SJ_CTA * sj_query_slots(1, true) / 32 <= TW, "a task's query groups fit the staged words");
+
+struct __align__(16) LineInfo {
+    uint32_t base;          // slot of the window's list entry 0 if it were this line's
+    uint32_t key, hi2, add; // the line's key and its part of the pair hash
+};
 
 struct WarpSmem {
-    uint16_t ent[EM_CAP];   // staged entries in slot order: rows (query << 11) | chunk position,
-                            // columns (lane << 5) | query bit
-    uint32_t base[32];      // slot of entry 0 of the window for each query (rows) / lane (columns)
-    uint32_t start[32];     // rows: slot of each query's first pair of the chunk
+    uint32_t tile[TW][33];  // [staged word][line]
+    uint32_t val[TW * 32];  // value of bit i of staged word j: val[32 j + i]
+    uint16_t ent[1024];     // one window's list: byte offset into val; with more than two lines a window
+                            // (line in window << 10) | index into val
+    LineInfo line[32];
 };
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x, uint32_t lane)
@@ -97,10 +91,47 @@ __device__ __forceinline__ uint32_t top_bit(uint32_t m)
     return b;
 }
 
-// Writes tag | (index of each set bit of m) to buf[k .. k + n), lowest bit
-// first, where n = popc(m).  The bits are taken highest first and the entries
-// filled from the end, two per round (a lone last bit on its own).
-__device__ __forceinline__ void decode_bits(uint32_t m, uint32_t n, uint32_t tag, uint16_t *buf, uint32_t k)
+// The pair hash, splitmix64(key << 32 | value), with the key's part separated:
+// both are point ids below 2^31, so adding the increment's low half to the
+// value never carries and the high half depends on the key alone.  Written in
+// 32-bit halves (18 integer instructions).
+struct KeyHash {
+    uint32_t hi2, add;   // high word << 2 (xored into the low word); high word's contribution to the first product
+};
+
+__device__ __forceinline__ KeyHash key_hash(uint32_t key)
+{
+    const uint32_t hi = key + 0x9e3779b9u;
+    return {hi << 2, (hi ^ (hi >> 30)) * 0x1ce4e5b9u};
+}
+
+__device__ __forceinline__ uint64_t pair_hash(KeyHash kh, uint32_t val)
+{
+    const uint32_t y = val + 0x7f4a7c15u;
+    const uint32_t lo = y ^ (y >> 30) ^ kh.hi2;
+    const uint64_t z = (uint64_t)lo * 0x1ce4e5b9u;
+    uint32_t zl = (uint32_t)z, zh = lo * 0xbf58476du + kh.add + (uint32_t)(z >> 32);
+    zl ^= __funnelshift_r(zl, zh, 27);
+    zh ^= zh >> 27;
+    const uint64_t p = (uint64_t)zl * 0x133111ebu;
+    const uint32_t ql = (uint32_t)p;
+    const uint32_t qh = zh * 0x133111ebu + (zl * 0x94d049bbu + (uint32_t)(p >> 32));
+    return ((uint64_t)(qh ^ (qh >> 31)) << 32) | (ql ^ __funnelshift_r(ql, qh, 31));
+}
+
+// Output of one warp: the arrays, and the hash of the pairs written so far.
+struct Out {
+    int32_t *__restrict__ key;
+    int32_t *__restrict__ val;
+    uint64_t cap;
+    unsigned long long hash;
+};
+
+// Writes tag + unit * (index of each set bit of m) to the list from entry k on,
+// lowest bit first; n = popc(m).  sparse: the bits highest first, two a step, filling
+// from the end.  dense: all 32 bits tested, no bit scans and no loop.
+__device__ __forceinline__ void decode_sparse(uint32_t m, uint32_t n, uint32_t tag, uint32_t unit, uint16_t *buf,
+                                              uint32_t k)
 {
     uint16_t *p = buf + k + n;
     for (; n >= 2; n -= 2) {
@@ -108,267 +139,239 @@ __device__ __forceinline__ void decode_bits(uint32_t m, uint32_t n, uint32_t tag
         m ^= 1u << b0;
         const uint32_t b1 = top_bit(m);
         m ^= 1u << b1;
-        p[-1] = (uint16_t)(tag | b0);
-        p[-2] = (uint16_t)(tag | b1);
+        p[-1] = (uint16_t)(tag + unit * b0);
+        p[-2] = (uint16_t)(tag + unit * b1);
         p -= 2;
     }
-    if (n) p[-1] = (uint16_t)(tag | top_bit(m));
+    if (n) p[-1] = (uint16_t)(tag + unit * top_bit(m));
 }
 
-// decode_bits for two words at once (two independent chains of bit scans):
-// word a's n_a entries go to buf[ka ..), word b's to buf[kb ..).
-__device__ __forceinline__ void decode_bits2(uint32_t ma, uint32_t na, uint32_t tagA, uint32_t ka, uint32_t mb,
-                                             uint32_t nb, uint32_t tagB, uint32_t kb, uint16_t *buf)
+__device__ __forceinline__ void decode_dense(uint32_t m, uint32_t tag, uint32_t unit, uint16_t *buf, uint32_t k)
 {
-    uint16_t *pa = buf + ka + na, *pb = buf + kb + nb;
-    while (na >= 2 || nb >= 2) {
-        if (na >= 2) {
-            const uint32_t b0 = top_bit(ma);
-            ma ^= 1u << b0;
-            const uint32_t b1 = top_bit(ma);
-            ma ^= 1u << b1;
-            pa[-1] = (uint16_t)(tagA | b0);
-            pa[-2] = (uint16_t)(tagA | b1);
-            pa -= 2;
-            na -= 2;
-        }
-        if (nb >= 2) {
-            const uint32_t b0 = top_bit(mb);
-            mb ^= 1u << b0;
-            const uint32_t b1 = top_bit(mb);
-            mb ^= 1u << b1;
-            pb[-1] = (uint16_t)(tagB | b0);
-            pb[-2] = (uint16_t)(tagB | b1);
-            pb -= 2;
-            nb -= 2;
-        }
-    }
-    if (na) pa[-1] = (uint16_t)(tagA | top_bit(ma));
-    if (nb) pb[-1] = (uint16_t)(tagB | top_bit(mb));
-}
-
-// Stores one value.  FITS: the caller has shown that every slot of the window
-// is below the capacity; otherwise each slot is checked.
-template <bool FITS>
-__device__ __forceinline__ void put(const sj_join_args &a, uint32_t slot, int32_t val)
-{
-    if (FITS || slot < a.capacity) {
-        a.outVal[slot] = val;
-    } else {
-        atomicMax(&a.stat[3], 1ULL);
+    uint32_t p = (uint32_t)__cvta_generic_to_shared(buf + k);
+#pragma unroll
+    for (int b = 0; b < 32; b++) {
+        asm volatile("{ .reg .pred q; .reg .b32 t;\n\t"
+                     "and.b32 t, %1, %3; setp.ne.u32 q, t, 0;\n\t"
+                     "@q st.shared.u16 [%0], %2;\n\t"
+                     "@q add.u32 %0, %0, 2; }"
+                     : "+r"(p)
+                     : "r"(m), "r"(tag), "r"(1u << b)
+                     : "memory");
+        tag += unit;
     }
 }
 
-// Copies the window's T staged entries out: entry e goes to slot
-// slotOf(ent[e], e) with value src[srcOf(ent[e])].  Whole rounds of 32 * CO
-// entries issue all their loads before any store; the rest goes 32 at a time,
-// so a window never pays for more than 31 idle lane slots.
-template <bool FITS, class SlotOf, class SrcOf>
-__device__ __forceinline__ void copy_out(const sj_join_args &a, const uint16_t *ent, uint32_t T,
-                                         const uint32_t *__restrict__ src, uint32_t lane, SlotOf slotOf,
-                                         SrcOf srcOf)
+// Copies the list's entries [e0, e0 + n) of one line (byte offsets into w.val) to
+// slots B, B + 1 ..
+template <bool KEYS>
+__device__ __forceinline__ void copy_line(Out &o, const WarpSmem &w, uint32_t lane, uint32_t e0, uint32_t n,
+                                          uint32_t B, uint32_t key, KeyHash kh)
 {
-    uint32_t e0 = 0;
-    for (; e0 + 32 * CO <= T; e0 += 32 * CO) {
-        uint32_t slot[CO], pos[CO], val[CO];
+    uint32_t ent = (uint32_t)__cvta_generic_to_shared(w.ent + e0 + lane);
+    const uint32_t val = (uint32_t)__cvta_generic_to_shared(w.val);
+    int32_t *pv = o.val + (uint64_t)B + lane;
+    int32_t *pk = KEYS ? o.key + (uint64_t)B + lane : nullptr;
+#pragma unroll 1
+    for (; n >= 128; n -= 128) {
+        uint32_t at[4], v[4];
 #pragma unroll
-        for (int i = 0; i < CO; i++) {
-            const uint32_t e = e0 + 32 * i + lane;
-            const uint32_t en = ent[e];
-            pos[i] = srcOf(en);
-            slot[i] = slotOf(en, e);
+        for (uint32_t i = 0; i < 4; i++) asm volatile("ld.shared.u16 %0, [%1];" : "=r"(at[i]) : "r"(ent + 64 * i));
+#pragma unroll
+        for (uint32_t i = 0; i < 4; i++) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v[i]) : "r"(val + at[i]));
+#pragma unroll
+        for (uint32_t i = 0; i < 4; i++) {
+            pv[32 * i] = (int32_t)v[i];
+            if (KEYS) pk[32 * i] = (int32_t)key;
+            o.hash += pair_hash(kh, v[i]);
         }
-#pragma unroll
-        for (int i = 0; i < CO; i++) val[i] = __ldg(src + pos[i]);
-#pragma unroll
-        for (int i = 0; i < CO; i++) put<FITS>(a, slot[i], (int32_t)val[i]);
+        ent += 256;
+        pv += 128;
+        if (KEYS) pk += 128;
     }
-    for (; e0 < T; e0 += 32) {
-        const uint32_t e = e0 + lane;
-        if (e < T) {
-            const uint32_t en = ent[e];
-            put<FITS>(a, slotOf(en, e), (int32_t)__ldg(src + srcOf(en)));
-        }
+#pragma unroll 1
+    for (uint32_t e = lane; e < n; e += 32) {
+        uint32_t at, v;
+        asm volatile("ld.shared.u16 %0, [%1];" : "=r"(at) : "r"(ent));
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(val + at));
+        *pv = (int32_t)v;
+        if (KEYS) *pk = (int32_t)key;
+        o.hash += pair_hash(kh, v);
+        ent += 64;
+        pv += 32;
+        if (KEYS) pk += 32;
     }
 }
 
-// Fields of the task an emission unit belongs to.
-struct UnitTask {
-    uint32_t t, qBegin, qc, L;
-};
-
-// Bits of a row word whose block starts at stream position p0 (< L) past the
-// stream end are never set by a consistent count pass: drop them and flag it.
-__device__ __forceinline__ uint32_t stream_checked(const sj_join_args &a, uint32_t word, uint32_t p0, uint32_t L)
+// Emits the hits of up to 32 lines (those of the mask `lines` have any) over the
+// nl staged words.  Lane l holds line
+// l's key, its hash part and its next slot (advanced past the line's pairs).
+// Lines without hits need no valid key.
+template <bool KEYS>
+__device__ __forceinline__ void emit_lines(const sj_join_args &a, Out &o, WarpSmem &w, uint32_t lane, uint32_t nl,
+                                           uint32_t lines, uint32_t key, KeyHash kh, uint32_t &next)
 {
-    const uint32_t rem = L - p0;
-    if (rem < 32u && (word >> rem) != 0u) {
-        atomicMax(&a.stat[6], 1ULL);
-        word &= (1u << rem) - 1u;
-    }
-    return word;
-}
-
-// Row unit: queries 32g .. 32g+nq-1 of task u.t (key = query, value = candidate).
-__device__ __forceinline__ void emit_rows(const sj_join_args &a, const UnitTask &u, uint32_t g, WarpSmem &w,
-                                          uint32_t lane)
-{
-    const uint32_t qc = u.qc;
-    const uint32_t q0 = g * 32;
-    const uint32_t nq = min(32u, qc - q0);
-    const uint32_t nBlk = (u.L + 31) / 32;
-    const uint32_t *const masks = a.masks + (a.maskOff[u.t] - a.maskOff[a.taskBegin]);
-    const uint32_t *const cid = a.candId + (a.candOff[u.t] - a.candOff[a.taskBegin]);
-    const uint32_t *const rel = a.rowRel + (a.rowOff[u.t] - a.rowOff[a.taskBegin]);
-    uint32_t next = 0;   // lane q: slot of query q's next pair
-    __syncwarp();        // the previous unit is done with the warp's shared memory
-    if (lane < nq) {
-        const uint32_t qid = a.ids[u.qBegin + q0 + lane];
-        next = a.keyStart[qid] + rel[q0 + lane];
-    }
-    for (uint32_t c0 = 0; c0 < nBlk; c0 += 64) {
-        const uint32_t cb = min(64u, nBlk - c0);          // blocks of this chunk
-        const uint32_t nw = nq * cb;                      // the group's words of this chunk
-        const uint32_t *const wq = masks + (uint64_t)c0 * qc + (uint64_t)q0 * cb;
-        const uint32_t *const pcid = cid + c0 * 32;
-        const auto srcOf = [](uint32_t en) { return en & 0x7ffu; };
-        // floor(f / cb) = (f * magic) >> 32 for f < 2^26 (error < 2^-6 <= 1/cb)
-        const uint64_t magic = ((1ULL << 32) + cb - 1) / cb;
-        __syncwarp();
-        w.start[lane] = next;
-        uint32_t carry = 0;   // entries of earlier windows of this chunk
-        // a window is 64 words: lane L holds words L and 32 + L; the words of
-        // the next PF windows are in flight while this one is written
-        uint32_t pw[PF][2];
-#pragma unroll
-        for (int k = 0; k < PF; k++) {
-            const uint32_t f = 64u * k + lane;
-            pw[k][0] = f < nw ? __ldg(wq + f) : 0u;
-            pw[k][1] = f + 32 < nw ? __ldg(wq + f + 32) : 0u;
-        }
-        for (uint32_t ws = 0; ws < nw; ws += 64) {
-            const uint32_t fa = ws + lane, fb = fa + 32;
-            uint32_t wa = pw[0][0], wb = pw[0][1];
-#pragma unroll
-            for (int k = 0; k + 1 < PF; k++) {
-                pw[k][0] = pw[k + 1][0];
-                pw[k][1] = pw[k + 1][1];
-            }
-            {
-                const uint32_t f = fa + 64u * PF;
-                pw[PF - 1][0] = f < nw ? __ldg(wq + f) : 0u;
-                pw[PF - 1][1] = f + 32 < nw ? __ldg(wq + f + 32) : 0u;
-            }
-            const uint32_t qa = (uint32_t)(((uint64_t)fa * magic) >> 32);
-            const uint32_t qb = (uint32_t)(((uint64_t)fb * magic) >> 32);
-            const uint32_t ra = fa - qa * cb, rb = fb - qb * cb;   // block of each word in the chunk
-            // words past the group's end are zero; a word's block is inside the stream
-            if (wa) wa = stream_checked(a, wa, (c0 + ra) * 32u, u.L);
-            if (wb) wb = stream_checked(a, wb, (c0 + rb) * 32u, u.L);
-            const uint32_t ca = __popc(wa), cbt = __popc(wb);
-            if (__ballot_sync(FULL, ca | cbt) == 0) {
-                // no pair in the window: only the bases of queries that start in it
-                __syncwarp();
-                if (fa < nw && ra == 0) w.base[qa] = w.start[qa] - carry;
-                if (fb < nw && rb == 0) w.base[qb] = w.start[qb] - carry;
-                continue;
-            }
-            // one scan of both halves' counts (each total <= 1024 fits 16 bits):
-            // word fa's entries start at exA, word fb's at TA + exB
-            const uint32_t incl = warp_incl_scan(ca | (cbt << 16), lane);
-            const uint32_t tot = __shfl_sync(FULL, incl, 31);
-            const uint32_t TA = tot & 0xffffu, T = TA + (tot >> 16);
-            const uint32_t exA = (incl & 0xffffu) - ca, exB = TA + (incl >> 16) - cbt;
-            __syncwarp();   // the previous window's copy-out is done with ent / base
-            // a query's first word: base = its chunk start slot minus its flat prefix
-            if (fa < nw && ra == 0) w.base[qa] = w.start[qa] - (carry + exA);
-            if (fb < nw && rb == 0) w.base[qb] = w.start[qb] - (carry + exB);
-            decode_bits2(wa, ca, (qa << 11) | (ra << 5), exA, wb, cbt, (qb << 11) | (rb << 5), exB, w.ent);
-            __syncwarp();
-            // copy-out.  Every entry is valid by construction (words of queries
-            // < nq, bits inside the stream).
-            const uint32_t qf = __shfl_sync(FULL, qa, 0);
-            if (ws - qf * cb + min(64u, nw - ws) <= cb) {
-                // the whole window is one query's: one base for every entry
-                const uint32_t B = w.base[qf] + carry;
-                const auto slotOf = [B](uint32_t, uint32_t e) { return B + e; };
-                if ((uint64_t)B + T <= a.capacity) copy_out<true>(a, w.ent, T, pcid, lane, slotOf, srcOf);
-                else copy_out<false>(a, w.ent, T, pcid, lane, slotOf, srcOf);
-            } else {
-                const uint32_t *const base = w.base;
-                const uint32_t cy = carry;
-                // each word's last entry has the largest slot of its run
-                const bool fits = (ca == 0 || (uint64_t)base[qa] + cy + exA + ca <= a.capacity) &&
-                                  (cbt == 0 || (uint64_t)base[qb] + cy + exB + cbt <= a.capacity);
-                const auto slotOf = [base, cy](uint32_t en, uint32_t e) { return base[en >> 11] + cy + e; };
-                if (__all_sync(FULL, fits)) copy_out<true>(a, w.ent, T, pcid, lane, slotOf, srcOf);
-                else copy_out<false>(a, w.ent, T, pcid, lane, slotOf, srcOf);
-            }
-            carry += T;
-        }
-        __syncwarp();
-        // query q's slot after this chunk: its base plus the flat prefix at its
-        // last word's end (the next query's start prefix, or the chunk total)
-        if (lane < nq) next = w.base[lane] + ((lane + 1 < nq) ? (w.start[lane + 1] - w.base[lane + 1]) : carry);
-    }
-}
-
-// Column unit: stream positions 32b .. 32b+31 of symmetric task u.t (key =
-// candidate, value = query).  A window is one query group: lane j's word of it.
-__device__ __forceinline__ void emit_cols(const sj_join_args &a, const UnitTask &u, uint32_t b, WarpSmem &w,
-                                          uint32_t lane)
-{
-    const uint32_t nG = (u.qc + 31) / 32;
-    const uint32_t s = b * 32 + lane;
-    const uint64_t rec = a.candOff[u.t] - a.candOff[a.taskBegin];
-    // words of positions past the stream end are zero (the count pass masks them)
-    const uint32_t *const cw = a.colMasks + (a.colOff[u.t] - a.colOff[a.taskBegin]) + (uint64_t)b * nG * 32 + lane;
-    const uint32_t *const qids = a.ids + u.qBegin;
-    uint32_t slot = 0;
-    __syncwarp();        // the previous unit is done with the warp's shared memory
-    if (s < u.L) {
-        slot = a.keyStart[a.candId[rec + s]] + a.candRel[rec + s];
-    }
-    // the words of the next PF query groups are in flight while one is written
-    uint32_t pw[PF];
-#pragma unroll
-    for (int k = 0; k < PF; k++) pw[k] = (uint32_t)k < nG ? __ldg(cw + k * 32) : 0u;
-    for (uint32_t g = 0; g < nG; g++) {
-        uint32_t cur = pw[0];
-#pragma unroll
-        for (int k = 0; k + 1 < PF; k++) pw[k] = pw[k + 1];
-        pw[PF - 1] = g + PF < nG ? __ldg(cw + (uint64_t)(g + PF) * 32) : 0u;
-        {
-            // positions past the stream end and queries past the tile have no
-            // bits in a consistent count pass
-            const uint32_t nq = u.qc - g * 32;
-            const uint32_t valid = s >= u.L ? 0u : (nq >= 32u ? FULL : (1u << nq) - 1u);
-            if (cur & ~valid) {
-                atomicMax(&a.stat[6], 1ULL);
-                cur &= valid;
-            }
-        }
-        const uint32_t cnt = __popc(cur);
-        if (__ballot_sync(FULL, cnt) == 0) continue;   // warp-uniform
+    const uint32_t sh = nl > 1 ? 32 - __clz(nl - 1) : 0u;   // words per line, rounded up to 2^sh
+    const uint32_t j = lane & ((1u << sh) - 1u), lw = lane >> sh, lpw = 32u >> sh;
+    const uint32_t unit = lpw > 2 ? 1u : 4u;
+    const uint32_t tag = lpw > 2 ? (j * 32) | (lw << 10) : j * 128;
+    const uint32_t inWindow = FULL >> (32u - lpw);
+#pragma unroll 1
+    for (uint32_t l0 = 0; l0 < 32; l0 += lpw) {
+        if (!((lines >> l0) & inWindow)) continue;
+        const uint32_t word = j < nl ? w.tile[j][l0 + lw] : 0u;
+        const uint32_t cnt = __popc(word);
+        const uint32_t most = __reduce_max_sync(FULL, cnt);
         const uint32_t incl = warp_incl_scan(cnt, lane);
         const uint32_t T = __shfl_sync(FULL, incl, 31);
         const uint32_t ex = incl - cnt;
-        __syncwarp();
-        w.base[lane] = slot - ex;   // lane L's entries [ex_L, ex_L + cnt_L) go to slot_L onwards
-        decode_bits(cur, cnt, lane << 5, w.ent, ex);
-        __syncwarp();
-        const uint32_t *const base = w.base;
-        const auto slotOf = [base](uint32_t en, uint32_t e) { return base[en >> 5] + e; };
-        const auto srcOf = [](uint32_t en) { return en & 31u; };
-        if (__all_sync(FULL, (uint64_t)slot + cnt <= a.capacity))
-            copy_out<true>(a, w.ent, T, qids + g * 32, lane, slotOf, srcOf);
-        else
-            copy_out<false>(a, w.ent, T, qids + g * 32, lane, slotOf, srcOf);
-        slot += cnt;
+        // every slot of the window's lines fits: a consistent count pass sees to that
+        const uint32_t first = (lane - l0) << sh;   // first word of this lane's line, for lanes of the window
+        const bool mine = lane - l0 < lpw;
+        const uint32_t exF = __shfl_sync(FULL, ex, first & 31u);
+        const uint32_t nLine = __shfl_sync(FULL, incl, (first + (1u << sh) - 1u) & 31u) - exF;
+        if (__any_sync(FULL, mine && (uint64_t)next + nLine > o.cap && nLine)) {
+            atomicMax(&a.stat[3], 1ULL);
+            if (mine) next += nLine;
+            continue;
+        }
+        __syncwarp();   // the previous window's copy-out is done with the list
+        if (most > DENSE) decode_dense(word, tag, unit, w.ent, ex);
+        else decode_sparse(word, cnt, tag, unit, w.ent, ex);
+        if (lpw <= 2) {
+            __syncwarp();
+#pragma unroll 1
+            for (uint32_t i = 0; i < lpw; i++) {
+                const uint32_t l = l0 + i;
+                const uint32_t n = __shfl_sync(FULL, nLine, l);
+                if (!n) continue;
+                copy_line<KEYS>(o, w, lane, __shfl_sync(FULL, exF, l), n, __shfl_sync(FULL, next, l),
+                                __shfl_sync(FULL, key, l),
+                                KeyHash{__shfl_sync(FULL, kh.hi2, l), __shfl_sync(FULL, kh.add, l)});
+            }
+        } else {
+            if (mine) w.line[lane - l0] = LineInfo{next - exF, key, kh.hi2, kh.add};
+            __syncwarp();
+            for (uint32_t e = lane; e < T; e += 32) {
+                const uint32_t en = w.ent[e];
+                const LineInfo l = w.line[en >> 10];
+                const uint32_t v = w.val[en & 0x3ffu];
+                o.val[l.base + e] = (int32_t)v;
+                if (KEYS) o.key[l.base + e] = (int32_t)l.key;
+                o.hash += pair_hash(KeyHash{l.hi2, l.add}, v);
+            }
+        }
+        if (mine) next += nLine;
     }
 }
 
-__global__ void __launch_bounds__(EW, SJ_EMIT_MINB) k_emit(sj_join_args a)
+// Unit k of task t: query group k (rows), or for k >= nG block k - nG of 32
+// positions of a symmetric task (columns).  Both are the same loop over live
+// words: word x of the unit is words[x * stride + lane] for line = lane and its
+// bit i selects value vals[32 x + i] of nv values.  (One code path, so that the
+// kernel stays inside the instruction caches with every warp at another place:
+// with rows and columns inlined apart the warps waited for instructions for 11 of
+// 19 cycles an issue.)
+template <bool KEYS>
+__device__ __forceinline__ void emit_unit(const sj_join_args &a, Out &o, uint32_t t, uint32_t k, WarpSmem &w,
+                                          uint32_t lane)
+{
+    const sj_task *const tp = a.tasks + t;
+    const uint32_t qBegin = tp->qBegin, qc = tp->qCount, L = tp->sEnd - tp->sBegin;
+    const uint32_t nBlk = (L + 31) / 32, nG = (qc + 31) / 32;
+    const uint32_t *const live = a.masks + (a.maskOff[t] - a.maskOff[a.taskBegin]);
+    const uint64_t rec = a.candOff[t] - a.candOff[a.taskBegin];
+    const bool row = k < nG;
+    const uint32_t *words, *vals;
+    uint32_t stride, nv, nLine, nLive;   // nLive: words of live bits
+    uint32_t key = 0, next = 0, colLive = 0;
+    if (row) {
+        nLine = min(32u, qc - 32 * k);
+        words = live + sj_live_words(nBlk, nG) + 32 * k;
+        stride = qc;
+        vals = a.candId + rec;
+        nv = L;
+        nLive = (nBlk + 31) / 32;
+        if (lane < nLine) {
+            key = a.ids[qBegin + 32 * k + lane];
+            next = a.keyStart[key] + a.rowRel[a.rowOff[t] - a.rowOff[a.taskBegin] + 32 * k + lane];
+        }
+    } else {
+        const uint32_t b = k - nG;
+        // the live bits of a block lie in one word per group (at most TW groups)
+        const bool lv = lane < nG && ((__ldg(live + (b >> 5) * nG + lane) >> (b & 31)) & 1u);
+        colLive = __ballot_sync(FULL, lv);
+        if (!colLive) return;
+        nLine = min(32u, L - 32 * b);
+        words = a.colMasks + (a.colOff[t] - a.colOff[a.taskBegin]) + (uint64_t)b * nG * 32;
+        stride = 32;
+        vals = a.ids + qBegin;
+        nv = qc;
+        nLive = 1;
+        if (lane < nLine) {
+            key = a.candId[rec + 32 * b + lane];
+            next = a.keyStart[key] + a.candRel[rec + 32 * b + lane];
+        }
+    }
+    const KeyHash kh = key_hash(key);
+    uint32_t c0 = 0, myLive = 0, chunks = 0, x0 = 0, m = 0, nl = 0, any = 0;
+    bool more = true;
+    do {
+        while (!m) {   // the next live words
+            if (!chunks) {
+                if (c0 >= nLive) {
+                    more = false;
+                    break;
+                }
+                myLive = row ? (c0 + lane < nLive ? __ldg(live + (uint64_t)(c0 + lane) * nG + k) : 0u)
+                             : (lane == 0 ? colLive : 0u);
+                chunks = __ballot_sync(FULL, myLive);
+                c0 += 32;
+                continue;
+            }
+            const uint32_t ci = __ffs(chunks) - 1;
+            chunks &= chunks - 1;
+            m = __shfl_sync(FULL, myLive, ci);
+            x0 = (c0 - 32 + ci) * 32;
+        }
+        // up to LD words (and their values) in flight
+        uint32_t v[LD], c[LD], got = 0;
+#pragma unroll
+        for (uint32_t i = 0; i < LD; i++) {
+            v[i] = c[i] = 0;
+            if (m && nl + i < TW) {   // warp-uniform
+                const uint32_t x = x0 + __ffs(m) - 1;
+                m &= m - 1;
+                got++;
+                const uint32_t rem = 32 * x < nv ? nv - 32 * x : 0u;   // values from the word's first on
+                if (lane < nLine && rem) v[i] = __ldg(words + (uint64_t)x * stride + lane);
+                if (lane < rem) c[i] = __ldg(vals + 32 * x + lane);
+                if (rem < 32u && (v[i] >> rem) != 0u) {   // bits past the stream end or the tile
+                    atomicMax(&a.stat[6], 1ULL);
+                    v[i] &= (1u << rem) - 1u;
+                }
+            }
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < LD; i++) {
+            if (i < got) {
+                w.tile[nl + i][lane] = v[i];
+                w.val[(nl + i) * 32 + lane] = c[i];
+                any |= v[i];
+            }
+        }
+        nl += got;
+        if (nl == TW || (!more && nl)) {
+            __syncwarp();
+            emit_lines<KEYS>(a, o, w, lane, nl, __ballot_sync(FULL, any), key, kh, next);
+            __syncwarp();
+            nl = any = 0;
+        }
+    } while (more);
+}
+
+template <bool KEYS>
+__global__ void __launch_bounds__(EW, EMIT_MINB) k_emit(sj_join_args a)
 {
     __shared__ WarpSmem smem[ENW];
     const uint32_t lane = threadIdx.x & 31u;
@@ -380,46 +383,40 @@ __global__ void __launch_bounds__(EW, SJ_EMIT_MINB) k_emit(sj_join_args a)
     }
     const uint64_t u0 = a.unitOff[a.taskBegin];
     const uint32_t nUnits = (uint32_t)(a.unitOff[a.taskEnd] - u0);
-#if SJ_EMIT_COOP
-    // the CTA's warps take consecutive units (mostly of one task), so the
-    // task's candidate ids and query ids are shared through L1
-    __shared__ uint32_t ctaBase;
-#endif
+    Out o{a.outKey, a.outVal, a.capacity, 0ULL};
+    const uint32_t endGame = 8 * UN * gridDim.x * ENW;   // units left below which warps take them one by one
+    uint32_t take = nUnits > endGame ? UN : 1u;
     for (;;) {
-#if SJ_EMIT_COOP
-        __syncthreads();   // every warp is done with the previous round's units
-        if (threadIdx.x == 0) ctaBase = atomicAdd(a.queueHead, (uint32_t)ENW);
-        __syncthreads();
-        if (ctaBase >= nUnits) break;   // uniform over the CTA
-        const uint32_t un = ctaBase + (threadIdx.x >> 5);
-        if (un >= nUnits) continue;
-#else
         uint32_t un = 0;
-        if (lane == 0) un = atomicAdd(a.queueHead, 1u);
+        if (lane == 0) un = atomicAdd(a.queueHead, take);
         un = __shfl_sync(FULL, un, 0);
         if (un >= nUnits) break;
-#endif
-        // the unit's task: the last t with unitOff[t] - u0 <= un
+        const uint32_t unEnd = nUnits - un < take ? nUnits : un + take;
+        if (nUnits - un < endGame) take = 1;
+        // the first unit's task: the last t with unitOff[t] - u0 <= un
         uint32_t lo = a.taskBegin, hi = a.taskEnd;
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) >> 1;
             if (a.unitOff[mid] - u0 <= un) lo = mid; else hi = mid;
         }
-        if (a.taskHits && a.taskHits[lo] == 0) continue;   // the count pass found no pair in this task
-        const sj_task *const tp = a.tasks + lo;
-        UnitTask u;
-        u.t = lo;
-        u.qBegin = tp->qBegin;
-        u.qc = tp->qCount;
-        u.L = tp->sEnd - tp->sBegin;
-        const bool sym = (tp->flags & SJ_TASK_SYM) != 0;
-        const uint32_t k = un - (uint32_t)(a.unitOff[lo] - u0);
-        const uint32_t nG = (u.qc + 31) / 32;
-        if (k < nG) emit_rows(a, u, k, w, lane);
-        else if (sym) emit_cols(a, u, k - nG, w, lane);
+        uint32_t tBeg = (uint32_t)(a.unitOff[lo] - u0), tEnd = (uint32_t)(a.unitOff[lo + 1] - u0);
+        for (; un < unEnd; un++) {
+            while (un >= tEnd) {   // the next task (every task has a unit)
+                lo++;
+                tBeg = tEnd;
+                tEnd = (uint32_t)(a.unitOff[lo + 1] - u0);
+            }
+            if (a.taskHits && a.taskHits[lo] == 0) continue;   // the count pass found no pair in this task
+            emit_unit<KEYS>(a, o, lo, un - tBeg, w, lane);
+        }
     }
+    unsigned long long h = o.hash;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) h += __shfl_xor_sync(FULL, h, d);
+    if (lane == 0 && h) atomicAdd(&a.stat[4], h);
 }
 
+template <bool KEYS>
 int emit_occupancy()
 {
     constexpr int MAXDEV = 64;
@@ -430,21 +427,27 @@ int emit_occupancy()
     int o = occ[dev].load();
     if (o == 0) {
         int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_emit, EW, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_emit<KEYS>, EW, 0);
         o = b > 0 ? b : 1;
         occ[dev].store(o);
     }
     return o;
 }
 
-}  // namespace
-
-cudaError_t sj_launch_emit(const sj_join_args &a, int numSM, int maxCtasPerSM, cudaStream_t s)
+template <bool KEYS>
+cudaError_t launch(const sj_join_args &a, int numSM, int maxCtasPerSM, cudaStream_t s)
 {
-    if (a.taskEnd == a.taskBegin) return cudaSuccess;
-    int perSM = emit_occupancy();
+    int perSM = emit_occupancy<KEYS>();
     if (maxCtasPerSM > 0 && maxCtasPerSM < perSM) perSM = maxCtasPerSM;
-    k_emit<<<(unsigned)(numSM * perSM), EW, 0, s>>>(a);
+    k_emit<KEYS><<<(unsigned)(numSM * perSM), EW, 0, s>>>(a);
     sj_note_launch();
     return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t sj_launch_emit(const sj_join_args &a, int keys, int numSM, int maxCtasPerSM, cudaStream_t s)
+{
+    if (a.taskEnd == a.taskBegin) return cudaSuccess;
+    return keys ? launch<true>(a, numSM, maxCtasPerSM, s) : launch<false>(a, numSM, maxCtasPerSM, s);
 }

@@ -9,6 +9,8 @@
 #define SJ_MAX_DIM 16        // data dimensions handled by the kernels (padded to a template width)
 #define SJ_MAX_K 16          // indexed dimensions
 #define SJ_CTA 128           // threads per join CTA (one query point per thread)
+#define SJ_SMALL_QUERIES 32  // tasks of at most this many query points go to the warp-per-task count pass
+#define SJ_SMALL_EVALS 65536u  // evaluations of such a task, about
 #define SJ_STAGE 256         // candidates staged in shared memory per step
 #define SJ_MAX_SEG 1024      // candidate segments (home + neighbour cells) per task
 #define SJ_NFEAT 16          // learned-estimator input features per cell
@@ -59,26 +61,32 @@ struct sj_task {
     uint32_t segCount;
     uint32_t sBegin;
     uint32_t sEnd;
-    uint32_t flags;   // bit0: symmetric emission, bit1: home segment included
+    uint32_t flags;   // bit0: symmetric emission, bit1: home segment included, bit2: sampled queries
 };
 
 #define SJ_TASK_SYM 1u
 #define SJ_TASK_HOME 2u
+#define SJ_TASK_SAMPLE 4u   // sampling estimate: the queries are the cell's points in the index's order
 
 // Device-side state of one join (all pointers device memory).
 struct sj_join_args {
     const double *xs;           // n x Dp cell-sorted coordinates (FP64)
-    const uint32_t *ids;        // n point ids in cell-sorted order (indexLookupArr)
+    const uint32_t *ids;        // n point ids in the join's order (by cell, in spatial order inside a cell)
+    const double *pts;          // the points as supplied (n x D) and their ids in the index's order (by cell, then
+    const uint32_t *indexIds;   // by id): the sampling estimate's queries
     const uint32_t *cellStart;  // nCells+1
     const uint32_t *nbrStart;   // nCells+1 (owned neighbour list, excludes home)
     const uint32_t *nbrCell;
     const uint32_t *cellCoord;  // nCells x k
     const sj_task *tasks;
     uint32_t taskBegin, taskEnd;
-    uint32_t *queueHead;        // persistent-queue cursor (work-queue modes)
+    // the tasks by kernel: number of small tasks (at most SJ_SMALL_QUERIES query points) before each task, and
+    // the lists of the others and of the small ones, in task order
+    const uint32_t *smallPre, *bigList, *smallList;
+    uint32_t *queueHead;        // persistent-queue cursors: [0] k_join / emission, [1] small tasks
     uint32_t *keyCount;         // count pass: per point-id pair counts
     const uint32_t *keyStart;   // emission: first slot of each point id's key run (exclusive scan)
-    int32_t *outKey, *outVal;   // batch output: keys by sj_expand_keys, values by the emission
+    int32_t *outKey, *outVal;   // batch output, written by the emission (outKey may be null without keys)
     uint64_t capacity;          // pairs the output buffers hold
     unsigned long long *stat;   // [2] pairs (count pass), [3] run past capacity, [4] set hash,
                                 // [5] batches skipped for overflow, [6] emission record out of range,
@@ -87,8 +95,8 @@ struct sj_join_args {
     uint32_t *taskHits;         // optional per-task measured pairs (count pass)
     // count-pass records consumed by the emission pass (null: not recorded).
     // Offsets are absolute over all tasks; a batch indexes from its first task's.
-    uint32_t *masks;            // per task: row hit masks, bit i = candidate 32*block+i, laid out
-                                // [chunk of 64 blocks][query][block in chunk] (sj_row_mask_index)
+    uint32_t *masks;            // per task: live bits and row hit masks, bit i = candidate 32*block+i
+                                // (layout: see sj_live_words)
     const uint64_t *maskOff;    // per task: first row-mask word
     uint32_t *colMasks;         // per symmetric task: column hit masks [block][query group][candidate],
                                 // bit i = query 32*group+i (the query itself dropped on the home diagonal)
@@ -104,18 +112,17 @@ struct sj_join_args {
     uint32_t *taskEvals;        // per task: candidate evaluations
     uint32_t *taskRefined;      // per task: FP32 borderline re-evaluations
     double margin;              // FP32 filter: bound M on |FP32 estimate - (FP64 d2 - T)|
+    float pruneT;               // squared distance of two boxes of local coordinates above which no pair of
+                                // their points satisfies the predicate
     float delta;                // FP32 filter: width of the borderline band (>= 2M plus threshold rounding)
 };
 
-// Row-mask word of query qi and block b of a task with qc queries and nBlk
-// blocks: chunks of 64 blocks, each [query][block in chunk], so one query's
-// words of a chunk are contiguous.
-__host__ __device__ inline uint64_t sj_row_mask_index(uint32_t b, uint32_t qi, uint32_t qc, uint32_t nBlk)
-{
-    const uint32_t c = b >> 6;
-    const uint32_t cb = (nBlk - 64 * c) < 64 ? (nBlk - 64 * c) : 64;
-    return (uint64_t)64 * c * qc + (uint64_t)qi * cb + (b & 63);
-}
+// Row-mask record of a task with qc queries in nG groups of 32 and nBlk blocks
+// of 32 stream positions: first the live bits, word [block / 32][group], bit
+// block % 32 set when any query of the group hits any position of the block;
+// then the hit words [block][query].  Only the hit words (row and column) of
+// live (block, group) tiles are written and read.
+__host__ __device__ inline uint32_t sj_live_words(uint32_t nBlk, uint32_t nG) { return ((nBlk + 31) / 32) * nG; }
 
 // Parameters of the device task builder (sj_tasks.cu).
 struct sj_taskgen {
@@ -132,7 +139,7 @@ struct sj_taskgen {
     double pairsPerTask;         // chunking target of policy 0
     double evalsPerTask;         // policy 0: evaluations per task at most (0: no limit)
     int sym;                     // symmetric traversal (owned neighbours, both directions emitted)
-    int policy;                  // 0 cost-proportional chunks, 1 fixed 65536, 2 mode-8 split by thirds of the work
+    int policy;                  // 0 cost-proportional chunks, 1 short fixed chunks, 2 mode-8 split by thirds of the work
     float sampleRate;            // > 0: tasks for the sampled queries of each cell only (sampling estimator)
     // spread != 0: a task's neighbour pairs follow the offset-class model
     // (sj_nbr_spread) instead of the cell's mean rate
@@ -163,27 +170,8 @@ cudaError_t sj_radix_sort_u64_u32(uint64_t *keys, uint32_t *vals, uint64_t *keys
                                   uint64_t n, int bits, void *temp, int *resultInAlt, cudaStream_t s);
 cudaError_t sj_radix_sort_u32_u32(uint32_t *keys, uint32_t *vals, uint32_t *keysAlt, uint32_t *valsAlt,
                                   uint64_t n, int bits, void *temp, int *resultInAlt, cudaStream_t s);
-cudaError_t sj_hash_pairs(const int32_t *key, const int32_t *val, uint64_t m,
-                          unsigned long long *hashOut, cudaStream_t s);
-
-// keys of a batch from its row structure: key k owns [excl[k], excl[k+1])
-// (excl[n] = *total); skipped when the batch's count exceeds cap.  longRuns
-// (16-byte records, sj_expand_long_slots(cap) of them) and longCount are
-// scratch for the runs too long for one warp.
-cudaError_t sj_expand_keys(const uint32_t *excl, const uint32_t *total, uint64_t n, int32_t *outKey,
-                           const unsigned long long *batchPairs, uint64_t cap, void *longRuns, uint32_t longCap,
-                           uint32_t *longCount, int numSM, cudaStream_t s);
-size_t sj_expand_long_slots(uint64_t cap);
-// consumer fold of a device-resident batch with the key array written in the
-// same pass: reads the values, writes the keys from the key runs (as
-// sj_expand_keys), adds the pairs' set hash to *hashOut; skipped when the
-// batch's count exceeds cap.  chunkKey: sj_fold_chunks(cap) entries of scratch.
-size_t sj_fold_chunks(uint64_t cap);
 // out[i] = (float)in[i]
 cudaError_t sj_u32_to_f32(const uint32_t *in, uint64_t n, float *out, cudaStream_t s);
-cudaError_t sj_fold(const uint32_t *excl, const uint32_t *total, uint64_t n, const int32_t *val, int32_t *outKey,
-                    const unsigned long long *batchPairs, uint64_t cap, uint32_t *chunkKey,
-                    unsigned long long *hashOut, int numSM, cudaStream_t s);
 // appends a batch (values vals, key runs start[0..n], start[n] = *total) to a
 // device CSR table rowPtr[n+1] / cols[colsCap]; fill[n] are the rows' cursors
 cudaError_t sj_csr_append(const uint32_t *start, const uint32_t *total, uint64_t n, const int32_t *vals,
@@ -202,6 +190,20 @@ cudaError_t sj_launch_gather(const double *pts, const uint32_t *ids, uint64_t n,
 cudaError_t sj_launch_cell_coords(const uint64_t *cellLid, uint32_t nCells, sj_grid_dev g, uint32_t *coord,
                                   cudaStream_t s);
 
+// Order of the points inside their cells for the join: which coordinate each
+// bit of a point's place halves, most significant first.
+struct sj_place_plan {
+    int bits;                        // of the place (0: the cells keep the id order)
+    uint8_t dim[32], shift[32];      // per bit: the dimension and the bit of its binary coordinate
+    uint8_t nb[SJ_MAX_DIM];          // bits of each dimension's binary coordinate
+    double lo[SJ_MAX_DIM], inv[SJ_MAX_DIM];   // non-indexed dimensions: data minimum and 1 / range
+};
+cudaError_t sj_launch_place_keys(const double *pts, const uint32_t *ids, const uint64_t *keys,
+                                 const uint32_t *cellExcl, uint64_t n, const sj_grid_dev &g, const sj_place_plan &pl,
+                                 uint32_t *out, uint32_t *vals, cudaStream_t s);
+cudaError_t sj_launch_place_spread(const uint32_t *placed, const uint32_t *ids, const uint32_t *cellStart, uint64_t n,
+                                   int bits, uint32_t *out, cudaStream_t s);
+
 // neighbour lists and features (sj_stencil.cu)
 // pass 0: owned-neighbour counts, full-stencil candidates per cell (and their
 // total, added to *candTotal) and features; pass 1: the owned lists
@@ -211,12 +213,14 @@ cudaError_t sj_launch_neighbours(const uint64_t *cellLid, const uint32_t *cellCo
                                  float *feat, int pass, cudaStream_t s);
 
 // join (sj_join.cu): the count pass (per-key pair counts, hit masks)
+// nBig / nSmall: at least the tasks of each kind in the range (0: none)
 // (persistent queue: numSM x resident CTAs per SM, at most maxCtasPerSM when > 0)
-cudaError_t sj_launch_join(const sj_join_args &a, const sj_grid_dev &g, int fp32, int queue, int numSM,
-                           int maxCtasPerSM, cudaStream_t s);
+cudaError_t sj_launch_join(const sj_join_args &a, const sj_grid_dev &g, int fp32, int queue, uint32_t nBig,
+                           uint32_t nSmall, int numSM, int maxCtasPerSM, cudaStream_t s);
 // emission (sj_emit.cu): the values of the pairs from the recorded hit masks
 // into their key runs; a.queueHead must be zero at launch
-cudaError_t sj_launch_emit(const sj_join_args &a, int numSM, int maxCtasPerSM, cudaStream_t s);
+// (keys: also write a.outKey); the pairs' set hash is added to a.stat[4]
+cudaError_t sj_launch_emit(const sj_join_args &a, int keys, int numSM, int maxCtasPerSM, cudaStream_t s);
 
 // emission units of a task: one per group of 32 queries, plus one per block of
 // 32 stream positions for a symmetric task
@@ -249,6 +253,10 @@ cudaError_t sj_tg_item_write(const sj_taskgen &g, const uint32_t *order, const u
                              sj_task *tasks, float *pred, cudaStream_t s);
 cudaError_t sj_tg_shard(const sj_task *in, const float *predIn, uint32_t nOut, uint32_t idx, uint32_t cnt,
                         sj_task *out, float *predOut, cudaStream_t s);
+// the tasks by count-pass kernel: pre[0..nt] (exclusive prefix of the small ones), lists of the others and
+// of the small ones; temp: sj_scan_temp_bytes(nt + 1)
+cudaError_t sj_task_lists(const sj_task *tasks, uint32_t nt, uint32_t *pre, uint32_t *bigList, uint32_t *smallList,
+                          void *temp, cudaStream_t s);
 // record offsets of a task list: out[0..6] = row-mask words, column-mask words,
 // row offsets, candidate records, emission units, planned pairs
 // (ceil(pred * (1 + alpha))), predicted pairs (rounded); each nt+1 entries
@@ -260,9 +268,9 @@ cudaError_t sj_task_offsets(const sj_task *tasks, const float *pred, uint32_t nt
 cudaError_t sj_plan_batches(unsigned long long *const off[7], uint32_t nt, unsigned long long cap,
                             unsigned long long maskLim, uint32_t *next, uint32_t *start, uint32_t *nBatches,
                             cudaStream_t s);
-// per batch: predicted pairs, row-mask words, column-mask words, row offsets, candidate records
+// per batch: predicted pairs, row-mask words, column-mask words, row offsets, candidate records, small tasks
 cudaError_t sj_plan_stats(const uint32_t *start, uint32_t nb, unsigned long long *const off[7],
-                          unsigned long long *stats, cudaStream_t s);
+                          const uint32_t *smallPre, unsigned long long *stats, cudaStream_t s);
 // learned estimator: rates (2 per cell: home, owned neighbours) from the
 // network's outputs (log2(1 + home hits), log2(1 + owned-neighbour hits))
 cudaError_t sj_rates_mlp(const float *out, const uint32_t *cellStart, const uint32_t *nbrStart,

@@ -1,7 +1,7 @@
 // The distance join's count pass over cell tasks.
 //
-// One CTA of 128 threads takes a task: up to 128*R query points of one cell
-// (R query "slots" of 128; thread t holds queries t, t+128, ... in registers)
+// One CTA of 128 threads takes a task: up to 128*R query points of one cell in
+// groups of 32 (warp w holds groups w, w + 4, .., lane = query, in registers)
 // against a stretch of that cell's candidate stream (home cell + owned
 // neighbour cells, kernel.cu:1403-1538 in the reference).  Candidates are
 // staged in shared memory in steps of SJ_STAGE and read as broadcasts; each
@@ -29,7 +29,9 @@
 #include "sj_internal.h"
 #include "sj_device.cuh"
 
+#include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #ifndef SJ_EVAL_UNROLL
 #define SJ_EVAL_UNROLL 2    // unrolling of the per-block candidate loop
@@ -62,10 +64,32 @@ __device__ __forceinline__ double ref_dist2(const double *c, const double *q)
     return acc;
 }
 
+// Coordinates and point id of a task's query qi.  The sampling estimate's
+// queries are the first of their cell in the index's order: its points in id
+// order, so the sample covers the cell whatever the join's order of its points.
 template <int DP>
-__device__ __forceinline__ bool exact_hit(const double *__restrict__ xs, uint32_t cpos, uint32_t qpos, double T)
+__device__ __forceinline__ uint32_t load_query(const sj_join_args &a, const sj_task &t, uint32_t qi, int D,
+                                               double (&x)[DP])
 {
-    return ref_dist2<DP>(xs + (uint64_t)cpos * DP, xs + (uint64_t)qpos * DP) <= T;
+    if (t.flags & SJ_TASK_SAMPLE) {
+        const uint32_t id = a.indexIds[t.qBegin + qi];
+#pragma unroll
+        for (int l = 0; l < DP; l++) x[l] = l < D ? a.pts[(uint64_t)id * D + l] : 0.0;
+        return id;
+    }
+    const uint64_t pos = t.qBegin + qi;
+#pragma unroll
+    for (int l = 0; l < DP; l++) x[l] = a.xs[pos * DP + l];
+    return a.ids[pos];
+}
+
+template <int DP>
+__device__ __forceinline__ bool exact_hit(const sj_join_args &a, uint32_t cpos, const sj_task &t, uint32_t qi, int D,
+                                          double T)
+{
+    double q[DP];
+    load_query<DP>(a, t, qi, D, q);
+    return ref_dist2<DP>(a.xs + (uint64_t)cpos * DP, q) <= T;
 }
 
 template <int DP>
@@ -98,7 +122,7 @@ __device__ __forceinline__ uint32_t push_sign(uint32_t mask, float v)
     return r;
 }
 
-// FP32 filter over one block of 32 staged candidates for slots 0..RR-1.
+// FP32 filter over one block of 32 staged candidates for slots R0..R0+RR-1.
 //   y = (|b|^2 - tLo) + sum_l (-2 a_l) b_l      (packed f32x2: two candidates per op)
 // hit bit <- sign(y): y < 0 proves the FP64 predicate true; y >= delta proves
 // it false; 0 <= y < delta is the borderline band.  Bits are shifted in from
@@ -108,7 +132,7 @@ __device__ __forceinline__ uint32_t push_sign(uint32_t mask, float v)
 // floats order like their bits; negative ones have the sign bit and never win
 // the unsigned minimum), so ymin < bits(delta) tells that the block has a
 // borderline candidate, which near_bits() then finds.
-template <int DP, int RR, int R>
+template <int DP, int R0, int RR, int R>
 __device__ __forceinline__ void eval_block_f32(const Stage32<DP> &st, uint32_t pb, const float2 (&qa)[R][DP],
                                                const float2 (&nt)[R], uint32_t (&hit)[R], uint32_t (&ymin)[R])
 {
@@ -121,11 +145,11 @@ __device__ __forceinline__ void eval_block_f32(const Stage32<DP> &st, uint32_t p
             const float4 v = row[0];
             const float2 nb = make_float2(v.x, v.y);
 #pragma unroll
-            for (int r = 0; r < RR; r++) y[r] = __fadd2_rn(nb, nt[r]);
+            for (int r = 0; r < RR; r++) y[r] = __fadd2_rn(nb, nt[R0 + r]);
             if (DP >= 1) {
                 const float2 b = make_float2(v.z, v.w);
 #pragma unroll
-                for (int r = 0; r < RR; r++) y[r] = __ffma2_rn(qa[r][0], b, y[r]);
+                for (int r = 0; r < RR; r++) y[r] = __ffma2_rn(qa[R0 + r][0], b, y[r]);
             }
         }
 #pragma unroll
@@ -134,19 +158,19 @@ __device__ __forceinline__ void eval_block_f32(const Stage32<DP> &st, uint32_t p
             if (2 * h - 1 < DP) {
                 const float2 b = make_float2(v.x, v.y);
 #pragma unroll
-                for (int r = 0; r < RR; r++) y[r] = __ffma2_rn(qa[r][2 * h - 1], b, y[r]);
+                for (int r = 0; r < RR; r++) y[r] = __ffma2_rn(qa[R0 + r][2 * h - 1], b, y[r]);
             }
             if (2 * h < DP) {
                 const float2 b = make_float2(v.z, v.w);
 #pragma unroll
-                for (int r = 0; r < RR; r++) y[r] = __ffma2_rn(qa[r][2 * h], b, y[r]);
+                for (int r = 0; r < RR; r++) y[r] = __ffma2_rn(qa[R0 + r][2 * h], b, y[r]);
             }
         }
 #pragma unroll
         for (int r = 0; r < RR; r++) {
-            hit[r] = push_sign(hit[r], y[r].y);
-            hit[r] = push_sign(hit[r], y[r].x);
-            ymin[r] = min(ymin[r], min(__float_as_uint(y[r].x), __float_as_uint(y[r].y)));
+            hit[R0 + r] = push_sign(hit[R0 + r], y[r].y);
+            hit[R0 + r] = push_sign(hit[R0 + r], y[r].x);
+            ymin[R0 + r] = min(ymin[R0 + r], min(__float_as_uint(y[r].x), __float_as_uint(y[r].y)));
         }
     }
 }
@@ -174,10 +198,10 @@ __device__ __forceinline__ uint32_t near_bits(const Stage32<DP> &st, uint32_t pb
     return m;
 }
 
-// FP64 predicate over one block of 32 staged candidates for slots 0..RR-1, in
+// FP64 predicate over one block of 32 staged candidates for slots R0..R0+RR-1, in
 // the reference's rounding order (ref_dist2).  acc >= 0, so acc <= T is the
 // sign of bits(acc) - (bits(T) + 1) as 64-bit integers.
-template <int DP, int RR, int R>
+template <int DP, int R0, int RR, int R>
 __device__ __forceinline__ void eval_block_f64(const Stage64<DP> &st, uint32_t jb, const double (&q)[R][DP],
                                                long long T1, uint32_t (&hit)[R])
 {
@@ -190,15 +214,15 @@ __device__ __forceinline__ void eval_block_f64(const Stage64<DP> &st, uint32_t j
             if (DP == 1) {
 #pragma unroll
                 for (int r = 0; r < RR; r++) {
-                    const double d0 = __dsub_rn(c0, q[r][0]);
+                    const double d0 = __dsub_rn(c0, q[R0 + r][0]);
                     acc[r] = __dmul_rn(d0, d0);
                 }
             } else {
                 const double c1 = cb[DP > 1 ? 1 : 0];
 #pragma unroll
                 for (int r = 0; r < RR; r++) {
-                    const double d0 = __dsub_rn(c0, q[r][0]);
-                    const double d1 = __dsub_rn(c1, q[r][DP > 1 ? 1 : 0]);
+                    const double d0 = __dsub_rn(c0, q[R0 + r][0]);
+                    const double d1 = __dsub_rn(c1, q[R0 + r][DP > 1 ? 1 : 0]);
                     acc[r] = __fma_rn(d0, d0, __dmul_rn(d1, d1));
                 }
             }
@@ -208,16 +232,61 @@ __device__ __forceinline__ void eval_block_f64(const Stage64<DP> &st, uint32_t j
             const double cl = cb[l];
 #pragma unroll
             for (int r = 0; r < RR; r++) {
-                const double d = __dsub_rn(cl, q[r][l]);
+                const double d = __dsub_rn(cl, q[R0 + r][l]);
                 acc[r] = __fma_rn(d, d, acc[r]);
             }
         }
 #pragma unroll
         for (int r = 0; r < RR; r++) {
             const long long diff = __double_as_longlong(acc[r]) - T1;
-            hit[r] = push_sign(hit[r], __int_as_float((int)((unsigned long long)diff >> 32)));
+            hit[R0 + r] = push_sign(hit[R0 + r], __int_as_float((int)((unsigned long long)diff >> 32)));
         }
     }
+}
+
+// Minimum and maximum of v over the warp.
+__device__ __forceinline__ float2 warp_min_max(float lo, float hi)
+{
+    float2 r;
+    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r.x) : "f"(lo));
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r.y) : "f"(hi));
+    return r;
+}
+
+// Evaluates block jb of the stage for the slots of act (a subset of the warp's
+// nAct slots; other slots' results are undefined).  All slots, or three of four,
+// go through the code that loads each candidate once for all of them.
+template <int DP, bool F32, int R, class Eval>
+__device__ __forceinline__ void eval_slots(uint32_t act, uint32_t nAct, Eval eval)
+{
+    if (R == 1 || nAct == 1) {
+        eval(std::integral_constant<int, 0>{}, std::integral_constant<int, 1>{});
+        return;
+    }
+    if constexpr (R == 2) {
+        if (act == 3u) eval(std::integral_constant<int, 0>{}, std::integral_constant<int, 2>{});
+        else if (act == 1u) eval(std::integral_constant<int, 0>{}, std::integral_constant<int, 1>{});
+        else eval(std::integral_constant<int, 1>{}, std::integral_constant<int, 1>{});
+    }
+    if constexpr (R == 4) {
+        if (__popc(act) >= 3) {
+            eval(std::integral_constant<int, 0>{}, std::integral_constant<int, 4>{});
+            return;
+        }
+        if (act == 3u) {
+            eval(std::integral_constant<int, 0>{}, std::integral_constant<int, 2>{});
+            return;
+        }
+        if (act == 12u) {
+            eval(std::integral_constant<int, 2>{}, std::integral_constant<int, 2>{});
+            return;
+        }
+        if (act & 1u) eval(std::integral_constant<int, 0>{}, std::integral_constant<int, 1>{});
+        if (act & 2u) eval(std::integral_constant<int, 1>{}, std::integral_constant<int, 1>{});
+        if (act & 4u) eval(std::integral_constant<int, 2>{}, std::integral_constant<int, 1>{});
+        if (act & 8u) eval(std::integral_constant<int, 3>{}, std::integral_constant<int, 1>{});
+    }
+    static_assert(R == 1 || R == 2 || R == 4, "slot sets of eval_slots");
 }
 
 // Shared memory of one count-pass CTA.
@@ -230,7 +299,9 @@ struct __align__(16) JoinSmem {
     uint32_t segStart[SJ_MAX_SEG];
     uint32_t segPre[SJ_MAX_SEG + 1];
     uint32_t colCnt[NW][S];
-    double originS[F32 ? DP : 1];
+    float2 boxC[S / 32][DP];            // per staged block: (min, max) of each local coordinate
+    float2 boxQ[NW * R][DP];            // per group of 32 queries
+    double originS[DP];
     uint32_t scanTmp[NW];
     uint32_t curTask;
     unsigned long long taskPairs;
@@ -243,17 +314,14 @@ struct __align__(16) JoinSmem {
 // set -- every query's hit mask per block of 32 stream positions plus its row
 // count, which the emission pass turns into pairs without a second distance
 // evaluation.
-// Resident CTAs per SM the register allocation must allow: the FP32 filter
-// gains from a fifth CTA, the FP64 predicate from keeping its registers.
-#ifndef SJ_JOIN_MIN_BLOCKS_F32
-#define SJ_JOIN_MIN_BLOCKS_F32 5
-#endif
-#ifndef SJ_JOIN_MIN_BLOCKS_F64
-#define SJ_JOIN_MIN_BLOCKS_F64 1
-#endif
+// Resident CTAs per SM the register allocation must allow.  FP32 filter: four,
+// five at six dimensions (4-D: 41.2 ms of count passes with four, 45.7 with
+// five; 8-D 7.2 against 7.6; 6-D 82 against 79).  FP64: three up to six
+// dimensions (29.6 ms against 36.4 with two on 6-D data), two above.
+constexpr int sj_join_min_blocks(int DP, bool F32) { return F32 ? (DP == 6 ? 5 : 4) : (DP <= 6 ? 3 : 2); }
 
 template <int DP, bool F32, int R>
-__global__ void __launch_bounds__(SJ_CTA, F32 ? SJ_JOIN_MIN_BLOCKS_F32 : SJ_JOIN_MIN_BLOCKS_F64) k_join(sj_join_args a, sj_grid_dev g, int queue)
+__global__ void __launch_bounds__(SJ_CTA, sj_join_min_blocks(DP, F32)) k_join(sj_join_args a, sj_grid_dev g, int queue)
 {
     using Smem = JoinSmem<DP, F32, R>;
     constexpr int S = Smem::S;
@@ -273,20 +341,23 @@ __global__ void __launch_bounds__(SJ_CTA, F32 ? SJ_JOIN_MIN_BLOCKS_F32 : SJ_JOIN
 
     for (int j = tid; j < NW * S; j += SJ_CTA) (&colCnt[0][0])[j] = 0;
 
+    // this kernel's tasks of the range: entries [first, first + count) of bigList
+    const uint32_t first = a.taskBegin - a.smallPre[a.taskBegin];
+    const uint32_t count = (a.taskEnd - a.smallPre[a.taskEnd]) - first;
     uint32_t iter = 0;
     for (;;) {
         // ---- fetch the next task
         __syncthreads();
         if (tid == 0) {
-            uint32_t t = queue ? (a.taskBegin + atomicAdd(a.queueHead, 1u)) : (a.taskBegin + blockIdx.x + iter);
-            sm.curTask = t;
+            const uint32_t i = queue ? atomicAdd(a.queueHead, 1u) : blockIdx.x + iter;
+            sm.curTask = i < count ? a.bigList[first + i] : 0xffffffffu;
             sm.taskPairs = 0ULL;
             sm.taskEvals = 0ULL;
             sm.taskRefined = 0ULL;
         }
         __syncthreads();
         const uint32_t t = sm.curTask;
-        if (t >= a.taskEnd || (!queue && iter > 0)) break;
+        if (t == 0xffffffffu || (!queue && iter > 0)) break;
         iter++;
         const sj_task task = a.tasks[t];
         const bool sym = (task.flags & SJ_TASK_SYM) != 0;
@@ -319,13 +390,13 @@ __global__ void __launch_bounds__(SJ_CTA, F32 ? SJ_JOIN_MIN_BLOCKS_F32 : SJ_JOIN
             locLen[r] = len;
             mySum += len;
         }
-        if (F32 && (int)tid < DP) {
+        if ((int)tid < DP) {
             // local-coordinate origin: home cell centre (indexed dims), data centre (others)
             double o;
             if ((int)tid < g.k) o = g.minArr[tid] + ((double)a.cellCoord[(uint64_t)cellA * g.k + tid] + 0.5) * g.eps;
             else if ((int)tid < D) o = g.center[tid];
             else o = 0.0;
-            originS[F32 ? tid : 0] = o;
+            originS[tid] = o;
         }
         {
             // block exclusive scan of mySum
@@ -351,88 +422,126 @@ __global__ void __launch_bounds__(SJ_CTA, F32 ? SJ_JOIN_MIN_BLOCKS_F32 : SJ_JOIN
         __syncthreads();
         const uint32_t homeEnd = (task.segBase == 0 && (task.flags & SJ_TASK_HOME)) ? segPre[1] : 0u;
 
-        // ---- query points of this thread: slot r holds query r*128 + tid
-        // nAct: slots with at least one valid query in this warp (warp-uniform)
-        const uint32_t nAct = task.qCount > warp * 32
-                                  ? min((uint32_t)R, (task.qCount - warp * 32 + SJ_CTA - 1) / SJ_CTA)
-                                  : 0u;
+        // ---- query points of this warp: slot r holds group r * NW + warp, lane =
+        // query; nAct: the warp's groups (warp-uniform).  Neighbouring groups lie
+        // close together and go to different warps, so that the warps have about
+        // as many tiles left of a stage as each other.
+        const uint32_t nG = (task.qCount + 31) / 32;
+        const uint32_t nAct = nG > warp ? (nG - warp + NW - 1) / NW : 0u;
         uint32_t qid[R];
         double q64[F32 ? 1 : R][F32 ? 1 : DP];
         float2 qa[F32 ? R : 1][F32 ? DP : 1];   // (-2 a_l, -2 a_l)
         float2 nt[R];                           // (-tLo, -tLo)
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            const uint32_t qi = (uint32_t)r * SJ_CTA + tid;
-            const bool v = qi < task.qCount;
-            const uint32_t qpos = task.qBegin + (v ? qi : 0u);
-            qid[r] = a.ids[qpos];
-            const double *src = a.xs + (uint64_t)qpos * DP;
-            if (F32) {
-                double na = 0.0;
+            const uint32_t qi = ((uint32_t)r * NW + warp) * 32 + lane;
+            const bool v = (uint32_t)r < nAct && qi < task.qCount;
+            double src[DP];
+            qid[r] = load_query<DP>(a, task, v ? qi : 0u, D, src);
+            double na = 0.0;
 #pragma unroll
-                for (int l = 0; l < DP; l++) {
-                    const float ql = (l < D) ? __double2float_rn(src[l] - originS[F32 ? l : 0]) : 0.0f;
+            for (int l = 0; l < DP; l++) {
+                const double x = src[l];
+                const float ql = (l < D) ? __double2float_rn(x - originS[l]) : 0.0f;
+                if (F32) {
                     qa[F32 ? r : 0][F32 ? l : 0] = make_float2(-2.0f * ql, -2.0f * ql);
                     na += (double)ql * (double)ql;
+                } else {
+                    q64[F32 ? 0 : r][F32 ? 0 : l] = x;
                 }
+                if ((uint32_t)r < nAct) {
+                    const float2 mm = warp_min_max(v ? ql : INFINITY, v ? ql : -INFINITY);
+                    if (lane == 0) sm.boxQ[r * NW + warp][l] = mm;
+                }
+            }
+            if (F32) {
                 const float tLo = __double2float_rd(T - na - a.margin);
                 nt[r] = make_float2(-tLo, -tLo);
             } else {
-#pragma unroll
-                for (int l = 0; l < DP; l++) q64[F32 ? 0 : r][F32 ? 0 : l] = src[l];
                 nt[r] = make_float2(0.f, 0.f);
             }
         }
         const long long T1 = __double_as_longlong(T) + 1;
-        uint32_t *const maskBase = a.masks ? a.masks + (a.maskOff[t] - a.maskOff[a.taskBegin]) : nullptr;
+        uint32_t *const liveBase = a.masks ? a.masks + (a.maskOff[t] - a.maskOff[a.taskBegin]) : nullptr;
         uint32_t *const colBase = (a.colMasks && sym) ? a.colMasks + (a.colOff[t] - a.colOff[a.taskBegin]) : nullptr;
         const uint64_t candRecOff = a.candOff ? a.candOff[t] - a.candOff[a.taskBegin] : 0;
         uint32_t *const candIdRec = a.candId ? a.candId + candRecOff : nullptr;
         uint32_t *const candRelRec = (a.candRel && sym) ? a.candRel + candRecOff : nullptr;
 
         uint32_t rowCount[R];   // pairs keyed by each query
+        uint32_t live[R];       // blocks of the current 32 in which the group has a hit
         uint32_t evals = 0;     // candidate evaluations
         uint32_t refined = 0;   // FP32 borderline re-evaluations
 #pragma unroll
-        for (int r = 0; r < R; r++) rowCount[r] = 0;
+        for (int r = 0; r < R; r++) rowCount[r] = live[r] = 0;
 
         // the stream can never extend past the segments actually present
         const uint32_t sEnd = min(task.sEnd, segPre[nSeg]);
         const uint32_t nBlk = (sEnd - task.sBegin + 31) / 32;
-        const uint32_t nG = (task.qCount + 31) / 32;
+        uint32_t *const rowBase = liveBase ? liveBase + sj_live_words(nBlk, nG) : nullptr;
         for (uint32_t sBase = task.sBegin; sBase < sEnd; sBase += S) {
             const uint32_t nIn = min((uint32_t)S, sEnd - sBase);
             __syncthreads();
             // ---- stage candidates
-            for (uint32_t j = tid; j < nIn; j += SJ_CTA) {
-                uint32_t s = sBase + j;
-                uint32_t lo = 0, hi = nSeg;   // largest seg with segPre[seg] <= s
-                while (hi - lo > 1) {
-                    uint32_t mid = (lo + hi) >> 1;
-                    if (segPre[mid] <= s) lo = mid; else hi = mid;
-                }
-                uint32_t pos = segStart[lo] + (s - segPre[lo]);
-                const uint32_t cid = a.ids[pos];
-                candId[j] = cid;
-                if (candIdRec) candIdRec[s - task.sBegin] = cid;   // the emission's candidate record
-                const double *src = a.xs + (uint64_t)pos * DP;
-                if constexpr (F32) {
-                    float *dst = reinterpret_cast<float *>(&st.c[j >> 1][0]) + (j & 1);
+            for (uint32_t j0 = warp * 32; j0 < nIn; j0 += SJ_CTA) {   // a warp stages whole blocks
+                const uint32_t j = j0 + lane;
+                const bool in = j < nIn;
+                float bl[DP];
+                if (in) {
+                    uint32_t s = sBase + j;
+                    uint32_t lo = 0, hi = nSeg;   // largest seg with segPre[seg] <= s
+                    while (hi - lo > 1) {
+                        uint32_t mid = (lo + hi) >> 1;
+                        if (segPre[mid] <= s) lo = mid; else hi = mid;
+                    }
+                    uint32_t pos = segStart[lo] + (s - segPre[lo]);
+                    const uint32_t cid = a.ids[pos];
+                    candId[j] = cid;
+                    if (candIdRec) candIdRec[s - task.sBegin] = cid;   // the emission's candidate record
+                    const double *src = a.xs + (uint64_t)pos * DP;
                     double nb = 0.0;
 #pragma unroll
                     for (int l = 0; l < DP; l++) {
-                        float b = (l < D) ? __double2float_rn(src[l] - originS[F32 ? l : 0]) : 0.0f;
-                        dst[2 * (1 + l)] = b;
-                        nb += (double)b * (double)b;
+                        const double x = src[l];
+                        bl[l] = (l < D) ? __double2float_rn(x - originS[l]) : 0.0f;
+                        if constexpr (F32) {
+                            float *dst = reinterpret_cast<float *>(&st.c[j >> 1][0]) + (j & 1);
+                            dst[2 * (1 + l)] = bl[l];
+                            nb += (double)bl[l] * (double)bl[l];
+                        } else {
+                            st.c[j][l] = x;
+                        }
                     }
-                    dst[0] = __double2float_rn(nb);
-                } else {
-                    double *dst = reinterpret_cast<double *>(&st.c[j][0]);
+                    if constexpr (F32) reinterpret_cast<float *>(&st.c[j >> 1][0])[j & 1] = __double2float_rn(nb);
+                }
 #pragma unroll
-                    for (int l = 0; l < DP; l++) dst[l] = src[l];
+                for (int l = 0; l < DP; l++) {
+                    const float2 mm = warp_min_max(in ? bl[l] : INFINITY, in ? bl[l] : -INFINITY);
+                    if (lane == 0) sm.boxC[j0 >> 5][l] = mm;
                 }
             }
             __syncthreads();
+            // ---- which (group, block) tiles can hold a hit: lane = slot x 8 +
+            // block.  Ruled out: boxes further apart than the radius (pruneT
+            // covers the rounding of the local coordinates), and home blocks
+            // whose positions all come before the group's queries.
+            uint32_t tiles;
+            {
+                const uint32_t r = lane >> 3, bi = lane & 7;
+                const uint32_t blk = sBase + bi * 32;
+                bool alive = r < nAct && bi * 32 < nIn;
+                if (alive) {
+                    float d2 = 0.0f;
+#pragma unroll
+                    for (int l = 0; l < DP; l++) {
+                        const float2 q = sm.boxQ[r * NW + warp][l], cb = sm.boxC[bi][l];
+                        const float gap = fmaxf(0.0f, fmaxf(cb.x - q.y, q.x - cb.y));
+                        d2 = fmaf(gap, gap, d2);
+                    }
+                    alive = !(d2 > a.pruneT) && !(sym && blk + 32 <= min(homeEnd, (r * NW + warp) * 32));
+                }
+                tiles = __ballot_sync(0xffffffffu, alive);
+            }
             // ---- hit masks of every block of the stage.  A warp without
             // queries skips the evaluation (but not the barriers).
 #pragma unroll 1
@@ -442,28 +551,28 @@ __global__ void __launch_bounds__(SJ_CTA, F32 ? SJ_JOIN_MIN_BLOCKS_F32 : SJ_JOIN
                 uint32_t hits[R], ymin[R];
 #pragma unroll
                 for (int r = 0; r < R; r++) { hits[r] = 0; ymin[r] = 0xffffffffu; }
-                // branch-free evaluation of the warp's active slots (a partly
-                // active slot set rounds up; the extra slots are ignored below)
-                if constexpr (F32) {
-                    if (nAct == 1) eval_block_f32<DP, 1, R>(st, jb >> 1, qa, nt, hits, ymin);
-                    else eval_block_f32<DP, R, R>(st, jb >> 1, qa, nt, hits, ymin);
-                } else {
-                    if (nAct == 1) eval_block_f64<DP, 1, R>(st, jb, q64, T1, hits);
-                    else eval_block_f64<DP, R, R>(st, jb, q64, T1, hits);
+                const uint32_t col = (tiles >> (jb >> 5)) & 0x01010101u;   // bit 8 r: slot r
+                const uint32_t act = (col | (col >> 7) | (col >> 14) | (col >> 21)) & 15u;
+                if (act) {
+                    eval_slots<DP, F32, R>(act, nAct, [&](auto r0, auto rr) {
+                        if constexpr (F32)
+                            eval_block_f32<DP, decltype(r0)::value, decltype(rr)::value, R>(st, jb >> 1, qa, nt, hits, ymin);
+                        else
+                            eval_block_f64<DP, decltype(r0)::value, decltype(rr)::value, R>(st, jb, q64, T1, hits);
+                    });
                 }
                 const uint32_t blk = sBase + jb;
                 const uint32_t hb = home_bits(blk, homeEnd, sym);
                 const uint32_t bInTask = (blk - task.sBegin) >> 5;
-                // record addresses of this block: row masks [chunk][query][block in
-                // chunk], column masks [block][query group][candidate]
-                uint32_t *const rowRec = maskBase ? maskBase + sj_row_mask_index(bInTask, 0, task.qCount, nBlk) : nullptr;
-                const uint32_t rowStride = min(64u, nBlk - (bInTask & ~63u));
-                uint32_t *const colRec = colBase ? colBase + ((uint64_t)bInTask * nG + warp) * 32 + lane : nullptr;
+                // record addresses of this block: row words [block][query],
+                // column words [block][query group][candidate]
+                uint32_t *const rowRec = rowBase ? rowBase + (uint64_t)bInTask * task.qCount + tid : nullptr;
+                uint32_t *const colRec = colBase ? colBase + (uint64_t)bInTask * nG * 32 + tid : nullptr;
                 uint32_t colHits = 0;   // this lane's candidate: hits over the warp's slots
 #pragma unroll
                 for (int r = 0; r < R; r++) {
-                    if ((uint32_t)r >= nAct) continue;   // warp-uniform
-                    const uint32_t qi = (uint32_t)r * SJ_CTA + tid;
+                    if (!((act >> r) & 1u)) continue;   // warp-uniform
+                    const uint32_t qi = ((uint32_t)r * NW + warp) * 32 + lane;
                     const bool qValid = qi < task.qCount;
                     const uint32_t rowValid = qValid ? (hb ? (inRange & row_keep(qi, blk, hb)) : inRange) : 0u;
                     uint32_t h = hits[r];
@@ -481,20 +590,28 @@ __global__ void __launch_bounds__(SJ_CTA, F32 ? SJ_JOIN_MIN_BLOCKS_F32 : SJ_JOIN
                                 }
                                 const uint32_t cpos = segStart[lo] + (s - segPre[lo]);
                                 refined++;
-                                if (exact_hit<DP>(a.xs, cpos, task.qBegin + qi, T)) h |= 1u << jj;
+                                if (exact_hit<DP>(a, cpos, task, qi, D, T)) h |= 1u << jj;
                             }
                         }
                     }
                     const uint32_t rowMask = h & rowValid;   // lane = query, bit = candidate
-                    if (rowRec && qValid) rowRec[(uint64_t)qi * rowStride] = rowMask;
+                    if (!__any_sync(0xffffffffu, rowMask)) continue;   // no hit in the tile
+                    live[r] |= 1u << (bInTask & 31);
+                    if (rowRec && qValid) rowRec[r * SJ_CTA] = rowMask;
                     rowCount[r] += __popc(rowMask);
                     if (sym) {
-                        // the mirrored direction: lane L gets candidate L's hits (none
-                        // to transpose when the warp's block has no hit at all)
+                        // the mirrored direction: lane L gets candidate L's hits
                         const uint32_t mir = hb ? (rowMask & mir_keep(qi, blk, hb)) : rowMask;
-                        const uint32_t colW = __any_sync(0xffffffffu, mir) ? transpose32(mir, lane) : 0u;
+                        const uint32_t colW = transpose32(mir, lane);
                         colHits += __popc(colW);
-                        if (colRec) colRec[(uint32_t)r * NW * 32] = colW;
+                        if (colRec) colRec[r * SJ_CTA] = colW;
+                    }
+                }
+                if (liveBase && ((bInTask & 31) == 31 || bInTask + 1 == nBlk)) {
+#pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        if ((uint32_t)r < nAct && lane == 0) liveBase[(bInTask >> 5) * nG + r * NW + warp] = live[r];
+                        live[r] = 0;
                     }
                 }
                 if (sym && colHits) colCnt[warp][jb + lane] += colHits;
@@ -517,10 +634,11 @@ __global__ void __launch_bounds__(SJ_CTA, F32 ? SJ_JOIN_MIN_BLOCKS_F32 : SJ_JOIN
         }
         {
             uint32_t mine = 0;
-            uint32_t *const rowBase = a.rowRel ? a.rowRel + (a.rowOff[t] - a.rowOff[a.taskBegin]) : nullptr;
+            uint32_t *const relBase = a.rowRel ? a.rowRel + (a.rowOff[t] - a.rowOff[a.taskBegin]) : nullptr;
 #pragma unroll
             for (int r = 0; r < R; r++) {
-                const uint32_t qi = (uint32_t)r * SJ_CTA + tid;
+                if ((uint32_t)r >= nAct) continue;
+                const uint32_t qi = ((uint32_t)r * NW + warp) * 32 + lane;
                 // evaluations of this query: stream positions [sBegin, sEnd), in the
                 // symmetric home segment only those at or after the query itself
                 if (qi < task.qCount) {
@@ -530,7 +648,7 @@ __global__ void __launch_bounds__(SJ_CTA, F32 ? SJ_JOIN_MIN_BLOCKS_F32 : SJ_JOIN
                 // the key's count before this addition: where this task's row
                 // run starts inside the query's key run
                 const uint32_t rel = rowCount[r] ? atomicAdd(&a.keyCount[qid[r]], rowCount[r]) : 0u;
-                if (rowBase && qi < task.qCount) rowBase[qi] = rel;
+                if (relBase && qi < task.qCount) relBase[qi] = rel;
                 mine += rowCount[r];
             }
             if (mine) atomicAdd(&sm.taskPairs, (unsigned long long)mine);
@@ -560,18 +678,296 @@ __global__ void __launch_bounds__(SJ_CTA, F32 ? SJ_JOIN_MIN_BLOCKS_F32 : SJ_JOIN
     }
 }
 
+// ------------------------------------------------- tasks of few queries --
+// Count pass over the tasks of at most SJ_SMALL_QUERIES query points: one warp a
+// task, lane = candidate.  k_join's CTA would leave most of its lanes without a
+// query on sparse grids (two points a cell: 2 of 128); here every lane evaluates
+// its candidate against the task's queries in turn (packed two per FP32
+// instruction), a ballot is the query's row word, the lane's own bits are the
+// candidate's column word, and no barrier or segment table is needed: the
+// segments go by 32 at a time in registers.  Same operations in the same order
+// as k_join, same records.
+// Bound: instruction issue (per block of 32 candidates ~60 instructions and
+// ~12 + D per query).  Measured against k_join on the same tasks: see DESIGN.
 template <int DP, bool F32>
-int occupancy_of()
+struct __align__(16) SmallSmem {
+    static constexpr int CW2 = Stage32<DP>::CW2;
+    // FP32: per pair of queries the two (-tLo), then the two (-2 a_l) of each dimension
+    float2 q2[F32 ? SJ_SMALL_QUERIES / 2 : 1][CW2];
+    double q[F32 ? 1 : SJ_SMALL_QUERIES][DP];
+    float2 box[DP];             // (min, max) of the queries' local coordinates
+    double origin[DP];
+};
+
+constexpr uint32_t SMALL_BOX = 6;   // queries from which on testing a block against their box pays
+
+template <int DP, bool F32>
+__global__ void __launch_bounds__(SJ_CTA, DP <= 8 ? 6 : 4) k_join_small(sj_join_args a, sj_grid_dev g, int queue)
 {
-    constexpr int MAXDEV = 64;
-    static std::atomic<int> occ[MAXDEV];   // per device ordinal, 0 = not measured yet
+    constexpr uint32_t FULL = 0xffffffffu;
+    __shared__ SmallSmem<DP, F32> smem[NW];
+    const uint32_t lane = threadIdx.x & 31u;
+    SmallSmem<DP, F32> &sm = smem[threadIdx.x >> 5];
+    const int D = g.D;
+    const double T = g.thresh;
+    const uint32_t deltaBits = __float_as_uint(a.delta);
+    const uint32_t first = a.smallPre[a.taskBegin];
+    const uint32_t count = a.smallPre[a.taskEnd] - first;
+    const uint32_t warps = gridDim.x * NW;
+    unsigned long long pairsAll = 0;
+    uint32_t i = blockIdx.x * NW + (threadIdx.x >> 5);
+    for (;;) {
+        if (queue) {
+            if (lane == 0) i = atomicAdd(a.queueHead + 1, 1u);
+            i = __shfl_sync(FULL, i, 0);
+        }
+        if (i >= count) break;
+        const uint32_t t = a.smallList[first + i];
+        i += warps;
+        const sj_task task = a.tasks[t];
+        const bool sym = (task.flags & SJ_TASK_SYM) != 0;
+        const uint32_t qc = task.qCount;
+        const uint32_t aStart = a.cellStart[task.cell], aEnd = a.cellStart[task.cell + 1];
+        const uint32_t nbrBase = a.nbrStart[task.cell];
+        const uint32_t homeEnd = (task.segBase == 0 && (task.flags & SJ_TASK_HOME)) ? aEnd - (sym ? task.qBegin : aStart)
+                                                                                   : 0u;
+        __syncwarp();   // the previous task is done with the warp's shared memory
+        if ((int)lane < DP) {
+            // local-coordinate origin, as k_join's
+            double o;
+            if ((int)lane < g.k) o = g.minArr[lane] + ((double)a.cellCoord[(uint64_t)task.cell * g.k + lane] + 0.5) * g.eps;
+            else if ((int)lane < D) o = g.center[lane];
+            else o = 0.0;
+            sm.origin[lane] = o;
+        }
+        __syncwarp();
+        uint32_t qid;
+        {
+            double src[DP];
+            qid = load_query<DP>(a, task, lane < qc ? lane : 0u, D, src);
+            double na = 0.0;
+#pragma unroll
+            for (int l = 0; l < DP; l++) {
+                const double x = src[l];
+                const float ql = (l < D && lane < qc) ? __double2float_rn(x - sm.origin[l]) : 0.0f;
+                if (qc >= SMALL_BOX) {
+                    const float2 mm = warp_min_max(lane < qc ? ql : INFINITY, lane < qc ? ql : -INFINITY);
+                    if (lane == 0) sm.box[l] = mm;
+                }
+                if constexpr (F32) {
+                    reinterpret_cast<float *>(&sm.q2[lane >> 1][1 + l])[lane & 1] = -2.0f * ql;
+                    na += (double)ql * (double)ql;
+                } else {
+                    sm.q[lane][l] = x;
+                }
+            }
+            if constexpr (F32) {
+                const float tLo = __double2float_rd(T - na - a.margin);
+                reinterpret_cast<float *>(&sm.q2[lane >> 1][0])[lane & 1] = lane < qc ? -tLo : INFINITY;
+            }
+        }
+        __syncwarp();
+        uint32_t *const liveBase = a.masks ? a.masks + (a.maskOff[t] - a.maskOff[a.taskBegin]) : nullptr;
+        uint32_t *const colBase = (a.colMasks && sym) ? a.colMasks + (a.colOff[t] - a.colOff[a.taskBegin]) : nullptr;
+        const uint64_t candRecOff = a.candOff ? a.candOff[t] - a.candOff[a.taskBegin] : 0;
+        uint32_t *const candIdRec = a.candId ? a.candId + candRecOff : nullptr;
+        uint32_t *const candRelRec = (a.candRel && sym) ? a.candRel + candRecOff : nullptr;
+        const uint32_t nBlk = (task.sEnd - task.sBegin + 31) / 32;
+        uint32_t *const rowBase = liveBase ? liveBase + sj_live_words(nBlk, 1) : nullptr;
+
+        uint32_t rowCount = 0, colCount = 0, live = 0, refined = 0;
+        // the current 32 segments: lane's start, and prefix of their lengths (stream positions)
+        uint32_t seg = 0, segStart = 0, segLen = 0, segIncl = 0, segEnd = 0;   // segEnd: stream position after them
+        // candidate of stream position blk + lane, for ascending blocks
+        auto locate = [&](uint32_t blk) -> uint32_t {
+            const uint32_t s = blk + lane;
+            uint32_t cpos = 0;
+            for (;;) {
+                {
+                    // positions inside the current segments: the first with prefix > s
+                    const uint32_t base = segEnd - __shfl_sync(FULL, segIncl, 31);   // position of the first one
+                    uint32_t lo = 0;
+#pragma unroll
+                    for (int w = 16; w > 0; w >>= 1) {
+                        const uint32_t v = __shfl_sync(FULL, segIncl, lo + w - 1);
+                        if (base + v <= s) lo += w;
+                    }
+                    lo = min(lo, 31u);
+                    const uint32_t st = __shfl_sync(FULL, segStart, lo);
+                    const uint32_t ex = __shfl_sync(FULL, segIncl - segLen, lo);
+                    if (s >= base && s < segEnd) cpos = st + (s - base - ex);
+                }
+                if (segEnd > blk + 31 || segEnd >= task.sEnd || seg >= task.segCount) return cpos;   // warp-uniform
+                // ---- the next 32 segments
+                const uint32_t mySeg = seg + lane;
+                segStart = segLen = 0;
+                if (mySeg < task.segCount) {
+                    const uint32_t gs = task.segBase + mySeg;
+                    if (gs == 0) {
+                        segStart = sym ? task.qBegin : aStart;
+                        segLen = aEnd - segStart;
+                    } else {
+                        const uint32_t nb = a.nbrCell[nbrBase + gs - 1];
+                        segStart = a.cellStart[nb];
+                        segLen = a.cellStart[nb + 1] - segStart;
+                    }
+                }
+                segIncl = segLen;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(FULL, segIncl, o);
+                    if (lane >= (uint32_t)o) segIncl += y;
+                }
+                segEnd += __shfl_sync(FULL, segIncl, 31);
+                seg += 32;
+            }
+        };
+        // the next block's candidates are loaded while this one is evaluated
+        uint32_t nPos = locate(task.sBegin), nId = a.ids[nPos];
+        double nx[DP];
+#pragma unroll
+        for (int l = 0; l < DP; l++) nx[l] = a.xs[(uint64_t)nPos * DP + l];
+#pragma unroll 1
+        for (uint32_t b = 0; b < nBlk; b++) {
+            const uint32_t blk = task.sBegin + 32 * b;
+            const uint32_t s = blk + lane;
+            const bool in = s < task.sEnd;
+            const uint32_t cpos = nPos, cid = nId;
+            double c[DP];
+#pragma unroll
+            for (int l = 0; l < DP; l++) c[l] = nx[l];
+            if (b + 1 < nBlk) {
+                nPos = locate(blk + 32);
+                nId = a.ids[nPos];
+#pragma unroll
+                for (int l = 0; l < DP; l++) nx[l] = a.xs[(uint64_t)nPos * DP + l];
+            }
+            if (candIdRec && in) candIdRec[s - task.sBegin] = cid;
+            const bool home = sym && s < homeEnd;
+            const bool anyHome = sym && blk < homeEnd;   // warp-uniform
+            uint32_t rowWord = 0, colW = 0;
+            float bl[DP];
+#pragma unroll
+            for (int l = 0; l < DP; l++) {
+                bl[l] = (l < D) ? __double2float_rn(c[l] - sm.origin[l]) : 0.0f;
+            }
+            // the block is ruled out when every candidate lies further from the
+            // queries' box than the radius (as k_join's tiles)
+            bool alive = true;
+            if (qc >= SMALL_BOX) {
+                float d2 = 0.0f;
+#pragma unroll
+                for (int l = 0; l < DP; l++) {
+                    const float2 q = sm.box[l];
+                    const float gap = fmaxf(0.0f, fmaxf(bl[l] - q.y, q.x - bl[l]));
+                    d2 = fmaf(gap, gap, d2);
+                }
+                alive = __any_sync(FULL, in && !(d2 > a.pruneT));
+            }
+            if (!alive) {
+                // no hit: nothing to record but the candidates' ids
+            } else if constexpr (F32) {
+                float2 b2[DP];
+                double nbd = 0.0;
+#pragma unroll
+                for (int l = 0; l < DP; l++) {
+                    b2[l] = make_float2(bl[l], bl[l]);
+                    nbd += (double)bl[l] * (double)bl[l];
+                }
+                const float nbf = __double2float_rn(nbd);
+                for (uint32_t p = 0; 2 * p < qc; p++) {
+                    const float4 *const row4 = reinterpret_cast<const float4 *>(&sm.q2[p][0]);
+                    float4 v = row4[0];
+                    float2 y = __fadd2_rn(make_float2(nbf, nbf), make_float2(v.x, v.y));
+                    y = __ffma2_rn(make_float2(v.z, v.w), b2[0], y);
+#pragma unroll
+                    for (int h = 1; h < SmallSmem<DP, F32>::CW2 / 2; h++) {
+                        v = row4[h];
+                        if (2 * h - 1 < DP) y = __ffma2_rn(make_float2(v.x, v.y), b2[2 * h - 1 < DP ? 2 * h - 1 : 0], y);
+                        if (2 * h < DP) y = __ffma2_rn(make_float2(v.z, v.w), b2[2 * h < DP ? 2 * h : 0], y);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        const uint32_t q = 2 * p + e;
+                        const float ye = e ? y.y : y.x;
+                        bool keep = in && q < qc;
+                        if (anyHome) keep = keep && (!home || s >= q);
+                        bool h = __float_as_int(ye) < 0;
+                        if (__any_sync(FULL, keep && __float_as_uint(ye) < deltaBits)) {
+                            if (keep && __float_as_uint(ye) < deltaBits) {
+                                refined++;
+                                h = exact_hit<DP>(a, cpos, task, q, D, T);
+                            }
+                        }
+                        h = h && keep;
+                        const uint32_t word = __ballot_sync(FULL, h);
+                        if (lane == q) rowWord = word;
+                        colW |= (h ? 1u : 0u) << (q & 31u);
+                    }
+                }
+            } else {
+                for (uint32_t q = 0; q < qc; q++) {
+                    const double acc = ref_dist2<DP>(c, sm.q[q]);
+                    bool h = in && acc <= T;
+                    if (anyHome) h = h && (!home || s >= q);
+                    const uint32_t word = __ballot_sync(FULL, h);
+                    if (lane == q) rowWord = word;
+                    colW |= (h ? 1u : 0u) << q;
+                }
+            }
+            if (home) colW &= s < 32u ? ~(1u << s) : FULL;   // the mirrored direction drops the query itself
+            rowCount += __popc(rowWord);
+            const bool hit = __any_sync(FULL, rowWord);
+            if (hit) {
+                live |= 1u << (b & 31);
+                if (rowBase && lane < qc) rowBase[(uint64_t)b * qc + lane] = rowWord;
+            }
+            if (sym) {
+                const uint32_t n = __popc(colW);
+                const uint32_t rel = n ? atomicAdd(&a.keyCount[cid], n) : 0u;
+                if (candRelRec && in) candRelRec[s - task.sBegin] = rel;
+                if (hit && colBase) colBase[(uint64_t)b * 32 + lane] = colW;
+                colCount += n;
+            }
+            if (liveBase && ((b & 31) == 31 || b + 1 == nBlk)) {
+                if (lane == 0) liveBase[b >> 5] = live;
+                live = 0;
+            }
+        }
+        uint32_t evals = 0;
+        if (lane < qc) {
+            const uint32_t from = max(task.sBegin, min(lane, sym ? homeEnd : 0u));
+            evals = task.sEnd > from ? task.sEnd - from : 0u;
+            const uint32_t rel = rowCount ? atomicAdd(&a.keyCount[qid], rowCount) : 0u;
+            if (a.rowRel) a.rowRel[a.rowOff[t] - a.rowOff[a.taskBegin] + lane] = rel;
+        }
+        // a task's worst case is below 2^32 pairs and evaluations
+        const uint32_t hits = __reduce_add_sync(FULL, (sym ? colCount : 0u) + (lane < qc ? rowCount : 0u));
+        evals = __reduce_add_sync(FULL, evals);
+        if (F32) refined = __reduce_add_sync(FULL, refined);
+        if (lane == 0) {
+            pairsAll += hits;
+            if (a.taskHits) a.taskHits[t] = hits;
+            if (a.taskEvals) a.taskEvals[t] = evals;
+            if (a.taskRefined) a.taskRefined[t] = refined;
+        }
+    }
+    if (lane == 0 && pairsAll) {
+        atomicAdd(&a.stat[2], pairsAll);
+        if (a.batchPairs) atomicAdd(a.batchPairs, pairsAll);
+    }
+}
+
+template <class Kernel>
+int occupancy_of(Kernel k, std::atomic<int> (&occ)[64])
+{
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev < 0 || dev >= MAXDEV) dev = 0;
-    int o = occ[dev].load();
+    if (dev < 0 || dev >= 64) dev = 0;
+    int o = occ[dev].load();   // per device ordinal, 0 = not measured yet
     if (o == 0) {
         int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_join<DP, F32, sj_query_slots(DP, F32)>, SJ_CTA, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, SJ_CTA, 0);
         o = b > 0 ? b : 1;
         occ[dev].store(o);
     }
@@ -579,44 +975,51 @@ int occupancy_of()
 }
 
 template <int DP, bool F32>
-cudaError_t launch_one(const sj_join_args &a, const sj_grid_dev &g, int queue, int numSM, int maxCtasPerSM,
-                       cudaStream_t s)
+cudaError_t launch_one(const sj_join_args &a, const sj_grid_dev &g, int queue, uint32_t nBig, uint32_t nSmall,
+                       int numSM, int maxCtasPerSM, cudaStream_t s)
 {
-    const uint32_t nt = a.taskEnd - a.taskBegin;
-    if (nt == 0) return cudaSuccess;
+    static std::atomic<int> occBig[64], occSmall[64];
     // persistent queue: one full wave of resident CTAs (or fewer per SM, to
     // leave room for a kernel of the other stream)
-    int perSM = occupancy_of<DP, F32>();
-    if (maxCtasPerSM > 0 && maxCtasPerSM < perSM) perSM = maxCtasPerSM;
-    unsigned grid = queue ? (unsigned)(numSM * perSM) : nt;
-    if (queue && grid > nt) grid = nt;
-    k_join<DP, F32, sj_query_slots(DP, F32)><<<grid, SJ_CTA, 0, s>>>(a, g, queue);
-    sj_note_launch();
+    if (nBig) {
+        int perSM = occupancy_of(k_join<DP, F32, sj_query_slots(DP, F32)>, occBig);
+        if (maxCtasPerSM > 0 && maxCtasPerSM < perSM) perSM = maxCtasPerSM;
+        unsigned grid = queue ? (unsigned)(numSM * perSM) : nBig;
+        if (queue && grid > nBig) grid = nBig;
+        k_join<DP, F32, sj_query_slots(DP, F32)><<<grid, SJ_CTA, 0, s>>>(a, g, queue);
+        sj_note_launch();
+    }
+    if (nSmall) {
+        const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)numSM * occupancy_of(k_join_small<DP, F32>, occSmall),
+                                                           ((uint64_t)nSmall + NW - 1) / NW);
+        k_join_small<DP, F32><<<grid, SJ_CTA, 0, s>>>(a, g, queue);
+        sj_note_launch();
+    }
     return cudaGetLastError();
 }
 
 template <int DP>
-cudaError_t launch_dp(const sj_join_args &a, const sj_grid_dev &g, int fp32, int queue, int numSM, int maxCtas,
-                      cudaStream_t s)
+cudaError_t launch_dp(const sj_join_args &a, const sj_grid_dev &g, int fp32, int queue, uint32_t nBig, uint32_t nSmall,
+                      int numSM, int maxCtas, cudaStream_t s)
 {
-    return fp32 ? launch_one<DP, true>(a, g, queue, numSM, maxCtas, s)
-                : launch_one<DP, false>(a, g, queue, numSM, maxCtas, s);
+    return fp32 ? launch_one<DP, true>(a, g, queue, nBig, nSmall, numSM, maxCtas, s)
+                : launch_one<DP, false>(a, g, queue, nBig, nSmall, numSM, maxCtas, s);
 }
 
 }  // namespace
 
-cudaError_t sj_launch_join(const sj_join_args &a, const sj_grid_dev &g, int fp32, int queue, int numSM,
-                           int maxCtasPerSM, cudaStream_t s)
+cudaError_t sj_launch_join(const sj_join_args &a, const sj_grid_dev &g, int fp32, int queue, uint32_t nBig,
+                           uint32_t nSmall, int numSM, int maxCtasPerSM, cudaStream_t s)
 {
     switch (g.Dp) {
-    case 1: return launch_dp<1>(a, g, fp32, queue, numSM, maxCtasPerSM, s);
-    case 2: return launch_dp<2>(a, g, fp32, queue, numSM, maxCtasPerSM, s);
-    case 3: return launch_dp<3>(a, g, fp32, queue, numSM, maxCtasPerSM, s);
-    case 4: return launch_dp<4>(a, g, fp32, queue, numSM, maxCtasPerSM, s);
-    case 6: return launch_dp<6>(a, g, fp32, queue, numSM, maxCtasPerSM, s);
-    case 8: return launch_dp<8>(a, g, fp32, queue, numSM, maxCtasPerSM, s);
-    case 12: return launch_dp<12>(a, g, fp32, queue, numSM, maxCtasPerSM, s);
-    case 16: return launch_dp<16>(a, g, fp32, queue, numSM, maxCtasPerSM, s);
+    case 1: return launch_dp<1>(a, g, fp32, queue, nBig, nSmall, numSM, maxCtasPerSM, s);
+    case 2: return launch_dp<2>(a, g, fp32, queue, nBig, nSmall, numSM, maxCtasPerSM, s);
+    case 3: return launch_dp<3>(a, g, fp32, queue, nBig, nSmall, numSM, maxCtasPerSM, s);
+    case 4: return launch_dp<4>(a, g, fp32, queue, nBig, nSmall, numSM, maxCtasPerSM, s);
+    case 6: return launch_dp<6>(a, g, fp32, queue, nBig, nSmall, numSM, maxCtasPerSM, s);
+    case 8: return launch_dp<8>(a, g, fp32, queue, nBig, nSmall, numSM, maxCtasPerSM, s);
+    case 12: return launch_dp<12>(a, g, fp32, queue, nBig, nSmall, numSM, maxCtasPerSM, s);
+    case 16: return launch_dp<16>(a, g, fp32, queue, nBig, nSmall, numSM, maxCtasPerSM, s);
     }
     return cudaErrorInvalidValue;
 }

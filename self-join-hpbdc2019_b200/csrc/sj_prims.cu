@@ -1,4 +1,4 @@
-// Device primitives: exclusive scan (u32), stable LSD radix sort, pair-set hash.
+// Device primitives: exclusive scan (u32), stable LSD radix sort, CSR append.
 #include <atomic>
 
 #include "sj_internal.h"
@@ -268,240 +268,6 @@ cudaError_t radix_sort(K *keys, uint32_t *vals, K *keysAlt, uint32_t *valsAlt, u
     return cudaSuccess;
 }
 
-__device__ __forceinline__ unsigned long long splitmix64(unsigned long long z)
-{
-    z += 0x9e3779b97f4a7c15ULL;
-    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ULL;
-    z = (z ^ (z >> 27)) * 0x94d049bb133111ebULL;
-    return z ^ (z >> 31);
-}
-
-__global__ void __launch_bounds__(256) k_hash_pairs(const int32_t *__restrict__ key, const int32_t *__restrict__ val,
-                                                    uint64_t m, unsigned long long *out)
-{
-    unsigned long long h = 0;
-    uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += stride) {
-        unsigned long long z = ((unsigned long long)(uint32_t)key[i] << 32) | (uint32_t)val[i];
-        h += splitmix64(z);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
-    __shared__ unsigned long long ws[8];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = h;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long t = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += ws[w];
-        atomicAdd(out, t);
-    }
-}
-
-// Keys of a batch: key k owns slots [excl[k], excl[k+1]) (excl[n] = *total).
-// A warp takes 32 consecutive keys and writes each key's run with all lanes,
-// 128 contiguous bytes per store.  Runs longer than EXP_LONG slots (a dense
-// key can own a million slots of one batch) are queued instead and written by
-// whole CTAs in k_expand_long, so one warp never holds up the launch.
-constexpr uint32_t EXP_LONG = 16384;
-
-__device__ __forceinline__ void write_run(int32_t *__restrict__ outKey, uint32_t s0, uint32_t e0, int32_t key,
-                                          uint32_t t, uint32_t nt)
-{
-    // up to 3 single slots to a 16-byte boundary, 16-byte stores, the rest
-    const uint32_t a = min((s0 + 3u) & ~3u, e0);
-    const uint32_t b = a + ((e0 - a) & ~3u);
-    if (t < a - s0) outKey[s0 + t] = key;
-    const int4 kv = make_int4(key, key, key, key);
-    for (uint32_t pos = a + 4 * t; pos < b; pos += 4 * nt) *reinterpret_cast<int4 *>(outKey + pos) = kv;
-    if (t < e0 - b) outKey[b + t] = key;
-}
-
-__global__ void __launch_bounds__(256) k_expand_keys(const uint32_t *__restrict__ excl,
-                                                     const uint32_t *__restrict__ total, uint64_t n,
-                                                     int32_t *__restrict__ outKey,
-                                                     const unsigned long long *__restrict__ batchPairs, uint64_t cap,
-                                                     uint4 *__restrict__ longRuns, uint32_t longCap,
-                                                     uint32_t *__restrict__ longCount)
-{
-    if (*batchPairs > cap) return;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t k0 = ((uint64_t)blockIdx.x * 256 + (threadIdx.x & ~31u));
-    if (k0 >= n) return;
-    const uint64_t k = k0 + lane;
-    const uint32_t tot = *total;
-    const uint32_t st = k < n ? excl[k] : tot;
-    const uint32_t en = k + 1 < n ? excl[k + 1] : tot;
-    uint32_t live = __ballot_sync(0xffffffffu, en > st);
-    while (live) {
-        const int i = __ffs(live) - 1;
-        live &= live - 1;
-        const uint32_t s0 = __shfl_sync(0xffffffffu, st, i);
-        const uint32_t e0 = __shfl_sync(0xffffffffu, en, i);
-        const int32_t key = (int32_t)(k0 + i);
-        if (e0 - s0 > EXP_LONG) {
-            uint32_t j = 0;
-            if (lane == 0) j = atomicAdd(longCount, 1u);
-            j = __shfl_sync(0xffffffffu, j, 0);
-            if (j < longCap) {
-                if (lane == 0) longRuns[j] = make_uint4((uint32_t)key, s0, e0, 0u);
-                continue;
-            }
-        }
-        write_run(outKey, s0, e0, key, lane, 32);
-    }
-}
-
-// The queued long runs, one CTA per run at a time.
-__global__ void __launch_bounds__(256) k_expand_long(int32_t *__restrict__ outKey,
-                                                     const unsigned long long *__restrict__ batchPairs, uint64_t cap,
-                                                     const uint4 *__restrict__ longRuns, uint32_t longCap,
-                                                     const uint32_t *__restrict__ longCount)
-{
-    if (*batchPairs > cap) return;
-    const uint32_t cnt = min(*longCount, longCap);
-    for (uint32_t j = blockIdx.x; j < cnt; j += gridDim.x) {
-        const uint4 r = longRuns[j];
-        write_run(outKey, r.y, r.z, (int32_t)r.x, threadIdx.x, blockDim.x);
-    }
-}
-
-// The consumer fold of a device-resident batch, with the key array written in
-// the same pass.  Key k owns slots [excl[k], excl[k+1]) (excl[n] = *total).
-// The slots are cut into chunks of FOLD_CHUNK; k_fold_chunk_keys records the
-// key at each chunk's first slot (one thread per key writes the chunks its run
-// starts), and in k_fold a warp takes a chunk in rounds of 128 slots, lane L
-// holding slots 4L .. 4L+3 of the round.  The warp keeps a window of 32
-// consecutive keys, one per lane (its run start and end); each lane whose
-// non-empty run starts inside the round marks key + 1 at that slot in a
-// per-warp shared array, and an inclusive max-scan over the round (4 slots per
-// lane, then across the lanes, seeded with the key carried from the previous
-// round) gives every slot its key, since keys ascend with the slots.  When the
-// window's runs end inside the round, the window jumps to the key whose run
-// holds the first slot past it (a 32-ary search over the run starts, which
-// steps over stretches of empty runs: keys are point ids).  The values are
-// read back in 16-byte streaming loads, the keys stored in 16-byte streaming
-// stores, and splitmix64(key << 32 | value) is added to the set hash.  Every
-// chunk is the same size, so the work is balanced whatever the run lengths.
-// 8 bytes per pair move, against 12 for a key expansion followed by a fold
-// that reads both arrays.  Skipped when the batch's count exceeds cap.
-constexpr uint32_t FOLD_CHUNK = 4096;
-constexpr int FOLD_THREADS = 256;
-constexpr int FOLD_CTAS_PER_SM = 6;   // resident k_fold CTAs per SM (the register budget allows 6)
-
-__global__ void __launch_bounds__(256) k_fold_chunk_keys(const uint32_t *__restrict__ excl,
-                                                         const uint32_t *__restrict__ total, uint64_t n,
-                                                         const unsigned long long *__restrict__ batchPairs,
-                                                         uint64_t cap, uint32_t *__restrict__ chunkKey)
-{
-    if (*batchPairs > cap) return;
-    const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const uint32_t tot = *total;
-    const uint32_t st = excl[k];
-    const uint32_t en = k + 1 < n ? excl[k + 1] : tot;
-    for (uint32_t c = (st + FOLD_CHUNK - 1) / FOLD_CHUNK; (uint64_t)c * FOLD_CHUNK < en; c++) chunkKey[c] = (uint32_t)k;
-}
-
-__global__ void __launch_bounds__(FOLD_THREADS, FOLD_CTAS_PER_SM) k_fold(const uint32_t *__restrict__ excl,
-                                                       const uint32_t *__restrict__ total, uint64_t n,
-                                                       const int32_t *__restrict__ val, int32_t *__restrict__ outKey,
-                                                       const unsigned long long *__restrict__ batchPairs,
-                                                       uint64_t cap, const uint32_t *__restrict__ chunkKey,
-                                                       unsigned long long *__restrict__ hashOut)
-{
-    __shared__ __align__(16) uint32_t marks[FOLD_THREADS / 32][128];   // per warp: key + 1 at each run start
-    if (*batchPairs > cap) return;
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t *const mk = marks[threadIdx.x >> 5];
-    const uint32_t tot = *total;
-    const uint32_t nChunks = (tot + FOLD_CHUNK - 1) / FOLD_CHUNK;
-    const uint32_t warpsAll = (gridDim.x * blockDim.x) >> 5;
-    unsigned long long h = 0;
-    *reinterpret_cast<uint4 *>(mk + 4 * lane) = make_uint4(0u, 0u, 0u, 0u);
-    // run start and end of key kk (both the total for kk >= n)
-    auto runStart = [&](uint64_t kk) -> uint32_t { return kk < n ? excl[kk] : tot; };
-    auto runEnd = [&](uint64_t kk) -> uint32_t { return kk + 1 < n ? excl[kk + 1] : tot; };
-    for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nChunks; c += warpsAll) {
-        const uint32_t p0 = c * FOLD_CHUNK, p1 = min(p0 + FOLD_CHUNK, tot);
-        uint64_t k = chunkKey[c];         // its run holds slot p0
-        uint32_t carry = (uint32_t)k;     // key of the round's slots before its first marked start
-        uint32_t S = runStart(k + lane), R = runEnd(k + lane);
-        for (uint32_t base = p0; base < p1; base += 128) {
-            const uint32_t lim = min(base + 128u, p1);
-            const uint32_t p = base + 4 * lane;
-            const uint32_t cnt = p < lim ? min(4u, lim - p) : 0u;   // this lane's slots: p .. p + cnt - 1
-            int4 v = make_int4(0, 0, 0, 0);   // the values, loaded while the keys are found
-            if (cnt == 4) {
-                v = __ldcs(reinterpret_cast<const int4 *>(val + p));
-            } else {
-                if (cnt > 0) v.x = __ldcs(val + p);
-                if (cnt > 1) v.y = __ldcs(val + p + 1);
-                if (cnt > 2) v.z = __ldcs(val + p + 2);
-            }
-            __syncwarp();   // every lane has cleared its slots of the previous round
-            for (;;) {
-                if (R > S && S >= base && S < lim) mk[S - base] = (uint32_t)(k + lane) + 1u;
-                const uint32_t Rlast = __shfl_sync(0xffffffffu, R, 31);
-                if (Rlast >= lim || k + 32 >= n) break;   // warp-uniform
-                // the window's runs end inside the round: jump to the largest
-                // key k' with excl[k'] <= Rlast (the keys in between have empty
-                // runs).  Invariant: excl[lo] <= Rlast, and hi == n or
-                // excl[hi] > Rlast.
-                uint64_t lo = k + 32, hi = n;
-                while (hi - lo > 1) {
-                    const uint64_t step = (hi - lo + 31) / 32;
-                    const uint64_t probe = lo + (uint64_t)(lane + 1) * step;
-                    const bool ok = probe < hi && excl[probe] <= Rlast;
-                    const uint32_t cntOk = __popc(__ballot_sync(0xffffffffu, ok));   // a prefix of the lanes
-                    lo += (uint64_t)cntOk * step;
-                    hi = min(hi, lo + step);
-                }
-                k = lo;
-                S = runStart(k + lane);
-                R = runEnd(k + lane);
-            }
-            __syncwarp();
-            const uint4 m = *reinterpret_cast<const uint4 *>(mk + 4 * lane);
-            *reinterpret_cast<uint4 *>(mk + 4 * lane) = make_uint4(0u, 0u, 0u, 0u);
-            // keys ascend with the slots: each slot's key + 1 is the largest mark
-            // at or before it (or the carried key + 1)
-            const uint32_t m1 = max(m.x, m.y), m2 = max(m1, m.z), m3 = max(m2, m.w);
-            uint32_t x = m3;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= (uint32_t)o) x = max(x, y);
-            }
-            uint32_t pre = __shfl_up_sync(0xffffffffu, x, 1);
-            pre = max(lane ? pre : 0u, carry + 1u);
-            const uint32_t k0 = max(pre, m.x) - 1u, k1 = max(pre, m1) - 1u, k2 = max(pre, m2) - 1u,
-                           k3 = max(pre, m3) - 1u;
-            carry = __shfl_sync(0xffffffffu, k3, 31);
-            if (cnt == 4) {
-                __stcs(reinterpret_cast<int4 *>(outKey + p), make_int4((int)k0, (int)k1, (int)k2, (int)k3));
-            } else {
-                if (cnt > 0) outKey[p] = (int32_t)k0;
-                if (cnt > 1) outKey[p + 1] = (int32_t)k1;
-                if (cnt > 2) outKey[p + 2] = (int32_t)k2;
-            }
-            if (cnt > 0) h += splitmix64(((unsigned long long)k0 << 32) | (uint32_t)v.x);
-            if (cnt > 1) h += splitmix64(((unsigned long long)k1 << 32) | (uint32_t)v.y);
-            if (cnt > 2) h += splitmix64(((unsigned long long)k2 << 32) | (uint32_t)v.z);
-            if (cnt > 3) h += splitmix64(((unsigned long long)k3 << 32) | (uint32_t)v.w);
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
-    __shared__ unsigned long long ws[FOLD_THREADS / 32];
-    if (lane == 0) ws[threadIdx.x >> 5] = h;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long t = 0;
-        for (int w = 0; w < FOLD_THREADS / 32; w++) t += ws[w];
-        if (t) atomicAdd(hashOut, t);
-    }
-}
-
 // Appends a batch to a device CSR neighbour table: key k's run
 // [start[k], start[k+1]) of vals (start[n] = *total) goes to
 // cols[rowPtr[k] + fill[k] ...] and fill[k] grows by its length.  A warp takes
@@ -558,36 +324,6 @@ cudaError_t sj_u32_to_f32(const uint32_t *in, uint64_t n, float *out, cudaStream
     return cudaGetLastError();
 }
 
-cudaError_t sj_expand_keys(const uint32_t *excl, const uint32_t *total, uint64_t n, int32_t *outKey,
-                           const unsigned long long *batchPairs, uint64_t cap, void *longRuns, uint32_t longCap,
-                           uint32_t *longCount, int numSM, cudaStream_t s)
-{
-    if (n == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(longCount, 0, sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
-    k_expand_keys<<<(unsigned)ceil_div(n, 256), 256, 0, s>>>(excl, total, n, outKey, batchPairs, cap,
-                                                            (uint4 *)longRuns, longCap, longCount);
-    sj_note_launch();
-    k_expand_long<<<(unsigned)(numSM * 8), 256, 0, s>>>(outKey, batchPairs, cap, (const uint4 *)longRuns, longCap,
-                                                       longCount);
-    sj_note_launch();
-    return cudaGetLastError();
-}
-
-size_t sj_fold_chunks(uint64_t cap) { return (size_t)(cap / FOLD_CHUNK) + 2; }
-
-cudaError_t sj_fold(const uint32_t *excl, const uint32_t *total, uint64_t n, const int32_t *val, int32_t *outKey,
-                    const unsigned long long *batchPairs, uint64_t cap, uint32_t *chunkKey,
-                    unsigned long long *hashOut, int numSM, cudaStream_t s)
-{
-    if (n == 0) return cudaSuccess;
-    k_fold_chunk_keys<<<(unsigned)ceil_div(n, 256), 256, 0, s>>>(excl, total, n, batchPairs, cap, chunkKey);
-    sj_note_launch();
-    k_fold<<<(unsigned)(numSM * FOLD_CTAS_PER_SM), FOLD_THREADS, 0, s>>>(excl, total, n, val, outKey, batchPairs, cap, chunkKey, hashOut);
-    sj_note_launch();
-    return cudaGetLastError();
-}
-
 cudaError_t sj_csr_append(const uint32_t *start, const uint32_t *total, uint64_t n, const int32_t *vals,
                           const uint64_t *rowPtr, uint32_t *fill, int32_t *cols, uint64_t colsCap,
                           unsigned long long *err, cudaStream_t s)
@@ -597,8 +333,6 @@ cudaError_t sj_csr_append(const uint32_t *start, const uint32_t *total, uint64_t
     sj_note_launch();
     return cudaGetLastError();
 }
-
-size_t sj_expand_long_slots(uint64_t cap) { return (size_t)(cap / EXP_LONG) + 1; }
 
 static std::atomic<unsigned long long> g_launches{0};
 void sj_note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
@@ -634,14 +368,4 @@ cudaError_t sj_radix_sort_u32_u32(uint32_t *keys, uint32_t *vals, uint32_t *keys
                                   int bits, void *temp, int *resultInAlt, cudaStream_t s)
 {
     return radix_sort<uint32_t>(keys, vals, keysAlt, valsAlt, n, bits, temp, resultInAlt, s);
-}
-
-cudaError_t sj_hash_pairs(const int32_t *key, const int32_t *val, uint64_t m, unsigned long long *hashOut,
-                          cudaStream_t s)
-{
-    if (m == 0) return cudaSuccess;
-    uint64_t blocks = ceil_div(m, 256 * 16);
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    k_hash_pairs<<<(unsigned)blocks, 256, 0, s>>>(key, val, m, hashOut); sj_note_launch();
-    return cudaGetLastError();
 }

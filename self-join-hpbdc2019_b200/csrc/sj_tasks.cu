@@ -72,7 +72,7 @@ __device__ __forceinline__ uint64_t diag_evals(uint64_t s0, uint64_t s1, uint64_
 
 // Stream chunk (positions per task) of a tile of qc queries over a stream of
 // L positions.  policy 0: cost-proportional, the tile's predicted pairs per
-// task near pairsPerTask; 1: fixed 65536; 2: `workers` tasks share the
+// task near pairsPerTask; 1: about 5e5 evaluations; 2: `workers` tasks share the
 // stream (mode 8).  Never more positions than keep a task's worst case (every
 // evaluation a hit, both directions when symmetric) inside one batch.
 __device__ __forceinline__ uint32_t chunk_len(const sj_taskgen &g, float rate, uint32_t qc, uint32_t L, int workers)
@@ -83,7 +83,10 @@ __device__ __forceinline__ uint32_t chunk_len(const sj_taskgen &g, float rate, u
         s = (s + 31) / 32 * 32;
         if (s > 65536) s = 65536;
     } else if (g.policy == 1) {
-        s = 65536;
+        // the sampling estimate: few queries against whole streams, nothing
+        // recorded, so short tasks (about 5e5 evaluations) cost nothing and keep
+        // every CTA busy
+        s = min(16384u, max(512u, 524288u / qc));
     } else {
         const double perEval = fmax((double)rate, 1e-6) * (g.sym ? 2.0 : 1.0);
         double chunk = g.pairsPerTask / (perEval * (double)qc);
@@ -93,6 +96,9 @@ __device__ __forceinline__ uint32_t chunk_len(const sj_taskgen &g, float rate, u
         if (g.evalsPerTask > 0.0) chunk = fmin(chunk, g.evalsPerTask / (double)qc);
         s = (uint64_t)fmin(65536.0, fmax(256.0, chunk));
     }
+    // one warp runs a task of few queries: cut its stream so that none of them
+    // holds up a launch (8192 positions are about 0.1 ms of a warp)
+    if (qc <= SJ_SMALL_QUERIES) s = min(s, (uint64_t)min(8192u, SJ_SMALL_EVALS / qc));
     const uint64_t worst = g.cap / ((g.sym ? 2ULL : 1ULL) * (uint64_t)qc);
     if (s > worst) s = worst;
     s = (s / 32) * 32;
@@ -102,6 +108,7 @@ __device__ __forceinline__ uint32_t chunk_len(const sj_taskgen &g, float rate, u
 
 struct TileWork {
     uint32_t qBegin, qc, L, homeLen, sc, nChunks;
+    uint32_t occ;
     uint64_t evHome, evOther;   // evaluations against the home segment / the owned neighbours
 };
 
@@ -169,6 +176,7 @@ __device__ __forceinline__ TileWork tile_work(const sj_taskgen &g, uint32_t c, u
     const uint32_t nq = queries_of(g, c, occ);
     const uint32_t q0 = tile * g.tile;
     w.qBegin = aStart + q0;
+    w.occ = occ;
     w.qc = min(g.tile, nq - q0);
     w.homeLen = grp == 0 ? (g.sym ? occ - q0 : occ) : 0u;
     w.L = S + w.homeLen;
@@ -202,6 +210,11 @@ __device__ __forceinline__ uint32_t n_groups(const sj_taskgen &g, uint32_t c)
 {
     const uint32_t nSegAll = 1 + (g.nbrStart[c + 1] - g.nbrStart[c]);
     return (nSegAll + SJ_MAX_SEG - 1) / SJ_MAX_SEG;
+}
+
+__device__ __forceinline__ uint32_t n_queries(const sj_taskgen &g, uint32_t c)
+{
+    return queries_of(g, c, g.cellStart[c + 1] - g.cellStart[c]);
 }
 
 __device__ __forceinline__ uint32_t n_tiles(const sj_taskgen &g, uint32_t c)
@@ -423,7 +436,8 @@ __global__ void __launch_bounds__(256) k_tg_item_write(sj_taskgen g, const uint3
         k.segCount = min((uint32_t)SJ_MAX_SEG, nSegAll - segBase);
         k.sBegin = s0;
         k.sEnd = s1;
-        k.flags = (g.sym ? SJ_TASK_SYM : 0u) | (it.grp == 0 ? SJ_TASK_HOME : 0u);
+        k.flags = (g.sym ? SJ_TASK_SYM : 0u) | (it.grp == 0 ? SJ_TASK_HOME : 0u) |
+                  (g.sampleRate > 0.0f && n_queries(g, it.c) < w.occ ? SJ_TASK_SAMPLE : 0u);
         tasks[t] = k;
         pred[t] = (float)pairs_of(g, r, evH, evO, diag);
     }
@@ -441,6 +455,24 @@ __global__ void __launch_bounds__(256) k_tg_shard(const sj_task *__restrict__ in
     predOut[w] = predIn[i];
 }
 
+// ------------------------------------------------------- tasks by kernel --
+__global__ void __launch_bounds__(256) k_small_flags(const sj_task *__restrict__ tasks, uint32_t nt,
+                                                     uint32_t *__restrict__ flag)
+{
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < nt) flag[t] = tasks[t].qCount <= SJ_SMALL_QUERIES ? 1u : 0u;
+}
+
+__global__ void __launch_bounds__(256) k_task_lists(const uint32_t *__restrict__ pre, uint32_t nt,
+                                                    uint32_t *__restrict__ bigList, uint32_t *__restrict__ smallList)
+{
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nt) return;
+    const uint32_t p = pre[t];
+    if (pre[t + 1] != p) smallList[p] = t;
+    else bigList[t - p] = t;
+}
+
 // ------------------------------------------------------ record offsets ----
 constexpr int NC = 7;           // row masks, column masks, row offsets, candidate records, units,
                                 // planned pairs (rounded up, x (1 + alpha)), predicted pairs (rounded)
@@ -454,7 +486,7 @@ __device__ __forceinline__ void task_sizes(const sj_task &t, float pred, double 
     const bool sym = (t.flags & SJ_TASK_SYM) != 0;
     const uint64_t blocks = ((uint64_t)len + 31) / 32;
     const uint64_t groups = ((uint64_t)t.qCount + 31) / 32;
-    v[0] = blocks * t.qCount;
+    v[0] = blocks * t.qCount + sj_live_words((uint32_t)blocks, (uint32_t)groups);
     v[1] = sym ? blocks * groups * 32 : 0;
     v[2] = t.qCount;
     v[3] = len;
@@ -597,7 +629,7 @@ __global__ void __launch_bounds__(256) k_plan_next(const unsigned long long *__r
     uint32_t e = reach(planned, s, nt, cap);
     e = min(e, reach(maskOff, s, nt, maskLim));
     e = min(e, reach(colOff, s, nt, maskLim));
-    e = min(e, reach(unitOff, s, nt, 0xffffffffULL));
+    e = min(e, reach(unitOff, s, nt, 0xff000000ULL));   // the unit counter runs past the end by a few per warp
     next[s] = max(e, s + 1);
 }
 
@@ -617,17 +649,20 @@ __global__ void k_plan_chain(const uint32_t *__restrict__ next, uint32_t nt, uin
 
 // Per batch: predicted pairs and the sizes of its records.
 __global__ void __launch_bounds__(256) k_plan_stats(const uint32_t *__restrict__ start, uint32_t nb, OffOut off,
+                                                    const uint32_t *__restrict__ smallPre,
                                                     unsigned long long *__restrict__ stats)
 {
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nb) return;
     const uint32_t t0 = start[b], t1 = start[b + 1];
-    // [0] predicted pairs, [1] row-mask words, [2] column-mask words, [3] row offsets, [4] candidate records
-    stats[(uint64_t)b * 5 + 0] = off.p[6][t1] - off.p[6][t0];
-    stats[(uint64_t)b * 5 + 1] = off.p[0][t1] - off.p[0][t0];
-    stats[(uint64_t)b * 5 + 2] = off.p[1][t1] - off.p[1][t0];
-    stats[(uint64_t)b * 5 + 3] = off.p[2][t1] - off.p[2][t0];
-    stats[(uint64_t)b * 5 + 4] = off.p[3][t1] - off.p[3][t0];
+    // [0] predicted pairs, [1] row-mask words, [2] column-mask words, [3] row offsets, [4] candidate records,
+    // [5] small tasks
+    stats[(uint64_t)b * 6 + 0] = off.p[6][t1] - off.p[6][t0];
+    stats[(uint64_t)b * 6 + 1] = off.p[0][t1] - off.p[0][t0];
+    stats[(uint64_t)b * 6 + 2] = off.p[1][t1] - off.p[1][t0];
+    stats[(uint64_t)b * 6 + 3] = off.p[2][t1] - off.p[2][t0];
+    stats[(uint64_t)b * 6 + 4] = off.p[3][t1] - off.p[3][t0];
+    stats[(uint64_t)b * 6 + 5] = smallPre[t1] - smallPre[t0];
 }
 
 // ------------------------------------------------------------ estimates --
@@ -928,6 +963,19 @@ cudaError_t sj_tg_shard(const sj_task *in, const float *predIn, uint32_t nOut, u
     return cudaGetLastError();
 }
 
+cudaError_t sj_task_lists(const sj_task *tasks, uint32_t nt, uint32_t *pre, uint32_t *bigList, uint32_t *smallList,
+                          void *temp, cudaStream_t s)
+{
+    if (nt == 0) return cudaMemsetAsync(pre, 0, sizeof(uint32_t), s);
+    k_small_flags<<<blocks_for(nt, 256), 256, 0, s>>>(tasks, nt, pre);
+    sj_note_launch();
+    cudaError_t e = sj_exclusive_scan_u32(pre, pre, nt, temp, pre + nt, s);
+    if (e != cudaSuccess) return e;
+    k_task_lists<<<blocks_for(nt, 256), 256, 0, s>>>(pre, nt, bigList, smallList);
+    sj_note_launch();
+    return cudaGetLastError();
+}
+
 size_t sj_task_offsets_temp(uint32_t nt) { return (size_t)(blocks_for(nt ? nt : 1, OTILE)) * NC; }
 
 cudaError_t sj_task_offsets(const sj_task *tasks, const float *pred, uint32_t nt, double alpha,
@@ -966,12 +1014,12 @@ cudaError_t sj_plan_batches(unsigned long long *const off[7], uint32_t nt, unsig
 }
 
 cudaError_t sj_plan_stats(const uint32_t *start, uint32_t nb, unsigned long long *const off[7],
-                          unsigned long long *stats, cudaStream_t s)
+                          const uint32_t *smallPre, unsigned long long *stats, cudaStream_t s)
 {
     if (nb == 0) return cudaSuccess;
     OffOut o;
     for (int k = 0; k < NC; k++) o.p[k] = off[k];
-    k_plan_stats<<<blocks_for(nb, 256), 256, 0, s>>>(start, nb, o, stats);
+    k_plan_stats<<<blocks_for(nb, 256), 256, 0, s>>>(start, nb, o, smallPre, stats);
     sj_note_launch();
     return cudaGetLastError();
 }
