@@ -2,10 +2,20 @@
 //
 // The reference enumerates the clamped 3^k stencil per query POINT with a
 // binary search per neighbour (kernel.cu:1455-1534, 387-396).  Here the
-// stencil is enumerated once per non-empty CELL by a depth-first walk over the
+// stencil is enumerated once per non-empty CELL, by one warp, over the
 // linear-id ordering (dim k-1 most significant): each level narrows the range
-// of the sorted id array to the cells sharing the chosen coordinate prefix, so
-// empty sub-stencils are pruned early (sparse high-dimensional grids).
+// of the sorted id array to the cells sharing a coordinate prefix, so empty
+// sub-stencils drop out early (sparse high-dimensional grids).  The levels are
+// walked breadth first: eight prefixes at a time, four lanes each, the four
+// lanes searching the four bounds of the prefix's three children; the children
+// that hold cells are compacted, in id order, into the next level's list.  A
+// walk whose lowest TREE_DIMS dimensions are reached depth first (k > TREE_DIMS)
+// keeps the lists at 3^(TREE_DIMS-1) entries.
+// Bound: latency of the dependent searches (about 60 steps a cell at k = 6, which
+// the lanes of a warp take side by side).  One thread a cell, depth first with
+// six searches a prefix and its stack in local memory, took 10.3 ms a pass on
+// 466,982 cells at k = 6 (1M points, 16-D); this form's figures stand at
+// k_neighbours.
 //
 // Ownership rules decide which cell of an adjacent pair evaluates it:
 //   FULL      every neighbour (mode 3/7/9 semantics; one direction emitted)
@@ -28,144 +38,270 @@ __device__ __forceinline__ uint32_t lower_bound_u64(const uint64_t *__restrict__
     return lo;
 }
 
-__device__ __forceinline__ bool owns(int pattern, int k, const uint32_t *a, const int *off, unsigned long long myLid,
-                                     unsigned long long nbLid)
+// Offsets of a neighbour, two bits per dimension: 0, 1, 2 for -1, 0, +1.
+constexpr uint32_t CODE_HOME = 0x55555555u;   // every dimension 1
+
+// a: lane j holds the cell's coordinate of dimension j; odd: bit j set when it is odd
+__device__ __forceinline__ bool owns(int pattern, int k, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t odd,
+                                     uint32_t code, uint32_t c, uint32_t b)
 {
     switch (pattern) {
     case SJ_PAT_FULL:
         return true;
     case SJ_PAT_LID:
-        return nbLid > myLid;
+        return b > c;   // cells are sorted by linear id
     case SJ_PAT_UNICOMP: {
-        int d = k - 1;
-        while (d > 0 && off[d] == 0) d--;
-        return (a[d] & 1u) != 0;
+        const uint32_t diff = code ^ CODE_HOME;   // not home: some dimension differs
+        const int d = diff ? (31 - __clz(diff)) >> 1 : 0;
+        return (odd >> d) & 1u;
     }
     case SJ_PAT_BUNICOMP: {
+        const uint32_t v0 = a0 + (code & 3u) - 1u, v1 = a1 + ((code >> 2) & 3u) - 1u;
         if (k == 2) {
-            uint32_t v0 = a[0] + off[0], v1 = a[1] + off[1];
-            bool odd = ((a[0] + a[1]) & 1u) != 0;
-            if (odd) return (a[1] <= v1) && (a[0] != v0);
-            return (a[1] < v1) || (v1 < a[1] && v0 == a[0]);
+            if (((a0 + a1) & 1u) != 0) return (a1 <= v1) && (a0 != v0);
+            return (a1 < v1) || (v1 < a1 && v0 == a0);
         } else {
-            uint32_t v0 = a[0] + off[0], v1 = a[1] + off[1], v2 = a[2] + off[2];
-            bool odd = ((a[0] + a[1] + a[2]) & 1u) != 0;
-            if (odd)
-                return (a[0] != v0 && a[1] <= v1 && a[2] <= v2) || (a[0] == v0 && a[1] <= v1 && a[2] < v2) ||
-                       (a[1] < v1 && v2 < a[2]);
-            return (a[1] < v1 && a[2] <= v2) || (a[0] == v0 && v1 < a[1] && a[2] <= v2) ||
-                   (a[0] != v0 && a[1] < v1 && v2 < a[2]) || (a[1] == v1 && a[2] < v2);
+            const uint32_t v2 = a2 + ((code >> 4) & 3u) - 1u;
+            if (((a0 + a1 + a2) & 1u) != 0)
+                return (a0 != v0 && a1 <= v1 && a2 <= v2) || (a0 == v0 && a1 <= v1 && a2 < v2) ||
+                       (a1 < v1 && v2 < a2);
+            return (a1 < v1 && a2 <= v2) || (a0 == v0 && v1 < a1 && a2 <= v2) ||
+                   (a0 != v0 && a1 < v1 && v2 < a2) || (a1 == v1 && a2 < v2);
         }
     }
     }
     return false;
 }
 
+constexpr int TREE_DIMS = 6;                 // dimensions walked breadth first at most
+constexpr int NBR_THREADS = 128;
+
+constexpr int pow3(int e) { return e <= 0 ? 1 : 3 * pow3(e - 1); }
+
+// Prefixes of one level: their cells [lo, hi), the linear id of the first place,
+// the offsets.
+template <int N>
+struct TreeList {
+    uint32_t lo[N], hi[N], code[N];
+    unsigned long long base[N];
+};
+
+struct TreeRef {
+    uint32_t *lo, *hi, *code;
+    unsigned long long *base;
+};
+
+template <int N>
+__device__ __forceinline__ TreeRef ref(TreeList<N> &l)
+{
+    return {l.lo, l.hi, l.code, l.base};
+}
+
+// Two lists in turn: the last level's prefixes (3^(DIMS-1)) and the one's before.
+template <int DIMS>
+struct NbrSmem {
+    TreeList<pow3(DIMS - 1)> last;
+    TreeList<pow3(DIMS - 2)> before;
+    uint32_t hist[8];
+};
+
 // pass 0: count owned neighbours (out = counts), full-stencil candidates and
 //         features; pass 1: write owned neighbour cell indices (out = list).
-__global__ void __launch_bounds__(128) k_neighbours(const uint64_t *__restrict__ cellLid,
-                                                    const uint32_t *__restrict__ cellCoord,
-                                                    const uint32_t *__restrict__ cellStart, uint32_t nCells,
-                                                    sj_grid_dev g, int pattern,
-                                                    const uint32_t *__restrict__ nbrStart, uint32_t *__restrict__ out,
-                                                    uint64_t *__restrict__ candFull,
-                                                    unsigned long long *__restrict__ candTotal,
-                                                    float *__restrict__ feat, int pass)
+// Measured (both passes, one B200): 466,982 cells at k = 6 20.3 to 7 ms, 5,583 and
+// 6,980 cells at k = 6 3.7 to 0.1 ms.
+// GROUP lanes a cell: 32, or 8 where the tree has at most 27 leaves (two prefixes
+// at a time; a warp then has four cells).
+template <int DIMS, int GROUP>
+__global__ void __launch_bounds__(NBR_THREADS) k_neighbours(
+    const uint64_t *__restrict__ cellLid, const uint32_t *__restrict__ cellCoord,
+    const uint32_t *__restrict__ cellStart, uint32_t nCells, sj_grid_dev g, int pattern,
+    const uint32_t *__restrict__ nbrStart, uint32_t *__restrict__ out, uint64_t *__restrict__ candFull,
+    unsigned long long *__restrict__ candTotal, float *__restrict__ feat, int pass)
 {
-    uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int CELLS = NBR_THREADS / GROUP;
+    __shared__ NbrSmem<DIMS> smem[CELLS];
+    const uint32_t lane = threadIdx.x & (GROUP - 1);   // of the group
+    const uint32_t shift = threadIdx.x & 31u & ~(uint32_t)(GROUP - 1);
+    const uint32_t FULL = (GROUP == 32 ? 0xffffffffu : (1u << (GROUP & 31)) - 1u) << shift;   // the group's lanes
+    NbrSmem<DIMS> &sm = smem[threadIdx.x / GROUP];
+    const uint32_t c = blockIdx.x * CELLS + threadIdx.x / GROUP;
     if (c >= nCells) return;
+    const auto ballot = [&](bool v) { return __ballot_sync(FULL, v) >> shift; };
+    const auto shfl = [&](uint32_t v, int src) { return __shfl_sync(FULL, v, src, GROUP); };
     const int k = g.k;
-    uint32_t a[SJ_MAX_K];
-    for (int j = 0; j < k; j++) a[j] = cellCoord[(uint64_t)c * k + j];
-    const unsigned long long myLid = cellLid[c];
+    const uint32_t aj = (int)lane < k ? cellCoord[(uint64_t)c * k + lane] : 0u;   // lane j: coordinate j
+    const uint32_t odd = ballot(aj & 1u);
+    const uint32_t a0 = shfl(aj, 0), a1 = shfl(aj, 1), a2 = shfl(aj, 2);
     const uint32_t myOcc = cellStart[c + 1] - cellStart[c];
+    const uint32_t ltmask = (1u << lane) - 1u;
+    // bound q of the children of a prefix in dimension j: the first of its cells
+    // [lo, hi) at or after coordinate a_j - 1 + q (q = lane & 3)
+    const uint32_t q = lane & 3u;
+    auto bound = [&](int j, uint32_t a, unsigned long long base, uint32_t lo, uint32_t hi) -> uint32_t {
+        if (q == 0 && a == 0) return lo;   // no coordinate below 0
+        return lower_bound_u64(cellLid, lo, hi, base + ((unsigned long long)a + q - 1ULL) * g.mult[j]);
+    };
 
-    uint32_t lo[SJ_MAX_K + 1], hi[SJ_MAX_K + 1];
-    unsigned long long base[SJ_MAX_K + 1];
-    int t[SJ_MAX_K], off[SJ_MAX_K];
-    lo[k] = 0; hi[k] = nCells; base[k] = 0;
-    for (int j = 0; j < k; j++) off[j] = 0;
+    uint32_t owned = 0, writePos = pass == 1 ? nbrStart[c] : 0u;
+    unsigned long long stencilOcc = 0;            // this lane's part
+    float ownW = 0.0f, ownW1 = 0.0f, ownW2 = 0.0f;   // (as feat's f9, f13, f14; this lane's part)
+    if (feat && lane < 8) sm.hist[lane] = 0;
 
-    uint32_t owned = 0, writePos = (pass == 1) ? nbrStart[c] : 0u;
-    unsigned long long stencilOcc = 0;
-    uint32_t hist[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    // owned neighbours' occupancy weighted by the uniform-density hit
-    // probability of their offset class (all classes, classes 1 and 2)
-    float ownW = 0.0f, ownW1 = 0.0f, ownW2 = 0.0f;
-
-    int j = k - 1;
-    t[j] = 0;
-    while (j < k) {
-        if (t[j] == 3) {
-            j++;
-            if (j < k) t[j]++;
+    // prefixes of the dimensions above the tree, depth first (k > TREE_DIMS)
+    uint32_t dLo[SJ_MAX_K - TREE_DIMS + 1], dHi[SJ_MAX_K - TREE_DIMS + 1], dCode = 0;
+    unsigned long long dBase[SJ_MAX_K - TREE_DIMS + 1];
+    int t[SJ_MAX_K - TREE_DIMS + 1];
+    const int top = k > TREE_DIMS ? k - TREE_DIMS : 0;   // depth of the depth-first part
+    // the owned neighbours of the linear-id pattern come after the cell itself
+    dLo[0] = (pass == 1 && pattern == SJ_PAT_LID) ? c + 1 : 0u;
+    dHi[0] = nCells;
+    dBase[0] = 0;
+    t[0] = 0;
+    int depth = 0;
+    for (;;) {
+        if (depth < top) {
+            // the next child of the prefix at this depth
+            const int j = k - 1 - depth;
+            if (t[depth] == 3) {
+                if (depth == 0) break;
+                depth--;
+                t[depth]++;
+                continue;
+            }
+            const uint32_t a = shfl(aj, j);
+            const long long v = (long long)a + t[depth] - 1;
+            uint32_t l = 0, h = 0;
+            unsigned long long id = 0;
+            if (v >= 0 && v < (long long)g.nCells[j]) {
+                id = dBase[depth] + (unsigned long long)v * g.mult[j];
+                l = lower_bound_u64(cellLid, dLo[depth], dHi[depth], id);
+                h = lower_bound_u64(cellLid, l, dHi[depth], id + g.mult[j]);
+            }
+            if (l >= h) {
+                t[depth]++;
+                continue;
+            }
+            dCode = (dCode & ~(3u << (2 * j))) | ((uint32_t)t[depth] << (2 * j));
+            dLo[depth + 1] = l;
+            dHi[depth + 1] = h;
+            dBase[depth + 1] = id;
+            depth++;
+            t[depth] = 0;
             continue;
         }
-        long long v = (long long)a[j] + t[j] - 1;
-        if (v >= 0 && v < (long long)g.nCells[j]) {
-            unsigned long long idLo = base[j + 1] + (unsigned long long)v * g.mult[j];
-            unsigned long long idHi = idLo + g.mult[j];
-            uint32_t l = lower_bound_u64(cellLid, lo[j + 1], hi[j + 1], idLo);
-            uint32_t h = lower_bound_u64(cellLid, l, hi[j + 1], idHi);
-            if (l < h) {
-                off[j] = t[j] - 1;
-                if (j == 0) {
-                    // leaf: exactly one cell (mult[0] == 1)
-                    uint32_t b = l;
-                    uint32_t occ = cellStart[b + 1] - cellStart[b];
-                    stencilOcc += occ;
-                    bool home = (b == c);
-                    if (!home) {
-                        int bin = 31 - __clz(occ);
-                        hist[bin > 7 ? 7 : bin]++;
-                        if (owns(pattern, k, a, off, myLid, cellLid[b])) {
-                            if (pass == 1) out[writePos++] = b;
-                            owned++;
-                            if (feat) {
-                                int m = 0;
-                                for (int q = 0; q < k; q++) m += off[q] != 0;
-                                const float wo = (float)occ * g.offW[m];
+        // ---- the tree below the prefix, breadth first
+        uint32_t n = 1;
+        // dimension j reads `last` when j is even: dimension 0 has the longest list
+        const bool topEven = ((k - 1 - depth) & 1) == 0;
+        TreeRef L = topEven ? ref(sm.last) : ref(sm.before), N = topEven ? ref(sm.before) : ref(sm.last);
+        __syncwarp(FULL);
+        if (lane == 0) {
+            L.lo[0] = dLo[depth];
+            L.hi[0] = dHi[depth];
+            L.base[0] = dBase[depth];
+            L.code[0] = dCode;
+        }
+        __syncwarp(FULL);
+        for (int j = k - 1 - depth; j >= 0; j--) {
+            const uint32_t a = shfl(aj, j);
+            uint32_t made = 0;
+            for (uint32_t i0 = 0; i0 < n; i0 += GROUP / 4) {
+                const uint32_t i = i0 + (lane >> 2);
+                uint32_t r = 0, code = 0;
+                unsigned long long base = 0;
+                if (i < n) {
+                    base = L.base[i];
+                    code = L.code[i];
+                    r = bound(j, a, base, L.lo[i], L.hi[i]);
+                }
+                const uint32_t end = __shfl_down_sync(FULL, r, 1, GROUP);
+                const bool have = i < n && q < 3 && r < end && !(q == 0 && a == 0) && a + q - 1u < g.nCells[j];
+                const uint32_t m = ballot(have);
+                code |= q << (2 * j);
+                if (j > 0) {
+                    if (have) {
+                        const uint32_t at = made + __popc(m & ltmask);
+                        N.lo[at] = r;
+                        N.hi[at] = end;
+                        N.base[at] = base + ((unsigned long long)a + q - 1ULL) * g.mult[j];
+                        N.code[at] = code;
+                    }
+                    made += __popc(m);
+                    continue;
+                }
+                // leaves: one cell each (mult[0] == 1)
+                bool own = false;
+                if (have) {
+                    // dimensions at or above k count as unchanged
+                    const uint32_t full = k < 16 ? code | (CODE_HOME << (2 * k)) : code;
+                    const bool home = r == c;
+                    own = !home && owns(pattern, k, a0, a1, a2, odd, full, c, r);
+                    if (pass == 0) {
+                        const uint32_t occ = cellStart[r + 1] - cellStart[r];
+                        stencilOcc += occ;
+                        if (feat && !home) {
+                            const int bin = 31 - __clz(occ);
+                            atomicAdd(&sm.hist[bin > 7 ? 7 : bin], 1u);
+                            if (own) {
+                                const uint32_t diff = full ^ CODE_HOME;
+                                const int w = __popc((diff | (diff >> 1)) & CODE_HOME);   // dimensions that differ
+                                const float wo = (float)occ * g.offW[w];
                                 ownW += wo;
-                                if (m == 1) ownW1 += wo;
-                                else if (m == 2) ownW2 += wo;
+                                if (w == 1) ownW1 += wo;
+                                else if (w == 2) ownW2 += wo;
                             }
                         }
                     }
-                    t[0]++;
-                    continue;
                 }
-                lo[j] = l; hi[j] = h; base[j] = idLo;
-                j--;
-                t[j] = 0;
-                continue;
+                const uint32_t om = ballot(own);
+                if (pass == 1 && own) out[writePos + owned + __popc(om & ltmask)] = r;
+                owned += __popc(om);
             }
+            __syncwarp(FULL);
+            n = made;
+            const TreeRef x = L;
+            L = N;
+            N = x;
+            if (n == 0) break;
         }
-        t[j]++;
+        if (depth == 0) break;
+        depth--;
+        t[depth]++;
     }
-    if (pass == 0) {
+    if (pass != 0) return;
+#pragma unroll
+    for (int o = GROUP / 2; o > 0; o >>= 1) {
+        stencilOcc += __shfl_xor_sync(FULL, stencilOcc, o);
+        ownW += __shfl_xor_sync(FULL, ownW, o);
+        ownW1 += __shfl_xor_sync(FULL, ownW1, o);
+        ownW2 += __shfl_xor_sync(FULL, ownW2, o);
+    }
+    __syncwarp(FULL);
+    if (lane == 0) {
         out[c] = owned;
         candFull[c] = stencilOcc * (unsigned long long)myOcc;
         if (candTotal) atomicAdd(candTotal, stencilOcc * (unsigned long long)myOcc);
-        if (feat) {
-            float *f = feat + (uint64_t)c * SJ_NFEAT;
-            float nst = 1.0f;
-            for (int q = 0; q < k; q++) nst *= 3.0f;
-            nst -= 1.0f;
-            // occupancy, neighbour-occupancy histogram, eps / cell width,
-            // dimension; f9, f13, f14: the expected hits with the owned
-            // neighbours (all offset classes, face neighbours, edge neighbours)
-            // under a locally uniform density, log2(1 + occupancy x weighted sum)
-            const float o = (float)myOcc;
-            f[0] = log2f(1.0f + o);
-            for (int b = 0; b < 8; b++) f[1 + b] = (float)hist[b] / nst;
-            f[9] = log2f(1.0f + o * ownW);
-            f[10] = log2f(1.0f + (float)stencilOcc);
-            f[11] = 1.0f;                          // eps / cell width (cells are eps wide)
-            f[12] = (float)g.D / 16.0f;
-            f[13] = log2f(1.0f + o * ownW1);
-            f[14] = log2f(1.0f + o * ownW2);
-            f[15] = log2f((float)g.eps) / 8.0f;
-        }
+    }
+    for (uint32_t e = lane; feat && e < SJ_NFEAT; e += GROUP) {
+        float nst = 1.0f;
+        for (int d = 0; d < k; d++) nst *= 3.0f;
+        nst -= 1.0f;
+        // occupancy, neighbour-occupancy histogram, eps / cell width,
+        // dimension; f9, f13, f14: the expected hits with the owned
+        // neighbours (all offset classes, face neighbours, edge neighbours)
+        // under a locally uniform density, log2(1 + occupancy x weighted sum)
+        const float o = (float)myOcc;
+        float f;
+        if (e == 0) f = log2f(1.0f + o);
+        else if (e < 9) f = (float)sm.hist[e - 1] / nst;
+        else if (e == 9) f = log2f(1.0f + o * ownW);
+        else if (e == 10) f = log2f(1.0f + (float)stencilOcc);
+        else if (e == 11) f = 1.0f;                          // eps / cell width (cells are eps wide)
+        else if (e == 12) f = (float)g.D / 16.0f;
+        else if (e == 13) f = log2f(1.0f + o * ownW1);
+        else if (e == 14) f = log2f(1.0f + o * ownW2);
+        else f = log2f((float)g.eps) / 8.0f;
+        feat[(uint64_t)c * SJ_NFEAT + e] = f;
     }
 }
 
@@ -177,8 +313,21 @@ cudaError_t sj_launch_neighbours(const uint64_t *cellLid, const uint32_t *cellCo
                                  float *feat, int pass, cudaStream_t s)
 {
     if (nCells == 0) return cudaSuccess;
-    k_neighbours<<<(nCells + 127) / 128, 128, 0, s>>>(cellLid, cellCoord, cellStart, nCells, g, pattern, nbrStart,
-                                                      nbrCountOrCell, candFull, candTotal, feat, pass);
+    const auto go = [&](auto kernel, unsigned group) {
+        const unsigned cells = NBR_THREADS / group;
+        kernel<<<(nCells + cells - 1) / cells, NBR_THREADS, 0, s>>>(cellLid, cellCoord, cellStart, nCells, g, pattern,
+                                                                   nbrStart, nbrCountOrCell, candFull, candTotal,
+                                                                   feat, pass);
+    };
+    // the lists hold 3^(dimensions - 1) prefixes: small ones leave room for more warps
+    switch (g.k < TREE_DIMS ? g.k : TREE_DIMS) {
+    case 1:
+    case 2: go(k_neighbours<2, 8>, 8); break;
+    case 3: go(k_neighbours<3, 8>, 8); break;
+    case 4: go(k_neighbours<4, 32>, 32); break;
+    case 5: go(k_neighbours<5, 32>, 32); break;
+    default: go(k_neighbours<TREE_DIMS, 32>, 32); break;
+    }
     sj_note_launch();
     return cudaGetLastError();
 }

@@ -98,3 +98,20 @@ def test_device_delivery_keys_and_values():
     assert all(np.all(np.diff(k) >= 0) for k in ks)
     ck, cv = sjoin.canonical(np.concatenate(ks), np.concatenate(vs))
     assert np.array_equal(ck, ok) and np.array_equal(cv, ov)
+
+
+@pytest.mark.parametrize("dim,k", [(5, 5), (6, 6), (7, 7), (9, 9), (11, 10)])
+@pytest.mark.parametrize("mode", [3, 4, 6])
+def test_neighbour_walk_depths(dim, k, mode):
+    # up to six indexed dimensions are walked breadth first, the ones above depth first
+    r = np.random.default_rng(dim)
+    pts = np.clip(r.exponential(0.05, (900, dim)), 0.0, 1.0)
+    eps = 0.08
+    ix = oracle.OracleIndex(pts, eps, k)
+    ok, ov = ix.pairs()
+    with sjoin.SelfJoin(dim, eps, indexed_dims=k, mode=mode) as sj:
+        sj.set_points(pts)
+        sj.build_index()
+        st = sj.join(sjoin.DELIVER_NONE)
+    assert st.total_pairs == len(ok) and st.pair_hash == oracle.hash_pairs(ok, ov)
+    assert st.full_stencil_calcs == int(ix.cell_candidates().sum())
