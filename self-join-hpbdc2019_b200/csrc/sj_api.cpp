@@ -292,7 +292,11 @@ struct Ctx {
     uint64_t *csrRowPtr = nullptr;
     int32_t *csrCols = nullptr;
     uint64_t csrCap = 0;
+    bool csrDirect = false;    // rows not sized yet: a join of one batch emits straight into the caller's arrays
+    bool csrDone = false;      // ... and it did
+    uint64_t csrTotal = 0;
     DevBuf<uint32_t> csrFill;
+    DevBuf<unsigned long long> csrWide, csrScan;
     DevBuf<unsigned long long> batchTot;
     std::vector<cudaEvent_t> events;   // per-batch stage boundaries of the asynchronous phase
     PinBuf pinTotal, pinKey[2], pinVal[2], pinStart[2];
@@ -706,8 +710,10 @@ uint64_t mask_batch_words()
 // 0 cost-proportional stream chunks, 1 fixed chunks, 2 the mode-8 split by
 // thirds of the work (0 and 2 predict pairs from c.rate).  sampleRate > 0 builds the sampling
 // estimator's tasks.  With `shard`, keeps this context's shard of the list.
+// Without `rates` nothing is predicted and policy 0 cuts by evaluations alone.
 // Sets c.nTasks; the tasks are in c.dTasks, their predicted pairs in c.dTaskPred.
-sj_status build_tasks_dev(Ctx &c, bool sym, uint64_t cap, bool byCost, int policy, float sampleRate, bool shard)
+sj_status build_tasks_dev(Ctx &c, bool sym, uint64_t cap, bool byCost, int policy, float sampleRate, bool shard,
+                          bool rates = true)
 {
     const uint32_t nc = c.nCells;
     cudaStream_t s = c.s;
@@ -715,7 +721,7 @@ sj_status build_tasks_dev(Ctx &c, bool sym, uint64_t cap, bool byCost, int polic
     g.cellStart = c.cellStart.p;
     g.nbrStart = c.nbrStart.p;
     g.nbrCell = c.nbrCell.p;
-    g.rate = policy == 1 ? nullptr : c.rate.p;   // the split of policy 2 ignores it, its predictions do not
+    g.rate = policy == 1 || !rates ? nullptr : c.rate.p;   // the split of policy 2 ignores it, its predictions do not
     g.nCells = nc;
     g.tile = SJ_CTA * (uint32_t)sj_query_slots(c.g.Dp, c.p.precision == SJ_PREC_FP32_REFINE);
     g.cap = cap;
@@ -739,7 +745,7 @@ sj_status build_tasks_dev(Ctx &c, bool sym, uint64_t cap, bool byCost, int polic
     // the learned scheduler shares a cell's predicted neighbour pairs among its
     // tasks by the offset-class model its features use; the sampling estimate
     // keeps the cell's mean rate
-    g.spread = (c.rateLearned && policy != 1) ? 1 : 0;
+    g.spread = (c.rateLearned && policy != 1 && rates) ? 1 : 0;
     g.nbrPre = c.nbrPre.p;
     g.nbrPreW = c.nbrPreW.p;
     g.nbrWt = c.nbrWt.p;
@@ -962,7 +968,7 @@ sj_status estimate_rates(Ctx &c)
 }
 
 // ---------------------------------------------------------------- join --
-sj_status prepare_join(Ctx &c, int &pattern, bool &queue)
+sj_status prepare_join(Ctx &c, int &pattern, bool &queue, bool estimate = true)
 {
     if (!c.indexed) {
         set_error("index not built: call sj_build_index first");
@@ -975,7 +981,7 @@ sj_status prepare_join(Ctx &c, int &pattern, bool &queue)
     tm.start(c.s);
     CKS(build_neighbours(c, pattern));
     c.st.ms_tasks = tm.stop(c.s);
-    CKS(estimate_rates(c));
+    if (estimate) CKS(estimate_rates(c));
     return SJ_OK;
 }
 
@@ -1081,6 +1087,8 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
         CKS(plan_dev(c, cap, plan, maxes, predTotal));
         c.st.ms_tasks += tm.stop(c.s);
     }
+    // the rows of a table of several batches have to be sized first
+    if (delivery == SJ_DELIVER_CSR && c.csrDirect && plan.size() != 1) return SJ_OK;
     const uint32_t nt = c.nTasks;
     c.st.num_tasks = nt;
     c.st.estimated_pairs = predTotal;
@@ -1389,6 +1397,36 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
         CK(cudaStreamSynchronize(c.s));
         memcpy(&cnt, c.pinTotal.p, sizeof(cnt));
         noteErr(br, cnt);
+        if (c.csrDirect && delivery == SJ_DELIVER_CSR) {
+            // the join is this batch: its key runs are the table's rows
+            if (cnt > cap) return SJ_OK;   // more than one batch after all
+            CK(c.csrFill.ensure(n ? n : 1));
+            CK(sj_csr_rows(ksBuf, c.total.p, n, c.csrRowPtr, c.csrFill.p, c.s));
+            CK(c.dCellHits.ensure(c.nCells ? c.nCells : 1));
+            CK(sj_cell_hits(c.cellStart.p, c.ids.p, c.csrFill.p, c.nCells, c.dCellHits.p, c.s));
+            c.haveMeas = true;
+            c.csrDone = true;
+            c.csrTotal = cnt;
+            if (c.csrCap < cnt) {
+                CK(cudaStreamSynchronize(c.s));
+                set_error("cols holds %llu values, the table needs %llu", (unsigned long long)c.csrCap,
+                          (unsigned long long)cnt);
+                return SJ_ERR_BAD_INPUT;
+            }
+            a.outVal = c.csrCols;
+            a.outKey = nullptr;
+            a.capacity = std::min<uint64_t>(c.csrCap, 0xffffffffULL);
+            CK(cudaEventRecord(ev(3), c.s));
+            CK(cudaMemsetAsync(c.queueHead.p, 0, sizeof(uint32_t), c.s));
+            CK(sj_launch_emit(a, 0, c.numSM, 0, c.s));
+            CK(cudaEventRecord(ev(4), c.s));
+            CK(cudaEventRecord(ev(5), c.s));
+            iterFull.push_back(1);
+            iter++;
+            pairsTotal += cnt;
+            batches++;
+            continue;
+        }
         if (cnt > cap) {
             // estimate too low: re-plan the batch from the measured per-task
             // pairs (the scan already cleared the counts)
@@ -1545,14 +1583,16 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
     return result;
 }
 
-// Degrees only: count pass over all tasks, no capacity limit.
+// Degrees only: count pass over all tasks, no capacity limit and no batches, so
+// nothing to estimate.  They stay in c.keyCount (per point id).
 sj_status run_degrees(Ctx &c, uint32_t *degHost)
 {
     int pattern;
     bool queue;
-    CKS(prepare_join(c, pattern, queue));
+    CKS(prepare_join(c, pattern, queue, false));
+    c.st.ms_estimate = 0;
     const uint64_t n = c.n;
-    CKS(build_tasks_dev(c, pattern != SJ_PAT_FULL, 0xffffffffULL, false, 0, 0.0f, true));
+    CKS(build_tasks_dev(c, pattern != SJ_PAT_FULL, 0xffffffffULL, false, 0, 0.0f, true, false));
     const uint32_t nt = c.nTasks;
     CK(c.keyCount.ensure(n));
     CK(c.stat.ensure(8));
@@ -1586,16 +1626,13 @@ sj_status run_degrees(Ctx &c, uint32_t *degHost)
     CK(sj_cell_hits(c.cellStart.p, c.ids.p, c.keyCount.p, c.nCells, c.dCellHits.p, c.s));
     CK(c.sums.ensure(3));
     CK(sj_task_sums(c.dTaskEvals.p, c.dTaskRefined.p, nullptr, nullptr, nt, c.sums.p, nullptr, c.numSM, c.s));
-    std::vector<uint32_t> deg(n);
-    CK(cudaMemcpyAsync(deg.data(), c.keyCount.p, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, c.s));
-    unsigned long long sm[3];
+    if (degHost) CK(cudaMemcpyAsync(degHost, c.keyCount.p, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, c.s));
+    unsigned long long sm[3], hs[8];
     CK(cudaMemcpyAsync(sm, c.sums.p, sizeof(sm), cudaMemcpyDeviceToHost, c.s));
+    CK(cudaMemcpyAsync(hs, c.stat.p, sizeof(hs), cudaMemcpyDeviceToHost, c.s));
     CK(cudaStreamSynchronize(c.s));
-    if (degHost) memcpy(degHost, deg.data(), sizeof(uint32_t) * n);
     c.haveMeas = true;
-    uint64_t tot = 0;
-    for (uint64_t i = 0; i < n; i++) tot += deg[i];
-    c.st.total_pairs = tot;
+    c.st.total_pairs = hs[2];
     c.st.distance_calcs = sm[0];
     c.st.refined_pairs = sm[1];
     return SJ_OK;
@@ -1953,41 +1990,62 @@ sj_status sj_neighbor_csr(sj_ctx *ctx, uint64_t *rowPtr, int32_t *cols, uint64_t
             return SJ_ERR_BAD_INPUT;
         }
     }
-    const uint64_t n = c.n;
-    std::vector<uint32_t> deg(n);
-    CKS(run_degrees(c, deg.data()));
-    std::vector<uint64_t> hp(n + 1);
-    hp[0] = 0;
-    for (uint64_t i = 0; i < n; i++) hp[i + 1] = hp[i] + deg[i];
-    if (total) *total = hp[n];
-    CK(cudaMemcpyAsync(rowPtr, hp.data(), sizeof(uint64_t) * (n + 1), cudaMemcpyHostToDevice, c.s));
-    CK(cudaStreamSynchronize(c.s));
-    if (!cols) return SJ_OK;
-    if (cols_capacity < hp[n]) {
-        set_error("cols holds %llu values, the table needs %llu", (unsigned long long)cols_capacity,
-                  (unsigned long long)hp[n]);
-        return SJ_ERR_BAD_INPUT;
+    if (!c.indexed) {
+        set_error("index not built: call sj_build_index first");
+        return SJ_ERR_STATE;
     }
+    const uint64_t n = c.n;
     CK(c.csrFill.ensure(n ? n : 1));
-    CK(cudaMemsetAsync(c.csrFill.p, 0, sizeof(uint32_t) * (n ? n : 1), c.s));
     c.csrRowPtr = rowPtr;
     c.csrCols = cols;
     c.csrCap = cols_capacity;
-    const sj_status s = run_join(c, SJ_DELIVER_CSR, nullptr, nullptr);
-    c.csrRowPtr = nullptr;
-    c.csrCols = nullptr;
-    c.csrCap = 0;
-    if (s != SJ_OK) return s;
-    // every row must be exactly full
-    std::vector<uint32_t> fill(n);
-    if (n) CK(cudaMemcpyAsync(fill.data(), c.csrFill.p, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, c.s));
-    CK(cudaStreamSynchronize(c.s));
-    for (uint64_t i = 0; i < n; i++)
-        if (fill[i] != deg[i]) {
-            set_error("internal: neighbour-table row %llu holds %u of %u values", (unsigned long long)i, fill[i],
-                      deg[i]);
-            return SJ_ERR_INTERNAL;
+    c.csrDone = false;
+    struct Clear {
+        Ctx &c;
+        ~Clear()
+        {
+            c.csrRowPtr = nullptr;
+            c.csrCols = nullptr;
+            c.csrCap = 0;
+            c.csrDirect = false;
         }
+    } clear{c};
+    if (cols) {
+        // a join that is one batch needs no sizing pass: its key runs are the rows
+        c.csrDirect = true;
+        const sj_status s = run_join(c, SJ_DELIVER_CSR, nullptr, nullptr);
+        c.csrDirect = false;
+        if (c.csrDone && total) *total = c.csrTotal;
+        if (s != SJ_OK || c.csrDone) return s;
+    }
+    // row offsets from the degrees
+    CKS(run_degrees(c, nullptr));
+    CK(c.csrWide.ensure(n ? n : 1));
+    CK(c.csrScan.ensure(sj_scan64_temp(n)));
+    CK(sj_u32_to_u64(c.keyCount.p, n, c.csrWide.p, c.s));
+    CK(sj_exclusive_scan_u64(c.csrWide.p, reinterpret_cast<unsigned long long *>(rowPtr), n, c.csrScan.p, c.s));
+    uint64_t tot = 0;
+    CK(cudaMemcpyAsync(&tot, rowPtr + n, sizeof(tot), cudaMemcpyDeviceToHost, c.s));
+    CK(cudaStreamSynchronize(c.s));
+    if (total) *total = tot;
+    if (!cols) return SJ_OK;
+    if (cols_capacity < tot) {
+        set_error("cols holds %llu values, the table needs %llu", (unsigned long long)cols_capacity,
+                  (unsigned long long)tot);
+        return SJ_ERR_BAD_INPUT;
+    }
+    CK(cudaMemsetAsync(c.csrFill.p, 0, sizeof(uint32_t) * (n ? n : 1), c.s));
+    CKS(run_join(c, SJ_DELIVER_CSR, nullptr, nullptr));
+    // every row must be exactly full
+    CK(cudaMemsetAsync(c.stat.p + 7, 0, sizeof(unsigned long long), c.s));
+    CK(sj_csr_check(rowPtr, c.csrFill.p, n, c.stat.p + 7, c.s));
+    unsigned long long bad = 0;
+    CK(cudaMemcpyAsync(&bad, c.stat.p + 7, sizeof(bad), cudaMemcpyDeviceToHost, c.s));
+    CK(cudaStreamSynchronize(c.s));
+    if (bad) {
+        set_error("internal: neighbour-table row %llu is not full", bad - 1);
+        return SJ_ERR_INTERNAL;
+    }
     return SJ_OK;
 }
 

@@ -170,6 +170,14 @@ cudaError_t sj_radix_sort_u64_u32(uint64_t *keys, uint32_t *vals, uint64_t *keys
                                   uint64_t n, int bits, void *temp, int *resultInAlt, cudaStream_t s);
 cudaError_t sj_radix_sort_u32_u32(uint32_t *keys, uint32_t *vals, uint32_t *keysAlt, uint32_t *valsAlt,
                                   uint64_t n, int bits, void *temp, int *resultInAlt, cudaStream_t s);
+// table of one batch: rowPtr[n+1] and the rows' lengths from the key runs (as sj_csr_append's start / total)
+cudaError_t sj_csr_rows(const uint32_t *start, const uint32_t *total, uint64_t n, uint64_t *rowPtr, uint32_t *len,
+                        cudaStream_t s);
+// *bad (zero before) = 1 + a row whose fill differs from its length
+cudaError_t sj_csr_check(const uint64_t *rowPtr, const uint32_t *fill, uint64_t n, unsigned long long *bad,
+                         cudaStream_t s);
+// out[i] = in[i]
+cudaError_t sj_u32_to_u64(const uint32_t *in, uint64_t n, unsigned long long *out, cudaStream_t s);
 // out[i] = (float)in[i]
 cudaError_t sj_u32_to_f32(const uint32_t *in, uint64_t n, float *out, cudaStream_t s);
 // appends a batch (values vals, key runs start[0..n], start[n] = *total) to a

@@ -307,6 +307,36 @@ __global__ void __launch_bounds__(256) k_csr_append(const uint32_t *__restrict__
     }
 }
 
+// Rows of a table that is one batch: rowPtr[k] = start[k] (rowPtr[n] = *total) and
+// the rows' lengths.
+__global__ void __launch_bounds__(256) k_csr_rows(const uint32_t *__restrict__ start,
+                                                  const uint32_t *__restrict__ total, uint64_t n,
+                                                  uint64_t *__restrict__ rowPtr, uint32_t *__restrict__ len)
+{
+    const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const uint32_t s = start[k], e = k + 1 < n ? start[k + 1] : *total;
+    rowPtr[k] = s;
+    len[k] = e - s;
+    if (k + 1 == n) rowPtr[n] = e;
+}
+
+// *bad = 1 + a row whose fill is not its length (0: none)
+__global__ void __launch_bounds__(256) k_csr_check(const uint64_t *__restrict__ rowPtr,
+                                                   const uint32_t *__restrict__ fill, uint64_t n,
+                                                   unsigned long long *__restrict__ bad)
+{
+    const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n && rowPtr[k + 1] - rowPtr[k] != fill[k]) atomicMax(bad, (unsigned long long)k + 1ULL);
+}
+
+__global__ void __launch_bounds__(256) k_u32_to_u64(const uint32_t *__restrict__ in, uint64_t n,
+                                                    unsigned long long *__restrict__ out)
+{
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = in[i];
+}
+
 __global__ void __launch_bounds__(256) k_u32_to_f32(const uint32_t *__restrict__ in, uint64_t n,
                                                     float *__restrict__ out)
 {
@@ -315,6 +345,32 @@ __global__ void __launch_bounds__(256) k_u32_to_f32(const uint32_t *__restrict__
 }
 
 }  // namespace
+
+cudaError_t sj_csr_rows(const uint32_t *start, const uint32_t *total, uint64_t n, uint64_t *rowPtr, uint32_t *len,
+                        cudaStream_t s)
+{
+    if (n == 0) return cudaMemsetAsync(rowPtr, 0, sizeof(uint64_t), s);
+    k_csr_rows<<<(unsigned)ceil_div(n, 256), 256, 0, s>>>(start, total, n, rowPtr, len);
+    sj_note_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t sj_csr_check(const uint64_t *rowPtr, const uint32_t *fill, uint64_t n, unsigned long long *bad,
+                         cudaStream_t s)
+{
+    if (n == 0) return cudaSuccess;
+    k_csr_check<<<(unsigned)ceil_div(n, 256), 256, 0, s>>>(rowPtr, fill, n, bad);
+    sj_note_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t sj_u32_to_u64(const uint32_t *in, uint64_t n, unsigned long long *out, cudaStream_t s)
+{
+    if (n == 0) return cudaSuccess;
+    k_u32_to_u64<<<(unsigned)ceil_div(n, 256), 256, 0, s>>>(in, n, out);
+    sj_note_launch();
+    return cudaGetLastError();
+}
 
 cudaError_t sj_u32_to_f32(const uint32_t *in, uint64_t n, float *out, cudaStream_t s)
 {

@@ -115,3 +115,36 @@ def test_neighbour_walk_depths(dim, k, mode):
         st = sj.join(sjoin.DELIVER_NONE)
     assert st.total_pairs == len(ok) and st.pair_hash == oracle.hash_pairs(ok, ov)
     assert st.full_stencil_calcs == int(ix.cell_candidates().sum())
+
+
+@pytest.mark.parametrize("mode,prec", [(3, 0), (10, 1)])
+def test_csr_of_one_batch(mode, prec):
+    # one batch: the emission writes straight into the caller's rows
+    torch = pytest.importorskip("torch")
+    r = np.random.default_rng(9)
+    pts = r.random((5000, 3))
+    n, eps = len(pts), 0.07
+    ok, ov = oracle.OracleIndex(pts, eps, 3).pairs()
+    deg = np.bincount(ok, minlength=n)
+    with sjoin.SelfJoin(3, eps, mode=mode, precision=prec) as sj:
+        sj.set_points(pts)
+        sj.build_index()
+        row = torch.full((n + 1,), -1, dtype=torch.int64, device="cuda")
+        small = torch.full((len(ok) - 1,), -7, dtype=torch.int32, device="cuda")
+        with pytest.raises(sjoin.SJError) as e:
+            sj.neighbor_csr(row.data_ptr(), small.data_ptr(), len(ok) - 1)
+        assert e.value.status == sjoin.SJ_ERR_BAD_INPUT
+        assert bool((small == -7).all())          # refused before anything is written
+        want = np.concatenate([[0], np.cumsum(deg)])
+        assert np.array_equal(row.cpu().numpy(), want)   # the sizes are there all the same
+        cols = torch.full((len(ok) + 3,), -7, dtype=torch.int32, device="cuda")
+        assert sj.neighbor_csr(row.data_ptr(), cols.data_ptr(), len(ok) + 3) == len(ok)
+        st = sj.stats()
+        assert st.num_batches == 1 and st.total_pairs == len(ok)
+        _, hits, _ = sj.cell_features(with_hits=True)
+        assert int(hits.sum()) == len(ok)
+    c = cols.cpu().numpy()
+    assert np.all(c[len(ok):] == -7)
+    keys = np.repeat(np.arange(n), deg)
+    assert np.array_equal(c[:len(ok)][np.lexsort((c[:len(ok)], keys))], ov)
+    assert np.array_equal(row.cpu().numpy(), want)
