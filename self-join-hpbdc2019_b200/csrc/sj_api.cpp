@@ -110,26 +110,37 @@ struct PinBuf {
     }
 };
 
+// A stage's time: recorded as the stage is queued, read when someone asks (no
+// host round trip in between).
 struct Timer {
     cudaEvent_t a = nullptr, b = nullptr;
-    Timer()
-    {
-        cudaEventCreate(&a);
-        cudaEventCreate(&b);
-    }
+    bool pending = false;
     ~Timer()
     {
         if (a) cudaEventDestroy(a);
         if (b) cudaEventDestroy(b);
     }
-    void start(cudaStream_t s) { cudaEventRecord(a, s); }
-    float stop(cudaStream_t s)
+    void start(cudaStream_t s)
+    {
+        if (!a) {
+            cudaEventCreate(&a);
+            cudaEventCreate(&b);
+        }
+        pending = false;
+        cudaEventRecord(a, s);
+    }
+    void stop(cudaStream_t s)
     {
         cudaEventRecord(b, s);
+        pending = true;
+    }
+    float ms()
+    {
+        pending = false;
         cudaEventSynchronize(b);
-        float ms = 0;
-        cudaEventElapsedTime(&ms, a, b);
-        return ms;
+        float t = 0;
+        cudaEventElapsedTime(&t, a, b);
+        return t;
     }
 };
 
@@ -252,9 +263,9 @@ struct Ctx {
     DevBuf<float> dTaskPred, dTaskPredAlt;
     DevBuf<uint32_t> smallPre, bigList, smallList;   // the tasks by count-pass kernel (sj_task_lists)
     DevBuf<uint32_t> tgGroupCnt, tgGroupBase, tgGroupLen, tgPosCnt, tgOrder, tgOrderAlt, tgItemCnt, tgItemStart,
-        tgItemTasks, tgItemTaskStart, tgTot32;
-    DevBuf<uint64_t> tgKeys, tgKeysAlt;
-    DevBuf<unsigned long long> tgPosEv, tgEvExcl, tgTotals, tgScan64;
+        tgItemTasks, tgItemTaskStart;
+    DevBuf<uint32_t> tgKeys, tgKeysAlt;
+    DevBuf<unsigned long long> tgPosEv, tgEvExcl, tgScan64;
     DevBuf<uint8_t> tgWorkers;
     // per-task record offsets (exclusive prefix sums, nTasks + 1 each): row-mask
     // words, column-mask words, row offsets, candidate records, emission units,
@@ -262,7 +273,7 @@ struct Ctx {
     DevBuf<unsigned long long> off[7];
     DevBuf<unsigned long long> offTemp;
     // batch plan
-    DevBuf<uint32_t> planNext, planStart, planCount;
+    DevBuf<uint32_t> planNext, planStart;
     DevBuf<unsigned long long> planStats;
     // batch state
     DevBuf<uint32_t> keyCount, keyStart, keyStart2;
@@ -274,12 +285,16 @@ struct Ctx {
     std::vector<cudaEvent_t> syncEvents;   // stage boundaries of the synchronous phase
     DevBuf<uint8_t> scanTemp, scanTemp2;
     DevBuf<uint32_t> total;
-    DevBuf<unsigned long long> stat;   // see sj_join_args::stat
+    // small results side by side, so that one copy brings them to the host
+    DevBuf<unsigned long long> mail;
+    unsigned long long *stat() const { return mail.p; }                 // 8, see sj_join_args::stat
+    unsigned long long *sums() const { return mail.p + 8; }             // 4, see sj_task_sums
+    uint32_t *planCount() const { return reinterpret_cast<uint32_t *>(mail.p + 12); }
+    uint32_t *tgTot32() const { return reinterpret_cast<uint32_t *>(mail.p + 13); }   // work items, tasks by item
+    unsigned long long *tgTotals() const { return mail.p + 14; }        // 4, see sj_tg_cells
+    static constexpr size_t MAIL = 18;
     DevBuf<uint32_t> queueHead;
-    DevBuf<uint32_t> taskHits;
-    DevBuf<uint32_t> dTaskEvals, dTaskRefined;   // per task, written by the count pass
-    DevBuf<unsigned long long> sums;   // task sums: evaluations, refined, measured pairs
-    DevBuf<double> errSum;             // sum over tasks of |predicted - measured pairs|
+    DevBuf<uint32_t> taskRec;   // per task: measured pairs, evaluations, re-evaluations (of the count pass)
     // count-pass records for the emission pass: per task, row and column hit
     // masks, per-query row-run offsets and per-position candidate records
     DevBuf<uint32_t> masks, colMasks, rowRel, candId, candRel;
@@ -315,10 +330,89 @@ struct Ctx {
     DevBuf<float> sMlpOut;
     DevBuf<unsigned long long> sHits, sCands, sScalars;
     DevBuf<unsigned long long> dCellHits;   // measured hits per cell (after sj_degrees)
+    Timer tmUpload, tmIndex, tmNbr, tmTasks, tmEstimate, tmTotal;
     bool haveMeas = false;
     bool haveSamples = false;   // sHits / sCands hold the last sampling estimate's per-cell counts
+    bool spreadBuilt = false;   // nbrPre .. cellW belong to the current neighbour lists
+    bool mlpDirty = true;       // mlpW is newer than dMlpW
+    uint32_t expectTasks = 0;   // tasks per cell, summed; their count per item is compared with it later
+    bool checkTasks = false;
     sj_stats st{};
 };
+
+// Small results for the host go through one pinned page: read() queues a copy,
+// and the values are there after the stream is waited for.
+struct Readback {
+    static constexpr size_t BYTES = 65536;
+    Ctx &c;
+    size_t at = 0;
+    sj_status ready = SJ_OK;
+    explicit Readback(Ctx &ctx) : c(ctx)
+    {
+        if (c.pinTotal.ensure(BYTES) != cudaSuccess) ready = SJ_ERR_OOM;
+    }
+    template <typename T>
+    T *read(const T *dev, size_t count)
+    {
+        T *h = reinterpret_cast<T *>(static_cast<uint8_t *>(c.pinTotal.p) + at);
+        at += (count * sizeof(T) + 15) / 16 * 16;
+        if (at > BYTES) {
+            ready = SJ_ERR_INTERNAL;
+            set_error("internal: readback page too small");
+            return reinterpret_cast<T *>(c.pinTotal.p);
+        }
+        if (ready == SJ_OK && cudaMemcpyAsync(h, dev, count * sizeof(T), cudaMemcpyDeviceToHost, c.s) != cudaSuccess) {
+            ready = SJ_ERR_CUDA;
+            set_error("readback: %s", cudaGetErrorString(cudaGetLastError()));
+        }
+        return h;
+    }
+    sj_status wait()
+    {
+        if (ready != SJ_OK) return ready;
+        CK(cudaStreamSynchronize(c.s));
+        return SJ_OK;
+    }
+};
+
+// The context's small results as they were when the copy ran.
+struct Mail {
+    const unsigned long long *w;
+    explicit Mail(Readback &rb) : w(rb.read(rb.c.mail.p, Ctx::MAIL)) {}
+    unsigned long long word(size_t i) const { return w[i]; }
+    const unsigned long long *stat() const { return w; }
+    const unsigned long long *sums() const { return w + 8; }
+    double err() const
+    {
+        double e;
+        memcpy(&e, w + 11, sizeof(e));
+        return e;
+    }
+    uint32_t planCount() const { return (uint32_t)w[12]; }
+    uint32_t tot32(int i) const { return (uint32_t)(w[13] >> (32 * i)); }
+};
+
+// The stage times recorded so far go into the statistics.
+void settle(Ctx &c)
+{
+    if (c.tmUpload.pending) c.st.ms_upload = c.tmUpload.ms();
+    if (c.tmIndex.pending) c.st.ms_index = c.tmIndex.ms();
+    if (c.tmNbr.pending) c.st.ms_tasks = c.tmNbr.ms();
+    if (c.tmTasks.pending) c.st.ms_tasks += c.tmTasks.ms();
+    if (c.tmEstimate.pending) c.st.ms_estimate = c.tmEstimate.ms();
+    if (c.tmTotal.pending) c.st.ms_total = c.tmTotal.ms();
+}
+
+sj_status verify_tasks(Ctx &c, uint32_t perItem)
+{
+    if (!c.checkTasks) return SJ_OK;
+    c.checkTasks = false;
+    if (perItem != c.expectTasks) {
+        set_error("internal: task builder counted %u tasks per cell but %u per item", c.expectTasks, perItem);
+        return SJ_ERR_INTERNAL;
+    }
+    return SJ_OK;
+}
 
 
 sj_status check_params(const sj_params &p)
@@ -431,19 +525,25 @@ sj_status build_index(Ctx &c)
         set_error("no points: call sj_set_points or sj_import_csv first");
         return SJ_ERR_STATE;
     }
-    Timer tm;
-    tm.start(c.s);
+    c.tmIndex.start(c.s);
     const int D = c.p.gpunumdim, k = c.p.numindexeddim;
     const uint64_t n = c.n;
     // 1. min / max of every dimension
     DevBuf<double> &mm = c.sMinMax;
     CK(mm.ensure(2 * D + 1));
     CK(sj_launch_minmax(c.pts.p, n, D, mm.p, c.s));
-    std::vector<double> hmm(2 * D + 1);
-    CK(cudaMemcpyAsync(hmm.data(), mm.p, sizeof(double) * (2 * D + 1), cudaMemcpyDeviceToHost, c.s));
-    CK(cudaStreamSynchronize(c.s));
+    Readback rb(c);
+    const double *const raw = rb.read(mm.p, 2 * D + 1);
+    CKS(rb.wait());
+    double hmm[2 * SJ_MAX_DIM];
+    for (int j = 0; j < 2 * D; j++) {   // the kernel's order-preserving encoding
+        uint64_t u;
+        memcpy(&u, &raw[j], 8);
+        u = (u >> 63) ? (u & 0x7fffffffffffffffULL) : ~u;
+        memcpy(&hmm[j], &u, 8);
+    }
     uint64_t badBits;
-    memcpy(&badBits, &hmm[2 * D], 8);
+    memcpy(&badBits, &raw[2 * D], 8);
     if (badBits) {
         set_error("input contains non-finite coordinates");
         return SJ_ERR_BAD_INPUT;
@@ -504,9 +604,9 @@ sj_status build_index(Ctx &c)
     if (inAlt) c.ids.swap(valsAlt);
     CK(sj_launch_cell_flags(sk, n, flags.p, c.s));
     CK(sj_exclusive_scan_u32(flags.p, flags.p, n, tmp.p, nne.p, c.s));
-    uint32_t hn[2] = {0, 0};
-    CK(cudaMemcpyAsync(hn, nne.p, sizeof(hn), cudaMemcpyDeviceToHost, c.s));
-    CK(cudaStreamSynchronize(c.s));
+    Readback rn(c);
+    const uint32_t *const hn = rn.read(nne.p, 2);
+    CKS(rn.wait());
     if (hn[1]) {
         // a cell coordinate past its dimension's cell count would alias another cell
         set_error("internal: a point's cell coordinate lies outside the grid");
@@ -518,8 +618,6 @@ sj_status build_index(Ctx &c)
     CK(c.cellLid.ensure(nCells));
     CK(c.cellCoord.ensure((size_t)nCells * k));
     CK(sj_launch_cell_build(sk, flags.p, n, c.cellStart.p, c.cellLid.p, c.s));
-    uint32_t nn = (uint32_t)n;
-    CK(cudaMemcpyAsync(c.cellStart.p + nCells, &nn, sizeof(uint32_t), cudaMemcpyHostToDevice, c.s));
     CK(sj_launch_cell_coords(c.cellLid.p, nCells, g, c.cellCoord.p, c.s));
     // 4. the join's order inside the cells and the coordinates in that order
     c.jids = c.ids.p;
@@ -548,7 +646,7 @@ sj_status build_index(Ctx &c)
     c.haveMeas = false;
     c.st.n_points = (uint32_t)n;
     c.st.n_nonempty_cells = nCells;
-    c.st.ms_index = tm.stop(c.s);
+    c.tmIndex.stop(c.s);
     return SJ_OK;
 }
 
@@ -571,25 +669,36 @@ sj_status build_neighbours(Ctx &c, int pattern)
     CK(tmp.ensure(sj_scan_temp_bytes(nc)));
     CK(sj_exclusive_scan_u32(cnt.p, c.nbrStart.p, nc, tmp.p, c.nbrStart.p + nc, c.s));
     // the list length sizes the list; the candidate total is the work unit
+    Readback rb(c);
+    const uint32_t *const pTotal = rb.read(c.nbrStart.p + nc, 1);
+    const unsigned long long *const pFull = rb.read(sc.p, 1);
+    CKS(rb.wait());
     struct {
         uint32_t total;
         unsigned long long full;
-    } h{};
-    CK(cudaMemcpyAsync(&h.total, c.nbrStart.p + nc, sizeof(uint32_t), cudaMemcpyDeviceToHost, c.s));
-    CK(cudaMemcpyAsync(&h.full, sc.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c.s));
-    CK(cudaStreamSynchronize(c.s));
+    } h{*pTotal, *pFull};
     CK(c.nbrCell.ensure(h.total));
     CK(sj_launch_neighbours(c.cellLid.p, c.cellCoord.p, c.cellStart.p, nc, c.g, pattern, c.nbrStart.p, c.nbrCell.p,
                             nullptr, nullptr, nullptr, 1, c.s));
-    CK(c.nbrPre.ensure(h.total ? h.total : 1));
-    CK(c.nbrPreW.ensure(h.total ? h.total : 1));
-    CK(c.nbrWt.ensure(h.total ? h.total : 1));
-    CK(c.cellW.ensure(nc ? nc : 1));
-    CK(sj_nbr_spread(c.cellStart.p, c.cellCoord.p, c.nbrStart.p, c.nbrCell.p, nc, c.g, c.nbrPre.p, c.nbrPreW.p,
-                     c.nbrWt.p, c.cellW.p, c.s));
     c.nbrTotal = h.total;
     c.st.full_stencil_calcs = h.full;
     c.nbrPattern = pattern;
+    c.spreadBuilt = false;
+    return SJ_OK;
+}
+
+// The offset-class prefixes of the owned neighbours (the learned scheduler's).
+sj_status build_spread(Ctx &c)
+{
+    if (c.spreadBuilt) return SJ_OK;
+    const uint32_t nc = c.nCells, total = c.nbrTotal;
+    CK(c.nbrPre.ensure(total ? total : 1));
+    CK(c.nbrPreW.ensure(total ? total : 1));
+    CK(c.nbrWt.ensure(total ? total : 1));
+    CK(c.cellW.ensure(nc ? nc : 1));
+    CK(sj_nbr_spread(c.cellStart.p, c.cellCoord.p, c.nbrStart.p, c.nbrCell.p, nc, c.g, c.nbrPre.p, c.nbrPreW.p,
+                     c.nbrWt.p, c.cellW.p, c.s));
+    c.spreadBuilt = true;
     return SJ_OK;
 }
 
@@ -752,16 +861,15 @@ sj_status build_tasks_dev(Ctx &c, bool sym, uint64_t cap, bool byCost, int polic
     g.cellW = c.cellW.p;
     DevBuf<uint8_t> &tmp = c.sTemp;
     CK(tmp.ensure(std::max(sj_scan_temp_bytes(nc + 1), sj_radix_temp_bytes(nc))));
-    CK(c.tgTot32.ensure(2));
-    CK(c.tgTotals.ensure(4));
-    CK(cudaMemsetAsync(c.tgTotals.p, 0, sizeof(unsigned long long) * 4, s));
+    CK(c.mail.ensure(Ctx::MAIL));
+    CK(cudaMemsetAsync(c.tgTotals(), 0, sizeof(unsigned long long) * 4, s));
     // segment groups of every cell and their slots (at most one group per
     // SJ_MAX_SEG owned neighbours, plus one per cell)
     CK(c.tgGroupCnt.ensure(nc + 1));
     CK(c.tgGroupBase.ensure(nc + 1));
     CK(c.tgGroupLen.ensure((size_t)nc + c.nbrTotal / SJ_MAX_SEG + 1));
     CK(sj_tg_groups(g, c.tgGroupCnt.p, s));
-    CK(sj_exclusive_scan_u32(c.tgGroupCnt.p, c.tgGroupBase.p, nc, tmp.p, c.tgTot32.p, s));
+    CK(sj_exclusive_scan_u32(c.tgGroupCnt.p, c.tgGroupBase.p, nc, tmp.p, c.tgTot32(), s));
     g.groupBase = c.tgGroupBase.p;
     g.groupLen = c.tgGroupLen.p;
     // per-cell task counts, evaluations and cost keys, in cell order
@@ -771,63 +879,58 @@ sj_status build_tasks_dev(Ctx &c, bool sym, uint64_t cap, bool byCost, int polic
     CK(c.tgKeysAlt.ensure(nc));
     CK(c.tgOrder.ensure(nc));
     CK(c.tgOrderAlt.ensure(nc));
-    CK(sj_tg_cells(g, nullptr, nullptr, c.tgPosCnt.p, c.tgPosEv.p,
-                   byCost ? reinterpret_cast<unsigned long long *>(c.tgKeys.p) : nullptr, c.tgTotals.p, s));
-    CK(sj_iota_u32(c.tgOrder.p, nc, s));
+    CK(sj_tg_cells(g, nullptr, nullptr, c.tgPosCnt.p, c.tgPosEv.p, byCost ? c.tgKeys.p : nullptr, c.tgOrder.p,
+                   c.tgTotals(), s));
     uint32_t *order = c.tgOrder.p;
     if (byCost && nc > 1) {
         int inAlt = 0;
-        CK(sj_radix_sort_u64_u32(c.tgKeys.p, c.tgOrder.p, c.tgKeysAlt.p, c.tgOrderAlt.p, nc, 64, tmp.p, &inAlt, s));
+        CK(sj_radix_sort_u32_u32(c.tgKeys.p, c.tgOrder.p, c.tgKeysAlt.p, c.tgOrderAlt.p, nc, 16, tmp.p, &inAlt, s));
         if (inAlt) order = c.tgOrderAlt.p;
     }
     const uint8_t *workers = nullptr;
-    unsigned long long *taskTotal = c.tgTotals.p;
+    unsigned long long *taskTotal = c.tgTotals();
     if (policy == 2) {
         // mode 8: the evaluations in cost order decide each cell's third of the
         // work, which sets how many tasks share each of its tiles' streams
-        CK(sj_tg_cells(g, order, nullptr, c.tgPosCnt.p, c.tgPosEv.p, nullptr, c.tgTotals.p + 2, s));
+        CK(sj_tg_cells(g, order, nullptr, c.tgPosCnt.p, c.tgPosEv.p, nullptr, nullptr, c.tgTotals() + 2, s));
         CK(c.tgEvExcl.ensure(nc + 1));
         CK(c.tgScan64.ensure(sj_scan64_temp(nc)));
         CK(sj_exclusive_scan_u64(c.tgPosEv.p, c.tgEvExcl.p, nc, c.tgScan64.p, s));
         CK(c.tgWorkers.ensure(nc));
         CK(sj_tg_thirds(c.tgEvExcl.p, nc, c.tgWorkers.p, s));
         workers = c.tgWorkers.p;
-        CK(cudaMemsetAsync(c.tgTotals.p + 2, 0, sizeof(unsigned long long) * 2, s));
-        CK(sj_tg_cells(g, order, workers, c.tgPosCnt.p, c.tgPosEv.p, nullptr, c.tgTotals.p + 2, s));
-        taskTotal = c.tgTotals.p + 2;
+        CK(cudaMemsetAsync(c.tgTotals() + 2, 0, sizeof(unsigned long long) * 2, s));
+        CK(sj_tg_cells(g, order, workers, c.tgPosCnt.p, c.tgPosEv.p, nullptr, nullptr, c.tgTotals() + 2, s));
+        taskTotal = c.tgTotals() + 2;
     }
     // work items in order and their first tasks
     CK(c.tgItemCnt.ensure(nc + 1));
     CK(c.tgItemStart.ensure(nc + 1));
     CK(sj_tg_item_counts(g, order, c.tgItemCnt.p, s));
-    CK(sj_exclusive_scan_u32(c.tgItemCnt.p, c.tgItemStart.p, nc, tmp.p, c.tgTot32.p, s));
-    struct {
-        uint32_t items;
-        unsigned long long tasks;
-    } h{};
-    CK(cudaMemcpyAsync(&h.items, c.tgTot32.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(&h.tasks, taskTotal, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    if (h.tasks > 0xffffffffULL) {
-        set_error("%llu tasks exceed the 32-bit task index", h.tasks);
+    CK(sj_exclusive_scan_u32(c.tgItemCnt.p, c.tgItemStart.p, nc, tmp.p, c.tgTot32(), s));
+    Readback rb(c);
+    const Mail m(rb);
+    CKS(rb.wait());
+    CKS(verify_tasks(c, m.tot32(1)));   // the previous list's
+    const unsigned long long tasksTotal = m.word(taskTotal - c.mail.p);
+    if (tasksTotal > 0xffffffffULL) {
+        set_error("%llu tasks exceed the 32-bit task index", tasksTotal);
         return SJ_ERR_BAD_INPUT;
     }
-    const uint32_t nItems = h.items;
+    const uint32_t nItems = m.tot32(0);
+    uint32_t nt = (uint32_t)tasksTotal;
     CK(c.tgItemTasks.ensure((size_t)nItems + 1));
     CK(c.tgItemTaskStart.ensure((size_t)nItems + 1));
     CK(tmp.ensure(sj_scan_temp_bytes((uint64_t)nItems + 1)));
     CK(sj_tg_item_tasks(g, order, workers, c.tgItemStart.p, nItems, c.tgItemTasks.p, s));
-    CK(sj_exclusive_scan_u32(c.tgItemTasks.p, c.tgItemTaskStart.p, nItems, tmp.p, c.tgTot32.p + 1, s));
-    uint32_t nt = 0;
-    CK(cudaMemcpyAsync(&nt, c.tgTot32.p + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    if (nt != h.tasks) {
-        set_error("internal: task builder counted %llu tasks per cell but %u per item", h.tasks, nt);
-        return SJ_ERR_INTERNAL;
-    }
+    CK(sj_exclusive_scan_u32(c.tgItemTasks.p, c.tgItemTaskStart.p, nItems, tmp.p, c.tgTot32() + 1, s));
+    // the items' total is compared with the cells' at the next readback
+    c.expectTasks = nt;
+    c.checkTasks = true;
     CK(c.dTasks.ensure(nt ? nt : 1));
     CK(c.dTaskPred.ensure(nt ? nt : 1));
-    CK(sj_tg_item_write(g, order, workers, c.tgItemStart.p, nItems, c.tgItemTaskStart.p, c.dTasks.p, c.dTaskPred.p, s));
+    CK(sj_tg_item_write(g, order, workers, c.tgItemStart.p, nItems, c.tgItemTaskStart.p, c.dTasks.p, nt, c.dTaskPred.p,
+                        s));
     if (shard && c.p.shard_count > 1) {
         // round-robin over the ordered list: each shard gets a similar cost mix
         const uint32_t idx = (uint32_t)c.p.shard_index, cnt = (uint32_t)c.p.shard_count;
@@ -874,33 +977,35 @@ sj_status plan_dev(Ctx &c, uint64_t cap, std::vector<BatchRange> &plan, uint64_t
     for (int k = 0; k < 4; k++) maxes[k] = 1;
     unsigned long long *off[7];
     for (int k = 0; k < 7; k++) off[k] = c.off[k].p;
+    constexpr uint32_t FAST = 128;   // batches that come with the first readback
     CK(c.planNext.ensure(nt ? nt : 1));
     CK(c.planStart.ensure((size_t)nt + 1));
-    CK(c.planCount.ensure(1));
-    CK(sj_plan_batches(off, nt, cap, mask_batch_words(), c.planNext.p, c.planStart.p, c.planCount.p, c.s));
-    struct {
-        uint32_t nb;
-        unsigned long long pred;
-    } h{};
-    CK(cudaMemcpyAsync(&h.nb, c.planCount.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, c.s));
-    CK(cudaMemcpyAsync(&h.pred, c.off[6].p + nt, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c.s));
-    CK(cudaStreamSynchronize(c.s));
-    predTotal = (double)h.pred;
-    const uint32_t nb = h.nb;
-    if (nb == 0) return SJ_OK;
-    CK(c.planStats.ensure((size_t)nb * 6));
-    CK(sj_plan_stats(c.planStart.p, nb, off, c.smallPre.p, c.planStats.p, c.s));
-    std::vector<uint32_t> start(nb + 1);
-    std::vector<unsigned long long> st((size_t)nb * 6);
-    CK(cudaMemcpyAsync(start.data(), c.planStart.p, sizeof(uint32_t) * (nb + 1), cudaMemcpyDeviceToHost, c.s));
-    CK(cudaMemcpyAsync(st.data(), c.planStats.p, sizeof(unsigned long long) * nb * 6, cudaMemcpyDeviceToHost, c.s));
-    CK(cudaStreamSynchronize(c.s));
+    CK(c.planStats.ensure(1 + FAST * 8));
+    CK(sj_plan_batches(off, nt, cap, mask_batch_words(), c.planNext.p, c.planStart.p, c.planCount(), c.s));
+    CK(sj_plan_stats(c.planStart.p, FAST, c.planCount(), nt, off, c.smallPre.p, c.planStats.p, c.s));
+    Readback rb(c);
+    const Mail m(rb);
+    const unsigned long long *st = rb.read(c.planStats.p, 1 + FAST * 8);
+    CKS(rb.wait());
+    CKS(verify_tasks(c, m.tot32(1)));
+    predTotal = (double)st[0];
+    const uint32_t nb = m.planCount();
+    std::vector<unsigned long long> all;
+    if (nb > FAST) {
+        CK(c.planStats.ensure(1 + (size_t)nb * 8));
+        CK(sj_plan_stats(c.planStart.p, nb, c.planCount(), nt, off, c.smallPre.p, c.planStats.p, c.s));
+        all.resize(1 + (size_t)nb * 8);
+        CK(cudaMemcpyAsync(all.data(), c.planStats.p, sizeof(unsigned long long) * all.size(), cudaMemcpyDeviceToHost,
+                           c.s));
+        CK(cudaStreamSynchronize(c.s));
+        st = all.data();
+    }
     plan.resize(nb);
     for (uint32_t b = 0; b < nb; b++) {
-        const unsigned long long *const sb = &st[(size_t)b * 6];
-        const uint32_t n = start[b + 1] - start[b], small = (uint32_t)sb[5];
-        plan[b] = {start[b], start[b + 1], (double)sb[0], 0, n - small, small};
-        for (int k = 0; k < 4; k++) maxes[k] = std::max<uint64_t>(maxes[k], sb[1 + k]);
+        const unsigned long long *const sb = st + 1 + (size_t)b * 8;
+        const uint32_t t0 = (uint32_t)sb[0], t1 = (uint32_t)sb[1], small = (uint32_t)sb[7];
+        plan[b] = {t0, t1, (double)sb[2], 0, t1 - t0 - small, small};
+        for (int k = 0; k < 4; k++) maxes[k] = std::max<uint64_t>(maxes[k], sb[3 + k]);
     }
     return SJ_OK;
 }
@@ -914,15 +1019,17 @@ sj_status plan_dev(Ctx &c, uint64_t cap, std::vector<BatchRange> &plan, uint64_t
 // sampled point take the global rate.
 sj_status estimate_rates(Ctx &c)
 {
-    Timer tm;
-    tm.start(c.s);
+    c.tmEstimate.start(c.s);
     const uint32_t nc = c.nCells;
     CK(c.rate.ensure(2 * (size_t)(nc ? nc : 1)));
     if (c.p.scheduler == SJ_SCHED_LEARNED && !c.mlpW.empty()) {
         DevBuf<float> &out = c.sMlpOut;
         CK(out.ensure((size_t)nc * SJ_NOUT));
         CK(c.dMlpW.ensure(SJ_MLP_NPARAM));
-        CK(cudaMemcpyAsync(c.dMlpW.p, c.mlpW.data(), sizeof(float) * SJ_MLP_NPARAM, cudaMemcpyHostToDevice, c.s));
+        if (c.mlpDirty)
+            CK(cudaMemcpyAsync(c.dMlpW.p, c.mlpW.data(), sizeof(float) * SJ_MLP_NPARAM, cudaMemcpyHostToDevice, c.s));
+        c.mlpDirty = false;
+        CKS(build_spread(c));
         CK(sj_launch_mlp_infer(c.feat.p, nc, c.dMlpW.p, out.p, c.s));
         CK(sj_rates_mlp(out.p, c.cellStart.p, c.nbrStart.p, c.nbrCell.p, nc, c.rate.p, c.s));
         c.haveSamples = false;
@@ -932,11 +1039,9 @@ sj_status estimate_rates(Ctx &c)
         CKS(build_tasks_dev(c, false, 0xffffffffULL, false, 1, (float)c.p.sample_rate, false));
         const uint32_t nt = c.nTasks;
         CK(c.keyCount.ensure(c.n));
-        CK(c.stat.ensure(8));
+        CK(c.mail.ensure(Ctx::MAIL));
         CK(c.queueHead.ensure(2));
-        CK(c.taskHits.ensure(nt ? nt : 1));
-        CK(c.dTaskEvals.ensure(nt ? nt : 1));
-        CK(c.dTaskRefined.ensure(nt ? nt : 1));
+        CK(c.taskRec.ensure(3 * (size_t)(nt ? nt : 1)));
         sj_join_args a;
         join_args_base(c, a);
         a.tasks = c.dTasks.p;
@@ -945,10 +1050,10 @@ sj_status estimate_rates(Ctx &c)
         a.smallList = c.smallList.p;
         a.queueHead = c.queueHead.p;
         a.keyCount = c.keyCount.p;   // cleared before the join's first count pass
-        a.stat = c.stat.p;
-        a.taskHits = c.taskHits.p;
-        a.taskEvals = c.dTaskEvals.p;
-        a.taskRefined = c.dTaskRefined.p;
+        a.stat = c.stat();
+        a.taskHits = c.taskRec.p;
+        a.taskEvals = c.taskRec.p + nt;
+        a.taskRefined = c.taskRec.p + 2 * (size_t)nt;
         const FilterBounds fb = filter_bounds(c);
         a.margin = fb.margin;
         a.delta = fb.delta;
@@ -959,11 +1064,11 @@ sj_status estimate_rates(Ctx &c)
         CK(c.sHits.ensure(2 * (size_t)(nc ? nc : 1)));
         CK(c.sCands.ensure(2 * (size_t)(nc ? nc : 1)));
         CK(c.sScalars.ensure(2 + sj_sample_totals_len()));
-        CK(sj_sample_rates(c.dTasks.p, nt, c.taskHits.p, c.dTaskEvals.p, c.cellStart.p, c.sHits.p, c.sCands.p,
+        CK(sj_sample_rates(c.dTasks.p, nt, c.taskRec.p, c.taskRec.p + nt, c.cellStart.p, c.sHits.p, c.sCands.p,
                            c.sScalars.p + 2, nc, c.rate.p, c.s));
         c.haveSamples = true;
     }
-    c.st.ms_estimate = tm.stop(c.s);
+    c.tmEstimate.stop(c.s);
     return SJ_OK;
 }
 
@@ -977,10 +1082,10 @@ sj_status prepare_join(Ctx &c, int &pattern, bool &queue, bool estimate = true)
     pattern = pattern_of_mode(c.p.search_mode);
     // work queue: modes 9/10, or any mode when work is ordered by workload
     queue = (c.p.search_mode == 8 || c.p.search_mode == 9 || c.p.search_mode == 10 || c.p.sort_by_workload != 0);
-    Timer tm;
-    tm.start(c.s);
+    c.tmNbr.start(c.s);
     CKS(build_neighbours(c, pattern));
-    c.st.ms_tasks = tm.stop(c.s);
+    c.tmNbr.stop(c.s);
+    c.tmTasks.pending = false;
     if (estimate) CKS(estimate_rates(c));
     return SJ_OK;
 }
@@ -1013,7 +1118,10 @@ void expand_keys_host(const uint32_t *start, uint64_t n, uint64_t cnt, int32_t *
 {
     if (cnt == 0) return;
     static const bool avx2 = __builtin_cpu_supports("avx2");
-#pragma omp parallel
+    // a thread per half a million keys: with every core in the team, a small batch
+    // waits for whichever core is busy with something else
+    const int team = (int)std::min<uint64_t>((uint64_t)omp_get_max_threads(), 1 + cnt / (1u << 19));
+#pragma omp parallel num_threads(team)
     {
 #pragma omp for schedule(static)
         for (int64_t k = 0; k < (int64_t)n; k++) {
@@ -1064,8 +1172,7 @@ constexpr int SJ_DELIVER_CSR = 100;
 sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
 {
     const unsigned long long launches0 = sj_launch_total();
-    Timer total;
-    total.start(c.s);
+    c.tmTotal.start(c.s);
     int pattern;
     bool queue;
     CKS(prepare_join(c, pattern, queue));
@@ -1076,8 +1183,7 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
     uint64_t maxes[4];
     double predTotal = 0;
     {
-        Timer tm;
-        tm.start(c.s);
+        c.tmTasks.start(c.s);
         const bool byCost = c.p.sort_by_workload || c.p.search_mode == 7 || c.p.search_mode == 8 ||
                             c.p.search_mode == 9 || c.p.search_mode == 10;
         // mode 8 splits each tile's stream by the third of the work its cell is in
@@ -1085,7 +1191,7 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
         CKS(task_offsets_dev(c));
         // greedy batch plan on predicted pairs (and on hit-mask words)
         CKS(plan_dev(c, cap, plan, maxes, predTotal));
-        c.st.ms_tasks += tm.stop(c.s);
+        c.tmTasks.stop(c.s);
     }
     // the rows of a table of several batches have to be sized first
     if (delivery == SJ_DELIVER_CSR && c.csrDirect && plan.size() != 1) return SJ_OK;
@@ -1097,16 +1203,13 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
     CK(c.keyStart.ensure(n));
     CK(c.scanTemp.ensure(sj_scan_temp_bytes(n)));
     CK(c.total.ensure(1));
-    CK(c.stat.ensure(8));
+    CK(c.mail.ensure(Ctx::MAIL));
     CK(c.queueHead.ensure(2));
-    CK(c.taskHits.ensure(nt ? nt : 1));
-    CK(cudaMemsetAsync(c.taskHits.p, 0, sizeof(uint32_t) * (nt ? nt : 1), c.s));
-    CK(c.dTaskEvals.ensure(nt ? nt : 1));
-    CK(c.dTaskRefined.ensure(nt ? nt : 1));
-    CK(cudaMemsetAsync(c.dTaskEvals.p, 0, sizeof(uint32_t) * (nt ? nt : 1), c.s));
-    CK(cudaMemsetAsync(c.dTaskRefined.p, 0, sizeof(uint32_t) * (nt ? nt : 1), c.s));
-    CK(c.pinTotal.ensure(64));
-    CK(cudaMemsetAsync(c.stat.p, 0, sizeof(unsigned long long) * 8, c.s));
+    CK(c.taskRec.ensure(3 * (size_t)(nt ? nt : 1)));   // hits, evaluations, re-evaluations
+    CK(cudaMemsetAsync(c.taskRec.p, 0, sizeof(uint32_t) * 3 * (nt ? nt : 1), c.s));
+    uint32_t *const taskHits = c.taskRec.p, *const taskEvals = taskHits + nt, *const taskRefined = taskEvals + nt;
+    CK(c.pinTotal.ensure(Readback::BYTES));
+    CK(cudaMemsetAsync(c.stat(), 0, sizeof(unsigned long long) * 8, c.s));
 
     std::reverse(plan.begin(), plan.end());   // used as a stack
     CK(c.masks.ensure(maxMaskWords));
@@ -1127,10 +1230,10 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
     a.outKey = c.outKey.p;
     a.outVal = c.outVal.p;
     a.capacity = cap;
-    a.stat = c.stat.p;
-    a.taskHits = c.taskHits.p;
-    a.taskEvals = c.dTaskEvals.p;
-    a.taskRefined = c.dTaskRefined.p;
+    a.stat = c.stat();
+    a.taskHits = taskHits;
+    a.taskEvals = taskEvals;
+    a.taskRefined = taskRefined;
     a.masks = c.masks.p;
     a.maskOff = reinterpret_cast<const uint64_t *>(c.off[0].p);
     a.colMasks = c.colMasks.p;
@@ -1148,7 +1251,46 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
         a.pruneT = fb.pruneT;
     }
 
-    std::vector<uint32_t> hTaskHits(nt);
+    // measured pairs of tasks [t0, t1), for a batch that has to be re-planned
+    std::vector<uint32_t> hTaskHits;
+    auto readHits = [&](uint32_t t0, uint32_t t1) -> sj_status {
+        hTaskHits.resize(nt);
+        CK(cudaMemcpyAsync(hTaskHits.data() + t0, taskHits + t0, sizeof(uint32_t) * (t1 - t0), cudaMemcpyDeviceToHost,
+                           c.s));
+        CK(cudaStreamSynchronize(c.s));
+        return SJ_OK;
+    };
+    // the statistics of the tasks counted so far, queued behind them: evaluations,
+    // FP32 re-evaluations, measured pairs, the predictions' error, and the
+    // estimator-free reference count -- the same greedy plan with every task's
+    // measured pairs in place of its prediction (it rewrites the planned pairs
+    // among the record offsets, which nothing reads after the plan)
+    CK(c.exactPred.ensure(nt ? nt : 1));
+    auto queueSums = [&]() -> sj_status {
+        CK(sj_task_sums(taskEvals, taskRefined, taskHits, c.dTaskPred.p, nt, c.sums(), c.numSM, c.s));
+        if (nt) {
+            CK(sj_u32_to_f32(taskHits, nt, c.exactPred.p, c.s));
+            unsigned long long *o[7];
+            for (int k = 0; k < 7; k++) o[k] = c.off[k].p;
+            CK(sj_task_offsets(c.dTasks.p, c.exactPred.p, nt, c.p.alpha, c.offTemp.p, o, c.s));
+            CK(sj_plan_batches(o, nt, cap, mask_batch_words(), c.planNext.p, c.planStart.p, c.planCount(), c.s));
+        }
+        return SJ_OK;
+    };
+    struct {
+        unsigned long long stat[8], sums[3];
+        double err;
+        uint32_t exact;
+    } fin{};
+    auto takeSums = [&](Readback &rb) {   // queues the copies; `fin` is filled by the function it returns, after the wait
+        const Mail m(rb);
+        return [=, &fin]() {
+            memcpy(fin.stat, m.stat(), sizeof(fin.stat));
+            memcpy(fin.sums, m.sums(), sizeof(fin.sums));
+            fin.err = m.err();
+            fin.exact = m.planCount();
+        };
+    };
     uint64_t pairsTotal = 0, batches = 0, retries = 0, errBatches = 0;
     double relErrSum = 0;
     float msCount = 0, msScan = 0, msFill = 0, msDeliver = 0;
@@ -1272,11 +1414,21 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
             CK(cudaEventRecord(e[5], sB));
         }
         if (pipe) CK(cudaStreamWaitEvent(sA, ev[EV * (nplan - 1) + 5], 0));
+        // totals and statistics in one wait
+        CKS(queueSums());
         std::vector<unsigned long long> tot(nplan);
-        CK(cudaMemcpyAsync(tot.data(), c.batchTot.p, sizeof(unsigned long long) * nplan, cudaMemcpyDeviceToHost,
-                           c.s));
-        CK(cudaMemcpyAsync(hTaskHits.data(), c.taskHits.p, sizeof(uint32_t) * nt, cudaMemcpyDeviceToHost, c.s));
-        CK(cudaStreamSynchronize(c.s));
+        {
+            Readback rb(c);
+            const auto take = takeSums(rb);
+            const bool small = nplan <= 4096;
+            const unsigned long long *pt = small ? rb.read(c.batchTot.p, nplan) : nullptr;
+            if (!small)
+                CK(cudaMemcpyAsync(tot.data(), c.batchTot.p, sizeof(unsigned long long) * nplan,
+                                   cudaMemcpyDeviceToHost, c.s));
+            CKS(rb.wait());
+            take();
+            if (small) tot.assign(pt, pt + nplan);
+        }
         // stage times per batch (with two streams, each stage's time includes
         // sharing the device with the other stream's stage)
         for (size_t i = 0; i < nplan; i++) {
@@ -1323,6 +1475,7 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
                 // the count pass measured every task's pairs: re-plan this
                 // batch's tasks exactly against the capacity (the next round
                 // grows the buffers up to it; no task's worst case exceeds it)
+                CKS(readHits(br.t0, br.t1));
                 CKS(replan_exact(br, hTaskHits, cap, redo));
                 retries++;
                 continue;
@@ -1351,9 +1504,11 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
     auto finishPending = [&]() -> sj_status {
         if (!pend.live) return SJ_OK;
         pend.live = false;
-        CK(cudaEventSynchronize(c.evVals[pend.sel]));
         int32_t *hk = (int32_t *)c.pinKey[pend.sel].p, *hv = (int32_t *)c.pinVal[pend.sel].p;
+        // the run offsets come first: the keys are written while the values are copied
+        CK(cudaEventSynchronize(c.evStart[pend.sel]));
         expand_keys_host((const uint32_t *)c.pinStart[pend.sel].p, n, pend.cnt, hk);
+        CK(cudaEventSynchronize(c.evVals[pend.sel]));
         if (cb) {
             sj_batch b{pend.index, pend.cnt, hk, hv, 0};
             if (cb(&b, user)) return SJ_ERR_ABORTED;
@@ -1392,8 +1547,6 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
         CK(cudaEventRecord(ev(2), c.s));
         unsigned long long cnt = 0;
         CK(cudaMemcpyAsync(c.pinTotal.p, slot, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c.s));
-        CK(cudaMemcpyAsync(hTaskHits.data() + br.t0, c.taskHits.p + br.t0, sizeof(uint32_t) * (br.t1 - br.t0),
-                           cudaMemcpyDeviceToHost, c.s));
         CK(cudaStreamSynchronize(c.s));
         memcpy(&cnt, c.pinTotal.p, sizeof(cnt));
         noteErr(br, cnt);
@@ -1431,6 +1584,7 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
             // estimate too low: re-plan the batch from the measured per-task
             // pairs (the scan already cleared the counts)
             std::vector<BatchRange> parts;
+            CKS(readHits(br.t0, br.t1));
             CKS(replan_exact(br, hTaskHits, cap, parts));
             for (size_t i = parts.size(); i-- > 0;) stack.push_back(parts[i]);
             retries++;
@@ -1465,7 +1619,7 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
         CK(cudaEventRecord(ev(4), c.s));
         if (delivery == SJ_DELIVER_CSR) {
             CK(sj_csr_append(ksBuf, c.total.p, n, valBuf, c.csrRowPtr, c.csrFill.p, c.csrCols, c.csrCap,
-                             c.stat.p + 7, c.s));
+                             c.stat() + 7, c.s));
         } else if (delivery == SJ_DELIVER_DEVICE && cb) {
             CK(cudaStreamSynchronize(c.s));
             sj_batch b{batches, cnt, c.outKey.p, valBuf, 1};
@@ -1511,8 +1665,14 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
             if (ps != SJ_ERR_ABORTED) return ps;
         }
     }
-    CK(cudaStreamSynchronize(c.cs));
-    CK(cudaStreamSynchronize(c.s));
+    if (delivery != SJ_DELIVER_NONE) {
+        CKS(queueSums());
+        Readback rb(c);
+        const auto take = takeSums(rb);
+        CK(cudaStreamSynchronize(c.cs));
+        CKS(rb.wait());
+        take();
+    }
     for (size_t i = 0; i < iter; i++) {
         float t01 = 0, t12 = 0, t34 = 0, t45 = 0;
         cudaEvent_t *e = c.syncEvents.data() + 6 * i;
@@ -1527,47 +1687,18 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
             msDeliver += t45;
         }
     }
-    unsigned long long hs[8];
-    CK(cudaMemcpyAsync(hs, c.stat.p, sizeof(hs), cudaMemcpyDeviceToHost, c.s));
-    CK(cudaStreamSynchronize(c.s));
-    if (hs[3] || hs[6] || hs[7]) {
-        set_error(hs[3]   ? "internal: the emission exceeded the counted capacity"
-                  : hs[6] ? "internal: the emission met a count-pass record out of range"
+    if (fin.stat[3] || fin.stat[6] || fin.stat[7]) {
+        set_error(fin.stat[3]   ? "internal: the emission exceeded the counted capacity"
+                  : fin.stat[6] ? "internal: the emission met a count-pass record out of range"
                           : "internal: a neighbour-table row received more values than its degree");
         return SJ_ERR_INTERNAL;
     }
-    {
-        // evaluations, FP32 re-evaluations, measured pairs and the predicted
-        // pairs' error, summed over the tasks on the device
-        CK(c.sums.ensure(3));
-        CK(c.errSum.ensure(1));
-        CK(sj_task_sums(c.dTaskEvals.p, c.dTaskRefined.p, c.taskHits.p, c.dTaskPred.p, nt, c.sums.p, c.errSum.p,
-                        c.numSM, c.s));
-        unsigned long long sm[3];
-        double err = 0;
-        CK(cudaMemcpyAsync(sm, c.sums.p, sizeof(sm), cudaMemcpyDeviceToHost, c.s));
-        CK(cudaMemcpyAsync(&err, c.errSum.p, sizeof(double), cudaMemcpyDeviceToHost, c.s));
-        CK(cudaStreamSynchronize(c.s));
-        c.st.distance_calcs = sm[0];
-        c.st.refined_pairs = sm[1];
-        c.st.estimator_task_rel_err = sm[2] ? err / (double)sm[2] : 0.0;
-    }
-    if (nt) {
-        // the estimator-free reference count: the same greedy plan with every
-        // task's measured pairs in place of its prediction
-        CK(c.exactPred.ensure(nt));
-        CK(sj_u32_to_f32(c.taskHits.p, nt, c.exactPred.p, c.s));
-        unsigned long long *o[7];
-        for (int k = 0; k < 7; k++) o[k] = c.off[k].p;
-        CK(sj_task_offsets(c.dTasks.p, c.exactPred.p, nt, c.p.alpha, c.offTemp.p, o, c.s));
-        CK(sj_plan_batches(o, nt, cap, mask_batch_words(), c.planNext.p, c.planStart.p, c.planCount.p, c.s));
-        uint32_t nbExact = 0;
-        CK(cudaMemcpyAsync(&nbExact, c.planCount.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, c.s));
-        CK(cudaStreamSynchronize(c.s));
-        c.st.exact_plan_batches = nbExact;
-    }
+    c.st.distance_calcs = fin.sums[0];
+    c.st.refined_pairs = fin.sums[1];
+    c.st.estimator_task_rel_err = fin.sums[2] ? fin.err / (double)fin.sums[2] : 0.0;
+    if (nt) c.st.exact_plan_batches = fin.exact;
     c.st.total_pairs = pairsTotal;
-    c.st.pair_hash = hs[4];
+    c.st.pair_hash = fin.stat[4];
     c.st.num_batches = batches;
     c.st.overflow_retries = retries;
     c.st.estimator_mean_abs_rel_err = errBatches ? relErrSum / (double)errBatches : 0.0;
@@ -1578,7 +1709,7 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
     c.st.ms_join_kernels = msCount + msFill;
     c.st.ms_fill_kernel = msFill;
     c.st.ms_expand = 0;   // the emission writes the keys
-    c.st.ms_total = total.stop(c.s);
+    c.tmTotal.stop(c.s);   // read by sj_get_stats
     c.st.kernel_launches = sj_launch_total() - launches0;
     return result;
 }
@@ -1595,10 +1726,10 @@ sj_status run_degrees(Ctx &c, uint32_t *degHost)
     CKS(build_tasks_dev(c, pattern != SJ_PAT_FULL, 0xffffffffULL, false, 0, 0.0f, true, false));
     const uint32_t nt = c.nTasks;
     CK(c.keyCount.ensure(n));
-    CK(c.stat.ensure(8));
+    CK(c.mail.ensure(Ctx::MAIL));
     CK(c.queueHead.ensure(2));
     CK(cudaMemsetAsync(c.keyCount.p, 0, sizeof(uint32_t) * n, c.s));
-    CK(cudaMemsetAsync(c.stat.p, 0, sizeof(unsigned long long) * 8, c.s));
+    CK(cudaMemsetAsync(c.stat(), 0, sizeof(unsigned long long) * 8, c.s));
     sj_join_args a;
     join_args_base(c, a);
     a.tasks = c.dTasks.p;
@@ -1607,34 +1738,32 @@ sj_status run_degrees(Ctx &c, uint32_t *degHost)
     a.smallList = c.smallList.p;
     a.queueHead = c.queueHead.p;
     a.keyCount = c.keyCount.p;
-    a.stat = c.stat.p;
+    a.stat = c.stat();
     {
         const FilterBounds fb = filter_bounds(c);
         a.margin = fb.margin;
         a.delta = fb.delta;
         a.pruneT = fb.pruneT;
     }
-    CK(c.dTaskEvals.ensure(nt ? nt : 1));
-    CK(c.dTaskRefined.ensure(nt ? nt : 1));
-    a.taskEvals = c.dTaskEvals.p;
-    a.taskRefined = c.dTaskRefined.p;
+    CK(c.taskRec.ensure(2 * (size_t)(nt ? nt : 1)));
+    a.taskEvals = c.taskRec.p;
+    a.taskRefined = c.taskRec.p + nt;
     a.taskBegin = 0;
     a.taskEnd = nt;
     CKS(run_count(c, a, true, nt, nt));
     // per-cell measured hits (the sum of the cell's points' degrees)
     CK(c.dCellHits.ensure(c.nCells ? c.nCells : 1));
     CK(sj_cell_hits(c.cellStart.p, c.ids.p, c.keyCount.p, c.nCells, c.dCellHits.p, c.s));
-    CK(c.sums.ensure(3));
-    CK(sj_task_sums(c.dTaskEvals.p, c.dTaskRefined.p, nullptr, nullptr, nt, c.sums.p, nullptr, c.numSM, c.s));
+    CK(sj_task_sums(a.taskEvals, a.taskRefined, nullptr, nullptr, nt, c.sums(), c.numSM, c.s));
     if (degHost) CK(cudaMemcpyAsync(degHost, c.keyCount.p, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, c.s));
-    unsigned long long sm[3], hs[8];
-    CK(cudaMemcpyAsync(sm, c.sums.p, sizeof(sm), cudaMemcpyDeviceToHost, c.s));
-    CK(cudaMemcpyAsync(hs, c.stat.p, sizeof(hs), cudaMemcpyDeviceToHost, c.s));
-    CK(cudaStreamSynchronize(c.s));
+    Readback rb(c);
+    const Mail m(rb);
+    CKS(rb.wait());
+    CKS(verify_tasks(c, m.tot32(1)));
     c.haveMeas = true;
-    c.st.total_pairs = hs[2];
-    c.st.distance_calcs = sm[0];
-    c.st.refined_pairs = sm[1];
+    c.st.total_pairs = m.stat()[2];
+    c.st.distance_calcs = m.sums()[0];
+    c.st.refined_pairs = m.sums()[1];
     return SJ_OK;
 }
 
@@ -1648,8 +1777,7 @@ sj_status set_points(Ctx &c, const double *pts, uint64_t n, int onDevice)
         set_error("point count must be in 1..2^31-1 (got %llu)", (unsigned long long)n);
         return SJ_ERR_BAD_INPUT;
     }
-    Timer tm;
-    tm.start(c.s);
+    c.tmUpload.start(c.s);
     const size_t bytes = n * (size_t)c.p.gpunumdim * sizeof(double);
     CK(c.pts.ensure(n * (size_t)c.p.gpunumdim));
     CK(cudaMemcpyAsync(c.pts.p, pts, bytes, onDevice ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c.s));
@@ -1658,7 +1786,9 @@ sj_status set_points(Ctx &c, const double *pts, uint64_t n, int onDevice)
     c.indexed = false;
     c.nbrPattern = -1;
     c.st = sj_stats{};
-    c.st.ms_upload = tm.stop(c.s);
+    c.tmIndex.pending = c.tmNbr.pending = c.tmTasks.pending = c.tmEstimate.pending = c.tmTotal.pending = false;
+    c.tmUpload.stop(c.s);
+    CK(cudaStreamSynchronize(c.s));   // the caller's buffer is free again
     return SJ_OK;
 }
 
@@ -1824,6 +1954,7 @@ sj_status sj_index_sizes(sj_ctx *ctx, uint32_t *n_nonempty, uint32_t *n_mask_ele
         return SJ_ERR_STATE;
     }
     CKS(bind(c));
+    CK(cudaStreamSynchronize(c.s));
     if (n_nonempty) *n_nonempty = c.nCells;
     if (total_cells) *total_cells = c.st.total_cells;
     if (n_mask_elems) {
@@ -1851,6 +1982,7 @@ sj_status sj_index_export(sj_ctx *ctx, unsigned int *indexLookupArr, sj_grid *gr
         return SJ_ERR_STATE;
     }
     CKS(bind(c));
+    CK(cudaStreamSynchronize(c.s));
     const uint32_t nc = c.nCells;
     if (indexLookupArr) CK(cudaMemcpy(indexLookupArr, c.ids.p, sizeof(uint32_t) * c.n, cudaMemcpyDeviceToHost));
     if (grid) {
@@ -2037,10 +2169,10 @@ sj_status sj_neighbor_csr(sj_ctx *ctx, uint64_t *rowPtr, int32_t *cols, uint64_t
     CK(cudaMemsetAsync(c.csrFill.p, 0, sizeof(uint32_t) * (n ? n : 1), c.s));
     CKS(run_join(c, SJ_DELIVER_CSR, nullptr, nullptr));
     // every row must be exactly full
-    CK(cudaMemsetAsync(c.stat.p + 7, 0, sizeof(unsigned long long), c.s));
-    CK(sj_csr_check(rowPtr, c.csrFill.p, n, c.stat.p + 7, c.s));
+    CK(cudaMemsetAsync(c.stat() + 7, 0, sizeof(unsigned long long), c.s));
+    CK(sj_csr_check(rowPtr, c.csrFill.p, n, c.stat() + 7, c.s));
     unsigned long long bad = 0;
-    CK(cudaMemcpyAsync(&bad, c.stat.p + 7, sizeof(bad), cudaMemcpyDeviceToHost, c.s));
+    CK(cudaMemcpyAsync(&bad, c.stat() + 7, sizeof(bad), cudaMemcpyDeviceToHost, c.s));
     CK(cudaStreamSynchronize(c.s));
     if (bad) {
         set_error("internal: neighbour-table row %llu is not full", bad - 1);
@@ -2061,7 +2193,10 @@ sj_status sj_get_stream(sj_ctx *ctx, void **stream)
 sj_status sj_get_stats(sj_ctx *ctx, sj_stats *st)
 {
     if (!ctx || !st) return SJ_ERR_BAD_INPUT;
-    *st = as_ctx(ctx)->st;
+    Ctx &c = *as_ctx(ctx);
+    CKS(bind(c));
+    settle(c);
+    *st = c.st;
     return SJ_OK;
 }
 
@@ -2075,6 +2210,7 @@ sj_status sj_set_estimator_weights(sj_ctx *ctx, const float *w, uint32_t count)
     }
     Ctx &c = *as_ctx(ctx);
     c.mlpW.assign(w, w + count);
+    c.mlpDirty = true;
     return SJ_OK;
 }
 
@@ -2106,6 +2242,7 @@ sj_status sj_cell_features(sj_ctx *ctx, float *feat, double *hits, double *calcs
     }
     CKS(bind(c));
     if (c.nbrPattern < 0) CKS(build_neighbours(c, pattern_of_mode(c.p.search_mode)));
+    CK(cudaStreamSynchronize(c.s));
     if (feat)
         CK(cudaMemcpy(feat, c.feat.p, sizeof(float) * (size_t)c.nCells * SJ_NFEAT, cudaMemcpyDeviceToHost));
     const uint32_t nc = c.nCells;

@@ -65,16 +65,6 @@ __global__ void k_minmax_init(unsigned long long *mm, int D)
     if (j == 0) mm[2 * D] = 0ULL;
 }
 
-__global__ void k_minmax_decode(unsigned long long *mm, int D)
-{
-    int j = threadIdx.x;
-    if (j < 2 * D) {
-        unsigned long long u = mm[j];
-        u = (u >> 63) ? (u & 0x7fffffffffffffffULL) : ~u;
-        mm[j] = u;  // now the raw bits of the double
-    }
-}
-
 // Cell coordinate (main.cu:294, kernel.cu:1457) and linear id (main.cu:423-439).
 // A coordinate at or past its dimension's cell count (which the grid's eps
 // margins rule out up to rounding) would alias another cell's linear id: it
@@ -118,6 +108,7 @@ __global__ void __launch_bounds__(256) k_cell_build(const uint64_t *__restrict__
         cellStart[c] = (uint32_t)i;
         cellLid[c] = keys[i];
     }
+    if (i + 1 == n) cellStart[excl[i] + (start ? 1u : 0u)] = (uint32_t)n;   // the end of the last cell
 }
 
 __global__ void __launch_bounds__(256) k_gather(const double *__restrict__ pts, const uint32_t *__restrict__ ids,
@@ -245,7 +236,6 @@ cudaError_t sj_launch_minmax(const double *pts, uint64_t n, int D, double *minma
     if (blocks > 148 * 8) blocks = 148 * 8;
     if (blocks == 0) blocks = 1;
     k_minmax<<<(unsigned)blocks, 256, 0, s>>>(pts, n, D, mm); sj_note_launch();
-    k_minmax_decode<<<1, 64, 0, s>>>(mm, D); sj_note_launch();
     return cudaGetLastError();
 }
 

@@ -247,9 +247,8 @@ cudaError_t sj_nbr_spread(const uint32_t *cellStart, const uint32_t *cellCoord, 
                           const uint32_t *nbrCell, uint32_t nCells, const sj_grid_dev &g, uint32_t *nbrPre,
                           double *nbrPreW, float *nbrWt, double *cellW, cudaStream_t s);
 cudaError_t sj_tg_cells(const sj_taskgen &g, const uint32_t *order, const uint8_t *workersAt, uint32_t *posCnt,
-                        unsigned long long *posEv, unsigned long long *costKey, unsigned long long *totals,
+                        unsigned long long *posEv, uint32_t *costKey, uint32_t *iota, unsigned long long *totals,
                         cudaStream_t s);
-cudaError_t sj_iota_u32(uint32_t *v, uint32_t n, cudaStream_t s);
 // mode 8: workers per position from the exclusive prefix of the evaluations
 // in cost order (evExcl[n] = total): 16, 8 or 2 by third of the work
 cudaError_t sj_tg_thirds(const unsigned long long *evExcl, uint32_t n, uint8_t *workers, cudaStream_t s);
@@ -258,7 +257,7 @@ cudaError_t sj_tg_item_tasks(const sj_taskgen &g, const uint32_t *order, const u
                              const uint32_t *itemStart, uint32_t nItems, uint32_t *itemTasks, cudaStream_t s);
 cudaError_t sj_tg_item_write(const sj_taskgen &g, const uint32_t *order, const uint8_t *workersAt,
                              const uint32_t *itemStart, uint32_t nItems, const uint32_t *itemTaskStart,
-                             sj_task *tasks, float *pred, cudaStream_t s);
+                             sj_task *tasks, uint32_t nt, float *pred, cudaStream_t s);
 cudaError_t sj_tg_shard(const sj_task *in, const float *predIn, uint32_t nOut, uint32_t idx, uint32_t cnt,
                         sj_task *out, float *predOut, cudaStream_t s);
 // the tasks by count-pass kernel: pre[0..nt] (exclusive prefix of the small ones), lists of the others and
@@ -276,9 +275,11 @@ cudaError_t sj_task_offsets(const sj_task *tasks, const float *pred, uint32_t nt
 cudaError_t sj_plan_batches(unsigned long long *const off[7], uint32_t nt, unsigned long long cap,
                             unsigned long long maskLim, uint32_t *next, uint32_t *start, uint32_t *nBatches,
                             cudaStream_t s);
-// per batch: predicted pairs, row-mask words, column-mask words, row offsets, candidate records, small tasks
-cudaError_t sj_plan_stats(const uint32_t *start, uint32_t nb, unsigned long long *const off[7],
-                          const uint32_t *smallPre, unsigned long long *stats, cudaStream_t s);
+// stats[0] = predicted pairs; per batch, of the first nb at most, eight words: first task, task after the
+// last, predicted pairs, row-mask words, column-mask words, row offsets, candidate records, small tasks
+cudaError_t sj_plan_stats(const uint32_t *start, uint32_t nb, const uint32_t *nBatches, uint32_t nt,
+                          unsigned long long *const off[7], const uint32_t *smallPre, unsigned long long *stats,
+                          cudaStream_t s);
 // learned estimator: rates (2 per cell: home, owned neighbours) from the
 // network's outputs (log2(1 + home hits), log2(1 + owned-neighbour hits))
 cudaError_t sj_rates_mlp(const float *out, const uint32_t *cellStart, const uint32_t *nbrStart,
@@ -291,10 +292,9 @@ size_t sj_sample_totals_len();
 cudaError_t sj_sample_rates(const sj_task *tasks, uint32_t nt, const uint32_t *taskHits, const uint32_t *taskEvals,
                             const uint32_t *cellStart, unsigned long long *cellHits, unsigned long long *cellEvals,
                             unsigned long long *totals, uint32_t nCells, float *rate, cudaStream_t s);
-// sums[0] evaluations, [1] refined, [2] measured pairs; *errSum = sum |pred - measured|
+// sums[0] evaluations, [1] refined, [2] measured pairs, [3] (a double) sum |pred - measured|
 cudaError_t sj_task_sums(const uint32_t *taskEvals, const uint32_t *taskRefined, const uint32_t *taskHits,
-                         const float *pred, uint32_t nt, unsigned long long *sums, double *errSum, int numSM,
-                         cudaStream_t s);
+                         const float *pred, uint32_t nt, unsigned long long *sums, int numSM, cudaStream_t s);
 cudaError_t sj_cell_hits(const uint32_t *cellStart, const uint32_t *ids, const uint32_t *deg, uint32_t nCells,
                          unsigned long long *hits, cudaStream_t s);
 // exclusive scan of n u64 values (out has n+1 entries, out[n] = total); temp: sj_scan64_temp(n) entries

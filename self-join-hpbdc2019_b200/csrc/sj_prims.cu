@@ -131,6 +131,55 @@ __global__ void k_scan_total(const uint32_t *scannedSums, const uint32_t *sums, 
     if (threadIdx.x == 0 && blockIdx.x == 0 && total_dev) *total_dev = scannedSums[nb - 1] + sums[nb - 1];
 }
 
+// A scan of up to SCAN_ONE elements in one launch of one block (in place, or out
+// apart): the task builder and the small sorts scan a few thousand counts many
+// times a join, and a launch costs more than the block.
+constexpr int SCAN_ONE_THREADS = 1024;
+constexpr int SCAN_ONE_ITEMS = 16;
+constexpr uint64_t SCAN_ONE = (uint64_t)SCAN_ONE_THREADS * SCAN_ONE_ITEMS;
+
+__global__ void __launch_bounds__(SCAN_ONE_THREADS) k_scan_one(const uint32_t *in, uint32_t *out, uint32_t n,
+                                                               uint32_t *total_dev, uint32_t *zeroIn)
+{
+    __shared__ uint32_t ws[32];
+    const uint32_t per = (n + SCAN_ONE_THREADS - 1) / SCAN_ONE_THREADS;   // consecutive elements of a thread
+    const uint32_t base = threadIdx.x * per;
+    uint32_t v[SCAN_ONE_ITEMS], sum = 0;
+#pragma unroll
+    for (int i = 0; i < SCAN_ONE_ITEMS; i++) {
+        v[i] = ((uint32_t)i < per && base + i < n) ? in[base + i] : 0u;
+        sum += v[i];
+    }
+    uint32_t x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane_id() >= (uint32_t)o) x += y;
+    }
+    if (lane_id() == 31) ws[threadIdx.x >> 5] = x;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        uint32_t s = ws[threadIdx.x];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane_id() >= (uint32_t)o) s += y;
+        }
+        ws[threadIdx.x] = s;
+    }
+    __syncthreads();
+    uint32_t run = x - sum + (threadIdx.x >= 32 ? ws[(threadIdx.x >> 5) - 1] : 0u);
+#pragma unroll
+    for (int i = 0; i < SCAN_ONE_ITEMS; i++) {
+        if ((uint32_t)i < per && base + i < n) {
+            if (zeroIn) zeroIn[base + i] = 0u;
+            out[base + i] = run;
+            run += v[i];
+        }
+    }
+    if (total_dev && threadIdx.x == 0) *total_dev = ws[31];
+}
+
 uint64_t ceil_div(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 
 size_t scan_temp_elems(uint64_t n)
@@ -153,6 +202,10 @@ cudaError_t scan_rec(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *te
     }
     if (n <= (uint64_t)SCAN_TILE) {
         k_scan_tile<<<1, SCAN_THREADS, 0, s>>>(in, out, n, nullptr, total_dev, zeroIn); sj_note_launch();
+        return cudaGetLastError();
+    }
+    if (n <= SCAN_ONE) {
+        k_scan_one<<<1, SCAN_ONE_THREADS, 0, s>>>(in, out, (uint32_t)n, total_dev, zeroIn); sj_note_launch();
         return cudaGetLastError();
     }
     uint64_t nb = ceil_div(n, SCAN_TILE);

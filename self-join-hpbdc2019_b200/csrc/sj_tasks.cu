@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(256) k_tg_groups(sj_taskgen g, uint32_t *cnt)
 __global__ void __launch_bounds__(256) k_tg_cells(sj_taskgen g, const uint32_t *__restrict__ order,
                                                   const uint8_t *__restrict__ workersAt, uint32_t *__restrict__ posCnt,
                                                   unsigned long long *__restrict__ posEv,
-                                                  unsigned long long *__restrict__ costKey,
+                                                  uint32_t *__restrict__ costKey, uint32_t *__restrict__ iota,
                                                   unsigned long long *__restrict__ totals)
 {
     const uint32_t lane = threadIdx.x & 31u;
@@ -273,10 +273,13 @@ __global__ void __launch_bounds__(256) k_tg_cells(sj_taskgen g, const uint32_t *
     if (lane == 0) {
         posCnt[pos] = (uint32_t)min(cnt, (uint64_t)FULL);
         if (posEv) posEv[pos] = ev;
+        if (iota) iota[pos] = pos;
         if (costKey) {
-            // mean predicted task cost: evaluations plus a write cost per pair
+            // mean predicted task cost: evaluations plus a write cost per pair.  The
+            // key is its exponent and 8 bits of its mantissa, descending: two sort
+            // passes, and an order finer than 0.4 % would not be worth more
             const double cost = cnt ? ((double)ev + 4.0 * pred) / (double)cnt : 0.0;
-            costKey[pos] = ~(unsigned long long)__double_as_longlong(cost);   // cost >= 0: descending
+            costKey[pos] = 0xffffu - (__float_as_uint((float)cost) >> 15);   // cost >= 0
         }
         atomicAdd(&totals[0], (unsigned long long)cnt);
         atomicAdd(&totals[1], (unsigned long long)ev);
@@ -332,12 +335,6 @@ __global__ void __launch_bounds__(256) k_nbr_spread(const uint32_t *__restrict__
         carryW += __shfl_sync(FULL, iw, 31);
     }
     if (lane == 0) cellW[c] = carryW;
-}
-
-__global__ void __launch_bounds__(256) k_iota(uint32_t *v, uint32_t n)
-{
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) v[i] = i;
 }
 
 // Mode 8 (the reference's dynamic threads per point, kernel.cu:2072-2188 with
@@ -406,7 +403,8 @@ __global__ void __launch_bounds__(256) k_tg_item_write(sj_taskgen g, const uint3
                                                        const uint8_t *__restrict__ workersAt,
                                                        const uint32_t *__restrict__ itemStart, uint32_t nItems,
                                                        const uint32_t *__restrict__ itemTaskStart,
-                                                       sj_task *__restrict__ tasks, float *__restrict__ pred)
+                                                       sj_task *__restrict__ tasks, uint32_t nt,
+                                                       float *__restrict__ pred)
 {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= nItems) return;
@@ -417,7 +415,9 @@ __global__ void __launch_bounds__(256) k_tg_item_write(sj_taskgen g, const uint3
     const uint32_t segBase = it.grp * SJ_MAX_SEG;
     const float2 r = rates_of(g, it.c);
     uint32_t t = itemTaskStart[j];
-    for (uint32_t ch = 0; ch < w.nChunks; ch++, t++) {
+    // (t < nt: the lists are sized by the cells' task counts, and the two counts
+    // are compared on the host afterwards)
+    for (uint32_t ch = 0; ch < w.nChunks && t < nt; ch++, t++) {
         const uint2 sr = chunk_range(g, w, ch);
         const uint32_t s0 = sr.x, s1 = sr.y;
         // evaluations against the home segment (positions < homeLen) and the rest
@@ -477,8 +477,7 @@ __global__ void __launch_bounds__(256) k_task_lists(const uint32_t *__restrict__
 constexpr int NC = 7;           // row masks, column masks, row offsets, candidate records, units,
                                 // planned pairs (rounded up, x (1 + alpha)), predicted pairs (rounded)
 constexpr int OT = 256;         // threads per offsets block
-constexpr int OI = 8;           // tasks per thread
-constexpr int OTILE = OT * OI;
+constexpr uint32_t OFF_SHORT = 65536;   // tasks up to which a thread takes one (more blocks), 8 above
 
 __device__ __forceinline__ void task_sizes(const sj_task &t, float pred, double alpha1, uint64_t (&v)[NC])
 {
@@ -495,11 +494,12 @@ __device__ __forceinline__ void task_sizes(const sj_task &t, float pred, double 
     v[6] = (uint64_t)llrint((double)pred);
 }
 
+template <int OI>
 __global__ void __launch_bounds__(OT) k_off_reduce(const sj_task *__restrict__ tasks, const float *__restrict__ pred,
                                                    uint32_t nt, double alpha1, unsigned long long *__restrict__ sums)
 {
     uint64_t acc[NC] = {0, 0, 0, 0, 0, 0, 0};
-    const uint64_t base = (uint64_t)blockIdx.x * OTILE;
+    const uint64_t base = (uint64_t)blockIdx.x * (OT * OI);
     for (int i = 0; i < OI; i++) {
         const uint64_t t = base + (uint64_t)i * OT + threadIdx.x;
         if (t < nt) {
@@ -547,12 +547,13 @@ struct OffOut {
     unsigned long long *p[NC];
 };
 
+template <int OI>
 __global__ void __launch_bounds__(OT) k_off_write(const sj_task *__restrict__ tasks, const float *__restrict__ pred,
                                                   uint32_t nt, double alpha1,
                                                   const unsigned long long *__restrict__ blockBase, OffOut out)
 {
     // thread th handles tasks base + th*OI .. + OI-1 (consecutive)
-    const uint64_t base = (uint64_t)blockIdx.x * OTILE + (uint64_t)threadIdx.x * OI;
+    const uint64_t base = (uint64_t)blockIdx.x * (OT * OI) + (uint64_t)threadIdx.x * OI;
     uint64_t v[OI][NC];
     uint64_t tot[NC] = {0, 0, 0, 0, 0, 0, 0};
     for (int i = 0; i < OI; i++) {
@@ -647,22 +648,26 @@ __global__ void k_plan_chain(const uint32_t *__restrict__ next, uint32_t nt, uin
     *nBatches = b;
 }
 
-// Per batch: predicted pairs and the sizes of its records.
-__global__ void __launch_bounds__(256) k_plan_stats(const uint32_t *__restrict__ start, uint32_t nb, OffOut off,
+// stats[0]: predicted pairs of all tasks; then eight words per batch: its first
+// task and the one after its last, its predicted pairs and the sizes of its records.
+__global__ void __launch_bounds__(256) k_plan_stats(const uint32_t *__restrict__ start, uint32_t most,
+                                                    const uint32_t *__restrict__ nBatches, uint32_t nt, OffOut off,
                                                     const uint32_t *__restrict__ smallPre,
                                                     unsigned long long *__restrict__ stats)
 {
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
+    if (b == 0) stats[0] = off.p[6][nt];
+    if (b >= min(most, *nBatches)) return;
     const uint32_t t0 = start[b], t1 = start[b + 1];
-    // [0] predicted pairs, [1] row-mask words, [2] column-mask words, [3] row offsets, [4] candidate records,
-    // [5] small tasks
-    stats[(uint64_t)b * 6 + 0] = off.p[6][t1] - off.p[6][t0];
-    stats[(uint64_t)b * 6 + 1] = off.p[0][t1] - off.p[0][t0];
-    stats[(uint64_t)b * 6 + 2] = off.p[1][t1] - off.p[1][t0];
-    stats[(uint64_t)b * 6 + 3] = off.p[2][t1] - off.p[2][t0];
-    stats[(uint64_t)b * 6 + 4] = off.p[3][t1] - off.p[3][t0];
-    stats[(uint64_t)b * 6 + 5] = smallPre[t1] - smallPre[t0];
+    unsigned long long *const s = stats + 1 + (uint64_t)b * 8;
+    s[0] = t0;
+    s[1] = t1;
+    s[2] = off.p[6][t1] - off.p[6][t0];   // predicted pairs
+    s[3] = off.p[0][t1] - off.p[0][t0];   // row-mask words
+    s[4] = off.p[1][t1] - off.p[1][t0];   // column-mask words
+    s[5] = off.p[2][t1] - off.p[2][t0];   // row offsets
+    s[6] = off.p[3][t1] - off.p[3][t0];   // candidate records
+    s[7] = smallPre[t1] - smallPre[t0];   // small tasks
 }
 
 // ------------------------------------------------------------ estimates --
@@ -759,12 +764,12 @@ __global__ void __launch_bounds__(256) k_sample_rates(const unsigned long long *
 
 // ------------------------------------------------------------ statistics --
 // sums[0] evaluations, [1] FP32 borderline re-evaluations, [2] measured pairs;
-// errSum: sum over tasks of |predicted - measured pairs|.
+// [3], as a double: the sum over tasks of |predicted - measured pairs|.
 __global__ void __launch_bounds__(256) k_task_sums(const uint32_t *__restrict__ taskEvals,
                                                    const uint32_t *__restrict__ taskRefined,
                                                    const uint32_t *__restrict__ taskHits,
                                                    const float *__restrict__ pred, uint32_t nt,
-                                                   unsigned long long *__restrict__ sums, double *__restrict__ errSum)
+                                                   unsigned long long *__restrict__ sums)
 {
     uint64_t e = 0, r = 0, h = 0;
     double d = 0.0;
@@ -784,7 +789,7 @@ __global__ void __launch_bounds__(256) k_task_sums(const uint32_t *__restrict__ 
         if (e) atomicAdd(&sums[0], (unsigned long long)e);
         if (r) atomicAdd(&sums[1], (unsigned long long)r);
         if (h) atomicAdd(&sums[2], (unsigned long long)h);
-        if (d != 0.0 && errSum) atomicAdd(errSum, d);
+        if (d != 0.0) atomicAdd(reinterpret_cast<double *>(sums + 3), d);
     }
 }
 
@@ -900,20 +905,12 @@ cudaError_t sj_tg_groups(const sj_taskgen &g, uint32_t *cnt, cudaStream_t s)
 }
 
 cudaError_t sj_tg_cells(const sj_taskgen &g, const uint32_t *order, const uint8_t *workersAt, uint32_t *posCnt,
-                        unsigned long long *posEv, unsigned long long *costKey, unsigned long long *totals,
+                        unsigned long long *posEv, uint32_t *costKey, uint32_t *iota, unsigned long long *totals,
                         cudaStream_t s)
 {
     if (g.nCells == 0) return cudaSuccess;
     k_tg_cells<<<blocks_for((uint64_t)g.nCells * 32, 256), 256, 0, s>>>(g, order, workersAt, posCnt, posEv, costKey,
-                                                                        totals);
-    sj_note_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t sj_iota_u32(uint32_t *v, uint32_t n, cudaStream_t s)
-{
-    if (n == 0) return cudaSuccess;
-    k_iota<<<blocks_for(n, 256), 256, 0, s>>>(v, n);
+                                                                        iota, totals);
     sj_note_launch();
     return cudaGetLastError();
 }
@@ -945,11 +942,11 @@ cudaError_t sj_tg_item_tasks(const sj_taskgen &g, const uint32_t *order, const u
 
 cudaError_t sj_tg_item_write(const sj_taskgen &g, const uint32_t *order, const uint8_t *workersAt,
                              const uint32_t *itemStart, uint32_t nItems, const uint32_t *itemTaskStart,
-                             sj_task *tasks, float *pred, cudaStream_t s)
+                             sj_task *tasks, uint32_t nt, float *pred, cudaStream_t s)
 {
     if (nItems == 0) return cudaSuccess;
     k_tg_item_write<<<blocks_for(nItems, 256), 256, 0, s>>>(g, order, workersAt, itemStart, nItems, itemTaskStart,
-                                                            tasks, pred);
+                                                            tasks, nt, pred);
     sj_note_launch();
     return cudaGetLastError();
 }
@@ -976,7 +973,9 @@ cudaError_t sj_task_lists(const sj_task *tasks, uint32_t nt, uint32_t *pre, uint
     return cudaGetLastError();
 }
 
-size_t sj_task_offsets_temp(uint32_t nt) { return (size_t)(blocks_for(nt ? nt : 1, OTILE)) * NC; }
+inline uint32_t off_items(uint32_t nt) { return nt <= OFF_SHORT ? 1u : 8u; }
+
+size_t sj_task_offsets_temp(uint32_t nt) { return (size_t)(blocks_for(nt ? nt : 1, OT * off_items(nt))) * NC; }
 
 cudaError_t sj_task_offsets(const sj_task *tasks, const float *pred, uint32_t nt, double alpha,
                             unsigned long long *temp, unsigned long long *const out[7], cudaStream_t s)
@@ -990,13 +989,16 @@ cudaError_t sj_task_offsets(const sj_task *tasks, const float *pred, uint32_t nt
         }
         return cudaSuccess;
     }
-    const unsigned nb = blocks_for(nt, OTILE);
+    const unsigned nb = blocks_for(nt, OT * off_items(nt));
     const double alpha1 = 1.0 + alpha;
-    k_off_reduce<<<nb, OT, 0, s>>>(tasks, pred, nt, alpha1, temp);
+    const bool one = off_items(nt) == 1;
+    if (one) k_off_reduce<1><<<nb, OT, 0, s>>>(tasks, pred, nt, alpha1, temp);
+    else k_off_reduce<8><<<nb, OT, 0, s>>>(tasks, pred, nt, alpha1, temp);
     sj_note_launch();
     k_off_scan_blocks<<<1, 32 * NC, 0, s>>>(temp, nb);
     sj_note_launch();
-    k_off_write<<<nb, OT, 0, s>>>(tasks, pred, nt, alpha1, temp, o);
+    if (one) k_off_write<1><<<nb, OT, 0, s>>>(tasks, pred, nt, alpha1, temp, o);
+    else k_off_write<8><<<nb, OT, 0, s>>>(tasks, pred, nt, alpha1, temp, o);
     sj_note_launch();
     return cudaGetLastError();
 }
@@ -1013,13 +1015,13 @@ cudaError_t sj_plan_batches(unsigned long long *const off[7], uint32_t nt, unsig
     return cudaGetLastError();
 }
 
-cudaError_t sj_plan_stats(const uint32_t *start, uint32_t nb, unsigned long long *const off[7],
-                          const uint32_t *smallPre, unsigned long long *stats, cudaStream_t s)
+cudaError_t sj_plan_stats(const uint32_t *start, uint32_t nb, const uint32_t *nBatches, uint32_t nt,
+                          unsigned long long *const off[7], const uint32_t *smallPre, unsigned long long *stats, cudaStream_t s)
 {
     if (nb == 0) return cudaSuccess;
     OffOut o;
     for (int k = 0; k < NC; k++) o.p[k] = off[k];
-    k_plan_stats<<<blocks_for(nb, 256), 256, 0, s>>>(start, nb, o, smallPre, stats);
+    k_plan_stats<<<blocks_for(nb, 256), 256, 0, s>>>(start, nb, nBatches, nt, o, smallPre, stats);
     sj_note_launch();
     return cudaGetLastError();
 }
@@ -1056,15 +1058,13 @@ cudaError_t sj_sample_rates(const sj_task *tasks, uint32_t nt, const uint32_t *t
 }
 
 cudaError_t sj_task_sums(const uint32_t *taskEvals, const uint32_t *taskRefined, const uint32_t *taskHits,
-                         const float *pred, uint32_t nt, unsigned long long *sums, double *errSum, int numSM,
-                         cudaStream_t s)
+                         const float *pred, uint32_t nt, unsigned long long *sums, int numSM, cudaStream_t s)
 {
-    cudaError_t e = cudaMemsetAsync(sums, 0, sizeof(unsigned long long) * 3, s);
-    if (e == cudaSuccess && errSum) e = cudaMemsetAsync(errSum, 0, sizeof(double), s);
+    cudaError_t e = cudaMemsetAsync(sums, 0, sizeof(unsigned long long) * 4, s);
     if (e != cudaSuccess || nt == 0) return e;
     unsigned grid = blocks_for(nt, 256);
     if (grid > (unsigned)numSM * 8) grid = (unsigned)numSM * 8;
-    k_task_sums<<<grid, 256, 0, s>>>(taskEvals, taskRefined, taskHits, pred, nt, sums, errSum);
+    k_task_sums<<<grid, 256, 0, s>>>(taskEvals, taskRefined, taskHits, pred, nt, sums);
     sj_note_launch();
     return cudaGetLastError();
 }
