@@ -834,10 +834,13 @@ sj_status build_tasks_dev(Ctx &c, bool sym, uint64_t cap, bool byCost, int polic
     g.nCells = nc;
     g.tile = SJ_CTA * (uint32_t)sj_query_slots(c.g.Dp, c.p.precision == SJ_PREC_FP32_REFINE);
     g.cap = cap;
-    // predicted pairs per task: about 4096 tasks per full batch.  SJ_TASK_PAIRS
+    // predicted pairs per task: about 16384 tasks per full batch, so that the
+    // last ones leave little of the device idle (6-D FP64 data at 5e8 pairs a
+    // batch: 48 ms of count and emission with 60,000 pairs a task, 54 with
+    // 488,000; 2-D at 5e7: 70.4 with 3,000, 71.9 with 12,000).  SJ_TASK_PAIRS
     // overrides it (a tuning knob: profiling runs at a reduced batch capacity
     // use it to keep the task shapes of the full-capacity run)
-    g.pairsPerTask = std::max(4096.0, (double)cap / 4096.0);
+    g.pairsPerTask = std::max(4096.0, (double)cap / 16384.0);
     if (const char *ev = getenv("SJ_TASK_PAIRS")) {
         const double v = atof(ev);
         if (v >= 1.0) g.pairsPerTask = v;

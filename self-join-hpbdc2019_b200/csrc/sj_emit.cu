@@ -23,22 +23,23 @@
 //               candidates' ids;
 //   column unit (symmetric task, block of 32 positions): the words of the live
 //               groups; the lines are the candidates, the values the queries'.
-// Both stage up to TW words of every line and the values they select from in
-// shared memory and go through emit_lines: a window holds the words of one line
-// (or of 2, 4 .. lines when few words are live), one per lane; their popcounts
-// are scanned, the set bits decoded into a list in slot order, and the warp
-// copies the list out line by line: consecutive entries go to consecutive
-// slots, so the stores are coalesced.  Key, value and the hash of the pair are
-// produced in the same pass.
+// Both stage up to TW words of every line, and the values they select from, in
+// shared memory (asynchronous copies, all in flight together) and go out in one
+// of two ways, value, key and hash of every pair in the same pass:
+//   windows (many hits): the words of two lines across the lanes; popcounts
+//               scanned, the set bits decoded into one list a line in slot order,
+//               each list copied out with a uniform key: consecutive entries go
+//               to consecutive slots, so the stores are coalesced;
+//   lists (few hits, or few words): lane = line; each lane walks its own line's
+//               bits into its part of one packed list, which the warp copies out.
 //
-// Bound: instruction issue.  With the points of a cell in spatial order the
-// live words are dense (10 to 26 bits on average on the exponential sets, and
-// over 80 % of the pairs lie in words of 16 bits or more), so a window of 32
-// words yields 300 to 800 pairs and the copy-out -- two shared loads, two stores
-// and the ~19 integer operations of splitmix64 with the key's part taken out --
-// is most of the work.  Hence words across the lanes with one scan a window, and
-// not a list per line (lanes idle for the fullest line: 2.1 against 1.4 warp
-// instructions a pair on 6-D data).
+// Bound: instruction issue.  With the points of a cell in spatial order the hits
+// are bunched: on the exponential sets three quarters of the pairs lie in tiles
+// more than half full, and 60 % of the live tiles hold a tenth of them.  In a
+// full window the copy-out -- two shared loads, two stores and the ~19 integer
+// operations of splitmix64 with the key's part taken out -- is most of the work;
+// in sparse tiles a window's fixed ~100 instructions would be, so those go by
+// lists, whose decode is as long as the fullest line.
 // Every mask word is checked against its task's sizes before it is decoded (bits
 // past the stream end or for queries past the tile, which a consistent count
 // pass never sets, are dropped and raise an error flag that the host reports),
@@ -56,29 +57,41 @@ constexpr int EMIT_MINB = 7;        // resident CTAs per SM (26 KB of shared mem
 constexpr uint32_t UN = 4;          // consecutive units a warp takes at a time (1 near the end of the batch)
 constexpr uint32_t FULL = 0xffffffffu;
 constexpr uint32_t TW = 16;         // words per line staged together: windows of two lines
-constexpr uint32_t LD = 4;          // words whose loads are in flight together
+constexpr uint32_t LIM = 31;        // entries a line adds to a list per round: lane l of 32 full lines writes
+                                    // entry 31 l + k, (almost) all in different banks
+constexpr uint32_t SPARSE = 80;      // hits per staged word (of its 1024 over the lines) below which lists are used
+                                    // (20, 40, 80 and 160 within 1 % of each other but 160 on 6-D data: +4 %)
 constexpr uint32_t DENSE = 14;      // fullest word of a window above which every bit is tested in turn
 static_assert(SJ_CTA * sj_query_slots(1, true) / 32 <= TW, "a task's query groups fit the staged words");
 
 struct __align__(16) LineInfo {
-    uint32_t base;          // slot of the window's list entry 0 if it were this line's
+    uint32_t base;          // windows: the line's next slot; lists: slot of list entry 0 if it were this line's
     uint32_t key, hi2, add; // the line's key and its part of the pair hash
 };
 
 struct WarpSmem {
     uint32_t tile[TW][33];  // [staged word][line]
     uint32_t val[TW * 32];  // value of bit i of staged word j: val[32 j + i]
-    uint16_t ent[1024];     // one window's list: byte offset into val; with more than two lines a window
-                            // (line in window << 10) | index into val
+    uint16_t ent[1024];     // windows: two lists of up to 512 byte offsets into val; lists: (line << 9) | index
     LineInfo line[32];
 };
 
-__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x, uint32_t lane)
+// asynchronous copy of one word (or a zero when !have; src is not read then)
+__device__ __forceinline__ void copy_word(uint32_t *dst, const uint32_t *src, bool have)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(have ? 4 : 0)
+                 : "memory");
+}
+
+// inclusive scan over groups of W lanes
+template <int W>
+__device__ __forceinline__ uint32_t incl_scan(uint32_t x, uint32_t lane)
 {
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(FULL, x, o);
-        if (lane >= (uint32_t)o) x += y;
+    for (int o = 1; o < W; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULL, x, o, W);
+        if ((lane & (W - 1)) >= (uint32_t)o) x += y;
     }
     return x;
 }
@@ -127,11 +140,10 @@ struct Out {
     unsigned long long hash;
 };
 
-// Writes tag + unit * (index of each set bit of m) to the list from entry k on,
-// lowest bit first; n = popc(m).  sparse: the bits highest first, two a step, filling
-// from the end.  dense: all 32 bits tested, no bit scans and no loop.
-__device__ __forceinline__ void decode_sparse(uint32_t m, uint32_t n, uint32_t tag, uint32_t unit, uint16_t *buf,
-                                              uint32_t k)
+// Writes tag + 4 * (index of each set bit of m) to the list from entry k on,
+// lowest bit first; n = popc(m).  sparse: the bits highest first, two a step,
+// filling from the end.  dense: all 32 bits tested, no bit scans and no loop.
+__device__ __forceinline__ void decode_sparse(uint32_t m, uint32_t n, uint32_t tag, uint16_t *buf, uint32_t k)
 {
     uint16_t *p = buf + k + n;
     for (; n >= 2; n -= 2) {
@@ -139,26 +151,39 @@ __device__ __forceinline__ void decode_sparse(uint32_t m, uint32_t n, uint32_t t
         m ^= 1u << b0;
         const uint32_t b1 = top_bit(m);
         m ^= 1u << b1;
-        p[-1] = (uint16_t)(tag + unit * b0);
-        p[-2] = (uint16_t)(tag + unit * b1);
+        p[-1] = (uint16_t)(tag + 4 * b0);
+        p[-2] = (uint16_t)(tag + 4 * b1);
         p -= 2;
     }
-    if (n) p[-1] = (uint16_t)(tag + unit * top_bit(m));
+    if (n) p[-1] = (uint16_t)(tag + 4 * top_bit(m));
 }
 
-__device__ __forceinline__ void decode_dense(uint32_t m, uint32_t tag, uint32_t unit, uint16_t *buf, uint32_t k)
+__device__ __forceinline__ void decode_dense(uint32_t m, uint32_t n, uint32_t tag, uint32_t j, uint16_t *buf, uint32_t k)
 {
-    uint32_t p = (uint32_t)__cvta_generic_to_shared(buf + k);
+    // The lanes start at different bits (2 j for word j of the line) and wrap
+    // around: full words begin 64 bytes apart in the list, and lanes walking them
+    // in step would all hit two banks.
+    const uint32_t r = 2 * j;
+    uint32_t p = (uint32_t)__cvta_generic_to_shared(buf + k) + 2 * __popc(m & ((1u << r) - 1u));
+    uint32_t t = tag + 4 * r;
+    m = __funnelshift_r(m, m, r);
+    const uint32_t back = 2 * n;
 #pragma unroll
     for (int b = 0; b < 32; b++) {
+        if (b > 0 && b % 2 == 0)
+            asm volatile("{ .reg .pred q; setp.eq.u32 q, %2, %4;\n\t"
+                         "@q sub.u32 %0, %0, %3;\n\t"
+                         "@q sub.u32 %1, %1, 128; }"
+                         : "+r"(p), "+r"(t)
+                         : "r"(r), "r"(back), "r"(32 - b));
         asm volatile("{ .reg .pred q; .reg .b32 t;\n\t"
                      "and.b32 t, %1, %3; setp.ne.u32 q, t, 0;\n\t"
                      "@q st.shared.u16 [%0], %2;\n\t"
                      "@q add.u32 %0, %0, 2; }"
                      : "+r"(p)
-                     : "r"(m), "r"(tag), "r"(1u << b)
+                     : "r"(m), "r"(t), "r"(1u << b)
                      : "memory");
-        tag += unit;
+        t += 4;
     }
 }
 
@@ -166,8 +191,10 @@ __device__ __forceinline__ void decode_dense(uint32_t m, uint32_t tag, uint32_t 
 // slots B, B + 1 ..
 template <bool KEYS>
 __device__ __forceinline__ void copy_line(Out &o, const WarpSmem &w, uint32_t lane, uint32_t e0, uint32_t n,
-                                          uint32_t B, uint32_t key, KeyHash kh)
+                                          const LineInfo &li)
 {
+    const uint32_t B = li.base, key = li.key;
+    const KeyHash kh{li.hi2, li.add};
     uint32_t ent = (uint32_t)__cvta_generic_to_shared(w.ent + e0 + lane);
     const uint32_t val = (uint32_t)__cvta_generic_to_shared(w.val);
     int32_t *pv = o.val + (uint64_t)B + lane;
@@ -203,65 +230,79 @@ __device__ __forceinline__ void copy_line(Out &o, const WarpSmem &w, uint32_t la
     }
 }
 
-// Emits the hits of up to 32 lines (those of the mask `lines` have any) over the
-// nl staged words.  Lane l holds line
-// l's key, its hash part and its next slot (advanced past the line's pairs).
-// Lines without hits need no valid key.
+// Emits the hits of 32 lines over the nl staged words: a window holds 2 lines of
+// up to 16 words, 4 of up to 8, 8 of up to 4 or 16 of up to 2; lines: mask of the
+// lines with hits.  w.line holds the lines.
 template <bool KEYS>
-__device__ __forceinline__ void emit_lines(const sj_join_args &a, Out &o, WarpSmem &w, uint32_t lane, uint32_t nl,
-                                           uint32_t lines, uint32_t key, KeyHash kh, uint32_t &next)
+__device__ __forceinline__ void emit_windows(Out &o, WarpSmem &w, uint32_t lane, uint32_t nl, uint32_t lines)
 {
-    const uint32_t sh = nl > 1 ? 32 - __clz(nl - 1) : 0u;   // words per line, rounded up to 2^sh
-    const uint32_t j = lane & ((1u << sh) - 1u), lw = lane >> sh, lpw = 32u >> sh;
-    const uint32_t unit = lpw > 2 ? 1u : 4u;
-    const uint32_t tag = lpw > 2 ? (j * 32) | (lw << 10) : j * 128;
-    const uint32_t inWindow = FULL >> (32u - lpw);
+    const uint32_t sh = nl > 2 ? 32 - __clz(nl - 1) : 1u;   // words per line: 2^sh
+    const uint32_t W = 1u << sh, j = lane & (W - 1), lw = lane >> sh, lpw = 32u >> sh;
+    const uint32_t inWindow = (1u << lpw) - 1u;             // at most 16 lines
 #pragma unroll 1
     for (uint32_t l0 = 0; l0 < 32; l0 += lpw) {
         if (!((lines >> l0) & inWindow)) continue;
         const uint32_t word = j < nl ? w.tile[j][l0 + lw] : 0u;
         const uint32_t cnt = __popc(word);
-        const uint32_t most = __reduce_max_sync(FULL, cnt);
-        const uint32_t incl = warp_incl_scan(cnt, lane);
-        const uint32_t T = __shfl_sync(FULL, incl, 31);
-        const uint32_t ex = incl - cnt;
-        // every slot of the window's lines fits: a consistent count pass sees to that
-        const uint32_t first = (lane - l0) << sh;   // first word of this lane's line, for lanes of the window
-        const bool mine = lane - l0 < lpw;
-        const uint32_t exF = __shfl_sync(FULL, ex, first & 31u);
-        const uint32_t nLine = __shfl_sync(FULL, incl, (first + (1u << sh) - 1u) & 31u) - exF;
-        if (__any_sync(FULL, mine && (uint64_t)next + nLine > o.cap && nLine)) {
-            atomicMax(&a.stat[3], 1ULL);
-            if (mine) next += nLine;
-            continue;
-        }
-        __syncwarp();   // the previous window's copy-out is done with the list
-        if (most > DENSE) decode_dense(word, tag, unit, w.ent, ex);
-        else decode_sparse(word, cnt, tag, unit, w.ent, ex);
-        if (lpw <= 2) {
-            __syncwarp();
+        uint32_t incl = cnt;   // over the line's words
 #pragma unroll 1
-            for (uint32_t i = 0; i < lpw; i++) {
-                const uint32_t l = l0 + i;
-                const uint32_t n = __shfl_sync(FULL, nLine, l);
-                if (!n) continue;
-                copy_line<KEYS>(o, w, lane, __shfl_sync(FULL, exF, l), n, __shfl_sync(FULL, next, l),
-                                __shfl_sync(FULL, key, l),
-                                KeyHash{__shfl_sync(FULL, kh.hi2, l), __shfl_sync(FULL, kh.add, l)});
-            }
-        } else {
-            if (mine) w.line[lane - l0] = LineInfo{next - exF, key, kh.hi2, kh.add};
-            __syncwarp();
-            for (uint32_t e = lane; e < T; e += 32) {
-                const uint32_t en = w.ent[e];
-                const LineInfo l = w.line[en >> 10];
-                const uint32_t v = w.val[en & 0x3ffu];
-                o.val[l.base + e] = (int32_t)v;
-                if (KEYS) o.key[l.base + e] = (int32_t)l.key;
-                o.hash += pair_hash(KeyHash{l.hi2, l.add}, v);
-            }
+        for (uint32_t d = 1; d < W; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, incl, d, W);
+            if (j >= d) incl += y;
         }
-        if (mine) next += nLine;
+        const bool dense = __any_sync(FULL, cnt > DENSE);
+        const uint32_t at = lw * (W * 32) + incl - cnt;   // a list of W * 32 entries per line
+        __syncwarp();   // the previous window's copy-out is done with the lists
+        if (dense) decode_dense(word, cnt, j * 128, j, w.ent, at);
+        else decode_sparse(word, cnt, j * 128, w.ent, at);
+        __syncwarp();
+#pragma unroll 1
+        for (uint32_t i = 0; i < lpw; i++) {
+            const uint32_t n = __shfl_sync(FULL, incl, W * i + W - 1);
+            if (n) copy_line<KEYS>(o, w, lane, i * (W * 32), n, w.line[l0 + i]);
+        }
+    }
+}
+
+// Emits the hits of 32 lines, lane = line: cnt of them in the nonzero words nz,
+// slots up to `end`.
+template <bool KEYS>
+__device__ __forceinline__ void emit_lists(Out &o, WarpSmem &w, uint32_t lane, uint32_t cnt, uint32_t nz,
+                                           uint32_t end)
+{
+    uint32_t rem = cnt, word = 0, tag = 0;   // lines go from their last hit to the first
+#pragma unroll 1
+    while (__any_sync(FULL, rem)) {
+        const uint32_t c = min(rem, LIM);
+        const uint32_t incl = incl_scan<32>(c, lane);
+        const uint32_t T = __shfl_sync(FULL, incl, 31);
+        end -= c;
+        rem -= c;
+        w.line[lane].base = end - (incl - c);
+        uint16_t *p = w.ent + incl;
+#pragma unroll 1
+        for (uint32_t k = c; k; k--) {
+            if (!word) {
+                const uint32_t j = top_bit(nz);
+                nz ^= 1u << j;
+                word = w.tile[j][lane];
+                tag = (lane << 9) | (j << 5);
+            }
+            const uint32_t b = top_bit(word);
+            word ^= 1u << b;
+            *--p = (uint16_t)(tag + b);
+        }
+        __syncwarp();
+#pragma unroll 2
+        for (uint32_t e = lane; e < T; e += 32) {
+            const uint32_t en = w.ent[e];
+            const LineInfo l = w.line[en >> 9];
+            const uint32_t v = w.val[en & 0x1ffu];
+            o.val[l.base + e] = (int32_t)v;
+            if (KEYS) o.key[l.base + e] = (int32_t)l.key;
+            o.hash += pair_hash(KeyHash{l.hi2, l.add}, v);
+        }
+        __syncwarp();   // the list is read before the next round overwrites it
     }
 }
 
@@ -313,60 +354,72 @@ __device__ __forceinline__ void emit_unit(const sj_join_args &a, Out &o, uint32_
             next = a.keyStart[key] + a.candRel[rec + 32 * b + lane];
         }
     }
-    const KeyHash kh = key_hash(key);
-    uint32_t c0 = 0, myLive = 0, chunks = 0, x0 = 0, m = 0, nl = 0, any = 0;
+    __syncwarp();   // the previous unit is done with the lines
+    {
+        const KeyHash kh = key_hash(key);
+        w.line[lane] = LineInfo{next, key, kh.hi2, kh.add};
+    }
+    uint32_t c0 = 0, myLive = 0, chunks = 0, x0 = 0, m = 0;
     bool more = true;
+#pragma unroll 1
     do {
-        while (!m) {   // the next live words
-            if (!chunks) {
-                if (c0 >= nLive) {
-                    more = false;
-                    break;
+        // ---- stage the next live words, up to TW of them
+        uint32_t nl = 0, cut = 32;   // cut: values of the last word (32: all)
+#pragma unroll 1
+        while (nl < TW) {
+            if (!m) {
+                if (!chunks) {
+                    if (c0 >= nLive) {
+                        more = false;
+                        break;
+                    }
+                    myLive = row ? (c0 + lane < nLive ? __ldg(live + (uint64_t)(c0 + lane) * nG + k) : 0u)
+                                 : (lane == 0 ? colLive : 0u);
+                    chunks = __ballot_sync(FULL, myLive);
+                    c0 += 32;
+                    continue;
                 }
-                myLive = row ? (c0 + lane < nLive ? __ldg(live + (uint64_t)(c0 + lane) * nG + k) : 0u)
-                             : (lane == 0 ? colLive : 0u);
-                chunks = __ballot_sync(FULL, myLive);
-                c0 += 32;
-                continue;
+                const uint32_t ci = __ffs(chunks) - 1;
+                chunks &= chunks - 1;
+                m = __shfl_sync(FULL, myLive, ci);
+                x0 = (c0 - 32 + ci) * 32;
             }
-            const uint32_t ci = __ffs(chunks) - 1;
-            chunks &= chunks - 1;
-            m = __shfl_sync(FULL, myLive, ci);
-            x0 = (c0 - 32 + ci) * 32;
+            const uint32_t x = x0 + __ffs(m) - 1;
+            m &= m - 1;
+            const uint32_t rem = 32 * x < nv ? nv - 32 * x : 0u;   // values from the word's first on
+            copy_word(&w.tile[nl][lane], words + (uint64_t)x * stride + lane, lane < nLine && rem);
+            copy_word(&w.val[nl * 32 + lane], vals + 32 * x + lane, lane < rem);
+            if (rem < 32u) cut = rem;   // the stream's or the tile's last word
+            nl++;
         }
-        // up to LD words (and their values) in flight
-        uint32_t v[LD], c[LD], got = 0;
-#pragma unroll
-        for (uint32_t i = 0; i < LD; i++) {
-            v[i] = c[i] = 0;
-            if (m && nl + i < TW) {   // warp-uniform
-                const uint32_t x = x0 + __ffs(m) - 1;
-                m &= m - 1;
-                got++;
-                const uint32_t rem = 32 * x < nv ? nv - 32 * x : 0u;   // values from the word's first on
-                if (lane < nLine && rem) v[i] = __ldg(words + (uint64_t)x * stride + lane);
-                if (lane < rem) c[i] = __ldg(vals + 32 * x + lane);
-                if (rem < 32u && (v[i] >> rem) != 0u) {   // bits past the stream end or the tile
-                    atomicMax(&a.stat[6], 1ULL);
-                    v[i] &= (1u << rem) - 1u;
-                }
+        if (!nl) break;
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (cut < 32u) {   // this lane's own copy: the last word staged
+            const uint32_t v = w.tile[nl - 1][lane];
+            if (v >> cut) {   // bits past the stream end or the tile
+                atomicMax(&a.stat[6], 1ULL);
+                w.tile[nl - 1][lane] = v & ((1u << cut) - 1u);
             }
         }
-#pragma unroll
-        for (uint32_t i = 0; i < LD; i++) {
-            if (i < got) {
-                w.tile[nl + i][lane] = v[i];
-                w.val[(nl + i) * 32 + lane] = c[i];
-                any |= v[i];
-            }
+        uint32_t cnt = 0, nz = 0;   // lane = line
+#pragma unroll 4
+        for (uint32_t j = 0; j < nl; j++) {
+            const uint32_t v = w.tile[j][lane];
+            cnt += __popc(v);
+            if (v) nz |= 1u << j;
         }
-        nl += got;
-        if (nl == TW || (!more && nl)) {
+        if (__any_sync(FULL, cnt && (uint64_t)next + cnt > o.cap)) {   // a consistent count pass never gets here
+            atomicMax(&a.stat[3], 1ULL);
+        } else if (nl > 2 && __reduce_add_sync(FULL, cnt) >= SPARSE * nl) {
+            w.line[lane].base = next;
             __syncwarp();
-            emit_lines<KEYS>(a, o, w, lane, nl, __ballot_sync(FULL, any), key, kh, next);
+            emit_windows<KEYS>(o, w, lane, nl, __ballot_sync(FULL, cnt));
+        } else {
             __syncwarp();
-            nl = any = 0;
+            emit_lists<KEYS>(o, w, lane, cnt, nz, next + cnt);
         }
+        next += cnt;
+        __syncwarp();   // the words and lists are free again
     } while (more);
 }
 
@@ -387,17 +440,22 @@ __global__ void __launch_bounds__(EW, EMIT_MINB) k_emit(sj_join_args a)
     const uint32_t endGame = 8 * UN * gridDim.x * ENW;   // units left below which warps take them one by one
     uint32_t take = nUnits > endGame ? UN : 1u;
     for (;;) {
+        // (units are not taken ahead of their turn: a warp that holds one while it
+        // is busy with another costs more at the end than the counter's latency)
         uint32_t un = 0;
         if (lane == 0) un = atomicAdd(a.queueHead, take);
         un = __shfl_sync(FULL, un, 0);
         if (un >= nUnits) break;
         const uint32_t unEnd = nUnits - un < take ? nUnits : un + take;
         if (nUnits - un < endGame) take = 1;
-        // the first unit's task: the last t with unitOff[t] - u0 <= un
+        // the first unit's task: the last t with unitOff[t] - u0 <= un, 32 probes a step
         uint32_t lo = a.taskBegin, hi = a.taskEnd;
         while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (a.unitOff[mid] - u0 <= un) lo = mid; else hi = mid;
+            const uint32_t step = (hi - lo + 31) / 32;
+            const uint32_t probe = lo + (lane + 1) * step;
+            const bool below = probe < hi && a.unitOff[probe] - u0 <= un;   // a prefix of the lanes
+            lo += __popc(__ballot_sync(FULL, below)) * step;
+            hi = min(hi, lo + step);
         }
         uint32_t tBeg = (uint32_t)(a.unitOff[lo] - u0), tEnd = (uint32_t)(a.unitOff[lo + 1] - u0);
         for (; un < unEnd; un++) {
