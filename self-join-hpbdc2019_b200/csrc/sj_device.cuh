@@ -7,22 +7,39 @@
 
 namespace sjdev {
 
-__device__ __forceinline__ uint32_t transpose32(uint32_t x, uint32_t lane)
-{
-    // Lane i holds row i of a 32x32 bit matrix; afterwards lane j holds column j.
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-        const uint32_t lo = (s == 16) ? 0x0000ffffu
-                          : (s == 8)  ? 0x00ff00ffu
-                          : (s == 4)  ? 0x0f0f0f0fu
-                          : (s == 2)  ? 0x33333333u
-                                      : 0x55555555u;
-        uint32_t y = __shfl_xor_sync(0xffffffffu, x, s);
-        if (lane & s) x = (x & ~lo) | ((y & ~lo) >> s);
-        else x = (x & lo) | ((y & lo) << s);
+// 32x32 bit-matrix transpose over a warp: lane i holds row i; afterwards lane j
+// holds column j.  The usual five exchange steps; the halves of a step's result
+// are merged by one byte permute (distances 16 and 8), or by a rotation and one
+// three-input select (4, 2, 1), with the selectors, rotations and masks that
+// depend on the lane made once: 13 instructions a transpose, half of the
+// shift-and-mask form.
+struct Transpose {
+    uint32_t sel16, sel8, rot4, rot2, rot1, keep4, keep2, keep1;
+
+    __device__ __forceinline__ explicit Transpose(uint32_t lane)
+    {
+        sel16 = (lane & 16u) ? 0x3276u : 0x5410u;
+        sel8 = (lane & 8u) ? 0x3715u : 0x6240u;
+        rot4 = (lane & 4u) ? 28u : 4u;
+        rot2 = (lane & 2u) ? 30u : 2u;
+        rot1 = (lane & 1u) ? 31u : 1u;
+        keep4 = (lane & 4u) ? 0xf0f0f0f0u : 0x0f0f0f0fu;
+        keep2 = (lane & 2u) ? 0xccccccccu : 0x33333333u;
+        keep1 = (lane & 1u) ? 0xaaaaaaaau : 0x55555555u;
     }
-    return x;
-}
+
+    __device__ __forceinline__ uint32_t operator()(uint32_t x) const
+    {
+        x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 16), sel16);
+        x = __byte_perm(x, __shfl_xor_sync(0xffffffffu, x, 8), sel8);
+        uint32_t y = __shfl_xor_sync(0xffffffffu, x, 4);
+        x = (x & keep4) | (__funnelshift_l(y, y, rot4) & ~keep4);
+        y = __shfl_xor_sync(0xffffffffu, x, 2);
+        x = (x & keep2) | (__funnelshift_l(y, y, rot2) & ~keep2);
+        y = __shfl_xor_sync(0xffffffffu, x, 1);
+        return (x & keep1) | (__funnelshift_l(y, y, rot1) & ~keep1);
+    }
+};
 
 // Candidate-validity masks of a block of 32 stream positions starting at blk.
 // Inside a symmetric home segment (stream positions < homeEnd are the home

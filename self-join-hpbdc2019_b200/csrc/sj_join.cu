@@ -94,7 +94,7 @@ __device__ __forceinline__ bool exact_hit(const sj_join_args &a, uint32_t cpos, 
 
 template <int DP>
 struct __align__(16) Stage64 {
-    static constexpr int S = (DP <= 8) ? SJ_STAGE : ((SJ_STAGE * 8 / DP) / 32) * 32;
+    static constexpr int S = (DP <= 8) ? SJ_STAGE : SJ_STAGE / 2;   // divides 1024: 32 blocks of live bits
     double c[S][DP];
 };
 
@@ -339,6 +339,7 @@ __global__ void __launch_bounds__(SJ_CTA, sj_join_min_blocks(DP, F32)) k_join(sj
     const int D = g.D;
     const double T = g.thresh;
 
+    const Transpose transpose(lane);
     for (int j = tid; j < NW * S; j += SJ_CTA) (&colCnt[0][0])[j] = 0;
 
     // this kernel's tasks of the range: entries [first, first + count) of bigList
@@ -434,7 +435,7 @@ __global__ void __launch_bounds__(SJ_CTA, sj_join_min_blocks(DP, F32)) k_join(sj
         float2 nt[R];                           // (-tLo, -tLo)
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            const uint32_t qi = ((uint32_t)r * NW + warp) * 32 + lane;
+            const uint32_t qi = (uint32_t)r * SJ_CTA + tid;
             const bool v = (uint32_t)r < nAct && qi < task.qCount;
             double src[DP];
             qid[r] = load_query<DP>(a, task, v ? qi : 0u, D, src);
@@ -470,6 +471,7 @@ __global__ void __launch_bounds__(SJ_CTA, sj_join_min_blocks(DP, F32)) k_join(sj
 
         uint32_t rowCount[R];   // pairs keyed by each query
         uint32_t live[R];       // blocks of the current 32 in which the group has a hit
+        uint32_t colPairs = 0;  // pairs keyed by the candidates this thread adds up
         uint32_t evals = 0;     // candidate evaluations
         uint32_t refined = 0;   // FP32 borderline re-evaluations
 #pragma unroll
@@ -542,39 +544,42 @@ __global__ void __launch_bounds__(SJ_CTA, sj_join_min_blocks(DP, F32)) k_join(sj
                 }
                 tiles = __ballot_sync(0xffffffffu, alive);
             }
-            // ---- hit masks of every block of the stage.  A warp without
-            // queries skips the evaluation (but not the barriers).
+            // ---- hit masks of the blocks that have a tile left.  Only these are
+            // visited, and everything a tile needs beyond its distances waits for a
+            // hit (record addresses, counts) or for the end of the stage (live
+            // bits): with 32 blocks of distances at ~130 instructions a slot, the
+            // rest of a tile counts as much.  Count pass at 2-D 21.3 to 15.4 ms,
+            // 4-D 39.3 to 30.7, 6-D 74.6 to 62.2 (1M points), 8-D 6.56 to 6.34
+            // against visiting every block with all of it.
+            uint32_t blocks = (tiles | (tiles >> 8) | (tiles >> 16) | (tiles >> 24)) & 0xffu;
 #pragma unroll 1
-            for (uint32_t jb = 0; nAct != 0 && jb < nIn; jb += 32) {
+            while (blocks) {
+                const uint32_t bi = __ffs(blocks) - 1;
+                blocks &= blocks - 1;
+                const uint32_t jb = bi * 32, blk = sBase + jb;
                 const uint32_t nb = min(32u, nIn - jb);
-                const uint32_t inRange = (nb == 32) ? 0xffffffffu : ((1u << nb) - 1u);
+                const uint32_t inRange = 0xffffffffu >> (32u - nb);
+                const uint32_t col = (tiles >> bi) & 0x01010101u;   // bit 8 r: slot r
+                const uint32_t act = (col | (col >> 7) | (col >> 14) | (col >> 21)) & 15u;
                 uint32_t hits[R], ymin[R];
 #pragma unroll
                 for (int r = 0; r < R; r++) { hits[r] = 0; ymin[r] = 0xffffffffu; }
-                const uint32_t col = (tiles >> (jb >> 5)) & 0x01010101u;   // bit 8 r: slot r
-                const uint32_t act = (col | (col >> 7) | (col >> 14) | (col >> 21)) & 15u;
-                if (act) {
-                    eval_slots<DP, F32, R>(act, nAct, [&](auto r0, auto rr) {
-                        if constexpr (F32)
-                            eval_block_f32<DP, decltype(r0)::value, decltype(rr)::value, R>(st, jb >> 1, qa, nt, hits, ymin);
-                        else
-                            eval_block_f64<DP, decltype(r0)::value, decltype(rr)::value, R>(st, jb, q64, T1, hits);
-                    });
-                }
-                const uint32_t blk = sBase + jb;
+                eval_slots<DP, F32, R>(act, nAct, [&](auto r0, auto rr) {
+                    if constexpr (F32)
+                        eval_block_f32<DP, decltype(r0)::value, decltype(rr)::value, R>(st, jb >> 1, qa, nt, hits, ymin);
+                    else
+                        eval_block_f64<DP, decltype(r0)::value, decltype(rr)::value, R>(st, jb, q64, T1, hits);
+                });
                 const uint32_t hb = home_bits(blk, homeEnd, sym);
                 const uint32_t bInTask = (blk - task.sBegin) >> 5;
-                // record addresses of this block: row words [block][query],
-                // column words [block][query group][candidate]
-                uint32_t *const rowRec = rowBase ? rowBase + (uint64_t)bInTask * task.qCount + tid : nullptr;
-                uint32_t *const colRec = colBase ? colBase + (uint64_t)bInTask * nG * 32 + tid : nullptr;
                 uint32_t colHits = 0;   // this lane's candidate: hits over the warp's slots
 #pragma unroll
                 for (int r = 0; r < R; r++) {
                     if (!((act >> r) & 1u)) continue;   // warp-uniform
-                    const uint32_t qi = ((uint32_t)r * NW + warp) * 32 + lane;
+                    const uint32_t qi = (uint32_t)r * SJ_CTA + tid;
                     const bool qValid = qi < task.qCount;
-                    const uint32_t rowValid = qValid ? (hb ? (inRange & row_keep(qi, blk, hb)) : inRange) : 0u;
+                    uint32_t rowValid = qValid ? inRange : 0u;
+                    if (hb) rowValid &= row_keep(qi, blk, hb);
                     uint32_t h = hits[r];
                     if constexpr (F32) {
                         if (ymin[r] < __float_as_uint(a.delta)) {
@@ -597,28 +602,32 @@ __global__ void __launch_bounds__(SJ_CTA, sj_join_min_blocks(DP, F32)) k_join(sj
                     const uint32_t rowMask = h & rowValid;   // lane = query, bit = candidate
                     if (!__any_sync(0xffffffffu, rowMask)) continue;   // no hit in the tile
                     live[r] |= 1u << (bInTask & 31);
-                    if (rowRec && qValid) rowRec[r * SJ_CTA] = rowMask;
+                    // row words [block][query], column words [block][query group][candidate]
+                    if (rowBase && qValid) rowBase[bInTask * task.qCount + qi] = rowMask;
                     rowCount[r] += __popc(rowMask);
                     if (sym) {
                         // the mirrored direction: lane L gets candidate L's hits
-                        const uint32_t mir = hb ? (rowMask & mir_keep(qi, blk, hb)) : rowMask;
-                        const uint32_t colW = transpose32(mir, lane);
+                        uint32_t mir = rowMask;
+                        if (hb) mir &= mir_keep(qi, blk, hb);
+                        const uint32_t colW = transpose(mir);
                         colHits += __popc(colW);
-                        if (colRec) colRec[r * SJ_CTA] = colW;
+                        if (colBase) colBase[bInTask * nG * 32 + qi] = colW;
                     }
                 }
-                if (liveBase && ((bInTask & 31) == 31 || bInTask + 1 == nBlk)) {
+                if (sym) colCnt[warp][jb + lane] = colHits;
+            }
+            // the live bits of 32 blocks are complete (a stage never crosses them)
+            const uint32_t bEnd = (sBase + nIn - task.sBegin + 31) >> 5;   // blocks so far
+            if ((bEnd & 31) == 0 || bEnd == nBlk) {
 #pragma unroll
-                    for (int r = 0; r < R; r++) {
-                        if ((uint32_t)r < nAct && lane == 0) liveBase[(bInTask >> 5) * nG + r * NW + warp] = live[r];
-                        live[r] = 0;
-                    }
+                for (int r = 0; r < R; r++) {
+                    if (liveBase && (uint32_t)r < nAct && lane == 0)
+                        liveBase[((bEnd - 1) >> 5) * nG + r * NW + warp] = live[r];
+                    live[r] = 0;
                 }
-                if (sym && colHits) colCnt[warp][jb + lane] += colHits;
             }
             if (sym) {
                 __syncthreads();
-                uint32_t local = 0;
                 for (uint32_t j = tid; j < nIn; j += SJ_CTA) {
                     uint32_t tot = 0;
 #pragma unroll
@@ -627,18 +636,17 @@ __global__ void __launch_bounds__(SJ_CTA, sj_join_min_blocks(DP, F32)) k_join(sj
                     // these column pairs inside the candidate's key run
                     const uint32_t rel = tot ? atomicAdd(&a.keyCount[candId[j]], tot) : 0u;
                     if (candRelRec) candRelRec[sBase + j - task.sBegin] = rel;
-                    local += tot;
+                    colPairs += tot;
                 }
-                if (local) atomicAdd(&sm.taskPairs, (unsigned long long)local);
             }
         }
         {
-            uint32_t mine = 0;
+            unsigned long long mine = colPairs;
             uint32_t *const relBase = a.rowRel ? a.rowRel + (a.rowOff[t] - a.rowOff[a.taskBegin]) : nullptr;
 #pragma unroll
             for (int r = 0; r < R; r++) {
                 if ((uint32_t)r >= nAct) continue;
-                const uint32_t qi = ((uint32_t)r * NW + warp) * 32 + lane;
+                const uint32_t qi = (uint32_t)r * SJ_CTA + tid;
                 // evaluations of this query: stream positions [sBegin, sEnd), in the
                 // symmetric home segment only those at or after the query itself
                 if (qi < task.qCount) {
@@ -651,7 +659,9 @@ __global__ void __launch_bounds__(SJ_CTA, sj_join_min_blocks(DP, F32)) k_join(sj
                 if (relBase && qi < task.qCount) relBase[qi] = rel;
                 mine += rowCount[r];
             }
-            if (mine) atomicAdd(&sm.taskPairs, (unsigned long long)mine);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+            if (lane == 0 && mine) atomicAdd(&sm.taskPairs, mine);
         }
         // ---- statistics (per task: a re-run of the task overwrites them)
         unsigned long long e = evals, rf = refined;
