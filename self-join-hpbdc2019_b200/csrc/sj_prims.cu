@@ -41,16 +41,74 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *t
     return warpPrefix + x - v;
 }
 
+// A thread's SCAN_ITEMS consecutive elements as two 16-byte accesses where the
+// array allows them (base is a multiple of SCAN_ITEMS): a batch's key counts are
+// read twice and written twice per scan, and in 4-byte steps a warp's access
+// touches every 32-byte sector eight times.
+static_assert(SCAN_ITEMS == 8, "two 16-byte accesses a thread");
+
+__device__ __forceinline__ bool scan_wide(const uint32_t *p, uint64_t base, uint64_t n)
+{
+    return base + SCAN_ITEMS <= n && (reinterpret_cast<uintptr_t>(p) & 15u) == 0;
+}
+
+__device__ __forceinline__ void scan_load(const uint32_t *in, uint64_t base, uint64_t n, uint32_t (&v)[SCAN_ITEMS])
+{
+    if (scan_wide(in, base, n)) {
+        const uint4 x = *reinterpret_cast<const uint4 *>(in + base), y = *reinterpret_cast<const uint4 *>(in + base + 4);
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+        v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < SCAN_ITEMS; i++) v[i] = (base + i < n) ? in[base + i] : 0u;
+    }
+}
+
+__device__ __forceinline__ void scan_store(uint32_t *out, uint64_t base, uint64_t n, const uint32_t (&v)[SCAN_ITEMS])
+{
+    if (scan_wide(out, base, n)) {
+        *reinterpret_cast<uint4 *>(out + base) = make_uint4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<uint4 *>(out + base + 4) = make_uint4(v[4], v[5], v[6], v[7]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < SCAN_ITEMS; i++)
+            if (base + i < n) out[base + i] = v[i];
+    }
+}
+
+// Scans the block's tile with `off` as its offset; returns the tile's total.
+__device__ __forceinline__ uint32_t scan_tile(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *zeroIn,
+                                              uint32_t blockOff)
+{
+    const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + (uint64_t)threadIdx.x * SCAN_ITEMS;
+    uint32_t v[SCAN_ITEMS], s = 0;
+    scan_load(in, base, n, v);
+#pragma unroll
+    for (int i = 0; i < SCAN_ITEMS; i++) s += v[i];
+    if (zeroIn) {
+        const uint32_t zero[SCAN_ITEMS] = {};
+        scan_store(zeroIn, base, n, zero);
+    }
+    uint32_t tot;
+    uint32_t off = blockOff + block_exclusive_scan(s, &tot);
+#pragma unroll
+    for (int i = 0; i < SCAN_ITEMS; i++) {
+        const uint32_t x = v[i];
+        v[i] = off;
+        off += x;
+    }
+    scan_store(out, base, n, v);
+    return tot;
+}
+
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const uint32_t *__restrict__ in, uint64_t n,
                                                               uint32_t *__restrict__ sums)
 {
-    uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE;
-    uint32_t s = 0;
+    const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + (uint64_t)threadIdx.x * SCAN_ITEMS;
+    uint32_t v[SCAN_ITEMS], s = 0;
+    scan_load(in, base, n, v);
 #pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; i++) {
-        uint64_t idx = base + (uint64_t)i * SCAN_THREADS + threadIdx.x;
-        if (idx < n) s += in[idx];
-    }
+    for (int i = 0; i < SCAN_ITEMS; i++) s += v[i];
     uint32_t tot;
     block_exclusive_scan(s, &tot);
     if (threadIdx.x == 0) sums[blockIdx.x] = tot;
@@ -62,29 +120,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tile(const uint32_t *in, 
                                                             const uint32_t *__restrict__ blockOffsets,
                                                             uint32_t *total_dev, uint32_t *zeroIn)
 {
-    uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + (uint64_t)threadIdx.x * SCAN_ITEMS;
-    uint32_t v[SCAN_ITEMS];
-    uint32_t s = 0;
-#pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; i++) {
-        uint64_t idx = base + i;
-        v[i] = (idx < n) ? in[idx] : 0u;
-        s += v[i];
-    }
-    if (zeroIn) {
-#pragma unroll
-        for (int i = 0; i < SCAN_ITEMS; i++)
-            if (base + i < n) zeroIn[base + i] = 0u;
-    }
-    uint32_t tot;
-    uint32_t pre = block_exclusive_scan(s, &tot);
-    uint32_t off = (blockOffsets ? blockOffsets[blockIdx.x] : 0u) + pre;
-#pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; i++) {
-        uint64_t idx = base + i;
-        if (idx < n) out[idx] = off;
-        off += v[i];
-    }
+    const uint32_t tot = scan_tile(in, out, n, zeroIn, blockOffsets ? blockOffsets[blockIdx.x] : 0u);
     if (!blockOffsets && total_dev && threadIdx.x == 0) *total_dev = tot;
 }
 
@@ -101,28 +137,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tile_lookup(const uint32_
     for (uint32_t b = threadIdx.x; b < blockIdx.x; b += SCAN_THREADS) part += sums[b];
     uint32_t blockOff;   // sum of all earlier tiles (the block total of the parts)
     block_exclusive_scan(part, &blockOff);
-    const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + (uint64_t)threadIdx.x * SCAN_ITEMS;
-    uint32_t v[SCAN_ITEMS];
-    uint32_t sum = 0;
-#pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; i++) {
-        const uint64_t idx = base + i;
-        v[i] = (idx < n) ? in[idx] : 0u;
-        sum += v[i];
-    }
-    if (zeroIn) {
-#pragma unroll
-        for (int i = 0; i < SCAN_ITEMS; i++)
-            if (base + i < n) zeroIn[base + i] = 0u;
-    }
-    uint32_t tot;
-    uint32_t off = blockOff + block_exclusive_scan(sum, &tot);
-#pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; i++) {
-        const uint64_t idx = base + i;
-        if (idx < n) out[idx] = off;
-        off += v[i];
-    }
+    const uint32_t tot = scan_tile(in, out, n, zeroIn, blockOff);
     if (total_dev && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total_dev = blockOff + tot;
 }
 
