@@ -64,6 +64,34 @@ __device__ __forceinline__ double ref_dist2(const double *c, const double *q)
     return acc;
 }
 
+// N coordinates from dimension l0 on of the point at position pos of the join's
+// order, in the widest loads that rows of DP doubles allow (32 bytes, 16 bytes;
+// rows start on a multiple of that, the array on 256 bytes): a lane loads its own
+// point, so every load instruction touches 32 lines whatever its width.
+template <int DP, int L0 = 0, int N = DP>
+__device__ __forceinline__ void load_point(const double *__restrict__ xs, uint64_t pos, double *x)
+{
+    static_assert(L0 % 4 == 0 && L0 + N <= DP, "part of a point");
+    const double *const src = xs + pos * DP + L0;
+    if constexpr (DP % 4 == 0 && N % 4 == 0) {
+#pragma unroll
+        for (int l = 0; l < N; l += 4)
+            asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                : "=d"(x[l]), "=d"(x[l + 1]), "=d"(x[l + 2]), "=d"(x[l + 3])
+                : "l"(src + l));
+    } else if constexpr (DP % 2 == 0 && N % 2 == 0) {
+#pragma unroll
+        for (int l = 0; l < N; l += 2) {
+            const double2 v = __ldg(reinterpret_cast<const double2 *>(src + l));
+            x[l] = v.x;
+            x[l + 1] = v.y;
+        }
+    } else {
+#pragma unroll
+        for (int l = 0; l < N; l++) x[l] = __ldg(src + l);
+    }
+}
+
 // Coordinates and point id of a task's query qi.  The sampling estimate's
 // queries are the first of their cell in the index's order: its points in id
 // order, so the sample covers the cell whatever the join's order of its points.
@@ -78,8 +106,7 @@ __device__ __forceinline__ uint32_t load_query(const sj_join_args &a, const sj_t
         return id;
     }
     const uint64_t pos = t.qBegin + qi;
-#pragma unroll
-    for (int l = 0; l < DP; l++) x[l] = a.xs[pos * DP + l];
+    load_point<DP>(a.xs, pos, x);
     return a.ids[pos];
 }
 
@@ -500,7 +527,8 @@ __global__ void __launch_bounds__(SJ_CTA, sj_join_min_blocks(DP, F32)) k_join(sj
                     const uint32_t cid = a.ids[pos];
                     candId[j] = cid;
                     if (candIdRec) candIdRec[s - task.sBegin] = cid;   // the emission's candidate record
-                    const double *src = a.xs + (uint64_t)pos * DP;
+                    double src[DP];
+                    load_point<DP>(a.xs, pos, src);
                     double nb = 0.0;
 #pragma unroll
                     for (int l = 0; l < DP; l++) {
@@ -698,7 +726,19 @@ __global__ void __launch_bounds__(SJ_CTA, sj_join_min_blocks(DP, F32)) k_join(sj
 // segments go by 32 at a time in registers.  Same operations in the same order
 // as k_join, same records.
 // Bound: instruction issue (per block of 32 candidates ~60 instructions and
-// ~12 + D per query).  Measured against k_join on the same tasks: see DESIGN.
+// ~12 + D per query), and for wide points the conversions of the candidates'
+// coordinates to FP32 and back for |b|^2, four lanes a cycle each: what the test
+// of the first-loaded dimensions saves.  The tasks of 1M clustered points in 16-D
+// took k_join 20.4 ms more than its other tasks, this kernel 4.7 ms.
+// Dimensions that are loaded and tested first, the last of the padded width: a
+// point whose distance in these alone exceeds the radius is out.  The last
+// dimensions, because the grid has already put the first (indexed) ones close
+// together.  Points of 12 or 16 only: 1M clustered points in 16-D, 9.63 to 4.68 ms
+// (5.23 with four dimensions); 500k in 12-D 1.86 to 1.67 (1.87 with four); in 8-D
+// the test of the last four gives nothing (1.49 ms either way).
+template <int DP>
+constexpr int PRE_DIMS = DP >= 12 ? 8 : 0;
+
 template <int DP, bool F32>
 struct __align__(16) SmallSmem {
     static constexpr int CW2 = Stage32<DP>::CW2;
@@ -707,14 +747,32 @@ struct __align__(16) SmallSmem {
     double q[F32 ? 1 : SJ_SMALL_QUERIES][DP];
     float2 box[DP];             // (min, max) of the queries' local coordinates
     double origin[DP];
+    // per pair of queries the (-a_l) of the dimensions that are tested first
+    float2 pre[PRE_DIMS<DP> ? SJ_SMALL_QUERIES / 2 : 1][PRE_DIMS<DP> ? PRE_DIMS<DP> : 2];
 };
+
+// Squared distance of a point's dimensions [L0, L0 + N) to the box, in FP32.
+template <int L0, int N>
+__device__ __forceinline__ float box_dist2(const float2 *box, const float *x)
+{
+    float d2 = 0.0f;
+#pragma unroll
+    for (int l = L0; l < L0 + N; l++) {
+        const float2 q = box[l];
+        const float gap = fmaxf(0.0f, fmaxf(x[l] - q.y, q.x - x[l]));
+        d2 = fmaf(gap, gap, d2);
+    }
+    return d2;
+}
 
 constexpr uint32_t SMALL_BOX = 6;   // queries from which on testing a block against their box pays
 
 template <int DP, bool F32>
-__global__ void __launch_bounds__(SJ_CTA, DP <= 8 ? 6 : 4) k_join_small(sj_join_args a, sj_grid_dev g, int queue)
+__global__ void __launch_bounds__(SJ_CTA, DP <= 4 ? 6 : DP <= 8 ? 5 : 4) k_join_small(sj_join_args a, sj_grid_dev g, int queue)
 {
     constexpr uint32_t FULL = 0xffffffffu;
+    constexpr int PD = PRE_DIMS<DP>;
+    constexpr int ND = PD ? PD : DP;   // dimensions loaded ahead
     __shared__ SmallSmem<DP, F32> smem[NW];
     const uint32_t lane = threadIdx.x & 31u;
     SmallSmem<DP, F32> &sm = smem[threadIdx.x >> 5];
@@ -763,6 +821,10 @@ __global__ void __launch_bounds__(SJ_CTA, DP <= 8 ? 6 : 4) k_join_small(sj_join_
                 if (qc >= SMALL_BOX) {
                     const float2 mm = warp_min_max(lane < qc ? ql : INFINITY, lane < qc ? ql : -INFINITY);
                     if (lane == 0) sm.box[l] = mm;
+                }
+                if constexpr (PD > 0) {   // no query: infinitely far
+                    if (l >= DP - PD)
+                        reinterpret_cast<float *>(&sm.pre[lane >> 1][l - (DP - PD)])[lane & 1] = lane < qc ? -ql : INFINITY;
                 }
                 if constexpr (F32) {
                     reinterpret_cast<float *>(&sm.q2[lane >> 1][1 + l])[lane & 1] = -2.0f * ql;
@@ -834,9 +896,8 @@ __global__ void __launch_bounds__(SJ_CTA, DP <= 8 ? 6 : 4) k_join_small(sj_join_
         };
         // the next block's candidates are loaded while this one is evaluated
         uint32_t nPos = locate(task.sBegin), nId = a.ids[nPos];
-        double nx[DP];
-#pragma unroll
-        for (int l = 0; l < DP; l++) nx[l] = a.xs[(uint64_t)nPos * DP + l];
+        double nx[ND];
+        load_point<DP, DP - ND, ND>(a.xs, nPos, nx);
 #pragma unroll 1
         for (uint32_t b = 0; b < nBlk; b++) {
             const uint32_t blk = task.sBegin + 32 * b;
@@ -845,12 +906,11 @@ __global__ void __launch_bounds__(SJ_CTA, DP <= 8 ? 6 : 4) k_join_small(sj_join_
             const uint32_t cpos = nPos, cid = nId;
             double c[DP];
 #pragma unroll
-            for (int l = 0; l < DP; l++) c[l] = nx[l];
+            for (int l = 0; l < ND; l++) c[DP - ND + l] = nx[l];
             if (b + 1 < nBlk) {
                 nPos = locate(blk + 32);
                 nId = a.ids[nPos];
-#pragma unroll
-                for (int l = 0; l < DP; l++) nx[l] = a.xs[(uint64_t)nPos * DP + l];
+                load_point<DP, DP - ND, ND>(a.xs, nPos, nx);
             }
             if (candIdRec && in) candIdRec[s - task.sBegin] = cid;
             const bool home = sym && s < homeEnd;
@@ -858,22 +918,39 @@ __global__ void __launch_bounds__(SJ_CTA, DP <= 8 ? 6 : 4) k_join_small(sj_join_
             uint32_t rowWord = 0, colW = 0;
             float bl[DP];
 #pragma unroll
-            for (int l = 0; l < DP; l++) {
-                bl[l] = (l < D) ? __double2float_rn(c[l] - sm.origin[l]) : 0.0f;
-            }
+            for (int l = DP - ND; l < DP; l++) bl[l] = (l < D) ? __double2float_rn(c[l] - sm.origin[l]) : 0.0f;
             // the block is ruled out when every candidate lies further from the
-            // queries' box than the radius (as k_join's tiles)
+            // queries (few) or their box than the radius (as k_join's tiles: pruneT
+            // holds for single points, and for a part of the dimensions)
             bool alive = true;
-            if (qc >= SMALL_BOX) {
-                float d2 = 0.0f;
+            if constexpr (PD > 0) {
+                float m = INFINITY;
+                if (qc >= SMALL_BOX) {
+                    m = box_dist2<DP - PD, PD>(sm.box, bl);
+                } else {
+                    for (uint32_t p = 0; 2 * p < qc; p++) {
+                        float2 d2 = make_float2(0.0f, 0.0f);
+                        const float4 *const row4 = reinterpret_cast<const float4 *>(&sm.pre[p][0]);
 #pragma unroll
-                for (int l = 0; l < DP; l++) {
-                    const float2 q = sm.box[l];
-                    const float gap = fmaxf(0.0f, fmaxf(bl[l] - q.y, q.x - bl[l]));
-                    d2 = fmaf(gap, gap, d2);
+                        for (int l = 0; l < PD; l += 2) {
+                            const float4 v = row4[l / 2];
+                            const float b0 = bl[DP - PD + l], b1 = bl[DP - PD + l + 1];
+                            const float2 t0 = __fadd2_rn(make_float2(b0, b0), make_float2(v.x, v.y));
+                            const float2 t1 = __fadd2_rn(make_float2(b1, b1), make_float2(v.z, v.w));
+                            d2 = __ffma2_rn(t0, t0, d2);
+                            d2 = __ffma2_rn(t1, t1, d2);
+                        }
+                        m = fminf(m, fminf(d2.x, d2.y));
+                    }
                 }
-                alive = __any_sync(FULL, in && !(d2 > a.pruneT));
+                alive = __any_sync(FULL, in && !(m > a.pruneT));
+                if (alive) {
+                    load_point<DP, 0, DP - PD>(a.xs, cpos, c);
+#pragma unroll
+                    for (int l = 0; l < DP - PD; l++) bl[l] = (l < D) ? __double2float_rn(c[l] - sm.origin[l]) : 0.0f;
+                }
             }
+            if (alive && qc >= SMALL_BOX) alive = __any_sync(FULL, in && !(box_dist2<0, DP>(sm.box, bl) > a.pruneT));
             if (!alive) {
                 // no hit: nothing to record but the candidates' ids
             } else if constexpr (F32) {
