@@ -148,3 +148,10 @@ def test_csr_of_one_batch(mode, prec):
     keys = np.repeat(np.arange(n), deg)
     assert np.array_equal(c[:len(ok)][np.lexsort((c[:len(ok)], keys))], ov)
     assert np.array_equal(row.cpu().numpy(), want)
+
+
+def test_many_small_units():
+    # more than a million emission units of a few pairs each: warps take several
+    # at a time and step over the dead ones
+    pts = np.random.default_rng(5).random((750_000, 2))
+    _check(pts, 0.0006, 2, 6, sjoin.PREC_FP32_REFINE)
