@@ -8,8 +8,9 @@
 // sub-stencils drop out early (sparse high-dimensional grids).  The levels are
 // walked breadth first: eight prefixes at a time, four lanes each, the four
 // lanes searching the four bounds of the prefix's three children; the children
-// that hold cells are compacted, in id order, into the next level's list.  A
-// walk whose lowest TREE_DIMS dimensions are reached depth first (k > TREE_DIMS)
+// that hold cells are compacted, in id order, into the next level's list.  The
+// last dimension takes a lane a prefix: its up to three cells follow one another
+// in the id array, so one search finds them.  A walk whose lowest TREE_DIMS dimensions are reached depth first (k > TREE_DIMS)
 // keeps the lists at 3^(TREE_DIMS-1) entries.
 // Bound: latency of the dependent searches (about 60 steps a cell at k = 6, which
 // the lanes of a warp take side by side).  One thread a cell, depth first with
@@ -107,8 +108,10 @@ struct NbrSmem {
 
 // pass 0: count owned neighbours (out = counts), full-stencil candidates and
 //         features; pass 1: write owned neighbour cell indices (out = list).
-// Measured (both passes, one B200): 466,982 cells at k = 6 20.3 to 7 ms, 5,583 and
-// 6,980 cells at k = 6 3.7 to 0.1 ms.
+// Measured (both passes, one B200): 466,982 cells at k = 6 20.3 ms depth first,
+// 6.93 breadth first with four lanes a prefix at the leaves too, 5.88 with one;
+// 5,583 and 6,980 cells at k = 6 3.7 to 0.1 ms; 125k cells at k = 3 0.27 to 0.17 ms
+// with one lane a prefix at the leaves.
 // GROUP lanes a cell: 32, or 8 where the tree has at most 27 leaves (two prefixes
 // at a time; a warp then has four cells).
 template <int DIMS, int GROUP>
@@ -134,6 +137,7 @@ __global__ void __launch_bounds__(NBR_THREADS) k_neighbours(
     const uint32_t a0 = shfl(aj, 0), a1 = shfl(aj, 1), a2 = shfl(aj, 2);
     const uint32_t myOcc = cellStart[c + 1] - cellStart[c];
     const uint32_t ltmask = (1u << lane) - 1u;
+    const uint32_t highHome = k < 16 ? CODE_HOME << (2 * k) : 0u;   // dimensions at or above k are unchanged
     // bound q of the children of a prefix in dimension j: the first of its cells
     // [lo, hi) at or after coordinate a_j - 1 + q (q = lane & 3)
     const uint32_t q = lane & 3u;
@@ -202,7 +206,7 @@ __global__ void __launch_bounds__(NBR_THREADS) k_neighbours(
             L.code[0] = dCode;
         }
         __syncwarp(FULL);
-        for (int j = k - 1 - depth; j >= 0; j--) {
+        for (int j = k - 1 - depth; j > 0 && n; j--) {
             const uint32_t a = shfl(aj, j);
             uint32_t made = 0;
             for (uint32_t i0 = 0; i0 < n; i0 += GROUP / 4) {
@@ -218,24 +222,41 @@ __global__ void __launch_bounds__(NBR_THREADS) k_neighbours(
                 const bool have = i < n && q < 3 && r < end && !(q == 0 && a == 0) && a + q - 1u < g.nCells[j];
                 const uint32_t m = ballot(have);
                 code |= q << (2 * j);
-                if (j > 0) {
-                    if (have) {
-                        const uint32_t at = made + __popc(m & ltmask);
-                        N.lo[at] = r;
-                        N.hi[at] = end;
-                        N.base[at] = base + ((unsigned long long)a + q - 1ULL) * g.mult[j];
-                        N.code[at] = code;
-                    }
-                    made += __popc(m);
-                    continue;
-                }
-                // leaves: one cell each (mult[0] == 1)
-                bool own = false;
                 if (have) {
-                    // dimensions at or above k count as unchanged
-                    const uint32_t full = k < 16 ? code | (CODE_HOME << (2 * k)) : code;
+                    const uint32_t at = made + __popc(m & ltmask);
+                    N.lo[at] = r;
+                    N.hi[at] = end;
+                    N.base[at] = base + ((unsigned long long)a + q - 1ULL) * g.mult[j];
+                    N.code[at] = code;
+                }
+                made += __popc(m);
+            }
+            __syncwarp(FULL);
+            n = made;
+            const TreeRef x = L;
+            L = N;
+            N = x;
+        }
+        // ---- leaves, a lane a prefix: its cells with coordinate a0 - 1 to a0 + 1 in
+        // dimension 0 follow one another in the id array (mult[0] == 1), so one
+        // search finds them all
+        for (uint32_t i0 = 0; i0 < n; i0 += GROUP) {
+            const uint32_t i = i0 + lane;
+            uint32_t r0 = 0, ownBits = 0;
+            if (i < n) {
+                const unsigned long long base = L.base[i];
+                const uint32_t hi = L.hi[i], prefix = L.code[i] | highHome;
+                r0 = lower_bound_u64(cellLid, L.lo[i], hi, base + (a0 ? a0 - 1u : 0u));
+#pragma unroll
+                for (uint32_t e = 0; e < 3; e++) {
+                    const uint32_t r = r0 + e;
+                    if (r >= hi) break;
+                    const unsigned long long off = cellLid[r] - base;   // the cell's coordinate
+                    if (off > (unsigned long long)a0 + 1ULL) break;
+                    const uint32_t full = prefix | ((uint32_t)off + 1u - a0);
                     const bool home = r == c;
-                    own = !home && owns(pattern, k, a0, a1, a2, odd, full, c, r);
+                    const bool own = !home && owns(pattern, k, a0, a1, a2, odd, full, c, r);
+                    if (own) ownBits |= 1u << e;
                     if (pass == 0) {
                         const uint32_t occ = cellStart[r + 1] - cellStart[r];
                         stencilOcc += occ;
@@ -253,17 +274,23 @@ __global__ void __launch_bounds__(NBR_THREADS) k_neighbours(
                         }
                     }
                 }
-                const uint32_t om = ballot(own);
-                if (pass == 1 && own) out[writePos + owned + __popc(om & ltmask)] = r;
-                owned += __popc(om);
             }
-            __syncwarp(FULL);
-            n = made;
-            const TreeRef x = L;
-            L = N;
-            N = x;
-            if (n == 0) break;
+            const uint32_t cnt = __popc(ownBits);
+            uint32_t incl = cnt;
+#pragma unroll
+            for (int o = 1; o < GROUP; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULL, incl, o, GROUP);
+                if (lane >= (uint32_t)o) incl += y;
+            }
+            if (pass == 1) {
+                uint32_t at = writePos + owned + incl - cnt;
+#pragma unroll
+                for (uint32_t e = 0; e < 3; e++)
+                    if ((ownBits >> e) & 1u) out[at++] = r0 + e;
+            }
+            owned += shfl(incl, GROUP - 1);
         }
+        __syncwarp(FULL);
         if (depth == 0) break;
         depth--;
         t[depth]++;
