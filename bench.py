@@ -15,9 +15,9 @@ result batches of at most 2e9 pairs.
     hashes (the run exits non-zero if they differ).
 
 One step = grid-index build + estimate + batched join (per batch: count pass
-recording hit masks, scan of the per-key counts, key expansion, pair emission
-from the masks) + an on-device fold of every batch into the pair count and set
-hash, with the points already resident in HBM.  `e2e` is the same join through
+recording hit masks, scan of the per-key counts, emission of every pair from the
+masks: keys, values, and the set hash of what was written), with the points
+already resident in HBM.  `e2e` is the same join through
 the C ABI with host buffers: the points copied from pinned host memory and
 every batch's pairs delivered to host memory.
 
@@ -54,8 +54,7 @@ sys.path.insert(0, os.path.join(REPO, "self-join-hpbdc2019_b200"))
 ESTIMATOR_WEIGHTS = os.path.join(REPO, "self-join-hpbdc2019_b200", "sjoin", "estimator_c4.bin")
 
 # dram__bytes_read.sum + dram__bytes_write.sum per output pair of the emission
-# kernel (k_emit) in one ncu capture (profiles/k_emit_c4_n2M.md: the c4
-# generator at n = 2e6, one batch); the traffic grows with the pairs, so a
+# kernel (k_emit) when a capture has it; the traffic grows with the pairs, so a
 # full-size launch is scaled by its pairs
 EMIT_TRAFFIC_BYTES_PER_PAIR = None
 
@@ -438,7 +437,7 @@ def run_ours(args):
             e_ms = float(t.item())
         st_e = est[-1]
         if st_e["total_pairs"] != pairs or st_e["pair_hash"] != stats[-1]["pair_hash"]:
-            raise RuntimeError("host delivery produced a different pair set than the device fold")
+            raise RuntimeError("host delivery produced a different pair set than the device join")
         # host delivery copies each batch's values and its per-key run offsets
         # (the host expands the keys from them)
         e2e = {"value": job_pairs / (e_ms / 1e3), "unit": "pairs/s", "ms_per_step": e_ms, "steps": args.e2e_steps,
@@ -580,7 +579,7 @@ def main():
                     help="timed steps of the plain FP64 method on the same points (0: skip)")
     ap.add_argument("--e2e-steps", type=int, default=1, help="timed end-to-end steps with host delivery (0: skip)")
     ap.add_argument("--delivery", choices=["none", "device"], default="none",
-                    help="timed steps: on-device fold of every batch (none) or every batch handed to a "
+                    help="timed steps: batches written and hashed on the device (none) or every batch handed to a "
                          "device-memory consumer one at a time (device)")
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--no-stage-probe", action="store_true",

@@ -159,7 +159,7 @@ sj_status sj_index_export(sj_ctx *ctx, unsigned int *indexLookupArr, sj_grid *gr
 
 /* Replaces the batch loop of distanceTableNDGridBatches (GPU.cu:2086-2377):
  * estimates, plans batches, and streams every result batch to `cb`.
- * SJ_DELIVER_NONE runs the join and only folds each batch into the pair count
+ * SJ_DELIVER_NONE runs the join and only adds each batch to the pair count
  * and set hash (sj_stats). */
 sj_status sj_join(sj_ctx *ctx, int delivery, sj_batch_cb cb, void *user);
 

@@ -10,7 +10,8 @@
 //      for the work-queue / sorted modes (kernel.cu:33-250, GPU.cu:1660-1734)
 //   5. batches = consecutive tasks whose predicted pairs fit the capacity; per
 //      batch: count pass -> exclusive scan over point ids -> (split and retry
-//      on overflow) -> fill pass -> delivery (GPU.cu:2101-2377)
+//      on overflow) -> emission (keys, values, set hash) -> delivery
+//      (GPU.cu:2101-2377)
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -299,7 +300,7 @@ struct Ctx {
     // masks, per-query row-run offsets and per-position candidate records
     DevBuf<uint32_t> masks, colMasks, rowRel, candId, candRel;
     // the count pass of batch i + 1 writes this second record set while the
-    // emission of batch i reads the first (device-fold pipeline)
+    // emission of batch i reads the first (deliveries that stay on the device)
     DevBuf<uint32_t> masks2, colMasks2, rowRel2, candId2, candRel2;
     DevBuf<uint32_t> emitHead;   // the emission's work counter when it runs beside a count pass
     // device CSR neighbour table under construction (sj_neighbor_csr): the
@@ -1309,7 +1310,7 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
         }
     };
 
-    // ---- asynchronous phase: batches folded on the device (no host delivery).
+    // ---- asynchronous phase: batches that stay on the device (no host delivery).
     // Every batch runs count -> scan -> emission without a host round trip; a
     // batch whose count exceeds the output buffer skips its emission.  Such
     // batches are re-planned exactly from the count pass's

