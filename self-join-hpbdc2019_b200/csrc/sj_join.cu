@@ -343,9 +343,16 @@ struct __align__(16) JoinSmem {
 // evaluation.
 // Resident CTAs per SM the register allocation must allow.  FP32 filter: four,
 // five at six dimensions (4-D: 41.2 ms of count passes with four, 45.7 with
-// five; 8-D 7.2 against 7.6; 6-D 82 against 79).  FP64: three up to six
-// dimensions (29.6 ms against 36.4 with two on 6-D data), two above.
-constexpr int sj_join_min_blocks(int DP, bool F32) { return F32 ? (DP == 6 ? 5 : 4) : (DP <= 6 ? 3 : 2); }
+// five; 8-D 7.2 against 7.6; 6-D 82 against 79).  FP64: as many as leave the
+// queries in registers but for a few; its chain of dependent operations needs the
+// warps more than it minds the spills (with three, two above six dimensions: 2-D
+// 1.57 to 1.29 ms of count pass, 3-D 1.58 to 1.08, 4-D 3.91 to 3.02, 6-D 13.6 to
+// 12.1, 8-D 3.2 to 2.5).
+constexpr int sj_join_min_blocks(int DP, bool F32)
+{
+    if (F32) return DP == 6 ? 5 : 4;
+    return DP <= 4 ? 6 : DP <= 6 ? 5 : DP <= 8 ? 4 : 3;
+}
 
 template <int DP, bool F32, int R>
 __global__ void __launch_bounds__(SJ_CTA, sj_join_min_blocks(DP, F32)) k_join(sj_join_args a, sj_grid_dev g, int queue)
