@@ -271,12 +271,13 @@ __device__ __forceinline__ void eval_block_f64(const Stage64<DP> &st, uint32_t j
     }
 }
 
-// Minimum and maximum of v over the warp.
+// Minimum and maximum of v over the warp (every lane takes part).  volatile: its
+// callers use the result in one lane only, and a plain asm may be moved there.
 __device__ __forceinline__ float2 warp_min_max(float lo, float hi)
 {
     float2 r;
-    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r.x) : "f"(lo));
-    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r.y) : "f"(hi));
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r.x) : "f"(lo));
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r.y) : "f"(hi));
     return r;
 }
 
