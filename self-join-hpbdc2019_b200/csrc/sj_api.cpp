@@ -29,6 +29,7 @@
 #include <string>
 #include <vector>
 
+#include "sj_host.h"
 #include "sj_internal.h"
 
 namespace sj {
@@ -1122,9 +1123,7 @@ void expand_keys_host(const uint32_t *start, uint64_t n, uint64_t cnt, int32_t *
 {
     if (cnt == 0) return;
     static const bool avx2 = __builtin_cpu_supports("avx2");
-    // a thread per half a million keys: with every core in the team, a small batch
-    // waits for whichever core is busy with something else
-    const int team = (int)std::min<uint64_t>((uint64_t)omp_get_max_threads(), 1 + cnt / (1u << 19));
+    const int team = sj_expand_team(n, cnt, omp_get_max_threads());
 #pragma omp parallel num_threads(team)
     {
 #pragma omp for schedule(static)
