@@ -309,8 +309,8 @@ struct Ctx {
     uint64_t *csrRowPtr = nullptr;
     int32_t *csrCols = nullptr;
     uint64_t csrCap = 0;
-    bool csrDirect = false;    // rows not sized yet: a join of one batch emits straight into the caller's arrays
-    bool csrDone = false;      // ... and it did
+    bool csrDirect = false;    // the table is one batch, emitted straight into the caller's arrays
+    bool csrSized = false;     // its rows' lengths and offsets are known, csrTotal values in all
     uint64_t csrTotal = 0;
     DevBuf<uint32_t> csrFill;
     DevBuf<unsigned long long> csrWide, csrScan;
@@ -1196,8 +1196,6 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
         CKS(plan_dev(c, cap, plan, maxes, predTotal));
         c.tmTasks.stop(c.s);
     }
-    // the rows of a table of several batches have to be sized first
-    if (delivery == SJ_DELIVER_CSR && c.csrDirect && plan.size() != 1) return SJ_OK;
     const uint32_t nt = c.nTasks;
     c.st.num_tasks = nt;
     c.st.estimated_pairs = predTotal;
@@ -1524,6 +1522,50 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
     auto ev = [&](size_t k) -> cudaEvent_t { return c.syncEvents[6 * iter + k]; };
     const bool hostDel = delivery == SJ_DELIVER_HOST;
     if (hostDel) CK(c.keyStartAlt.ensure(n ? n : 1));
+    // The rows of a device table: their lengths are known (per point id).  A table
+    // that is appended to gets its row offsets here and empty rows; the offsets of
+    // a table of one batch are its run offsets already.
+    auto takeRows = [&](const uint32_t *len, uint64_t pairs) -> sj_status {
+        CK(c.dCellHits.ensure(c.nCells ? c.nCells : 1));
+        CK(sj_cell_hits(c.cellStart.p, c.ids.p, len, c.nCells, c.dCellHits.p, c.s));
+        c.haveMeas = true;
+        if (!c.csrDirect) {
+            // 64-bit offsets: a counted batch past the capacity may pass 2^32 pairs
+            CK(c.csrWide.ensure(n ? n : 1));
+            CK(c.csrScan.ensure(sj_scan64_temp(n)));
+            CK(sj_u32_to_u64(len, n, c.csrWide.p, c.s));
+            CK(sj_exclusive_scan_u64(c.csrWide.p, reinterpret_cast<unsigned long long *>(c.csrRowPtr), n, c.csrScan.p,
+                                     c.s));
+            CK(cudaMemsetAsync(c.csrFill.p, 0, sizeof(uint32_t) * (n ? n : 1), c.s));
+        }
+        c.csrTotal = pairs;
+        c.csrSized = true;
+        if (c.csrCap < pairs) {
+            CK(cudaStreamSynchronize(c.s));
+            set_error("cols holds %llu values, the table needs %llu", (unsigned long long)c.csrCap,
+                      (unsigned long long)pairs);
+            return SJ_ERR_BAD_INPUT;
+        }
+        return SJ_OK;
+    };
+    if (delivery == SJ_DELIVER_CSR && stack.size() != 1) {
+        // a table of several batches: its rows are sized by one count pass over the
+        // whole list, then the planned batches are appended
+        c.csrDirect = false;
+        sj_join_args b = a;
+        b.masks = b.colMasks = b.rowRel = b.candId = b.candRel = nullptr;
+        b.taskBegin = 0;
+        b.taskEnd = nt;
+        b.batchPairs = slot;
+        CK(cudaMemsetAsync(slot, 0, sizeof(unsigned long long), c.s));
+        CKS(run_count(c, b, true, nt, nt));
+        CK(cudaMemcpyAsync(c.pinTotal.p, slot, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c.s));
+        CK(cudaStreamSynchronize(c.s));
+        unsigned long long pairs = 0;
+        memcpy(&pairs, c.pinTotal.p, sizeof(pairs));
+        CKS(takeRows(c.keyCount.p, pairs));
+        CK(cudaMemsetAsync(c.keyCount.p, 0, sizeof(uint32_t) * n, c.s));
+    }
     while (!stack.empty() && result == SJ_OK) {
         BatchRange br = stack.back();
         stack.pop_back();
@@ -1555,20 +1597,11 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
         noteErr(br, cnt);
         if (c.csrDirect && delivery == SJ_DELIVER_CSR) {
             // the join is this batch: its key runs are the table's rows
-            if (cnt > cap) return SJ_OK;   // more than one batch after all
-            CK(c.csrFill.ensure(n ? n : 1));
             CK(sj_csr_rows(ksBuf, c.total.p, n, c.csrRowPtr, c.csrFill.p, c.s));
-            CK(c.dCellHits.ensure(c.nCells ? c.nCells : 1));
-            CK(sj_cell_hits(c.cellStart.p, c.ids.p, c.csrFill.p, c.nCells, c.dCellHits.p, c.s));
-            c.haveMeas = true;
-            c.csrDone = true;
-            c.csrTotal = cnt;
-            if (c.csrCap < cnt) {
-                CK(cudaStreamSynchronize(c.s));
-                set_error("cols holds %llu values, the table needs %llu", (unsigned long long)c.csrCap,
-                          (unsigned long long)cnt);
-                return SJ_ERR_BAD_INPUT;
-            }
+            if (cnt > cap) c.csrDirect = false;   // more than one batch after all; the rows hold what it counted
+            CKS(takeRows(c.csrFill.p, cnt));
+        }
+        if (c.csrDirect && delivery == SJ_DELIVER_CSR) {
             a.outVal = c.csrCols;
             a.outKey = nullptr;
             a.capacity = std::min<uint64_t>(c.csrCap, 0xffffffffULL);
@@ -2131,10 +2164,25 @@ sj_status sj_neighbor_csr(sj_ctx *ctx, uint64_t *rowPtr, int32_t *cols, uint64_t
     }
     const uint64_t n = c.n;
     CK(c.csrFill.ensure(n ? n : 1));
+    if (!cols) {
+        // row offsets alone: the degrees
+        CKS(run_degrees(c, nullptr));
+        CK(c.csrWide.ensure(n ? n : 1));
+        CK(c.csrScan.ensure(sj_scan64_temp(n)));
+        CK(sj_u32_to_u64(c.keyCount.p, n, c.csrWide.p, c.s));
+        CK(sj_exclusive_scan_u64(c.csrWide.p, reinterpret_cast<unsigned long long *>(rowPtr), n, c.csrScan.p, c.s));
+        uint64_t tot = 0;
+        CK(cudaMemcpyAsync(&tot, rowPtr + n, sizeof(tot), cudaMemcpyDeviceToHost, c.s));
+        CK(cudaStreamSynchronize(c.s));
+        if (total) *total = tot;
+        return SJ_OK;
+    }
     c.csrRowPtr = rowPtr;
     c.csrCols = cols;
     c.csrCap = cols_capacity;
-    c.csrDone = false;
+    c.csrSized = false;
+    // a join that is one batch needs no sizing pass: its key runs are the rows
+    c.csrDirect = true;
     struct Clear {
         Ctx &c;
         ~Clear()
@@ -2142,35 +2190,11 @@ sj_status sj_neighbor_csr(sj_ctx *ctx, uint64_t *rowPtr, int32_t *cols, uint64_t
             c.csrRowPtr = nullptr;
             c.csrCols = nullptr;
             c.csrCap = 0;
-            c.csrDirect = false;
         }
     } clear{c};
-    if (cols) {
-        // a join that is one batch needs no sizing pass: its key runs are the rows
-        c.csrDirect = true;
-        const sj_status s = run_join(c, SJ_DELIVER_CSR, nullptr, nullptr);
-        c.csrDirect = false;
-        if (c.csrDone && total) *total = c.csrTotal;
-        if (s != SJ_OK || c.csrDone) return s;
-    }
-    // row offsets from the degrees
-    CKS(run_degrees(c, nullptr));
-    CK(c.csrWide.ensure(n ? n : 1));
-    CK(c.csrScan.ensure(sj_scan64_temp(n)));
-    CK(sj_u32_to_u64(c.keyCount.p, n, c.csrWide.p, c.s));
-    CK(sj_exclusive_scan_u64(c.csrWide.p, reinterpret_cast<unsigned long long *>(rowPtr), n, c.csrScan.p, c.s));
-    uint64_t tot = 0;
-    CK(cudaMemcpyAsync(&tot, rowPtr + n, sizeof(tot), cudaMemcpyDeviceToHost, c.s));
-    CK(cudaStreamSynchronize(c.s));
-    if (total) *total = tot;
-    if (!cols) return SJ_OK;
-    if (cols_capacity < tot) {
-        set_error("cols holds %llu values, the table needs %llu", (unsigned long long)cols_capacity,
-                  (unsigned long long)tot);
-        return SJ_ERR_BAD_INPUT;
-    }
-    CK(cudaMemsetAsync(c.csrFill.p, 0, sizeof(uint32_t) * (n ? n : 1), c.s));
-    CKS(run_join(c, SJ_DELIVER_CSR, nullptr, nullptr));
+    const sj_status s = run_join(c, SJ_DELIVER_CSR, nullptr, nullptr);
+    if (c.csrSized && total) *total = c.csrTotal;
+    if (s != SJ_OK || c.csrDirect) return s;
     // every row must be exactly full
     CK(cudaMemsetAsync(c.stat() + 7, 0, sizeof(unsigned long long), c.s));
     CK(sj_csr_check(rowPtr, c.csrFill.p, n, c.stat() + 7, c.s));
