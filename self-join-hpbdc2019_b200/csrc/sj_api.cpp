@@ -1541,7 +1541,14 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
         c.csrTotal = pairs;
         c.csrSized = true;
         if (c.csrCap < pairs) {
-            CK(cudaStreamSynchronize(c.s));
+            // the caller learns the table's size, from the statistics too
+            CK(sj_task_sums(taskEvals, taskRefined, nullptr, nullptr, nt, c.sums(), c.numSM, c.s));
+            Readback rb(c);
+            const Mail m(rb);
+            CKS(rb.wait());
+            c.st.total_pairs = pairs;
+            c.st.distance_calcs = m.sums()[0];
+            c.st.refined_pairs = m.sums()[1];
             set_error("cols holds %llu values, the table needs %llu", (unsigned long long)c.csrCap,
                       (unsigned long long)pairs);
             return SJ_ERR_BAD_INPUT;

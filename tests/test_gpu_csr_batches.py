@@ -4,6 +4,7 @@
     for the spatial order of their points; the same points as a host list;
   * several batches, whose plan is made once: the launches above those of the
     same join without a table are the appends and a fixed few;
+  * too small an array: refused, with the table's size in the statistics;
   * planned as one batch and counted as several (an untrained network predicts
     next to nothing), up to more than 2^32 pairs in that one batch.
 
@@ -112,3 +113,27 @@ def test_more_than_32_bits_of_pairs_in_the_planned_batch():
     for i in range(0, n, 6000):   # every row holds every point once
         rows, _ = torch.sort(cols.view(n, n)[i:i + 6000], dim=1)
         assert torch.equal(rows, every.expand_as(rows))
+
+
+@pytest.mark.parametrize("capacity", [0, 65536])
+def test_refused_table_reports_its_size(capacity):
+    torch = pytest.importorskip("torch")
+    pts = exp_points(4000, 2, 33)
+    ok, _ = oracle.OracleIndex(pts, 0.01, 2).pairs()
+    row = torch.zeros(len(pts) + 1, dtype=torch.int64, device="cuda")
+    cols = torch.zeros(len(ok) - 1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    with sjoin.SelfJoin(2, 0.01, mode=9, precision=sjoin.PREC_FP32_REFINE, capacity=capacity) as sj:
+        sj.set_points(pts)
+        sj.build_index()
+        sj.degrees()
+        ref = sj.stats()
+        sj.set_points(pts)   # statistics start anew
+        sj.build_index()
+        with pytest.raises(sjoin.SJError) as e:
+            sj.neighbor_csr(row.data_ptr(), cols.data_ptr(), len(ok) - 1)
+        st = sj.stats()
+    assert e.value.status == sjoin.SJ_ERR_BAD_INPUT
+    assert row[-1].item() == len(ok) and not torch.any(cols)
+    assert (st.total_pairs, st.distance_calcs) == (len(ok), ref.distance_calcs)
+    assert st.refined_pairs <= st.distance_calcs
