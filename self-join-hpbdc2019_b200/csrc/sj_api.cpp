@@ -394,15 +394,21 @@ struct Mail {
     uint32_t tot32(int i) const { return (uint32_t)(w[13] >> (32 * i)); }
 };
 
-// The stage times recorded so far go into the statistics.
-void settle(Ctx &c)
+// The stage times recorded so far go into the statistics: those of the last join,
+// degree count or sampling estimate (which have ended), and all of them.
+void settle_join(Ctx &c)
 {
-    if (c.tmUpload.pending) c.st.ms_upload = c.tmUpload.ms();
-    if (c.tmIndex.pending) c.st.ms_index = c.tmIndex.ms();
     if (c.tmNbr.pending) c.st.ms_tasks = c.tmNbr.ms();
     if (c.tmTasks.pending) c.st.ms_tasks += c.tmTasks.ms();
     if (c.tmEstimate.pending) c.st.ms_estimate = c.tmEstimate.ms();
     if (c.tmTotal.pending) c.st.ms_total = c.tmTotal.ms();
+}
+
+void settle(Ctx &c)
+{
+    if (c.tmUpload.pending) c.st.ms_upload = c.tmUpload.ms();
+    if (c.tmIndex.pending) c.st.ms_index = c.tmIndex.ms();
+    settle_join(c);
 }
 
 sj_status verify_tasks(Ctx &c, uint32_t perItem)
@@ -1175,6 +1181,7 @@ constexpr int SJ_DELIVER_CSR = 100;
 sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
 {
     const unsigned long long launches0 = sj_launch_total();
+    settle_join(c);
     c.tmTotal.start(c.s);
     int pattern;
     bool queue;
@@ -1763,6 +1770,7 @@ sj_status run_degrees(Ctx &c, uint32_t *degHost)
 {
     int pattern;
     bool queue;
+    settle_join(c);   // an earlier call's times, not to be read as this one's
     CKS(prepare_join(c, pattern, queue, false));
     c.st.ms_estimate = 0;
     const uint64_t n = c.n;
@@ -2312,6 +2320,7 @@ sj_status sj_cell_samples(sj_ctx *ctx, double *homeHits, double *homeEvals, doub
     CKS(bind(c));
     int pattern;
     bool queue;
+    settle_join(c);
     CKS(prepare_join(c, pattern, queue));   // owned-neighbour lists and the sampling estimate
     if (!c.haveSamples) {
         set_error("internal: no sampling estimate");
