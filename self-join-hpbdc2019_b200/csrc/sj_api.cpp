@@ -266,7 +266,7 @@ struct Ctx {
     DevBuf<uint32_t> smallPre, bigList, smallList;   // the tasks by count-pass kernel (sj_task_lists)
     DevBuf<uint32_t> tgGroupCnt, tgGroupBase, tgGroupLen, tgPosCnt, tgOrder, tgOrderAlt, tgItemCnt, tgItemStart,
         tgItemTasks, tgItemTaskStart;
-    DevBuf<uint32_t> tgKeys, tgKeysAlt;
+    DevBuf<uint64_t> tgKeys, tgKeysAlt;
     DevBuf<unsigned long long> tgPosEv, tgEvExcl, tgScan64;
     DevBuf<uint8_t> tgWorkers;
     // per-task record offsets (exclusive prefix sums, nTasks + 1 each): row-mask
@@ -890,12 +890,13 @@ sj_status build_tasks_dev(Ctx &c, bool sym, uint64_t cap, bool byCost, int polic
     CK(c.tgKeysAlt.ensure(nc));
     CK(c.tgOrder.ensure(nc));
     CK(c.tgOrderAlt.ensure(nc));
-    CK(sj_tg_cells(g, nullptr, nullptr, c.tgPosCnt.p, c.tgPosEv.p, byCost ? c.tgKeys.p : nullptr, c.tgOrder.p,
-                   c.tgTotals(), s));
+    CK(sj_tg_cells(g, nullptr, nullptr, c.tgPosCnt.p, c.tgPosEv.p,
+                   byCost ? reinterpret_cast<unsigned long long *>(c.tgKeys.p) : nullptr, c.tgOrder.p, c.tgTotals(),
+                   s));
     uint32_t *order = c.tgOrder.p;
     if (byCost && nc > 1) {
         int inAlt = 0;
-        CK(sj_radix_sort_u32_u32(c.tgKeys.p, c.tgOrder.p, c.tgKeysAlt.p, c.tgOrderAlt.p, nc, 16, tmp.p, &inAlt, s));
+        CK(sj_radix_sort_u64_u32(c.tgKeys.p, c.tgOrder.p, c.tgKeysAlt.p, c.tgOrderAlt.p, nc, 64, tmp.p, &inAlt, s));
         if (inAlt) order = c.tgOrderAlt.p;
     }
     const uint8_t *workers = nullptr;

@@ -247,8 +247,8 @@ cudaError_t sj_nbr_spread(const uint32_t *cellStart, const uint32_t *cellCoord, 
                           const uint32_t *nbrCell, uint32_t nCells, const sj_grid_dev &g, uint32_t *nbrPre,
                           double *nbrPreW, float *nbrWt, double *cellW, cudaStream_t s);
 cudaError_t sj_tg_cells(const sj_taskgen &g, const uint32_t *order, const uint8_t *workersAt, uint32_t *posCnt,
-                        unsigned long long *posEv, uint32_t *costKey, uint32_t *iota, unsigned long long *totals,
-                        cudaStream_t s);
+                        unsigned long long *posEv, unsigned long long *costKey, uint32_t *iota,
+                        unsigned long long *totals, cudaStream_t s);
 // mode 8: workers per position from the exclusive prefix of the evaluations
 // in cost order (evExcl[n] = total): 16, 8 or 2 by third of the work
 cudaError_t sj_tg_thirds(const unsigned long long *evExcl, uint32_t n, uint8_t *workers, cudaStream_t s);

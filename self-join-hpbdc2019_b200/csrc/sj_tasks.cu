@@ -235,7 +235,8 @@ __global__ void __launch_bounds__(256) k_tg_groups(sj_taskgen g, uint32_t *cnt)
 __global__ void __launch_bounds__(256) k_tg_cells(sj_taskgen g, const uint32_t *__restrict__ order,
                                                   const uint8_t *__restrict__ workersAt, uint32_t *__restrict__ posCnt,
                                                   unsigned long long *__restrict__ posEv,
-                                                  uint32_t *__restrict__ costKey, uint32_t *__restrict__ iota,
+                                                  unsigned long long *__restrict__ costKey,
+                                                  uint32_t *__restrict__ iota,
                                                   unsigned long long *__restrict__ totals)
 {
     const uint32_t lane = threadIdx.x & 31u;
@@ -275,11 +276,9 @@ __global__ void __launch_bounds__(256) k_tg_cells(sj_taskgen g, const uint32_t *
         if (posEv) posEv[pos] = ev;
         if (iota) iota[pos] = pos;
         if (costKey) {
-            // mean predicted task cost: evaluations plus a write cost per pair.  The
-            // key is its exponent and 8 bits of its mantissa, descending: two sort
-            // passes, and an order finer than 0.4 % would not be worth more
+            // mean predicted task cost: evaluations plus a write cost per pair
             const double cost = cnt ? ((double)ev + 4.0 * pred) / (double)cnt : 0.0;
-            costKey[pos] = 0xffffu - (__float_as_uint((float)cost) >> 15);   // cost >= 0
+            costKey[pos] = ~(unsigned long long)__double_as_longlong(cost);   // cost >= 0: descending
         }
         atomicAdd(&totals[0], (unsigned long long)cnt);
         atomicAdd(&totals[1], (unsigned long long)ev);
@@ -905,8 +904,8 @@ cudaError_t sj_tg_groups(const sj_taskgen &g, uint32_t *cnt, cudaStream_t s)
 }
 
 cudaError_t sj_tg_cells(const sj_taskgen &g, const uint32_t *order, const uint8_t *workersAt, uint32_t *posCnt,
-                        unsigned long long *posEv, uint32_t *costKey, uint32_t *iota, unsigned long long *totals,
-                        cudaStream_t s)
+                        unsigned long long *posEv, unsigned long long *costKey, uint32_t *iota,
+                        unsigned long long *totals, cudaStream_t s)
 {
     if (g.nCells == 0) return cudaSuccess;
     k_tg_cells<<<blocks_for((uint64_t)g.nCells * 32, 256), 256, 0, s>>>(g, order, workersAt, posCnt, posEv, costKey,
