@@ -386,7 +386,8 @@ __device__ __forceinline__ Item find_item(const sj_taskgen &g, const uint32_t *_
 __global__ void __launch_bounds__(256) k_tg_item_tasks(sj_taskgen g, const uint32_t *__restrict__ order,
                                                        const uint8_t *__restrict__ workersAt,
                                                        const uint32_t *__restrict__ itemStart, uint32_t nItems,
-                                                       uint32_t *__restrict__ itemTasks)
+                                                       uint32_t *__restrict__ itemTasks, uint4 *__restrict__ tiles,
+                                                       uint32_t *__restrict__ nTiles)
 {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= nItems) return;
@@ -394,6 +395,45 @@ __global__ void __launch_bounds__(256) k_tg_item_tasks(sj_taskgen g, const uint3
     const uint32_t S = g.groupLen[g.groupBase[it.c] + it.grp];
     const TileWork w = tile_work(g, it.c, it.grp, it.tile, S, workersAt ? (int)workersAt[it.pos] : 0);
     itemTasks[j] = w.nChunks;
+    if (tiles && n_tiles(g, it.c) > 1) tiles[atomicAdd(nTiles, 1u)] = make_uint4(j, it.c, it.grp, it.tile);
+}
+
+// Weights of the tiles of a cell that has several: each tile's sampled rates over
+// the cell's mean of them (by evaluations), so that the cell's predicted pairs stay
+// what its rates make them and are shared among its tiles as sampled.  One warp a
+// position; the sums have a fixed order.
+__global__ void __launch_bounds__(256) k_tg_tile_weights(sj_taskgen g, const uint32_t *__restrict__ order,
+                                                         const uint32_t *__restrict__ itemStart,
+                                                         float2 *__restrict__ rates)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t pos = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (pos >= g.nCells) return;
+    const uint32_t c = order[pos], T = n_tiles(g, c);
+    if (T <= 1) return;
+    const uint32_t n = n_groups(g, c) * T, j0 = itemStart[pos];
+    double ev[2] = {0.0, 0.0}, hits[2] = {0.0, 0.0};   // home, neighbours
+    for (uint32_t i = lane; i < n; i += 32) {
+        const uint32_t grp = i / T;
+        const TileWork w = tile_work(g, c, grp, i - grp * T, g.groupLen[g.groupBase[c] + grp], 0);
+        const float2 r = rates[j0 + i];
+        ev[0] += (double)w.evHome;
+        ev[1] += (double)w.evOther;
+        hits[0] += (double)w.evHome * (double)r.x;
+        hits[1] += (double)w.evOther * (double)r.y;
+    }
+    double per[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        ev[k] = warp_sum_f64(ev[k]);
+        hits[k] = warp_sum_f64(hits[k]);
+        per[k] = hits[k] > 0.0 ? ev[k] / hits[k] : 0.0;
+    }
+    for (uint32_t i = lane; i < n; i += 32) {
+        const float2 r = rates[j0 + i];
+        rates[j0 + i] = make_float2(per[0] > 0.0 ? (float)(r.x * per[0]) : 1.0f,
+                                    per[1] > 0.0 ? (float)(r.y * per[1]) : 1.0f);
+    }
 }
 
 // Writes every item's tasks (in item order, chunks ascending) and their
@@ -402,6 +442,7 @@ __global__ void __launch_bounds__(256) k_tg_item_write(sj_taskgen g, const uint3
                                                        const uint8_t *__restrict__ workersAt,
                                                        const uint32_t *__restrict__ itemStart, uint32_t nItems,
                                                        const uint32_t *__restrict__ itemTaskStart,
+                                                       const float2 *__restrict__ weights,
                                                        sj_task *__restrict__ tasks, uint32_t nt,
                                                        float *__restrict__ pred)
 {
@@ -412,7 +453,11 @@ __global__ void __launch_bounds__(256) k_tg_item_write(sj_taskgen g, const uint3
     const TileWork w = tile_work(g, it.c, it.grp, it.tile, S, workersAt ? (int)workersAt[it.pos] : 0);
     const uint32_t nSegAll = 1 + (g.nbrStart[it.c + 1] - g.nbrStart[it.c]);
     const uint32_t segBase = it.grp * SJ_MAX_SEG;
-    const float2 r = rates_of(g, it.c);
+    float2 r = rates_of(g, it.c);
+    if (weights && n_tiles(g, it.c) > 1) {
+        r.x = fminf(1.0f, r.x * weights[j].x);
+        r.y = fminf(1.0f, r.y * weights[j].y);
+    }
     uint32_t t = itemTaskStart[j];
     // (t < nt: the lists are sized by the cells' task counts, and the two counts
     // are compared on the host afterwards)
@@ -931,21 +976,32 @@ cudaError_t sj_tg_item_counts(const sj_taskgen &g, const uint32_t *order, uint32
 }
 
 cudaError_t sj_tg_item_tasks(const sj_taskgen &g, const uint32_t *order, const uint8_t *workersAt,
-                             const uint32_t *itemStart, uint32_t nItems, uint32_t *itemTasks, cudaStream_t s)
+                             const uint32_t *itemStart, uint32_t nItems, uint32_t *itemTasks, uint4 *tiles,
+                             uint32_t *nTiles, cudaStream_t s)
 {
     if (nItems == 0) return cudaSuccess;
-    k_tg_item_tasks<<<blocks_for(nItems, 256), 256, 0, s>>>(g, order, workersAt, itemStart, nItems, itemTasks);
+    k_tg_item_tasks<<<blocks_for(nItems, 256), 256, 0, s>>>(g, order, workersAt, itemStart, nItems, itemTasks, tiles,
+                                                            nTiles);
+    sj_note_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t sj_tg_tile_weights(const sj_taskgen &g, const uint32_t *order, const uint32_t *itemStart, float2 *rates,
+                               cudaStream_t s)
+{
+    if (g.nCells == 0) return cudaSuccess;
+    k_tg_tile_weights<<<blocks_for((uint64_t)g.nCells * 32, 256), 256, 0, s>>>(g, order, itemStart, rates);
     sj_note_launch();
     return cudaGetLastError();
 }
 
 cudaError_t sj_tg_item_write(const sj_taskgen &g, const uint32_t *order, const uint8_t *workersAt,
                              const uint32_t *itemStart, uint32_t nItems, const uint32_t *itemTaskStart,
-                             sj_task *tasks, uint32_t nt, float *pred, cudaStream_t s)
+                             const float2 *weights, sj_task *tasks, uint32_t nt, float *pred, cudaStream_t s)
 {
     if (nItems == 0) return cudaSuccess;
     k_tg_item_write<<<blocks_for(nItems, 256), 256, 0, s>>>(g, order, workersAt, itemStart, nItems, itemTaskStart,
-                                                            tasks, nt, pred);
+                                                            weights, tasks, nt, pred);
     sj_note_launch();
     return cudaGetLastError();
 }
