@@ -185,7 +185,9 @@ __device__ __forceinline__ TileWork tile_work(const sj_taskgen &g, uint32_t c, u
     w.evOther = qc * (uint64_t)S;
     const float2 r = rates_of(g, c);
     const double ev = (double)(w.evHome + w.evOther);
-    const float rate = ev > 0 ? (float)(((double)w.evHome * r.x + (double)w.evOther * r.y) / ev) : 0.0f;
+    // (explicit rounding: three kernels evaluate this, and their chunk counts must agree)
+    const double hits = __dadd_rn(__dmul_rn((double)w.evHome, (double)r.x), __dmul_rn((double)w.evOther, (double)r.y));
+    const float rate = ev > 0 ? (float)__ddiv_rn(hits, ev) : 0.0f;
     w.sc = chunk_len(g, rate, w.qc, w.L, workers);
     if (g.policy == 1)
         w.nChunks = (w.homeLen + w.sc - 1) / w.sc + (S + w.sc - 1) / w.sc;
@@ -459,8 +461,9 @@ __global__ void __launch_bounds__(256) k_tg_item_write(sj_taskgen g, const uint3
         r.y = fminf(1.0f, r.y * weights[j].y);
     }
     uint32_t t = itemTaskStart[j];
-    // (t < nt: the lists are sized by the cells' task counts, and the two counts
-    // are compared on the host afterwards)
+    // (the lists are sized by the cells' task counts; the host compares the two counts
+    // after a count pass may have run on the list, so that is written whole and not
+    // past its end whatever the items' counts are: tasks left over are empty)
     for (uint32_t ch = 0; ch < w.nChunks && t < nt; ch++, t++) {
         const uint2 sr = chunk_range(g, w, ch);
         const uint32_t s0 = sr.x, s1 = sr.y;
@@ -484,6 +487,12 @@ __global__ void __launch_bounds__(256) k_tg_item_write(sj_taskgen g, const uint3
                   (g.sampleRate > 0.0f && n_queries(g, it.c) < w.occ ? SJ_TASK_SAMPLE : 0u);
         tasks[t] = k;
         pred[t] = (float)pairs_of(g, r, evH, evO, diag);
+    }
+    if (j + 1 == nItems) {
+        for (; t < nt; t++) {
+            tasks[t] = sj_task{};
+            pred[t] = 0.0f;
+        }
     }
 }
 
