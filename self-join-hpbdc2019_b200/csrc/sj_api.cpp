@@ -726,58 +726,10 @@ void join_args_base(Ctx &c, sj_join_args &a)
     a.cellCoord = c.cellCoord.p;
 }
 
-// FP32 filter bounds.  Queries are taken relative to their home cell's centre
-// (indexed dims) or the data centre (others): |a| <= Ra; candidates lie in the
-// home cell or a neighbour: |b| <= Rb.  The kernel evaluates in FP32
-//     y = fl(|b|^2 - tLo) + sum_l fl(-2 a_l) b_l     (D+2 roundings),
-// with tLo = RD(T - |a|^2 - M).  With u = 2^-24 and r = Ra + Rb:
-//   * chain rounding <= (D+2) u (r^2 + T + M),
-//   * rounding the local coordinates moves |b - a|^2 by <= 2 u r^2,
-//   * the FP64 predicate's own rounding (d2 vs the exact |dx|^2) <= 2^-49 r^2,
-// so M = 2 (D+4) u (r^2 + T) + 2^-39 (r^2 + T) exceeds their sum: y <= 0 proves
-// d2 <= T.  y >= delta proves d2 > T when delta >= 2M + 2u (T + Ra^2 + M) (the
-// second term covers rounding tLo down).  Pairs with 0 < y < delta are
-// re-evaluated in FP64.
-// pruneT: two boxes of local FP32 coordinates whose squared distance s, in FP32,
-// exceeds T + 2M hold no pair that satisfies the predicate: rounding the
-// coordinates and the sum moves it by less than (D+6) u r^2 < M, the predicate's
-// own rounding by less than M.  Outside the range in which FP32 squares keep
-// that accuracy nothing is ruled out.
-struct FilterBounds {
-    double margin;
-    float delta;
-    float pruneT;
-};
-
-FilterBounds filter_bounds(const Ctx &c)
+// The filter's and the box test's bounds for the context's grid and data (sj_host.h).
+sj_filter_bounds filter_bounds(const Ctx &c)
 {
-    const sj_grid_dev &g = c.g;
-    double ra2 = 0, rb2 = 0;
-    for (int j = 0; j < g.D; j++) {
-        if (j < g.k) {
-            ra2 += (0.5 * g.eps * 1.01) * (0.5 * g.eps * 1.01);
-            rb2 += (1.5 * g.eps * 1.01) * (1.5 * g.eps * 1.01);
-        } else {
-            double h = 0.5 * (c.dataMax[j] - c.dataMin[j]) * 1.01 + 1e-300;
-            ra2 += h * h;
-            rb2 += h * h;
-        }
-    }
-    const double r = std::sqrt(ra2) + std::sqrt(rb2);
-    const double u = std::ldexp(1.0, -24);
-    const double T = g.thresh;
-    FilterBounds b;
-    b.margin = 2.0 * (g.D + 4) * u * (r * r + T) + std::ldexp(r * r + T, -39);
-    const double d = (2.0 * b.margin + 2.0 * u * (T + ra2 + b.margin)) * (1.0 + std::ldexp(1.0, -20));
-    float df = (float)d;
-    if ((double)df < d) df = std::nextafter(df, INFINITY);
-    b.delta = df;
-    b.pruneT = INFINITY;
-    if (g.eps >= 1e-15 && g.eps <= 1e15) {
-        const double pt = (T + 2.0 * b.margin) * (1.0 + std::ldexp(1.0, -20));
-        if (pt < 3.0e38) b.pruneT = std::nextafter((float)pt, INFINITY);
-    }
-    return b;
+    return sj_filter_bounds_of(c.g.D, c.g.k, c.g.eps, c.g.thresh, c.dataMin, c.dataMax);
 }
 
 // --------------------------------------------------------------- tasks --
@@ -1081,7 +1033,7 @@ sj_status estimate_rates(Ctx &c)
         a.taskHits = c.taskRec.p;
         a.taskEvals = c.taskRec.p + nt;
         a.taskRefined = c.taskRec.p + 2 * (size_t)nt;
-        const FilterBounds fb = filter_bounds(c);
+        const sj_filter_bounds fb = filter_bounds(c);
         a.margin = fb.margin;
         a.delta = fb.delta;
         a.pruneT = fb.pruneT;
@@ -1269,7 +1221,7 @@ sj_status run_join(Ctx &c, int delivery, sj_batch_cb cb, void *user)
     a.candOff = reinterpret_cast<const uint64_t *>(c.off[3].p);
     a.unitOff = reinterpret_cast<const uint64_t *>(c.off[4].p);
     {
-        const FilterBounds fb = filter_bounds(c);
+        const sj_filter_bounds fb = filter_bounds(c);
         a.margin = fb.margin;
         a.delta = fb.delta;
         a.pruneT = fb.pruneT;
@@ -1807,7 +1759,7 @@ sj_status run_degrees(Ctx &c, uint32_t *degHost)
     a.keyCount = c.keyCount.p;
     a.stat = c.stat();
     {
-        const FilterBounds fb = filter_bounds(c);
+        const sj_filter_bounds fb = filter_bounds(c);
         a.margin = fb.margin;
         a.delta = fb.delta;
         a.pruneT = fb.pruneT;
