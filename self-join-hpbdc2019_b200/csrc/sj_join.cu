@@ -31,6 +31,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cfloat>
 #include <type_traits>
 
 #ifndef SJ_EVAL_UNROLL
@@ -1065,7 +1066,10 @@ __global__ void __launch_bounds__(SJ_CTA, DP <= 4 ? 6 : DP <= 8 ? 5 : 4) k_join_
 // One CTA an item: its queries in registers, the sampled candidates staged 128 at
 // a time, every query against every candidate in FP32.  All tiles of a cell meet
 // the same candidates, so the sample's own error cancels in their ratios.
-constexpr uint32_t TILE_SAMPLE_MIN = 128, TILE_SAMPLE_MAX = 2048, TILE_SAMPLE_PART = 64;
+// A 64th of the points, 4096 at most: 1e7 points in 6-D, batches of 2e9 pairs, sampled
+// estimate 22 of 1730 batches counted twice (34 with 2048, 24 with 8192; what is left
+// is the stretch of a stream that a batch ends in), 0.1 % of the join's time.
+constexpr uint32_t TILE_SAMPLE_MIN = 128, TILE_SAMPLE_MAX = 4096, TILE_SAMPLE_PART = 64;
 
 __device__ __forceinline__ uint32_t tile_samples(uint32_t len)
 {
@@ -1277,7 +1281,7 @@ cudaError_t sj_launch_tile_rates(const sj_taskgen &g, const sj_grid_dev &gd, con
 {
     if (nItems == 0) return cudaSuccess;
     const unsigned grid = std::min<uint64_t>((uint64_t)numSM * 8, nItems);
-    const float T = (float)gd.thresh;
+    const float T = std::min((float)gd.thresh, FLT_MAX);   // (a slot without a query is infinitely far)
     switch (gd.Dp) {
     case 1: k_tile_rates<1><<<grid, SJ_CTA, 0, s>>>(g, xs, T, tiles, nTiles, rates); break;
     case 2: k_tile_rates<2><<<grid, SJ_CTA, 0, s>>>(g, xs, T, tiles, nTiles, rates); break;
