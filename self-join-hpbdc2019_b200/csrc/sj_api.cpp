@@ -269,8 +269,8 @@ struct Ctx {
     DevBuf<uint64_t> tgKeys, tgKeysAlt;
     DevBuf<unsigned long long> tgPosEv, tgEvExcl, tgScan64;
     DevBuf<uint8_t> tgWorkers;
-    DevBuf<uint4> tgTiles;       // work items of several tiles a cell, and per item the tile's sampled rates
-    DevBuf<float2> tgTileRate;
+    DevBuf<float2> tgSample;     // per task: its evaluations and its sample's hits
+    DevBuf<double2> tgItemSum;   // per work item: sums of them
     // per-task record offsets (exclusive prefix sums, nTasks + 1 each): row-mask
     // words, column-mask words, row offsets, candidate records, emission units,
     // planned pairs, predicted pairs
@@ -296,8 +296,7 @@ struct Ctx {
     uint32_t *planCount() const { return reinterpret_cast<uint32_t *>(mail.p + 12); }
     uint32_t *tgTot32() const { return reinterpret_cast<uint32_t *>(mail.p + 13); }   // work items, tasks by item
     unsigned long long *tgTotals() const { return mail.p + 14; }        // 4, see sj_tg_cells
-    uint32_t *tgTileCount() const { return reinterpret_cast<uint32_t *>(mail.p + 18); }
-    static constexpr size_t MAIL = 19;
+    static constexpr size_t MAIL = 18;
     DevBuf<uint32_t> queueHead;
     DevBuf<uint32_t> taskRec;   // per task: measured pairs, evaluations, re-evaluations (of the count pass)
     // count-pass records for the emission pass: per task, row and column hit
@@ -821,6 +820,7 @@ sj_status build_tasks_dev(Ctx &c, bool sym, uint64_t cap, bool byCost, int polic
     // tasks by the offset-class model its features use; the sampling estimate
     // keeps the cell's mean rate
     g.spread = (c.rateLearned && policy != 1 && rates) ? 1 : 0;
+    if (g.rate && c.jids != c.ids.p) CKS(build_spread(c));   // the prefixes locate the tasks' samples
     g.nbrPre = c.nbrPre.p;
     g.nbrPreW = c.nbrPreW.p;
     g.nbrWt = c.nbrWt.p;
@@ -828,7 +828,7 @@ sj_status build_tasks_dev(Ctx &c, bool sym, uint64_t cap, bool byCost, int polic
     DevBuf<uint8_t> &tmp = c.sTemp;
     CK(tmp.ensure(std::max(sj_scan_temp_bytes(nc + 1), sj_radix_temp_bytes(nc))));
     CK(c.mail.ensure(Ctx::MAIL));
-    CK(cudaMemsetAsync(c.tgTotals(), 0, sizeof(unsigned long long) * 5, s));   // and the tile count
+    CK(cudaMemsetAsync(c.tgTotals(), 0, sizeof(unsigned long long) * 4, s));
     // segment groups of every cell and their slots (at most one group per
     // SJ_MAX_SEG owned neighbours, plus one per cell)
     CK(c.tgGroupCnt.ensure(nc + 1));
@@ -889,27 +889,29 @@ sj_status build_tasks_dev(Ctx &c, bool sym, uint64_t cap, bool byCost, int polic
     CK(c.tgItemTasks.ensure((size_t)nItems + 1));
     CK(c.tgItemTaskStart.ensure((size_t)nItems + 1));
     CK(tmp.ensure(sj_scan_temp_bytes((uint64_t)nItems + 1)));
-    // In the spatial order the tiles of a cell differ, and batches hold few of them:
-    // each is predicted by a sample of its own (without it, tiles are alike but for chance)
-    const bool tiled = g.rate && c.jids != c.ids.p;
-    if (tiled) {
-        CK(c.tgTiles.ensure(nItems ? nItems : 1));
-        CK(c.tgTileRate.ensure(nItems ? nItems : 1));
-    }
-    CK(sj_tg_item_tasks(g, order, workers, c.tgItemStart.p, nItems, c.tgItemTasks.p, tiled ? c.tgTiles.p : nullptr,
-                        c.tgTileCount(), s));
-    if (tiled) {
-        CK(sj_launch_tile_rates(g, c.g, c.xs.p, c.tgTiles.p, c.tgTileCount(), nItems, c.numSM, c.tgTileRate.p, s));
-        CK(sj_tg_tile_weights(g, order, c.tgItemStart.p, c.tgTileRate.p, s));
-    }
+    CK(sj_tg_item_tasks(g, order, workers, c.tgItemStart.p, nItems, c.tgItemTasks.p, s));
     CK(sj_exclusive_scan_u32(c.tgItemTasks.p, c.tgItemTaskStart.p, nItems, tmp.p, c.tgTot32() + 1, s));
     // the items' total is compared with the cells' at the next readback
     c.expectTasks = nt;
     c.checkTasks = true;
     CK(c.dTasks.ensure(nt ? nt : 1));
     CK(c.dTaskPred.ensure(nt ? nt : 1));
-    CK(sj_tg_item_write(g, order, workers, c.tgItemStart.p, nItems, c.tgItemTaskStart.p,
-                        tiled ? c.tgTileRate.p : nullptr, c.dTasks.p, nt, c.dTaskPred.p, s));
+    // In the spatial order the tasks of a cell differ, and batches hold few of its
+    // tiles: each is predicted by a sample of its own (in id order they are alike but
+    // for chance)
+    float2 *sample = nullptr;
+    if (g.rate && c.jids != c.ids.p) {
+        CK(c.tgSample.ensure(nt ? nt : 1));
+        CK(c.tgItemSum.ensure(nItems ? nItems : 1));
+        sample = c.tgSample.p;
+    }
+    CK(sj_tg_item_write(g, order, workers, c.tgItemStart.p, nItems, c.tgItemTaskStart.p, c.dTasks.p, nt, c.dTaskPred.p,
+                        s, sample));
+    if (sample) {
+        CK(sj_launch_task_sample(g, c.g, c.xs.p, c.dTasks.p, nt, sample, s));
+        CK(sj_tg_share(g, order, c.tgItemStart.p, nItems, c.tgItemTaskStart.p, c.dTasks.p, nt, sample, c.tgItemSum.p,
+                       c.dTaskPred.p, s));
+    }
     if (shard && c.p.shard_count > 1) {
         // round-robin over the ordered list: each shard gets a similar cost mix
         const uint32_t idx = (uint32_t)c.p.shard_index, cnt = (uint32_t)c.p.shard_count;

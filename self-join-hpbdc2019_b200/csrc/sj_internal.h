@@ -124,6 +124,15 @@ struct sj_join_args {
 // live (block, group) tiles are written and read.
 __host__ __device__ inline uint32_t sj_live_words(uint32_t nBlk, uint32_t nG) { return ((nBlk + 31) / 32) * nG; }
 
+// Pairs that a task's sample evaluates: up to SJ_PROBE_QUERIES x SJ_PROBE_POS of its queries and positions.
+#define SJ_PROBE_QUERIES 64
+#define SJ_PROBE_POS 64
+__host__ __device__ inline uint32_t sj_probe_pairs(const sj_task &t)
+{
+    const uint32_t len = t.sEnd - t.sBegin;
+    return (len < SJ_PROBE_POS ? len : SJ_PROBE_POS) * (t.qCount < SJ_PROBE_QUERIES ? t.qCount : SJ_PROBE_QUERIES);
+}
+
 // Parameters of the device task builder (sj_tasks.cu).
 struct sj_taskgen {
     const uint32_t *cellStart;   // nCells+1
@@ -253,21 +262,19 @@ cudaError_t sj_tg_cells(const sj_taskgen &g, const uint32_t *order, const uint8_
 // in cost order (evExcl[n] = total): 16, 8 or 2 by third of the work
 cudaError_t sj_tg_thirds(const unsigned long long *evExcl, uint32_t n, uint8_t *workers, cudaStream_t s);
 cudaError_t sj_tg_item_counts(const sj_taskgen &g, const uint32_t *order, uint32_t *items, cudaStream_t s);
-// tiles (may be null): the items whose tiles are one of several of their cell, (item, cell, segment group, tile)
-// each, nTiles of them (zero before); the order is arbitrary
 cudaError_t sj_tg_item_tasks(const sj_taskgen &g, const uint32_t *order, const uint8_t *workersAt,
-                             const uint32_t *itemStart, uint32_t nItems, uint32_t *itemTasks, uint4 *tiles,
-                             uint32_t *nTiles, cudaStream_t s);
-// sampled hits per evaluation of those items' tiles against the home cell's and the group's neighbours' points
-// (sj_join.cu); then, per cell, each relative to the cell's mean
-cudaError_t sj_launch_tile_rates(const sj_taskgen &g, const sj_grid_dev &gd, const double *xs, const uint4 *tiles,
-                                 const uint32_t *nTiles, uint32_t nItems, int numSM, float2 *rates, cudaStream_t s);
-cudaError_t sj_tg_tile_weights(const sj_taskgen &g, const uint32_t *order, const uint32_t *itemStart, float2 *rates,
-                               cudaStream_t s);
-// weights (may be null): per item, of the items of several tiles a cell
+                             const uint32_t *itemStart, uint32_t nItems, uint32_t *itemTasks, cudaStream_t s);
+// sample (may be null): per task of a cell with several query tiles (evaluations, -), 0 of the others
 cudaError_t sj_tg_item_write(const sj_taskgen &g, const uint32_t *order, const uint8_t *workersAt,
                              const uint32_t *itemStart, uint32_t nItems, const uint32_t *itemTaskStart,
-                             const float2 *weights, sj_task *tasks, uint32_t nt, float *pred, cudaStream_t s);
+                             sj_task *tasks, uint32_t nt, float *pred, cudaStream_t s, float2 *sample = nullptr);
+// the hits of those tasks' samples (needs sj_nbr_spread's nbrPre; sj_join.cu)
+cudaError_t sj_launch_task_sample(const sj_taskgen &g, const sj_grid_dev &gd, const double *xs, const sj_task *tasks,
+                                  uint32_t nt, float2 *sample, cudaStream_t s);
+// the predicted pairs of each such cell shared among its tasks as their samples say (itemSum: nItems of scratch)
+cudaError_t sj_tg_share(const sj_taskgen &g, const uint32_t *order, const uint32_t *itemStart, uint32_t nItems,
+                        const uint32_t *itemTaskStart, const sj_task *tasks, uint32_t nt, float2 *sample,
+                        double2 *itemSum, float *pred, cudaStream_t s);
 cudaError_t sj_tg_shard(const sj_task *in, const float *predIn, uint32_t nOut, uint32_t idx, uint32_t cnt,
                         sj_task *out, float *predOut, cudaStream_t s);
 // the tasks by count-pass kernel: pre[0..nt] (exclusive prefix of the small ones), lists of the others and

@@ -1054,160 +1054,119 @@ __global__ void __launch_bounds__(SJ_CTA, DP <= 4 ? 6 : DP <= 8 ? 5 : 4) k_join_
     }
 }
 
-// ------------------------------------------------------- tile sampling --
-// Hits per evaluation of the query tiles of cells that have several, each against
-// a sample of its cell's points and of its segment group's neighbours' points.  The
-// spatial order inside the cells makes a tile (four runs of 128 neighbouring
-// points) unlike the cell, and a batch of a dense join holds a few tiles of one
-// cell.  Mean error of a batch's prediction with the cell's mean for every tile and
-// with these: 2M points in 6-D, learned 2.1 and 0.8 %, sampled 2.3 and 0.9; 60k in
-// 7-D 10 and 2.9 (18 of 65 batches counted twice, 4 of 51); 200k in 3-D 7.2 and 1.8:
-// what it is with the cells' points in id order.
-// One CTA an item: its queries in registers, the sampled candidates staged 128 at
-// a time, every query against every candidate in FP32.  All tiles of a cell meet
-// the same candidates, so the sample's own error cancels in their ratios.
-// A 64th of the points, 4096 at most: 1e7 points in 6-D, batches of 2e9 pairs, sampled
-// estimate 22 of 1730 batches counted twice (34 with 2048, 24 with 8192; what is left
-// is the stretch of a stream that a batch ends in), 0.1 % of the join's time.
-constexpr uint32_t TILE_SAMPLE_MIN = 128, TILE_SAMPLE_MAX = 4096, TILE_SAMPLE_PART = 64;
+// ------------------------------------------------------- task sampling --
+// Hits of the tasks of cells that have several query tiles, as a sample of each
+// task's own queries and candidates says.  In the spatial order inside the cells a
+// tile (four runs of 128 neighbouring points) and a stretch of a stream are unlike
+// the cell, and a batch of a dense join holds a few tiles of one cell: the cell's
+// mean rate for every task does not predict its batches (figures at k_task_pool).
+// One warp a task: up to 64 of its queries, two a lane, against up to 64 of its
+// stream positions, both evenly spread, in FP32.
+// Bound: the FP32 pipe and the candidates' loads: 0.46 ms for 156k tasks in 6-D, whose
+// count pass takes 24 ms.  32 x 32 pairs: 3.6 ms less for 2.2M tasks (count pass 471
+// ms), task error 9.3 % in place of 5.4.
+constexpr int TASK_SAMPLE_WARPS = 8;
 
-__device__ __forceinline__ uint32_t tile_samples(uint32_t len)
+// Place of sample i of m over len: `phase` of the way (in 2^-16) through its part.
+__device__ __forceinline__ uint32_t sample_at(uint32_t i, uint32_t m, uint32_t len, uint32_t phase)
 {
-    return min(len, min(TILE_SAMPLE_MAX, max(TILE_SAMPLE_MIN, len / TILE_SAMPLE_PART)));
+    return (uint32_t)(((((uint64_t)i << 16) + phase) * len) / ((uint64_t)m << 16));
 }
 
-// Position of sample i of m over len places (the middle of its share).
-__device__ __forceinline__ uint32_t sample_at(uint32_t i, uint32_t m, uint32_t len)
-{
-    return (uint32_t)(((2ULL * i + 1ULL) * len) / (2ULL * m));
-}
-
-template <int DP>   // query slots a thread: the most that a tile of this width has
-constexpr int TILE_SLOTS = sj_query_slots(DP, true) > sj_query_slots(DP, false) ? sj_query_slots(DP, true)
-                                                                               : sj_query_slots(DP, false);
-
+// sample: per task (evaluations, -), evaluations 0: not sampled; the second is set
+// to the hits of sj_probe_pairs' pairs.
 template <int DP>
-__global__ void __launch_bounds__(SJ_CTA) k_tile_rates(sj_taskgen g, const double *__restrict__ xs, float T,
-                                                       const uint4 *__restrict__ tiles,
-                                                       const uint32_t *__restrict__ nTiles, float2 *__restrict__ rates)
+__global__ void __launch_bounds__(32 * TASK_SAMPLE_WARPS) k_task_sample(sj_taskgen g, const double *__restrict__ xs,
+                                                                        float T, const sj_task *__restrict__ tasks,
+                                                                        uint32_t nt, float2 *__restrict__ sample)
 {
-    constexpr int QS = TILE_SLOTS<DP>;
-    __shared__ float cand[SJ_CTA][DP];
-    __shared__ double origin[DP];
-    __shared__ uint32_t segPos[SJ_CTA], segPre[SJ_CTA + 1], warpSum[NW];
-    __shared__ uint32_t hits[2];
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t n = *nTiles;
-    for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
-        const uint4 it = tiles[i];   // item, cell, segment group, tile
-        const uint32_t aStart = g.cellStart[it.y], occ = g.cellStart[it.y + 1] - aStart;
-        const uint32_t q0 = it.w * g.tile, qc = min(g.tile, occ - q0);
-        __syncthreads();   // the previous item is done with the shared memory
-        if (tid < DP) origin[tid] = xs[(uint64_t)(aStart + q0) * DP + tid];
-        if (tid < 2) hits[tid] = 0;
-        __syncthreads();
-        float q[QS][DP];
+    constexpr int ROW = (DP + 3) / 4 * 4;
+    constexpr int QS = SJ_PROBE_QUERIES / 32;   // queries a lane
+    __shared__ __align__(16) float cand[TASK_SAMPLE_WARPS][SJ_PROBE_POS][ROW];
+    __shared__ uint32_t candPos[TASK_SAMPLE_WARPS][SJ_PROBE_POS];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t t = blockIdx.x * TASK_SAMPLE_WARPS + warp;
+    if (t >= nt) return;
+    if (!(sample[t].x > 0.0f)) return;
+    const sj_task task = tasks[t];
+    const bool sym = (task.flags & SJ_TASK_SYM) != 0;
+    const uint32_t aStart = g.cellStart[task.cell], aEnd = g.cellStart[task.cell + 1];
+    const uint32_t homePos = sym ? task.qBegin : aStart;
+    const uint32_t homeLen = (task.segBase == 0 && (task.flags & SJ_TASK_HOME)) ? aEnd - homePos : 0u;
+    const uint32_t len = task.sEnd - task.sBegin;
+    const uint32_t m = min((uint32_t)SJ_PROBE_POS, len), mq = min((uint32_t)SJ_PROBE_QUERIES, task.qCount);
+    // the tasks of a tile take other queries each (golden-ratio phases), so that together they cover it
+    const uint32_t phase = (t * 40503u) & 0xffffu;
+    // local coordinates around the task's first query
+    double o[DP];
+    load_point<DP>(xs, task.qBegin, o);
+    float q[QS][DP];
+    uint32_t qPos[QS];
 #pragma unroll
-        for (int r = 0; r < QS; r++) {
-            const uint32_t qi = (uint32_t)r * SJ_CTA + tid;
-            double x[DP];
-            load_point<DP>(xs, (uint64_t)aStart + q0 + (qi < qc ? qi : 0u), x);
+    for (int r = 0; r < QS; r++) {
+        const uint32_t i = 32 * r + lane;
+        qPos[r] = task.qBegin + (i < mq ? sample_at(i, mq, task.qCount, phase) : 0u);
+        double x[DP];
+        load_point<DP>(xs, qPos[r], x);
 #pragma unroll
-            for (int l = 0; l < DP; l++) q[r][l] = qi < qc ? (float)(x[l] - origin[l]) : INFINITY;   // no query: no hit
+        for (int l = 0; l < DP; l++) q[r][l] = i < mq ? (float)(x[l] - o[l]) : INFINITY;   // no query: no hit
+    }
+    for (uint32_t i = lane; i < m; i += 32) {
+        const uint32_t s = task.sBegin + sample_at(i, m, len, 0x8000u);
+        uint32_t pos;
+        if (s < homeLen) {
+            pos = homePos + s;
+        } else {
+            // the owned neighbour that holds the position: the last entry that starts at or before it
+            uint32_t lo = g.nbrStart[task.cell], hi = g.nbrStart[task.cell + 1];
+            const uint32_t at = g.nbrPre[lo + (task.segBase ? task.segBase - 1u : 0u)] + (s - homeLen);
+            while (hi - lo > 1) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (g.nbrPre[mid] <= at) lo = mid; else hi = mid;
+            }
+            pos = g.cellStart[g.nbrCell[lo]] + (at - g.nbrPre[lo]);
         }
-        const auto stage = [&](uint32_t pos) {
-            double x[DP];
-            load_point<DP>(xs, pos, x);
+        candPos[warp][i] = pos;
+        double x[DP];
+        load_point<DP>(xs, pos, x);
 #pragma unroll
-            for (int l = 0; l < DP; l++) cand[tid][l] = (float)(x[l] - origin[l]);
-        };
-        const auto count = [&](uint32_t m) {   // the first m staged candidates
-            uint32_t h = 0;
+        for (int l = 0; l < DP; l++) cand[warp][i][l] = (float)(x[l] - o[l]);
+    }
+    __syncwarp();
+    // a point and itself are counted apart: only where the stretch holds queries
+    const uint32_t at = task.qBegin - homePos;
+    const bool own = homeLen && task.sBegin < at + task.qCount && task.sEnd > at;
+    uint32_t hits = 0;
+    const auto count = [&](auto skipSelf) {
 #pragma unroll 2
-            for (uint32_t j = 0; j < m; j++) {
-                float d2[QS];
+        for (uint32_t j = 0; j < m; j++) {
+            float b[ROW];
 #pragma unroll
-                for (int r = 0; r < QS; r++) d2[r] = 0.0f;
+            for (int l = 0; l < ROW; l += 4) {
+                const float4 v = *reinterpret_cast<const float4 *>(&cand[warp][j][l]);
+                b[l] = v.x;
+                b[l + 1] = v.y;
+                b[l + 2] = v.z;
+                b[l + 3] = v.w;
+            }
+#pragma unroll
+            for (int r = 0; r < QS; r++) {
+                float d2 = 0.0f;
 #pragma unroll
                 for (int l = 0; l < DP; l++) {
-                    const float b = cand[j][l];
-#pragma unroll
-                    for (int r = 0; r < QS; r++) {
-                        const float d = b - q[r][l];
-                        d2[r] = fmaf(d, d, d2[r]);
-                    }
+                    const float d = b[l] - q[r][l];
+                    d2 = fmaf(d, d, d2);
                 }
-#pragma unroll
-                for (int r = 0; r < QS; r++) h += d2[r] <= T ? 1u : 0u;
+                bool hit = d2 <= T;
+                if constexpr (decltype(skipSelf)::value) hit = hit && candPos[warp][j] != qPos[r];
+                hits += hit ? 1u : 0u;
             }
-            return h;
-        };
-        uint32_t hHome = 0, hNbr = 0;
-        const uint32_t mHome = it.z == 0 ? tile_samples(occ) : 0u;
-        for (uint32_t b = 0; b < mHome; b += SJ_CTA) {
-            __syncthreads();
-            if (b + tid < mHome) stage(aStart + sample_at(b + tid, mHome, occ));
-            __syncthreads();
-            hHome += count(min((uint32_t)SJ_CTA, mHome - b));
         }
-        // the group's neighbour stream, 128 segments at a time
-        const uint32_t S = g.groupLen[g.groupBase[it.y] + it.z], mNbr = tile_samples(S);
-        const uint32_t nb0 = g.nbrStart[it.y];
-        const uint32_t eEnd = min(g.nbrStart[it.y + 1], nb0 + (it.z + 1) * SJ_MAX_SEG - 1);
-        uint32_t done = 0, base = 0;   // samples taken; stream position of the first segment here
-        for (uint32_t e0 = nb0 + (it.z ? it.z * SJ_MAX_SEG - 1 : 0u); e0 < eEnd && done < mNbr; e0 += SJ_CTA) {
-            uint32_t len = 0, from = 0;
-            if (e0 + tid < eEnd) {
-                const uint32_t b = g.nbrCell[e0 + tid];
-                from = g.cellStart[b];
-                len = g.cellStart[b + 1] - from;
-            }
-            uint32_t x = len;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= (uint32_t)o) x += y;
-            }
-            __syncthreads();   // the previous segments are done with
-            if (lane == 31) warpSum[warp] = x;
-            __syncthreads();
-            for (uint32_t w = 0; w < warp; w++) x += warpSum[w];
-            segPos[tid] = from;
-            segPre[tid + 1] = x;
-            if (tid == 0) segPre[0] = 0;
-            __syncthreads();
-            const uint32_t total = segPre[SJ_CTA];
-            uint32_t m;
-            do {
-                const uint32_t k = done + tid;
-                const uint32_t at = k < mNbr ? sample_at(k, mNbr, S) : 0u;
-                const bool have = k < mNbr && at < base + total;   // the first m threads (also a barrier)
-                m = (uint32_t)__syncthreads_count(have);
-                if (have) {
-                    uint32_t lo = 0, hi = SJ_CTA;   // the last segment that starts at or before the sample
-                    while (hi - lo > 1) {
-                        const uint32_t mid = (lo + hi) >> 1;
-                        if (segPre[mid] <= at - base) lo = mid; else hi = mid;
-                    }
-                    stage(segPos[lo] + (at - base - segPre[lo]));
-                }
-                __syncthreads();
-                hNbr += count(m);
-                done += m;
-            } while (m == SJ_CTA);
-            base += total;
-        }
-        hHome = __reduce_add_sync(0xffffffffu, hHome);
-        hNbr = __reduce_add_sync(0xffffffffu, hNbr);
-        if (lane == 0) {
-            if (hHome) atomicAdd(&hits[0], hHome);
-            if (hNbr) atomicAdd(&hits[1], hNbr);
-        }
-        __syncthreads();
-        if (tid == 0)   // (half a hit more: a tile without one is not predicted to have none)
-            rates[it.x] = make_float2(mHome ? ((float)hits[0] + 0.5f) / ((float)qc * (float)mHome) : 0.0f,
-                                      mNbr ? ((float)hits[1] + 0.5f) / ((float)qc * (float)mNbr) : 0.0f);
-    }
+    };
+    if (own) count(std::true_type{});
+    else count(std::false_type{});
+    hits = __reduce_add_sync(0xffffffffu, hits);
+    if (lane == 0) sample[t].y = (float)hits;
 }
 
 template <class Kernel>
@@ -1276,21 +1235,22 @@ cudaError_t sj_launch_join(const sj_join_args &a, const sj_grid_dev &g, int fp32
     return cudaErrorInvalidValue;
 }
 
-cudaError_t sj_launch_tile_rates(const sj_taskgen &g, const sj_grid_dev &gd, const double *xs, const uint4 *tiles,
-                                 const uint32_t *nTiles, uint32_t nItems, int numSM, float2 *rates, cudaStream_t s)
+cudaError_t sj_launch_task_sample(const sj_taskgen &g, const sj_grid_dev &gd, const double *xs, const sj_task *tasks,
+                                  uint32_t nt, float2 *sample, cudaStream_t s)
 {
-    if (nItems == 0) return cudaSuccess;
-    const unsigned grid = std::min<uint64_t>((uint64_t)numSM * 8, nItems);
-    const float T = std::min((float)gd.thresh, FLT_MAX);   // (a slot without a query is infinitely far)
+    if (nt == 0) return cudaSuccess;
+    const unsigned grid = (nt + TASK_SAMPLE_WARPS - 1) / TASK_SAMPLE_WARPS;
+    constexpr unsigned B = 32 * TASK_SAMPLE_WARPS;
+    const float T = std::min((float)gd.thresh, FLT_MAX);   // (a lane without a query is infinitely far)
     switch (gd.Dp) {
-    case 1: k_tile_rates<1><<<grid, SJ_CTA, 0, s>>>(g, xs, T, tiles, nTiles, rates); break;
-    case 2: k_tile_rates<2><<<grid, SJ_CTA, 0, s>>>(g, xs, T, tiles, nTiles, rates); break;
-    case 3: k_tile_rates<3><<<grid, SJ_CTA, 0, s>>>(g, xs, T, tiles, nTiles, rates); break;
-    case 4: k_tile_rates<4><<<grid, SJ_CTA, 0, s>>>(g, xs, T, tiles, nTiles, rates); break;
-    case 6: k_tile_rates<6><<<grid, SJ_CTA, 0, s>>>(g, xs, T, tiles, nTiles, rates); break;
-    case 8: k_tile_rates<8><<<grid, SJ_CTA, 0, s>>>(g, xs, T, tiles, nTiles, rates); break;
-    case 12: k_tile_rates<12><<<grid, SJ_CTA, 0, s>>>(g, xs, T, tiles, nTiles, rates); break;
-    case 16: k_tile_rates<16><<<grid, SJ_CTA, 0, s>>>(g, xs, T, tiles, nTiles, rates); break;
+    case 1: k_task_sample<1><<<grid, B, 0, s>>>(g, xs, T, tasks, nt, sample); break;
+    case 2: k_task_sample<2><<<grid, B, 0, s>>>(g, xs, T, tasks, nt, sample); break;
+    case 3: k_task_sample<3><<<grid, B, 0, s>>>(g, xs, T, tasks, nt, sample); break;
+    case 4: k_task_sample<4><<<grid, B, 0, s>>>(g, xs, T, tasks, nt, sample); break;
+    case 6: k_task_sample<6><<<grid, B, 0, s>>>(g, xs, T, tasks, nt, sample); break;
+    case 8: k_task_sample<8><<<grid, B, 0, s>>>(g, xs, T, tasks, nt, sample); break;
+    case 12: k_task_sample<12><<<grid, B, 0, s>>>(g, xs, T, tasks, nt, sample); break;
+    case 16: k_task_sample<16><<<grid, B, 0, s>>>(g, xs, T, tasks, nt, sample); break;
     default: return cudaErrorInvalidValue;
     }
     sj_note_launch();

@@ -388,8 +388,7 @@ __device__ __forceinline__ Item find_item(const sj_taskgen &g, const uint32_t *_
 __global__ void __launch_bounds__(256) k_tg_item_tasks(sj_taskgen g, const uint32_t *__restrict__ order,
                                                        const uint8_t *__restrict__ workersAt,
                                                        const uint32_t *__restrict__ itemStart, uint32_t nItems,
-                                                       uint32_t *__restrict__ itemTasks, uint4 *__restrict__ tiles,
-                                                       uint32_t *__restrict__ nTiles)
+                                                       uint32_t *__restrict__ itemTasks)
 {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= nItems) return;
@@ -397,45 +396,6 @@ __global__ void __launch_bounds__(256) k_tg_item_tasks(sj_taskgen g, const uint3
     const uint32_t S = g.groupLen[g.groupBase[it.c] + it.grp];
     const TileWork w = tile_work(g, it.c, it.grp, it.tile, S, workersAt ? (int)workersAt[it.pos] : 0);
     itemTasks[j] = w.nChunks;
-    if (tiles && n_tiles(g, it.c) > 1) tiles[atomicAdd(nTiles, 1u)] = make_uint4(j, it.c, it.grp, it.tile);
-}
-
-// Weights of the tiles of a cell that has several: each tile's sampled rates over
-// the cell's mean of them (by evaluations), so that the cell's predicted pairs stay
-// what its rates make them and are shared among its tiles as sampled.  One warp a
-// position; the sums have a fixed order.
-__global__ void __launch_bounds__(256) k_tg_tile_weights(sj_taskgen g, const uint32_t *__restrict__ order,
-                                                         const uint32_t *__restrict__ itemStart,
-                                                         float2 *__restrict__ rates)
-{
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t pos = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (pos >= g.nCells) return;
-    const uint32_t c = order[pos], T = n_tiles(g, c);
-    if (T <= 1) return;
-    const uint32_t n = n_groups(g, c) * T, j0 = itemStart[pos];
-    double ev[2] = {0.0, 0.0}, hits[2] = {0.0, 0.0};   // home, neighbours
-    for (uint32_t i = lane; i < n; i += 32) {
-        const uint32_t grp = i / T;
-        const TileWork w = tile_work(g, c, grp, i - grp * T, g.groupLen[g.groupBase[c] + grp], 0);
-        const float2 r = rates[j0 + i];
-        ev[0] += (double)w.evHome;
-        ev[1] += (double)w.evOther;
-        hits[0] += (double)w.evHome * (double)r.x;
-        hits[1] += (double)w.evOther * (double)r.y;
-    }
-    double per[2];
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        ev[k] = warp_sum_f64(ev[k]);
-        hits[k] = warp_sum_f64(hits[k]);
-        per[k] = hits[k] > 0.0 ? ev[k] / hits[k] : 0.0;
-    }
-    for (uint32_t i = lane; i < n; i += 32) {
-        const float2 r = rates[j0 + i];
-        rates[j0 + i] = make_float2(per[0] > 0.0 ? (float)(r.x * per[0]) : 1.0f,
-                                    per[1] > 0.0 ? (float)(r.y * per[1]) : 1.0f);
-    }
 }
 
 // Writes every item's tasks (in item order, chunks ascending) and their
@@ -444,9 +404,8 @@ __global__ void __launch_bounds__(256) k_tg_item_write(sj_taskgen g, const uint3
                                                        const uint8_t *__restrict__ workersAt,
                                                        const uint32_t *__restrict__ itemStart, uint32_t nItems,
                                                        const uint32_t *__restrict__ itemTaskStart,
-                                                       const float2 *__restrict__ weights,
                                                        sj_task *__restrict__ tasks, uint32_t nt,
-                                                       float *__restrict__ pred)
+                                                       float *__restrict__ pred, float2 *__restrict__ sample)
 {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= nItems) return;
@@ -455,11 +414,8 @@ __global__ void __launch_bounds__(256) k_tg_item_write(sj_taskgen g, const uint3
     const TileWork w = tile_work(g, it.c, it.grp, it.tile, S, workersAt ? (int)workersAt[it.pos] : 0);
     const uint32_t nSegAll = 1 + (g.nbrStart[it.c + 1] - g.nbrStart[it.c]);
     const uint32_t segBase = it.grp * SJ_MAX_SEG;
-    float2 r = rates_of(g, it.c);
-    if (weights && n_tiles(g, it.c) > 1) {
-        r.x = fminf(1.0f, r.x * weights[j].x);
-        r.y = fminf(1.0f, r.y * weights[j].y);
-    }
+    const float2 r = rates_of(g, it.c);
+    const bool several = n_tiles(g, it.c) > 1;
     uint32_t t = itemTaskStart[j];
     // (the lists are sized by the cells' task counts; the host compares the two counts
     // after a count pass may have run on the list, so that is written whole and not
@@ -487,13 +443,111 @@ __global__ void __launch_bounds__(256) k_tg_item_write(sj_taskgen g, const uint3
                   (g.sampleRate > 0.0f && n_queries(g, it.c) < w.occ ? SJ_TASK_SAMPLE : 0u);
         tasks[t] = k;
         pred[t] = (float)pairs_of(g, r, evH, evO, diag);
+        if (sample)
+            sample[t] = make_float2(several ? (float)evH + (float)w.qc * (float)(s1 - max(s0, h1)) : 0.0f, 0.0f);
     }
     if (j + 1 == nItems) {
         for (; t < nt; t++) {
             tasks[t] = sj_task{};
             pred[t] = 0.0f;
+            if (sample) sample[t] = make_float2(0.0f, 0.0f);
         }
     }
+}
+
+// Predicted pairs of the tasks of cells with several query tiles, from their samples.
+// First, one warp an item: a task's hits per evaluation are its sample's, drawn by
+// TASK_PRIOR hits towards the cell's rate for it times how the item's samples compare
+// with that rate (few hits in a sample say little); (evaluations, hits of the sample)
+// become (-, expected hits).  itemSum: the item's predicted pairs by the cell's rates
+// and its expected hits.
+// Mean error of a batch's prediction, and of a task's, with the points in id order /
+// with the cell's mean for every task / with these: 2M points in 6-D, learned 0.7, 2.1,
+// 0.7 % and 4, 37, 5 %; sampled 0.9, 2.3, 0.65 and 47, 62, 5; 100k in 8-D 5.2, 5.7, 5.2
+// and 12, 49, 9; 60k in 7-D 2.8, 10.2, 2.6 and 8, 46, 7; 200k in 3-D 2.0, 7.2, 1.4 and
+// 6, 92, 6; 300k in 16-D 2.0, 2.5, 1.3 and 11, 25, 21.  Batches counted twice, 1e7 points
+// in 6-D: learned 0, 195, 0 of 1720; sampled 3, 267, 0 of 1708.
+constexpr double TASK_PRIOR = 8.0;
+
+__global__ void __launch_bounds__(256) k_task_pool(const uint32_t *__restrict__ itemTaskStart, uint32_t nItems,
+                                                   const sj_task *__restrict__ tasks, uint32_t nt,
+                                                   const float *__restrict__ pred, float2 *__restrict__ sample,
+                                                   double2 *__restrict__ itemSum)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (j >= nItems) return;
+    const uint32_t t0 = itemTaskStart[j], t1 = j + 1 < nItems ? min(nt, itemTaskStart[j + 1]) : nt;
+    if (t0 >= t1 || !(sample[t0].x > 0.0f)) {
+        if (lane == 0) itemSum[j] = make_double2(0.0, 0.0);
+        return;
+    }
+    double evals = 0.0, hits = 0.0, rated = 0.0;   // rated: hits by the cell's rates, but for a factor
+    for (uint32_t t = t0 + lane; t < t1; t += 32) {
+        const float2 e = sample[t];
+        if (e.x > 0.0f) hits += (double)e.x * ((double)e.y + 1.0 / 32.0) / (double)sj_probe_pairs(tasks[t]);
+        evals += (double)e.x;
+        rated += (double)pred[t];
+    }
+    evals = warp_sum_f64(evals);
+    hits = warp_sum_f64(hits);
+    rated = warp_sum_f64(rated);
+    const double least = 0.1 * hits / evals, factor = rated > 0.0 ? hits / rated : 0.0;
+    double expected = 0.0;
+    for (uint32_t t = t0 + lane; t < t1; t += 32) {
+        const float2 e = sample[t];
+        if (!(e.x > 0.0f)) continue;
+        const double rate = fmax(least, factor * (double)pred[t] / (double)e.x);
+        const double x = (double)e.x * ((double)e.y + TASK_PRIOR) /
+                         ((double)sj_probe_pairs(tasks[t]) + TASK_PRIOR / rate);
+        sample[t].y = (float)x;
+        expected += x;
+    }
+    expected = warp_sum_f64(expected);
+    if (lane == 0) itemSum[j] = make_double2(rated, expected);
+}
+
+// A task's pairs of a point and itself: queries whose own position is in its stretch.
+__device__ __forceinline__ uint32_t self_pairs(const sj_taskgen &g, const sj_task &k)
+{
+    if (!(k.flags & SJ_TASK_HOME)) return 0;
+    const uint32_t at = (k.flags & SJ_TASK_SYM) ? 0u : k.qBegin - g.cellStart[k.cell];   // of the first query
+    const uint32_t lo = max(k.sBegin, at), hi = min(k.sEnd, at + k.qCount);
+    return hi > lo ? hi - lo : 0u;
+}
+
+// Then, one warp an item: the cell's predicted pairs, as its rates make them, are
+// shared among its tasks: a point and itself where they are, the others in proportion
+// to the tasks' expected hits.  (The estimators' own totals stay: the samples alone
+// would predict most sets better, but not as the scheduler that was asked for.)
+// Every warp adds up its cell's items, at most some thousand, for itself; the sums
+// have a fixed order.
+__global__ void __launch_bounds__(256) k_task_share(sj_taskgen g, const uint32_t *__restrict__ order,
+                                                    const uint32_t *__restrict__ itemStart, uint32_t nItems,
+                                                    const uint32_t *__restrict__ itemTaskStart,
+                                                    const sj_task *__restrict__ tasks, uint32_t nt,
+                                                    const float2 *__restrict__ sample,
+                                                    const double2 *__restrict__ itemSum, float *__restrict__ pred)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (j >= nItems) return;
+    const uint32_t t0 = itemTaskStart[j], t1 = j + 1 < nItems ? min(nt, itemTaskStart[j + 1]) : nt;
+    if (t0 >= t1 || !(sample[t0].x > 0.0f)) return;
+    const Item it = find_item(g, order, itemStart, j);
+    const uint32_t j0 = itemStart[it.pos], j1 = j0 + n_groups(g, it.c) * n_tiles(g, it.c);
+    double rated = 0.0, expected = 0.0;
+    for (uint32_t i = j0 + lane; i < j1; i += 32) {
+        const double2 x = itemSum[i];
+        rated += x.x;
+        expected += x.y;
+    }
+    rated = warp_sum_f64(rated);
+    expected = warp_sum_f64(expected);
+    const double self = (double)(g.cellStart[it.c + 1] - g.cellStart[it.c]);   // every point is a query of one tile
+    const double own = fmin(1.0, rated / self), scale = expected > 0.0 ? fmax(0.0, rated - self) / expected : 0.0;
+    for (uint32_t t = t0 + lane; t < t1; t += 32)
+        if (sample[t].x > 0.0f) pred[t] = (float)(own * (double)self_pairs(g, tasks[t]) + scale * (double)sample[t].y);
 }
 
 // Shard `idx` of `cnt` keeps every cnt-th task of the ordered list.
@@ -985,32 +1039,34 @@ cudaError_t sj_tg_item_counts(const sj_taskgen &g, const uint32_t *order, uint32
 }
 
 cudaError_t sj_tg_item_tasks(const sj_taskgen &g, const uint32_t *order, const uint8_t *workersAt,
-                             const uint32_t *itemStart, uint32_t nItems, uint32_t *itemTasks, uint4 *tiles,
-                             uint32_t *nTiles, cudaStream_t s)
+                             const uint32_t *itemStart, uint32_t nItems, uint32_t *itemTasks, cudaStream_t s)
 {
     if (nItems == 0) return cudaSuccess;
-    k_tg_item_tasks<<<blocks_for(nItems, 256), 256, 0, s>>>(g, order, workersAt, itemStart, nItems, itemTasks, tiles,
-                                                            nTiles);
-    sj_note_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t sj_tg_tile_weights(const sj_taskgen &g, const uint32_t *order, const uint32_t *itemStart, float2 *rates,
-                               cudaStream_t s)
-{
-    if (g.nCells == 0) return cudaSuccess;
-    k_tg_tile_weights<<<blocks_for((uint64_t)g.nCells * 32, 256), 256, 0, s>>>(g, order, itemStart, rates);
+    k_tg_item_tasks<<<blocks_for(nItems, 256), 256, 0, s>>>(g, order, workersAt, itemStart, nItems, itemTasks);
     sj_note_launch();
     return cudaGetLastError();
 }
 
 cudaError_t sj_tg_item_write(const sj_taskgen &g, const uint32_t *order, const uint8_t *workersAt,
                              const uint32_t *itemStart, uint32_t nItems, const uint32_t *itemTaskStart,
-                             const float2 *weights, sj_task *tasks, uint32_t nt, float *pred, cudaStream_t s)
+                             sj_task *tasks, uint32_t nt, float *pred, cudaStream_t s, float2 *sample)
 {
     if (nItems == 0) return cudaSuccess;
     k_tg_item_write<<<blocks_for(nItems, 256), 256, 0, s>>>(g, order, workersAt, itemStart, nItems, itemTaskStart,
-                                                            weights, tasks, nt, pred);
+                                                            tasks, nt, pred, sample);
+    sj_note_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t sj_tg_share(const sj_taskgen &g, const uint32_t *order, const uint32_t *itemStart, uint32_t nItems,
+                        const uint32_t *itemTaskStart, const sj_task *tasks, uint32_t nt, float2 *sample,
+                        double2 *itemSum, float *pred, cudaStream_t s)
+{
+    if (nItems == 0 || nt == 0) return cudaSuccess;
+    const unsigned grid = blocks_for((uint64_t)nItems * 32, 256);
+    k_task_pool<<<grid, 256, 0, s>>>(itemTaskStart, nItems, tasks, nt, pred, sample, itemSum);
+    sj_note_launch();
+    k_task_share<<<grid, 256, 0, s>>>(g, order, itemStart, nItems, itemTaskStart, tasks, nt, sample, itemSum, pred);
     sj_note_launch();
     return cudaGetLastError();
 }

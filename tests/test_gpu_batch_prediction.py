@@ -1,11 +1,13 @@
 """Predicted against measured pairs of the planned batches (GPU).
 
-The points of a dense cell are in spatial order, so its tiles differ, and a batch
-holds few of them: each tile is predicted by a sample of its own.  Bounds: half
-again the mean batch error that the same predictions have with the cells' points
-in id order, where the tiles are alike (learned, 6-D 0.7 to 1.1 %; sampled, 6-D
-1.5 %, 3-D 2.0 %).  The cell's mean rate for every tile gave 2.1, 2.9 and 7.2 %, and
-up to a quarter of the batches overflowed.
+The points of a dense cell are in spatial order, so its tasks differ, and a batch
+holds few of its tiles: each task is predicted by a sample of its own.  Bounds:
+half again the mean batch error that the same predictions have with the cells'
+points in id order, where the tiles are alike (learned, 6-D 0.7 to 1.1 %; sampled,
+6-D 1.5 %, 3-D 2.0 %).  The cell's mean rate for every tile gave 2.1, 2.9 and 7.2 %,
+and up to a quarter of the batches overflowed.  In id order none of the 6-D batches
+overflow on these points and 4 of 96 (4.2 %) in 3-D, where the estimate itself is
+off by more than the margin in one cell: half again that for the 3-D set.
 """
 import os
 
@@ -17,11 +19,11 @@ from conftest import exp_points
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,dim,k,eps,mode,prec,learned,capacity,bound", [
-    (600_000, 6, 6, 0.03, 10, sjoin.PREC_FP32_REFINE, True, 200_000_000, 0.016),
-    (600_000, 6, 6, 0.03, 10, sjoin.PREC_FP32_REFINE, False, 200_000_000, 0.023),
-    (200_000, 3, 1, 0.01, 3, sjoin.PREC_FP32_REFINE, False, 10_000_000, 0.030)])
-def test_batches_as_predicted(n, dim, k, eps, mode, prec, learned, capacity, bound):
+@pytest.mark.parametrize("n,dim,k,eps,mode,prec,learned,capacity,bound,over", [
+    (600_000, 6, 6, 0.03, 10, sjoin.PREC_FP32_REFINE, True, 200_000_000, 0.016, 0.04),
+    (600_000, 6, 6, 0.03, 10, sjoin.PREC_FP32_REFINE, False, 200_000_000, 0.023, 0.04),
+    (200_000, 3, 1, 0.01, 3, sjoin.PREC_FP32_REFINE, False, 10_000_000, 0.030, 0.0625)])
+def test_batches_as_predicted(n, dim, k, eps, mode, prec, learned, capacity, bound, over):
     with sjoin.SelfJoin(dim, eps, indexed_dims=k, mode=mode, precision=prec, capacity=capacity,
                         scheduler=sjoin.SCHED_LEARNED if learned else sjoin.SCHED_SAMPLING) as sj:
         if learned:
@@ -31,4 +33,4 @@ def test_batches_as_predicted(n, dim, k, eps, mode, prec, learned, capacity, bou
         st = sj.join(sjoin.DELIVER_NONE)
     assert st.num_batches >= 30
     assert st.estimator_mean_abs_rel_err <= bound
-    assert st.overflow_retries <= 0.04 * st.num_batches
+    assert st.overflow_retries <= over * st.num_batches

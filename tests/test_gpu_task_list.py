@@ -50,7 +50,7 @@ int main()
     sj_task *dTasks = dev(tasks, nt);
     float *dPred = dev(pred, nt);
     const uint32_t *zero = dev(none, 2);
-    cudaError_t e = sj_tg_item_write(g, zero, nullptr, zero, 1, zero, nullptr, dTasks, nt, dPred, 0);
+    cudaError_t e = sj_tg_item_write(g, zero, nullptr, zero, 1, zero, dTasks, nt, dPred, 0);
     if (e == cudaSuccess) e = cudaMemcpy(tasks, dTasks, sizeof(tasks), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(pred, dPred, sizeof(pred), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return 2;
