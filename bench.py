@@ -53,11 +53,6 @@ sys.path.insert(0, os.path.join(REPO, "self-join-hpbdc2019_b200"))
 
 ESTIMATOR_WEIGHTS = os.path.join(REPO, "self-join-hpbdc2019_b200", "sjoin", "estimator_c4.bin")
 
-# dram__bytes_read.sum + dram__bytes_write.sum per output pair of the emission
-# kernel (k_emit) when a capture has it; the traffic grows with the pairs, so a
-# full-size launch is scaled by its pairs
-EMIT_TRAFFIC_BYTES_PER_PAIR = None
-
 # CUDA-core lanes per SM (B200): FP64 FMA and FP32 FMA per clock
 FP64_LANES, FP32_LANES, NUM_SM = 64, 128, 148
 
@@ -481,7 +476,6 @@ def run_ours(args):
     nb = max(1, ps["num_batches"])
     emit_ms = ps["ms_fill_kernel"]
     achieved = (8 * pairs) / (emit_ms / 1e3) / 1e9 if emit_ms > 0 else None
-    traffic = EMIT_TRAFFIC_BYTES_PER_PAIR * pairs / nb if EMIT_TRAFFIC_BYTES_PER_PAIR else None
     cpu = None
     if not args.no_cpu and ws == 1:   # the CPU baseline is rank 0's at N = 1 only
         rate, cores, sample, _ = cpu_oracle_rate(pts, eps, k, target_s=args.cpu_seconds)
@@ -500,7 +494,7 @@ def run_ours(args):
         "roofline": {"bound": "hbm", "kernel": "k_emit: keys, values and set hash of the pairs from the hit masks",
                      "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None, "peak_kind": peak_kind,
-                     "algorithmic_bytes_per_launch": 8 * pairs / nb, "launches": nb, "traffic": traffic,
+                     "algorithmic_bytes_per_launch": 8 * pairs / nb, "launches": nb, "traffic": None,   # not measured in a run
                      "note": ("key and value (8 B) written per pair; launch times from CUDA events around each launch "
                               "in the stage probe (every stage on one stream)" if probe else
                               "key and value (8 B) written per pair; launch times from CUDA events on the emission's "

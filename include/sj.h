@@ -108,6 +108,8 @@ typedef struct {
     double estimated_pairs;     /* scheduler's prediction of the total pair count */
     double estimator_mean_abs_rel_err; /* mean |pred-meas|/meas over batches */
     double estimator_task_rel_err;     /* sum|pred-meas| / sum(meas) over tasks */
+    /* stage times of the last call that ran the stage (a degree count has no estimate: 0); ms_total: the
+       last join's */
     float ms_upload, ms_index, ms_tasks, ms_estimate, ms_count, ms_scan, ms_fill, ms_deliver, ms_total;
     float ms_join_kernels;      /* count + fill kernel time */
     float ms_fill_kernel;       /* fill kernel time alone */

@@ -494,7 +494,10 @@ int bits_for(uint64_t count)
 // which the bins are widest so far (a cell is eps wide in the indexed
 // dimensions, the data's range in the others).
 // Only where the cells hold 16 points or more on average: with fewer, 32
-// consecutive points span cells anyway and the extra sort does not pay.
+// consecutive points span cells anyway.  The extra sort takes 0.14 ms on 400k points
+// and pays where a cell's points are not uniform (300k exponential points in 5-D, 21 a
+// cell, count pass 5.7 against 7.5 ms in FP64, 3.7 against 4.9 in FP32); on uniform 2-D
+// and 3-D sets of 24 to 95 a cell the count pass is the same with and without it.
 sj_place_plan place_plan(const Ctx &c)
 {
     sj_place_plan pl{};
@@ -778,7 +781,7 @@ uint64_t mask_batch_words()
 // The task list, built on the device (sj_tasks.cu): per-cell workload and cost
 // key, the cost order (stable radix sort, heaviest first, ties in cell order),
 // one work item per (cell, segment group, query tile) and its tasks.  policy:
-// 0 cost-proportional stream chunks, 1 fixed chunks, 2 the mode-8 split by
+// 0 cost-proportional stream chunks, 1 about 5e5 evaluations each, 2 the mode-8 split by
 // thirds of the work (0 and 2 predict pairs from c.rate).  sampleRate > 0 builds the sampling
 // estimator's tasks.  With `shard`, keeps this context's shard of the list.
 // Without `rates` nothing is predicted and policy 0 cuts by evaluations alone.

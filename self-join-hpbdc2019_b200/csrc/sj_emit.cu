@@ -33,13 +33,16 @@
 //   lists (few hits, or few words): lane = line; each lane walks its own line's
 //               bits into its part of one packed list, which the warp copies out.
 //
-// Bound: instruction issue.  With the points of a cell in spatial order the hits
-// are bunched: on the exponential sets three quarters of the pairs lie in tiles
-// more than half full, and 60 % of the live tiles hold a tenth of them.  In a
+// Bound: latency and instruction issue together.  In the 6-D capture 69 % of the issue
+// slots are used; the largest stall is the wait for a unit's staged words and values
+// (long_scoreboard, 3.5 of 10 cycles an issue: a unit stages, waits for all of it, then
+// emits), then the fixed-latency chains (2.1).  With the points of a cell in spatial
+// order the hits are bunched: on the exponential sets three quarters of the pairs lie
+// in tiles more than half full, and 60 % of the live tiles hold a tenth of them.  In a
 // full window the copy-out -- two shared loads, two stores and the ~19 integer
-// operations of splitmix64 with the key's part taken out -- is most of the work;
-// in sparse tiles a window's fixed ~100 instructions would be, so those go by
-// lists, whose decode is as long as the fullest line.
+// operations of splitmix64 with the key's part taken out -- is most of the
+// instructions; in sparse tiles a window's fixed ~100 would be, so those go by lists,
+// whose decode is as long as the fullest line.
 // Measured (one stream): 6-D, 1e7 points, 3.18e12 pairs 10.2 s, 2.5 TB/s of keys
 // and values, where the emission of values (11.4 s) and a second pass that read
 // them back, wrote the keys and hashed (6.9 s) took 18.2 s; 2-D, 2M points 34.2 ms.

@@ -148,7 +148,7 @@ struct sj_taskgen {
     double pairsPerTask;         // chunking target of policy 0
     double evalsPerTask;         // policy 0: evaluations per task at most (0: no limit)
     int sym;                     // symmetric traversal (owned neighbours, both directions emitted)
-    int policy;                  // 0 cost-proportional chunks, 1 short fixed chunks, 2 mode-8 split by thirds of the work
+    int policy;                  // 0 cost-proportional chunks, 1 about 5e5 evaluations each, 2 mode-8 split by thirds of the work
     float sampleRate;            // > 0: tasks for the sampled queries of each cell only (sampling estimator)
     // spread != 0: a task's neighbour pairs follow the offset-class model
     // (sj_nbr_spread) instead of the cell's mean rate

@@ -343,13 +343,20 @@ struct __align__(16) JoinSmem {
 // set -- every query's hit mask per block of 32 stream positions plus its row
 // count, which the emission pass turns into pairs without a second distance
 // evaluation.
-// Resident CTAs per SM the register allocation must allow.  FP32 filter: four,
-// five at six dimensions (4-D: 41.2 ms of count passes with four, 45.7 with
-// five; 8-D 7.2 against 7.6; 6-D 82 against 79).  FP64: as many as leave the
-// queries in registers but for a few; its chain of dependent operations needs the
-// warps more than it minds the spills (with three, two above six dimensions: 2-D
-// 1.57 to 1.29 ms of count pass, 3-D 1.58 to 1.08, 4-D 3.91 to 3.02, 6-D 13.6 to
-// 12.1, 8-D 3.2 to 2.5).
+// Resident CTAs per SM the register allocation must allow.  Count passes in ms on
+// exponential sets of 60k to 1M points, batches of 2e8 pairs (1-D: 0.06 to 0.08, a
+// launch's latency):
+//                               2-D   3-D   4-D   6-D   8-D   12-D  16-D
+//   FP32  three                 3.48  2.92  5.28  10.8  2.83  4.57  5.78
+//         four (not 6-D)        3.13  2.60  4.55        2.76  4.18  5.54
+//         five (6-D)            2.94  2.45  4.35  9.12  2.78  4.12  5.59
+//   FP64  one fewer             3.29  3.05  6.06  15.6  4.18  9.04  12.4
+//         6, 6, 6, 5, 4, 3, 3   3.17  2.91  6.01  15.3  3.94  8.22  11.7
+//         one more              3.12  2.84  6.06  16.2  4.10  8.29  11.4
+// (Five have become the better choice for FP32 at two to four dimensions: the kernel
+// was another when the line was drawn.)  FP64's chain of dependent operations needs the
+// warps more than it minds a few spilled registers (4-D 52 / 60 bytes of stores / loads,
+// 6-D 52 / 64, 8-D 8 / 8).
 constexpr int sj_join_min_blocks(int DP, bool F32)
 {
     if (F32) return DP == 6 ? 5 : 4;
@@ -774,8 +781,15 @@ __device__ __forceinline__ float box_dist2(const float2 *box, const float *x)
     return d2;
 }
 
-constexpr uint32_t SMALL_BOX = 6;   // queries from which on testing a block against their box pays
+// Queries from which on testing a block against their box pays: clusters of two points
+// a cell, 12-D / 16-D 2.03 / 2.37 ms of count pass with 6, 2.12 / 2.44 with 3, 1.99 /
+// 2.32 with 12; below 12 dimensions no difference.
+constexpr uint32_t SMALL_BOX = 6;
 
+// Resident CTAs per SM: 3-D / 2-D / 6-D / 8-D / 12-D / 16-D, FP32, 0.173 / 0.364 / 1.60 /
+// 1.95 / 2.03 / 2.37 ms with these, 0.191 / 0.420 / 1.80 / 2.04 / 2.42 / 2.72 with one
+// fewer, 0.168 / 0.329 / 1.70 / 2.31 / 2.26 / 2.90 with one more (spills; 8-D FP32 spills
+// 92 / 68 bytes of stores / loads as it is).
 template <int DP, bool F32>
 __global__ void __launch_bounds__(SJ_CTA, DP <= 4 ? 6 : DP <= 8 ? 5 : 4) k_join_small(sj_join_args a, sj_grid_dev g, int queue)
 {

@@ -14,7 +14,9 @@
 //   2. the cost order: the engine's stable LSD radix sort on the keys;
 //   3. work items = (cell, segment group, query tile) in that order; per item
 //      its chunk count; exclusive scans give every item's first task;
-//   4. one thread per item writes its tasks and their predicted pairs;
+//   4. one thread per item writes its tasks and their predicted pairs; those of
+//      cells with several query tiles, whose points are in spatial order, are
+//      shared among the cell's tasks by a sample of each (k_task_sample, sj_join.cu);
 //   5. per task the sizes of its count-pass records and emission units; their
 //      exclusive prefix sums are the record offsets the kernels index by;
 //   6. the batch plan: from every task s the end of a batch starting at s
